@@ -1,0 +1,846 @@
+// Prompts of the matrix-state recurrences (state-space scan, decay per key channel, gated delta rule), sixteen tokens at a time.
+//
+// Walked token by token (recurrent.cu) a prompt is a chain: every token waits for the sums over a state's rows of the one
+// before it, and a 2,048-token prompt took 1.1 to 1.8 ms for work that the multiprocessors' fp32 units can do in 0.07.  Here
+// a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 228, state-space scan
+// of 64 heads of 128 x 64 1,116 -> 218, delta rule of 16 heads of 128 x 128 over 1,501 + 500 tokens 1,224 -> 214).  With P(i..j) the product of the decays of the tokens i..j (per row, or
+// one number per head) and S the state in front of the chunk:
+//     out_j  = (P(0..j) q_j)^T S + sum_(i <= j) A_ji x_i,     A_ji = sum_rows q_j P(i+1..j) k_i
+//     S'     = P(0..15) S + sum_j (P(j+1..15) k_j) x_j^T
+// x is the value, or for the delta rule the corrected value: x = T (v - (P(0..j) k_j)^T S), T = (I + beta C)^-1 beta with
+// C_ji = k_j . P(i+1..j) k_i below the diagonal, so that the sixteen corrections, each of which waits for the one before it,
+// are one small triangular product.  Every factor is a product of at most 16 decays, never a quotient of two: nothing
+// overflows however strong a decay is, and all of it is fp32 multiply-adds, as in the walk.
+//
+// Two launches.  What does not depend on the state (decayed rows, A, T) is formed for all chunks at once; then a block owns
+// (sequence, head, 16 or 32 value columns), holds its part of S in registers, and walks the sequence's chunks, while one more
+// warp brings the next chunk into shared memory (cp.async).
+#include "common.cuh"
+
+BLM_API const char* blm_scan_chunks_last_error() { return g_blm_error; }
+
+constexpr int kQ = 16;            // tokens of a chunk
+constexpr int kMs = 20;           // floats a row of the 16 x 16 matrices: rows that lanes read side by side start in different banks
+constexpr int kMat = kQ * kMs;
+
+enum { kSsm = 0, kDecay = 1, kDelta = 2 };
+
+__device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
+__device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
+__device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
+
+// Chunk c of sequence s has the index cu[s] / 16 + s + c: distinct for all chunks, below n_tokens / 16 + n_seqs.
+__host__ __device__ inline int chunk_bound(int n_tokens, int n_seqs) { return n_tokens / kQ + n_seqs; }
+__device__ __forceinline__ int chunk_base(int cu, int seq) { return cu / kQ + seq; }
+
+// Floats of one (chunk, head) in scratch: [decayed k for the correction (delta)] [decayed q] [k decayed to the chunk's end]
+// [the chunk's decay], rows of NP (not for the state-space scan, whose rows are shared by heads and read where they lie);
+// then A (delta: A T), [T (delta)], [16 factors of q, 16 of x, the chunk's decay, 15 unused (state-space scan)].
+__host__ __device__ constexpr int rows_floats(int kind, int np) { return kind == kSsm ? 0 : (kind == kDelta ? 3 : 2) * kQ * np + np; }
+__host__ __device__ constexpr int small_floats(int kind) { return kMat * (kind == kDelta ? 2 : 1) + (kind == kSsm ? 48 : 0); }
+__host__ __device__ constexpr int part_floats(int kind, int np) { return rows_floats(kind, np) + small_floats(kind); }
+
+// Which sequence and chunk a chunk index names; false when none.  All threads of the block call it.
+__device__ __forceinline__ bool find_chunk(int idx, const int* __restrict__ cu, int n_seqs, int* found, int& seq, int& chunk) {
+    if (threadIdx.x == 0) found[0] = -1;
+    __syncthreads();
+    for (int s = threadIdx.x; s < n_seqs; s += blockDim.x) {
+        const int lo = cu[s], n = cu[s + 1] - lo, base = chunk_base(lo, s);
+        if (n > 0 && idx >= base && idx < base + (n + kQ - 1) / kQ) {
+            found[0] = s;
+            found[1] = idx - base;
+        }
+    }
+    __syncthreads();
+    seq = found[0];
+    chunk = found[1];
+    return seq >= 0;
+}
+
+// Sixteen values a lane, summed over the warp: lane l gets the sum of value l / 2.
+__device__ __forceinline__ float sum_sixteen(float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int n = 8, m = 16; n >= 1; n >>= 1, m >>= 1) {
+        const bool up = lane & m;
+#pragma unroll
+        for (int x = 0; x < n; ++x) {
+            const float give = up ? v[x] : v[x + n], keep = up ? v[x + n] : v[x];
+            v[x] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+struct RowsIn {                    // a column range of a float32 [N, *] tensor
+    const float* p;
+    long long stride;
+    int col0;
+};
+
+// ---------------------------------------------------------------------------------------------
+// a decay per row (kDecay) and the delta rule (kDelta): a block per (chunk, head), a thread per row of the state
+//
+// A_ji = sum_rows q_j P(i+1..j) k_i over the 120 pairs i < j as plain dot products: let 2^b be the highest bit in which j and i
+// differ.  Then j lies in an odd and i in the even neighbour of two blocks of 2^b tokens, and P(i+1..j) is the product of the
+// decays behind i up to its block's end and those from the start of j's block up to j.  So for each of the four levels b a
+// token's row is kept in shared memory once with that factor (its q in an odd block, its k in an even one), and a thread
+// takes a pair: 16-byte loads, no exchange between lanes.  (Running products and a sum over the lanes for each pair took
+// 63 us for 2,048 tokens of 32 heads x 128 rows.)
+// ---------------------------------------------------------------------------------------------
+struct PrepArgs {
+    RowsIn q, k, a, b;
+    const float *bias, *extra, *A_log;
+    const int* cu;
+    int n_seqs, heads, qk_heads, dk;
+    float* scratch;
+};
+
+__host__ __device__ constexpr int prep_threads(int np) { return np < 128 ? 128 : np; }
+__host__ __device__ constexpr int prep_smem(int np, bool delta) { return (4 * kQ + (delta ? 4 * kQ / 2 : 0)) * (np + 4) * 4; }
+
+// What the raw rows mean (blm_decay_scan): the delta rule; w = exp(-exp(a + bias)), the state read last, or first; a lower bound
+enum { kModeDelta = 0, kModeExp = 1, kModeExpFirst = 2, kModeLower = 3 };
+
+template <int NP, int MODE>
+__global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepArgs a) {
+    constexpr bool DELTA = MODE == kModeDelta, kFirst = MODE == kModeExpFirst;
+    constexpr int T = prep_threads(NP), W = T / 32, NS = NP + 4;
+    extern __shared__ __align__(16) float levels[];          // [4][16][NS], then (delta) the odd blocks' k [4][8][NS]
+    float* level_k = levels + 4 * kQ * NS;
+    __shared__ int found[2];
+    __shared__ float sums[3][W][16];                          // k . k, q . q, q . k of the sixteen tokens
+    __shared__ float As[kQ][kMs], Cs[kQ][kMs], Ts[kQ][kMs], betas[kQ];
+    const int h = blockIdx.y, r = threadIdx.x, lane = r & 31, warp = r >> 5;
+    int seq, chunk;
+    if (!find_chunk(blockIdx.x, a.cu, a.n_seqs, found, seq, chunk)) return;
+    const int first = a.cu[seq] + chunk * kQ, nt = min(kQ, a.cu[seq + 1] - first);
+    const int c = h / (a.heads / a.qk_heads);
+    float w[kQ], kk[kQ], qq[kQ];
+    const bool live = r < a.dk;
+    const float rate = DELTA ? -expf(a.A_log[h]) : 0.f;
+    const float bias = live ? a.bias[h * a.dk + r] : 0.f, extra = live && a.extra ? a.extra[h * a.dk + r] : 0.f;
+#pragma unroll
+    for (int t = 0; t < kQ; ++t) {             // every load first
+        const bool on = live && t < nt;
+        const size_t row = (size_t)(first + t);
+        w[t] = on ? a.a.p[row * a.a.stride + a.a.col0 + h * a.dk + r] : 0.f;
+        qq[t] = on ? a.q.p[row * a.q.stride + a.q.col0 + c * a.dk + r] : 0.f;
+        kk[t] = on && a.k.p ? a.k.p[row * a.k.stride + a.k.col0 + c * a.dk + r] : 0.f;
+    }
+    if (DELTA && r < kQ) betas[r] = r < nt ? sigmoid_f(a.b.p[(size_t)(first + r) * a.b.stride + a.b.col0 + h]) : 0.f;
+    for (int e = r; e < kMat; e += T) {
+        (&As[0][0])[e] = 0.f;
+        (&Cs[0][0])[e] = 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < kQ; ++t) {             // a token beyond the chunk's end keeps the state and writes nothing
+        const bool on = live && t < nt;
+        if (DELTA) {
+            w[t] = on ? expf(rate * softplus_r(w[t] + bias)) : 1.f;
+        } else if (MODE == kModeLower) {
+            const float f = extra + (1.0f - extra) * sigmoid_f(w[t] + bias);
+            w[t] = on ? f : 1.f;
+            kk[t] = on ? 1.0f - f : 0.f;
+            qq[t] = on ? silu_f(qq[t]) : 0.f;
+        } else {
+            w[t] = on ? expf(-expf(w[t] + bias)) : 1.f;
+        }
+    }
+    float v[16];
+    if (DELTA) {                               // unit vectors
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) v[t] = kk[t] * kk[t];
+        float s = sum_sixteen(v);
+        if (!(lane & 1)) sums[0][warp][lane >> 1] = s;
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) v[t] = qq[t] * qq[t];
+        s = sum_sixteen(v);
+        if (!(lane & 1)) sums[1][warp][lane >> 1] = s;
+        __syncthreads();
+        if (r < 32) {
+            const int t = r & 15, set = r >> 4;
+            float x = 0.f;
+            for (int y = 0; y < W; ++y) x += sums[set][y][t];
+            x = 1.0f / sqrtf(x + 1e-6f);
+            if (set) x *= 1.0f / sqrtf((float)a.dk);
+            __syncwarp();
+            sums[set][0][t] = x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) {
+            kk[t] *= sums[0][0][t];
+            qq[t] *= sums[1][0][t];
+        }
+    }
+    // the diagonal: q_t . k_t, with the current token's bonus where the state is read before the write
+#pragma unroll
+    for (int t = 0; t < kQ; ++t) v[t] = kFirst ? qq[t] * kk[t] * extra : qq[t] * kk[t];
+    {
+        const float s = sum_sixteen(v);
+        if (!(lane & 1)) sums[2][warp][lane >> 1] = s;
+    }
+    float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h) * part_floats(DELTA ? kDelta : kDecay, NP);
+    if (r < NP) {
+        float p = 1.f;
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) {
+            if (kFirst) out[t * NP + r] = qq[t] * p;
+            p *= w[t];
+            if (DELTA) {
+                out[t * NP + r] = kk[t] * p;
+                out[(kQ + t) * NP + r] = qq[t] * p;
+            } else if (!kFirst) {
+                out[t * NP + r] = qq[t] * p;
+            }
+        }
+        float* kd = out + (DELTA ? 2 : 1) * kQ * NP;
+        p = 1.f;
+#pragma unroll
+        for (int t = kQ - 1; t >= 0; --t) {
+            kd[t * NP + r] = kk[t] * p;
+            p *= w[t];
+        }
+        kd[kQ * NP + r] = p;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            constexpr int kAll = kQ;
+            const int B = 1 << b;
+#pragma unroll
+            for (int t0 = 0; t0 < kAll; t0 += 1 << b) {
+                float f = 1.f;
+                if (t0 & B) {                  // an odd block: from its start on
+#pragma unroll
+                    for (int t = t0; t < t0 + B; ++t) {
+                        if (!kFirst) f *= w[t];
+                        levels[(b * kQ + t) * NS + r] = qq[t] * f;
+                        if (DELTA) level_k[(b * 8 + ((t >> (b + 1)) << b) + (t & (B - 1))) * NS + r] = kk[t] * f;
+                        if (kFirst) f *= w[t];
+                    }
+                } else {                       // an even one: up to its end
+#pragma unroll
+                    for (int t = t0 + B - 1; t >= t0; --t) {
+                        levels[(b * kQ + t) * NS + r] = kk[t] * f;
+                        f *= w[t];
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int pair = r; pair < 120; pair += T) {
+        // pairs of level 3, then 2, 1, 0: 64, 32, 16, 8 of them, 4^b for each two neighbouring blocks
+        const int b = pair < 64 ? 3 : (pair < 96 ? 2 : (pair < 112 ? 1 : 0));
+        const int x = pair - (pair < 64 ? 0 : (pair < 96 ? 64 : (pair < 112 ? 96 : 112))), B = 1 << b;
+        const int two = x >> (2 * b), y = x & (B * B - 1);
+        const int j = two * 2 * B + B + (y >> b), i = two * 2 * B + (y & (B - 1));
+        const float4* pq = reinterpret_cast<const float4*>(levels + (b * kQ + j) * NS);
+        const float4* pk = reinterpret_cast<const float4*>(levels + (b * kQ + i) * NS);
+        const float4* pj = reinterpret_cast<const float4*>(level_k + (b * 8 + ((j >> (b + 1)) << b) + (j & (B - 1))) * NS);
+        float sa[4] = {0.f, 0.f, 0.f, 0.f}, sc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+        for (int n = 0; n < NP / 4; ++n) {
+            const float4 q4 = pq[n], k4 = pk[n];
+            sa[0] += q4.x * k4.x;
+            sa[1] += q4.y * k4.y;
+            sa[2] += q4.z * k4.z;
+            sa[3] += q4.w * k4.w;
+            if (DELTA) {
+                const float4 j4 = pj[n];
+                sc[0] += j4.x * k4.x;
+                sc[1] += j4.y * k4.y;
+                sc[2] += j4.z * k4.z;
+                sc[3] += j4.w * k4.w;
+            }
+        }
+        As[j][i] = (sa[0] + sa[1]) + (sa[2] + sa[3]);
+        if (DELTA) Cs[j][i] = (sc[0] + sc[1]) + (sc[2] + sc[3]);
+    }
+    if (r < kQ) {
+        float s = 0.f;
+        for (int y = 0; y < W; ++y) s += sums[2][y][r];
+        As[r][r] = s;
+    }
+    __syncthreads();
+    float* m = out + rows_floats(DELTA ? kDelta : kDecay, NP);
+    if (!DELTA) {
+        for (int e = r; e < kMat; e += T) m[e] = (&As[0][0])[e];
+        return;
+    }
+    // T = (I + beta C)^-1 beta: column i by forward substitution, a lane a column
+    if (r < kQ) {
+        float x[kQ];
+#pragma unroll
+        for (int j = 0; j < kQ; ++j) {
+            float s = 0.f;
+#pragma unroll
+            for (int y = 0; y < j; ++y) s += Cs[j][y] * x[y];
+            x[j] = (j == r ? betas[j] : 0.f) - betas[j] * s;
+        }
+#pragma unroll
+        for (int j = 0; j < kQ; ++j) Ts[j][r] = x[j];
+    }
+    __syncthreads();
+    for (int e = r; e < kMat; e += T) {
+        const int j = e / kMs, i = e % kMs;
+        float s = 0.f;
+        if (i < kQ) {
+#pragma unroll
+            for (int y = 0; y < kQ; ++y) s += As[j][y] * Ts[y][i];
+        }
+        m[e] = s;
+        m[kMat + e] = i < kQ ? Ts[j][i] : 0.f;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the state-space scan: B and C are shared by the heads of a group and the decay is one number a head and token, so only the
+// 16 x 16 products and numbers are kept.  A block per (chunk, group, eight heads of it), a thread per pair.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSsmHeads = 8;
+
+struct SsmPrepArgs {
+    RowsIn x, dt;                  // x names the tensor; B at b_col0, C at c_col0
+    int b_col0, c_col0;
+    const float *dt_bias, *A_log, *D;
+    const int* cu;
+    int n_seqs, heads, groups, N;
+    float* scratch;
+};
+
+__global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
+    __shared__ int found[2];
+    __shared__ float Bs[kQ][65], Cs[kQ][65];   // 64 rows of the state at a time
+    __shared__ float dts[kSsmHeads][kQ], decs[kSsmHeads][kQ], run[kSsmHeads][kQ][kQ + 1];
+    const int per = a.heads / a.groups, tiles = (per + kSsmHeads - 1) / kSsmHeads;
+    const int g = blockIdx.y / tiles, h0 = g * per + blockIdx.y % tiles * kSsmHeads, nh = min(kSsmHeads, (g + 1) * per - h0);
+    const int tid = threadIdx.x, j = tid >> 4, i = tid & 15;
+    int seq, chunk;
+    if (!find_chunk(blockIdx.x, a.cu, a.n_seqs, found, seq, chunk)) return;
+    const int first = a.cu[seq] + chunk * kQ, nt = min(kQ, a.cu[seq + 1] - first);
+    if (tid < kSsmHeads * kQ) {
+        const int hh = tid >> 4, t = tid & 15;
+        float dt = 0.f, dec = 1.f;             // a token beyond the chunk's end changes nothing
+        if (hh < nh && t < nt) {
+            dt = softplus_r(a.dt.p[(size_t)(first + t) * a.dt.stride + a.dt.col0 + h0 + hh] + a.dt_bias[h0 + hh]);
+            dec = expf(-expf(a.A_log[h0 + hh]) * dt);
+        }
+        dts[hh][t] = dt;
+        decs[hh][t] = dec;
+    }
+    float cb = 0.f;
+    for (int n0 = 0; n0 < a.N; n0 += 64) {
+        __syncthreads();
+        for (int e = tid; e < kQ * 64; e += 256) {
+            const int t = e >> 6, n = e & 63;
+            const bool on = t < nt && n0 + n < a.N;
+            const float* row = a.x.p + (size_t)(first + t) * a.x.stride + (size_t)g * a.N + n0 + n;
+            Bs[t][n] = on ? row[a.b_col0] : 0.f;
+            Cs[t][n] = on ? row[a.c_col0] : 0.f;
+        }
+        __syncthreads();
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int n = 0; n < 64; ++n) s[n & 3] += Cs[j][n] * Bs[i][n];
+        cb += (s[0] + s[1]) + (s[2] + s[3]);
+    }
+    // decays of the tokens i + 1 .. j of every head: a running product a (head, i)
+    __syncthreads();
+    if (tid < kSsmHeads * kQ) {
+        const int hh = tid >> 4, from = tid & 15;
+        float p = 1.f;
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) {
+            if (t > from) p *= decs[hh][t];
+            run[hh][t][from] = p;
+        }
+    }
+    __syncthreads();
+    for (int hh = 0; hh < nh; ++hh) {
+        const float p = run[hh][j][i];
+        float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h0 + hh) * part_floats(kSsm, 0);
+        out[j * kMs + i] = i > j ? 0.f : cb * p * dts[hh][i] + (i == j ? a.D[h0 + hh] : 0.f);
+        if (i < kMs - kQ) out[j * kMs + kQ + i] = 0.f;
+        if (i == 0) {                          // token j's factor of the read-out
+            out[kMat + j] = p * decs[hh][0];
+            if (j == kQ - 1) out[kMat + 32] = p * decs[hh][0];
+        }
+        if (j == kQ - 1) out[kMat + kQ + i] = p * dts[hh][i];       // and of what it writes
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the walk
+//
+// What bounds it: fp32 multiply-adds (2 a state element and token, 3 for the delta rule) on as many multiprocessors as there
+// are column tiles.  A thread holds NP / 16 rows of one or two columns.  Rows come from shared memory in 16-byte pieces, two
+// rows go into an instruction (fma.rn.f32x2: the rate of fma, half the issue slots, the same roundings).  The sums over the
+// sixteen row groups of a column: lane g keeps token x ^ g in place x, so that every exchange halves the values a lane
+// still holds and both partners give the same places away, without a select; lane g ends with token g.
+// ---------------------------------------------------------------------------------------------
+constexpr int kStages = 4;                     // chunks in shared memory: the one before, the one worked on, two on their way
+
+struct WalkArgs {
+    RowsIn v;
+    const float* scratch;
+    const float* rows;             // state-space scan: B and C where they lie
+    long long rows_stride;
+    int b_col0, c_col0, per_group, N;
+    float* y;
+    long long y_stride;
+    int heads, dv, vec;            // vec: B and C can be copied in 16-byte pieces
+    const int *cu, *slot_of_seq, *start_pos;
+    float* state;
+    long long slot_stride, copy_stride, state_off;
+};
+
+__device__ __forceinline__ void cp16(float* dst, const float* src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(float* dst, const float* src, int bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+typedef unsigned long long f32x2;              // two floats side by side
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// floats of a chunk in shared memory: the rows, the matrices and numbers, the values [16][columns]
+__host__ __device__ constexpr int stage_floats(int kind, int np, int ct) {
+    return (kind == kSsm ? 2 * kQ * np : rows_floats(kind, np)) + small_floats(kind) + kQ * ct;
+}
+
+// Dot products of the thread's rows with the sixteen tokens' rows, summed over the row groups of a column: the thread gets
+// token g's (with eight row groups g + 8's too) for each of its columns; of 32 row groups the lower 16 get the first half of
+// their columns and the upper 16, which hold the halves the other way round, theirs.
+template <int NP, int C, int RG>
+__device__ __forceinline__ void dots(const float* src, const f32x2 (&s)[NP / RG / 2][C], int g, float (&res)[RG < kQ ? kQ / RG : 1][RG == 32 ? C / 2 : C]) {
+    constexpr int P4 = NP / RG / 4, TG = RG < kQ ? RG : kQ, CK = RG == 32 ? C / 2 : C;
+    float v[kQ][C];
+#pragma unroll
+    for (int x = 0; x < kQ; ++x) {
+        const float* row = src + (x ^ (g % TG)) * NP + g * 4;
+        f32x2 acc[C];
+#pragma unroll
+        for (int m = 0; m < P4; ++m) {
+            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(row + m * 4 * RG);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                acc[c] = m == 0 ? mul2(s[0][c], k.x) : fma2(s[2 * m][c], k.x, acc[c]);
+                acc[c] = fma2(s[2 * m + 1][c], k.y, acc[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const float2 f = unpack2(acc[c]);
+            v[x][c] = f.x + f.y;
+        }
+    }
+#pragma unroll
+    for (int m = TG / 2; m >= 1; m >>= 1) {
+#pragma unroll
+        for (int x = 0; x < kQ; ++x) {
+            if (x % TG < m) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) v[x][c] += __shfl_xor_sync(0xffffffffu, v[x + m][c], m);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < kQ / TG; ++t)
+#pragma unroll
+        for (int c = 0; c < CK; ++c) res[t][c] = RG == 32 ? v[t * TG][c] + __shfl_xor_sync(0xffffffffu, v[t * TG][CK + c], 16) : v[t * TG][c];
+}
+
+template <int NP, int C, int RG, int CT, int KIND>
+__global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArgs a) {
+    constexpr int kWalkers = RG * CT / C;      // threads that compute; one more warp loads
+    constexpr int P4 = NP / RG / 4, TG = RG < kQ ? RG : kQ, TL = kQ / TG, CK = RG == 32 ? C / 2 : C;
+    constexpr int kRows = KIND == kSsm ? 2 * kQ * NP : rows_floats(KIND, NP), kSmall = small_floats(KIND);
+    constexpr int kPart = part_floats(KIND, NP), kStage = stage_floats(KIND, NP, CT);
+    extern __shared__ __align__(16) float sm[];
+    float* Ws = sm + kStages * kStage;               // delta: v - acc, then the corrected values, [2][16][CT]
+    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
+    const int first = a.cu[seq], n_new = a.cu[seq + 1] - first;
+    if (n_new <= 0) return;
+    const int chunks = (n_new + kQ - 1) / kQ, base = chunk_base(first, seq), start = a.start_pos[seq];
+    const int tid = threadIdx.x;
+
+    if (tid >= kWalkers) {                     // the loading warp, two chunks ahead of the others
+        const int lane = tid - kWalkers;
+        for (int chunk = 0; chunk < chunks + 2; ++chunk) {
+            if (chunk < chunks) {
+                float* st = sm + chunk % kStages * kStage;
+                const float* src = a.scratch + ((size_t)(base + chunk) * a.heads + h) * kPart;
+                const int at = first + chunk * kQ, nt = min(kQ, n_new - chunk * kQ);
+                if (KIND == kSsm) {
+                    const float* rows = a.rows + (size_t)at * a.rows_stride + (size_t)(h / a.per_group) * a.N;
+                    if (a.vec) {
+                        constexpr int kPieces = NP / 4, kAtOnce = kPieces < 32 ? 32 / kPieces : 1;      // rows a pass of the warp
+                        const int t0 = lane / kPieces, n0 = lane % kPieces * 4;
+                        const float *c = rows + t0 * a.rows_stride + a.c_col0 + n0, *b = c - a.c_col0 + a.b_col0;
+                        const long long step = kAtOnce * a.rows_stride;
+#pragma unroll
+                        for (int t = 0; t < kQ; t += kAtOnce) {
+#pragma unroll
+                            for (int n = 0; n < NP; n += 128) {
+                                const int on = t + t0 < nt && n + n0 < a.N ? 16 : 0;
+                                float* to = st + (t + t0) * NP + n + n0;
+                                cp16(to, on ? c + n : a.scratch, on);
+                                cp16(to + kQ * NP, on ? b + n : a.scratch, on);
+                            }
+                            c += step;
+                            b += step;
+                        }
+                    } else {
+                        for (int e = lane; e < 2 * kQ * NP; e += 32) {
+                            const int n = e % NP, t = e / NP % kQ, which = e / (NP * kQ);
+                            const bool on = t < nt && n < a.N;
+                            cp4(st + e, on ? rows + t * a.rows_stride + n + (which ? a.b_col0 : a.c_col0) : a.scratch, on ? 4 : 0);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < (kSmall / 4 + 31) / 32; ++i)
+                        if (lane + 32 * i < kSmall / 4) cp16(st + kRows + (lane + 32 * i) * 4, src + (lane + 32 * i) * 4, 16);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < (kPart / 4 + 31) / 32; ++i)
+                        if (lane + 32 * i < kPart / 4) cp16(st + (lane + 32 * i) * 4, src + (lane + 32 * i) * 4, 16);
+                }
+                const float* v = a.v.p + (size_t)at * a.v.stride + a.v.col0 + (size_t)h * a.dv + col0;
+#pragma unroll
+                for (int i = 0; i < kQ * CT / 32; ++i) {
+                    const int t = (lane + 32 * i) / CT, c = (lane + 32 * i) % CT;
+                    const bool on = t < nt && col0 + c < a.dv;
+                    cp4(st + kRows + kSmall + lane + 32 * i, on ? v + t * a.v.stride + c : a.scratch, on ? 4 : 0);
+                }
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 2;\n" ::: "memory");
+            if (chunk >= 2) __syncthreads();   // chunk - 2 is there, and the others are done with the one before it
+        }
+        return;
+    }
+
+    const int g = tid % RG, tg = g % TG, cl = tid / RG * C;     // row group, token, first column of the thread
+    const int turn = RG == 32 && g >= 16 ? C / 2 : 0;           // column p of the thread is cl + (p ^ turn)
+    // the state as it lies: [head][row / 8][column][row % 8]; the thread's rows are m * 4 RG + 4 g .. + 3
+    float* both = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off + (size_t)h * NP * a.dv;
+    const float* old = both + (size_t)(start & 1) * a.copy_stride;
+    float* fresh = both + (size_t)((start + n_new) & 1) * a.copy_stride;
+    f32x2 s[2 * P4][C];
+#pragma unroll
+    for (int m = 0; m < P4; ++m)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const int col = col0 + cl + (c ^ turn);
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (start > 0 && col < a.dv) {
+                const float* p = old + ((size_t)(m * (RG / 2) + (g >> 1)) * a.dv + col) * 8 + (g & 1) * 4;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = p[e];
+            }
+            s[2 * m][c] = pack2(v[0], v[1]);
+            s[2 * m + 1][c] = pack2(v[2], v[3]);
+        }
+    // the thread's columns of sixteen rows [16][CT]
+    auto columns = [&](const float* from, float (&x)[kQ][C]) {
+#pragma unroll
+        for (int i = 0; i < kQ; ++i) {
+            if (C == 1) {
+                x[i][0] = from[i * CT + cl];
+            } else {
+#pragma unroll
+                for (int c = 0; c < C; c += 2) {
+                    const float2 f = *reinterpret_cast<const float2*>(from + i * CT + cl + (c ^ turn));
+                    x[i][c] = f.x;
+                    x[i][C > 1 ? c + 1 : 0] = f.y;
+                }
+            }
+        }
+    };
+
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+        __syncthreads();
+        const float* st = sm + chunk % kStages * kStage;
+        const float* q = st + (KIND == kDelta ? kQ * NP : 0);
+        const float* kd = q + kQ * NP;
+        const float* M = st + kRows;
+        const float* V = st + kRows + kSmall;
+        const int nt = min(kQ, n_new - chunk * kQ);
+        float o[TL][CK];
+        dots<NP, C, RG>(q, s, g, o);
+        if (KIND == kSsm) {
+#pragma unroll
+            for (int t = 0; t < TL; ++t)
+#pragma unroll
+                for (int c = 0; c < CK; ++c) o[t][c] *= M[kMat + t * TG + tg];
+        }
+        float x[kQ][C];                        // what the matrices are applied to, and then what is written
+        if (KIND == kDelta) {
+            float acc[TL][CK];
+            dots<NP, C, RG>(st, s, g, acc);
+#pragma unroll
+            for (int t = 0; t < TL; ++t)
+#pragma unroll
+                for (int c = 0; c < CK; ++c) {
+                    const int at = (t * TG + tg) * CT + cl + turn + c;
+                    Ws[at] = V[at] - acc[t][c];
+                }
+            __syncwarp();                      // a column's values are written and read by the same warp
+            columns(Ws, x);
+        } else {
+            columns(V, x);
+        }
+        float u[TL][CK];
+#pragma unroll
+        for (int t = 0; t < TL; ++t) {
+#pragma unroll
+            for (int c = 0; c < CK; ++c) u[t][c] = 0.f;
+#pragma unroll
+            for (int i = 0; i < kQ; i += 4) {
+                const float4 mm = *reinterpret_cast<const float4*>(M + (t * TG + tg) * kMs + i);
+#pragma unroll
+                for (int c = 0; c < CK; ++c) o[t][c] += (mm.x * x[i][c] + mm.y * x[i + 1][c]) + (mm.z * x[i + 2][c] + mm.w * x[i + 3][c]);
+                if (KIND == kDelta) {
+                    const float4 tt = *reinterpret_cast<const float4*>(M + kMat + (t * TG + tg) * kMs + i);
+#pragma unroll
+                    for (int c = 0; c < CK; ++c) u[t][c] += (tt.x * x[i][c] + tt.y * x[i + 1][c]) + (tt.z * x[i + 2][c] + tt.w * x[i + 3][c]);
+                }
+            }
+        }
+        if (KIND == kDelta) {
+            float* U = Ws + kQ * CT;
+#pragma unroll
+            for (int t = 0; t < TL; ++t)
+#pragma unroll
+                for (int c = 0; c < CK; ++c) U[(t * TG + tg) * CT + cl + turn + c] = u[t][c];
+            __syncwarp();
+            columns(U, x);
+        }
+#pragma unroll
+        for (int t = 0; t < TL; ++t) {
+            if (t * TG + tg < nt) {
+                float* row = a.y + (size_t)(first + chunk * kQ + t * TG + tg) * a.y_stride + (size_t)h * a.dv + col0 + cl + turn;
+#pragma unroll
+                for (int c = 0; c < CK; ++c)
+                    if (col0 + cl + turn + c < a.dv) row[c] = o[t][c];
+            }
+        }
+        // the state behind the chunk
+#pragma unroll
+        for (int m = 0; m < P4; ++m) {
+            ulonglong2 G;
+            if (KIND == kSsm) G.x = G.y = pack2(M[kMat + 32], M[kMat + 32]);
+            else G = *reinterpret_cast<const ulonglong2*>(kd + kQ * NP + m * 4 * RG + g * 4);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                s[2 * m][c] = mul2(s[2 * m][c], G.x);
+                s[2 * m + 1][c] = mul2(s[2 * m + 1][c], G.y);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kQ; ++t) {
+            const float f = KIND == kSsm ? M[kMat + kQ + t] : 1.f;
+            f32x2 xx[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float v = KIND == kSsm ? x[t][c] * f : x[t][c];
+                xx[c] = pack2(v, v);
+            }
+#pragma unroll
+            for (int m = 0; m < P4; ++m) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(kd + t * NP + m * 4 * RG + g * 4);
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    s[2 * m][c] = fma2(k.x, xx[c], s[2 * m][c]);
+                    s[2 * m + 1][c] = fma2(k.y, xx[c], s[2 * m + 1][c]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < P4; ++m)
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const int col = col0 + cl + (c ^ turn);
+            if (col < a.dv) {
+                float* p = fresh + ((size_t)(m * (RG / 2) + (g >> 1)) * a.dv + col) * 8 + (g & 1) * 4;
+                const float2 lo = unpack2(s[2 * m][c]), hi = unpack2(s[2 * m + 1][c]);
+                p[0] = lo.x;
+                p[1] = lo.y;
+                p[2] = hi.x;
+                p[3] = hi.y;
+            }
+        }
+}
+
+// Rows of a state as the scans keep them: eight times a power of two.
+static int padded_rows(int rows) {
+    int n = 8;
+    while (n < rows) n *= 2;
+    return n;
+}
+
+template <typename K>
+static int allow_smem(K kernel, size_t smem) {
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "scan_chunks: %s", cudaGetErrorString(e));
+    }
+    return BLM_OK;
+}
+
+template <int NP, int C, int RG, int CT, int KIND>
+static int launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+    const size_t smem = ((size_t)kStages * stage_floats(KIND, NP, CT) + (KIND == kDelta ? 2 * kQ * CT : 0)) * sizeof(float);
+    if (int rc = allow_smem(walk_kernel<NP, C, RG, CT, KIND>, smem)) return rc;
+    walk_kernel<NP, C, RG, CT, KIND><<<dim3((a.dv + CT - 1) / CT, a.heads, n_seqs), RG * CT / C + 32, smem, stream>>>(a);
+    return blm_check_launch("scan_chunks (walk)");
+}
+
+// Rows and columns of a thread, columns of a block.  Four columns a thread: a row piece that comes from shared memory serves four
+// multiply-adds a row; 16 columns a block: a prompt of few heads still has a block for most multiprocessors.  2,048 tokens, states
+// of 128 rows (decay of 32 heads x 128 columns / state-space scan of 64 x 64 / delta rule of 16 x 128, 2,001 tokens), us:
+// 4 columns, 4 rows, 16 a block 177 / 202 / 174; 32 a block 198 / 208 / 249; 2 columns, 8 rows, 16 a block 206 / 216 / 188;
+// 4 columns, 8 rows, 16 a block (64 threads) 237 / 260 / 211, 32 a block 184 / 200 / 216.
+template <int KIND>
+static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
+    switch (np) {
+        case 32: return launch_walk<32, 2, 8, 32, KIND>(a, n_seqs, stream);
+        case 64: return launch_walk<64, 2, 16, 16, KIND>(a, n_seqs, stream);
+        case 128: return launch_walk<128, 4, 32, 16, KIND>(a, n_seqs, stream);
+        case 256: return launch_walk<256, 4, 32, 16, KIND>(a, n_seqs, stream);
+    }
+    return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
+}
+
+// Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows).
+BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs) {
+    const int np = padded_rows(rows);
+    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta) return 0;
+    return (long long)chunk_bound(n_tokens, n_seqs) * heads * part_floats(kind, np);
+}
+
+static int check_step(int n_tokens, int n_seqs, int heads) {
+    BLM_REQUIRE(heads > 0 && heads <= 65535 && n_seqs <= 65535 && n_tokens > 0, "scan_chunks: %d heads, %d sequences", heads, n_seqs);
+    return BLM_OK;
+}
+
+BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
+                                long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
+                                long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
+                                const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, float* state,
+                                long long slot_stride, long long copy_stride, long long state_off, float* scratch, cudaStream_t stream) {
+    if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
+    BLM_REQUIRE(groups > 0 && heads % groups == 0 && dv > 0, "scan_chunks: bad head counts");
+    if (int rc = check_step(n_tokens, n_seqs, heads)) return rc;
+    const int np = padded_rows(N), per = heads / groups;
+    SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, cu_seqlens, n_seqs, heads,
+                     groups, N, scratch};
+    prep_ssm_kernel<<<dim3(chunk_bound(n_tokens, n_seqs), groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
+    if (int rc = blm_check_launch("scan_chunks (state-space scan)")) return rc;
+    WalkArgs a = {};
+    a.v = {xbc, xbc_stride, x_col0};
+    a.scratch = scratch;
+    a.rows = xbc;
+    a.rows_stride = xbc_stride;
+    a.b_col0 = b_col0;
+    a.c_col0 = c_col0;
+    a.per_group = per;
+    a.N = N;
+    a.y = y;
+    a.y_stride = y_stride;
+    a.heads = heads;
+    a.dv = dv;
+    a.vec = ((size_t)xbc & 15) == 0 && xbc_stride % 4 == 0 && b_col0 % 4 == 0 && c_col0 % 4 == 0 && N % 4 == 0;
+    a.cu = cu_seqlens;
+    a.slot_of_seq = slot_of_seq;
+    a.start_pos = start_pos;
+    a.state = state;
+    a.slot_stride = slot_stride;
+    a.copy_stride = copy_stride;
+    a.state_off = state_off;
+    return walk<kSsm>(a, np, n_seqs, stream);
+}
+
+template <int NP, int MODE>
+static int launch_prep(const PrepArgs& p, dim3 grid, cudaStream_t stream) {
+    constexpr int smem = prep_smem(NP, MODE == kModeDelta);
+    if (int rc = allow_smem(prep_rows_kernel<NP, MODE>, smem)) return rc;
+    prep_rows_kernel<NP, MODE><<<grid, prep_threads(NP), smem, stream>>>(p);
+    return blm_check_launch("scan_chunks (rows)");
+}
+
+template <int NP>
+static int prep(const PrepArgs& p, int mode, dim3 grid, cudaStream_t stream) {
+    if (mode == kModeDelta) return launch_prep<NP, kModeDelta>(p, grid, stream);
+    if (mode == kModeExp) return launch_prep<NP, kModeExp>(p, grid, stream);
+    if (mode == kModeExpFirst) return launch_prep<NP, kModeExpFirst>(p, grid, stream);
+    return launch_prep<NP, kModeLower>(p, grid, stream);
+}
+
+// The decays per row and the delta rule.  b_raw null: the former (kinds and `extra` as in blm_decay_scan); else the latter.
+BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0, const float* k, long long k_stride, int k_col0,
+                                 const float* v, long long v_stride, int v_col0, const float* b_raw, long long b_stride, int b_col0,
+                                 const float* a_raw, long long a_stride, int a_col0, const float* bias, const float* extra,
+                                 const float* A_log, float* o, long long o_stride, int heads, int qk_heads, int dk, int dv,
+                                 int lower_bound, int read_first, const int* cu_seqlens, const int* slot_of_seq, const int* start_pos,
+                                 int n_tokens, int n_seqs, float* state, long long slot_stride, long long copy_stride,
+                                 long long state_off, float* scratch, cudaStream_t stream) {
+    if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
+    BLM_REQUIRE(qk_heads > 0 && heads % qk_heads == 0 && dk > 0 && dv > 0, "scan_chunks: bad head counts");
+    if (int rc = check_step(n_tokens, n_seqs, heads)) return rc;
+    const bool delta = b_raw != nullptr;
+    BLM_REQUIRE(delta ? k != nullptr && A_log != nullptr && !read_first && !lower_bound : (k != nullptr || lower_bound), "scan_chunks: no keys");
+    BLM_REQUIRE(!lower_bound || (extra != nullptr && !read_first), "scan_chunks: a lower bound, and the state read last");
+    const int np = padded_rows(dk);
+    PrepArgs p = {{q, q_stride, q_col0}, {k, k_stride, k_col0}, {a_raw, a_stride, a_col0}, {b_raw, b_stride, b_col0}, bias, extra, A_log,
+                  cu_seqlens, n_seqs, heads, qk_heads, dk, scratch};
+    const int mode = delta ? kModeDelta : (lower_bound ? kModeLower : (read_first ? kModeExpFirst : kModeExp));
+    const dim3 grid(chunk_bound(n_tokens, n_seqs), heads);
+    int rc = BLM_OK;
+    switch (np) {
+        case 32: rc = prep<32>(p, mode, grid, stream); break;
+        case 64: rc = prep<64>(p, mode, grid, stream); break;
+        case 128: rc = prep<128>(p, mode, grid, stream); break;
+        case 256: rc = prep<256>(p, mode, grid, stream); break;
+        default: return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
+    }
+    if (rc != BLM_OK) return rc;
+    WalkArgs a = {};
+    a.v = {v, v_stride, v_col0};
+    a.scratch = scratch;
+    a.y = o;
+    a.y_stride = o_stride;
+    a.heads = heads;
+    a.dv = dv;
+    a.cu = cu_seqlens;
+    a.slot_of_seq = slot_of_seq;
+    a.start_pos = start_pos;
+    a.state = state;
+    a.slot_stride = slot_stride;
+    a.copy_stride = copy_stride;
+    a.state_off = state_off;
+    return delta ? walk<kDelta>(a, np, n_seqs, stream) : walk<kDecay>(a, np, n_seqs, stream);
+}

@@ -142,6 +142,16 @@ _protos = {
         "blm_gated_group_norm": [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                  c_float, c_void_p, c_int, c_longlong, c_int, c_void_p],
     },
+    "scan_chunks": {
+        "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int],
+        "blm_scan_chunks_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
+                                c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                                c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+        "blm_scan_chunks_rows": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p,
+                                 c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong,
+                                 c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                                 c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+    },
     "retention": {
         "blm_retention_scan": _RETENTION + [c_void_p, c_longlong, c_void_p],
         "blm_retention_step": _RETENTION + [c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_longlong, c_void_p],
@@ -232,6 +242,9 @@ _protos = {
 _bound: dict[str, ctypes.CDLL] = {}
 
 
+_LONG_RESULTS = ("blm_scan_chunks_scratch",)     # entry points that return a number of floats instead of a status
+
+
 def _lib(module: str) -> ctypes.CDLL:
     lib = _bound.get(module)
     if lib is None:
@@ -239,7 +252,7 @@ def _lib(module: str) -> ctypes.CDLL:
         for name, argtypes in _protos.get(module, {}).items():
             fn = getattr(lib, name)
             fn.argtypes = argtypes
-            fn.restype = c_int
+            fn.restype = c_longlong if name in _LONG_RESULTS else c_int
         err = getattr(lib, f"blm_{module}_last_error")
         err.restype = ctypes.c_char_p
         err.argtypes = []
@@ -1336,6 +1349,24 @@ def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, sta
           kernels=2 if k > 1 and not single else 1)
 
 
+# From this many new tokens of a sequence on, a step's recurrences run in chunks of sixteen tokens (scan_chunks.cu): the two
+# launches cost what walking some 24 tokens does (a part of 2,048 lanes, chunks against the walk: 16 tokens 56 / 51 us for the
+# state-space scan, 32 / 33 for the lower-bounded decay; 32 tokens 52 / 52 and 28 / 38; 64 tokens 61 / 73 and 30 / 57).  A single
+# token costs a chunk all the same (64 of them: 241 / 121 and 104 / 53 us), so steps that are mostly single tokens are walked.
+SCAN_CHUNK_TOKENS = 32
+SCAN_CHUNK_MEAN = 4
+_SCAN_SSM, _SCAN_DECAY, _SCAN_DELTA = 0, 1, 2
+
+
+def _scan_chunks_scratch(kind, heads, rows, step, device):
+    """Scratch for a step whose recurrence runs in chunks, or None where it is walked token by token: single tokens and
+    short portions, states of up to 16 rows."""
+    if getattr(step, "max_q_len", 0) < SCAN_CHUNK_TOKENS or step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs:
+        return None
+    floats = int(_lib("scan_chunks").blm_scan_chunks_scratch(kind, heads, rows, step.n_tokens, step.n_seqs))
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
+
+
 def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y, heads, groups, n_state, value_dim, step, state,
              state_offset, wide_sums=False):
     """The state-space scan per head: S <- exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x with dt = softplus(dt_raw +
@@ -1351,6 +1382,12 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     dp, ds, dc = _cols(dt, dt_col0, heads)
     if tuple(y.shape) != (step.n_tokens, heads * value_dim) or not y.is_contiguous():
         raise KernelError("ssm_scan: y float32 [N, heads * value_dim]")
+    scratch = None if wide_sums else _scan_chunks_scratch(_SCAN_SSM, heads, n_state, step, y.device)
+    if scratch is not None:
+        _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
+              _ptr(d_skip), _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+        return
     _call("recurrent", "blm_ssm_scan", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
           _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
           _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, _stream())
@@ -1371,6 +1408,12 @@ def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a
     aa = _cols(a, a_col0, heads * key_dim)
     if tuple(out.shape) != (step.n_tokens, heads * value_dim) or not out.is_contiguous() or dt_bias.numel() != heads * key_dim:
         raise KernelError("delta_scan: out float32 [N, heads * value_dim], dt_bias [heads * key_dim]")
+    scratch = _scan_chunks_scratch(_SCAN_DELTA, heads, key_dim, step, out.device)
+    if scratch is not None:
+        _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(None), _ptr(a_log), _ptr(out),
+              c_longlong(out.stride(0)), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+        return
     _call("recurrent", "blm_delta_scan", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(a_log), _ptr(out), c_longlong(out.stride(0)),
           heads, qk_heads, key_dim, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_seqs,
           *_state_args(state, state_offset), _stream())
@@ -1414,6 +1457,13 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
         raise KernelError("decay_scan: out float32 [N, heads * value_dim], bias [heads * key_dim]")
     if extra is not None and extra.numel() != heads * key_dim:
         raise KernelError("decay_scan: extra [heads * key_dim]")
+    scratch = None if wide_sums else _scan_chunks_scratch(_SCAN_DECAY, heads, key_dim, step, out.device)
+    if scratch is not None:
+        _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, c_void_p(0), c_longlong(0), 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
+              _ptr(out), c_longlong(out.stride(0)), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
+              1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs,
+              *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+        return
     _call("recurrent", "blm_decay_scan", *qa, *ka, *va, *aa, _ptr(bias), _ptr(extra), _ptr(out), c_longlong(out.stride(0)), heads,
           key_dim, value_dim, int(kind), 1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos),
           step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, _stream())

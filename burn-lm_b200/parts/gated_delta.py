@@ -41,7 +41,7 @@ class GatedDelta(Part):
     family = "mixer"
     graph_safe = True
     roles = ("q", "q_conv", "k", "k_conv", "v", "v_conv", "b", "A_log", "norm", "a1", "a2", "dt_bias", "g1", "g2", "o")
-    kernel_modules = ("recurrent",)
+    kernel_modules = ("recurrent", "scan_chunks")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

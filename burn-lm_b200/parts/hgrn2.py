@@ -34,7 +34,7 @@ class Hgrn2(Part):
     family = "mixer"
     graph_safe = True
     roles = ("q", "f", "f_bias", "lower", "v", "norm", "o")
-    kernel_modules = ("recurrent",)
+    kernel_modules = ("recurrent", "scan_chunks")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

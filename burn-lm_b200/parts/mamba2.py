@@ -40,7 +40,7 @@ class Mamba2(Part):
     family = "mixer"
     graph_safe = True
     roles = ("in", "conv", "conv_bias", "dt_bias", "A_log", "D", "norm", "o")
-    kernel_modules = ("recurrent",)
+    kernel_modules = ("recurrent", "scan_chunks")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

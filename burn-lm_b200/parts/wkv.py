@@ -40,7 +40,7 @@ class Wkv(Part):
     graph_safe = True
     takes_float32_input = True           # the mixes are taken from the unrounded input
     roles = tuple("mu_" + m for m in MIXES) + ("r", "k", "v", "g", "w1", "w2", "w0", "u", "norm", "o")
-    kernel_modules = ("recurrent", "stream_ops", "gemm")
+    kernel_modules = ("recurrent", "scan_chunks", "stream_ops", "gemm")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

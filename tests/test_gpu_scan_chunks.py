@@ -1,0 +1,124 @@
+"""The recurrences in chunks of sixteen tokens (scan_chunks.cu) against the walk in float64, at the edges of chunks, of row
+and column tiles, through used states, and beside single tokens in one step."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from burn_lm_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def step_of(lens, starts):
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return SimpleNamespace(cu_seqlens=i32(cu), slot_of_seq=i32([len(lens) + 1 - s for s in range(len(lens))]), start_pos=i32(starts),
+                           n_tokens=cu[-1], n_seqs=len(lens), max_q_len=max(lens))
+
+
+def state_of(step, heads, rows, dv, offset, gen):
+    """A state block per slot whose unused rows hold zeros, as the scans leave them; everything else is drawn."""
+    floats = K.scan_state_floats(heads, rows, dv)
+    slots = step.n_seqs + 2
+    state = torch.randn((slots, 2, offset + floats), generator=gen, device="cuda")
+    padded = floats // heads // dv
+    lanes = state[:, :, offset:].view(slots, 2, heads, padded // 8, dv, 8)
+    lanes *= (torch.arange(padded, device="cuda").view(padded // 8, 1, 8) < rows)
+    return state
+
+
+def read_state(state, slot, copy, offset, heads, dv):
+    lanes = state[slot, copy, offset:].view(heads, -1, dv, 8)
+    return lanes.permute(0, 1, 3, 2).reshape(heads, -1, dv)
+
+
+def walk(q, k, v, w, beta, bonus, S):
+    """float64, token by token: (outputs [T, H, dv], the state behind the last token)."""
+    out = []
+    for t in range(q.shape[0]):
+        if bonus is not None:
+            kv = k[t][:, :, None] * v[t][:, None, :]
+            out.append(torch.einsum("hrv,hr->hv", S + bonus[:, :, None] * kv, q[t]))
+            S = w[t][:, :, None] * S + kv
+            continue
+        S = w[t][:, :, None] * S
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hrv,hr->hv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None, :]
+        out.append(torch.einsum("hrv,hr->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+STEPS = [([33], [0]), ([160, 1, 47], [0, 5, 64]), ([16, 32, 17, 15], [1, 0, 2, 3]), ([513], [7])]
+SIZES = [(2, 20, 5), (3, 64, 64), (4, 128, 100), (1, 200, 33), (40, 48, 48)]      # heads, rows, columns: every instance and its edges
+
+
+@pytest.mark.parametrize("lens,starts", STEPS)
+@pytest.mark.parametrize("heads,rows,dv", SIZES)
+@pytest.mark.parametrize("kind", ["ssm", "wkv", "lower", "delta"])
+def test_chunks_against_the_walk_in_float64(kind, heads, rows, dv, lens, starts):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(heads * 1000 + rows + len(lens))
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    step, n, offset = step_of(lens, starts), sum(lens), 7                    # (an odd offset: the state is not 16-byte aligned)
+    state = state_of(step, heads, rows, dv, offset, gen)
+    before = state.double()
+    out = torch.zeros((n, heads * dv), device="cuda")
+    f64 = lambda t, *shape: t.double().reshape(n, *shape)
+    beta = bonus = None
+    if kind == "ssm":
+        groups = 2 if heads % 2 == 0 else 1
+        odd = 1 if heads == 2 else 0                                          # (rows that cannot be copied in 16-byte pieces)
+        b0 = (heads * dv + 3) // 4 * 4 + odd
+        x, dt = rnd(n, b0 + 2 * groups * rows), rnd(n, heads)
+        dt_bias, a_log, skip = rnd(heads) - 2, rnd(heads), rnd(heads)
+        K.ssm_scan(x, 0, b0, b0 + groups * rows, dt, 0, dt_bias, a_log, skip, out, heads, groups, rows, dv, step, state, offset)
+        d = torch.nn.functional.softplus(dt.double() + dt_bias.double())
+        v = f64(x[:, :heads * dv], heads, dv)
+        k = f64(x[:, b0:b0 + groups * rows], groups, rows).repeat_interleave(heads // groups, 1) * d[..., None]
+        q = f64(x[:, b0 + groups * rows:], groups, rows).repeat_interleave(heads // groups, 1)
+        w = torch.exp(-torch.exp(a_log.double()) * d)[..., None].expand(n, heads, rows)
+    else:
+        qr, kr, v32, a = rnd(n, heads * rows), rnd(n, heads * rows), rnd(n, heads * dv), rnd(n, heads * rows)
+        bias, v = rnd(heads * rows), f64(v32, heads, dv)
+        if kind == "delta":
+            b, a_log = rnd(n, heads), rnd(heads)
+            K.delta_scan(qr, 0, kr, 0, v32, 0, b, 0, a, 0, bias, a_log, out, heads, heads, rows, dv, step, state, offset)
+            unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+            q, k, beta = unit(f64(qr, heads, rows)) * rows ** -0.5, unit(f64(kr, heads, rows)), torch.sigmoid(b.double())
+            w = torch.exp(-torch.exp(a_log.double())[:, None] * torch.nn.functional.softplus((a.double() + bias.double()).view(n, heads, rows)))
+        elif kind == "wkv":
+            extra = rnd(heads * rows)
+            K.decay_scan(qr, 0, kr, 0, v32, 0, a, 0, bias, extra, out, heads, rows, dv, K.DECAY_EXP_EXP, True, step, state, offset)
+            q, k, bonus = f64(qr, heads, rows), f64(kr, heads, rows), extra.double().view(heads, rows)
+            w = torch.exp(-torch.exp(a.double() + bias.double())).view(n, heads, rows)       # (from one to none left in a token)
+        else:
+            low = torch.rand(heads * rows, generator=gen, device="cuda")
+            K.decay_scan(qr, 0, None, 0, v32, 0, a, 0, bias, low, out, heads, rows, dv, K.DECAY_LOWER_BOUND, False, step, state, offset)
+            w = (low.double() + (1 - low.double()) * torch.sigmoid(a.double() + bias.double())).view(n, heads, rows)
+            q, k = torch.nn.functional.silu(f64(qr, heads, rows)), 1 - w
+    at = 0
+    for s, (m, start) in enumerate(zip(lens, starts)):
+        slot = int(step.slot_of_seq[s])
+        S = read_state(before, slot, start & 1, offset, heads, dv)[:, :rows]
+        if start == 0:
+            S = torch.zeros_like(S)
+        sl = slice(at, at + m)
+        want, S = walk(q[sl], k[sl], v[sl], w[sl], None if beta is None else beta[sl], bonus, S)
+        if kind == "ssm":
+            want = want + skip.double()[:, None] * v[sl]
+        got = read_state(state, slot, (start + m) & 1, offset, heads, dv).double()
+        # fp32 sums of a few hundred terms and decays of at most sixteen factors: a few units of 2^-23 of the largest value;
+        # the lower bound's written row 1 - w is formed in fp32 from a w close to 1
+        tol = 2e-5 if kind == "lower" else 1e-5
+        assert (out[sl].double().view(m, heads, dv) - want).abs().max() <= tol * want.abs().max()
+        assert (got[:, :rows] - S).abs().max() <= tol * S.abs().max()
+        assert not got[:, rows:].any()
+        if (start + m) & 1 != start & 1:                                     # the other copy, what lies in front, and other slots stay
+            assert torch.equal(state[slot, start & 1], before[slot, start & 1].float())
+        assert torch.equal(state[slot, :, :offset], before[slot, :, :offset].float())
+        at += m
+    for slot in set(range(state.shape[0])) - set(step.slot_of_seq.tolist()):
+        assert torch.equal(state[slot], before[slot].float())
