@@ -202,9 +202,10 @@ _protos = {
     },
     "gemm": {
         "blm_gemm_f32": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
-                         c_longlong, c_void_p],
+                         c_longlong, c_void_p, c_void_p],
         "blm_gemm_f32_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                                 c_longlong, c_longlong, c_longlong, c_void_p],
+                                 c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+        "blm_gemm_f32_scratch": [c_int, c_int, c_int, c_int],
     },
     "gemv": {
         "blm_gemv": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
@@ -242,7 +243,7 @@ _protos = {
 _bound: dict[str, ctypes.CDLL] = {}
 
 
-_LONG_RESULTS = ("blm_scan_chunks_scratch",)     # entry points that return a number of floats instead of a status
+_LONG_RESULTS = ("blm_scan_chunks_scratch", "blm_gemm_f32_scratch")     # entry points that return a number of floats instead of a status
 
 
 def _lib(module: str) -> ctypes.CDLL:
@@ -850,8 +851,15 @@ def gemm_f32(x, w, out=None):
         out = torch.empty((n, m), dtype=torch.float32, device=x.device)
     elif tuple(out.shape) != (n, m) or out.dtype != torch.float32:
         raise KernelError("gemm_f32: out must be float32 [N, M]")
-    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _stream())
+    scratch = _gemm_f32_scratch(1, n, m, k, x.device)
+    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _stream(), kernels=2 if scratch is not None else 1)
     return out
+
+
+def _gemm_f32_scratch(batch, n, m, k, device):
+    """A plane of sums for every share of K that the float32 product cuts its sums into; None where there is one share."""
+    floats = int(_lib("gemm").blm_gemm_f32_scratch(batch, n, m, k))
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
 
 
 def batched_product(x, w, out=None, out_dtype=None):
@@ -872,8 +880,10 @@ def batched_product(x, w, out=None, out_dtype=None):
             out = torch.empty((b, n, m), dtype=torch.float32, device=x.device)
         if out.dtype != torch.float32 or tuple(out.shape) != (b, n, m) or any(t.stride(2) != 1 for t in (x, w, out)):
             raise KernelError("batched_product: float32 out [B, N, M]; unit stride along the last axis")
+        scratch = _gemm_f32_scratch(b, n, m, k, x.device)
         _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, c_longlong(x.stride(1)), c_longlong(w.stride(1)),
-              c_longlong(out.stride(1)), c_longlong(x.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)), _stream())
+              c_longlong(out.stride(1)), c_longlong(x.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)), _ptr(scratch),
+              _stream(), kernels=2 if scratch is not None else 1)
         return out
     if out is not None:
         return torch.bmm(x, w.transpose(1, 2), out=out)

@@ -1,0 +1,27 @@
+"""The float32 product at the edges of its tiles and of its shares of K, against float64; a row's bits depend on nothing but
+the row and the weights."""
+import pytest
+import torch
+
+from burn_lm_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 16, 17, 32, 33, 65, 130])
+@pytest.mark.parametrize("m,k", [(33, 5), (128, 1023), (129, 1024), (300, 1025), (64, 2600), (40, 4096)])
+def test_product_at_the_edges(n, m, k):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n * 100003 + m * 31 + k)
+    x, w = (torch.randn(shape, generator=gen, device="cuda") for shape in ((n, k), (m, k)))
+    want = x.double() @ w.double().T
+    y = K.gemm_f32(x, w)
+    # sums of K products of unit normals: rounding errors of at most sqrt(K) 2^-24 times partial sums of size sqrt(K)
+    assert (y.double() - want).abs().max() <= 4 * k * 2.0 ** -24
+    assert torch.equal(K.gemm_f32(x[:1].contiguous(), w), y[:1])
+    assert torch.equal(K.gemm_f32(x, w[3:20].contiguous()), y[:, 3:20])
+    # the same as one of a batch of strided operands
+    wide = torch.zeros((n, 2, k + 3), device="cuda")
+    wide[:, 1, :k] = x
+    both = K.batched_product(wide[:, :, :k].transpose(0, 1), torch.stack([w, w]), out=torch.empty((n, 2, m), device="cuda").transpose(0, 1))
+    assert torch.equal(both[1], y) and not both[0].any()
