@@ -434,9 +434,6 @@ def nufolix_kernels(z, pk):
 
     def attention_case(n_seqs, new, cached):
         total = cached + new
-        # the key ranges the mixer takes at this size (parts.sigmoid_attention.SigmoidAttention._ranges)
-        tiles, sms = n_seqs * (-(-new // 16)), K.sm_count()
-        ranges = max(1, min(-(-(4 if new == 1 else 2) * sms // tiles), total // (K.PAGE if new == 1 else 256), 64))
         pages_each = -(-total // K.PAGE)
         n = n_seqs * new
         bt = torch.arange(n_seqs * pages_each, dtype=torch.int32, device=dev).reshape(n_seqs, pages_each)
@@ -447,6 +444,7 @@ def nufolix_kernels(z, pk):
         ms_llama = _time(lambda: K.attention(q, q.shape[1], pool5, bt, st.cu_seqlens, st.slot_of_seq, st.start_pos, o, n, n_seqs, new,
                                              H, G, hd, hd ** -0.5, window=0, n_splits=1, max_kv_len=total))
         pool = pool5.reshape(n_seqs * pages_each, -1)
+        ranges = K.sigmoid_attention_ranges(st, H, G, hd, hd, bf, torch.device(dev))        # the key ranges the mixer takes at this size
         talk = torch.randn((H, H), dtype=torch.float32, device=dev) * 0.2
         pb = torch.randn(H, dtype=torch.float32, device=dev) - 3.0
         partial = torch.empty(ranges * n * H * hd, dtype=torch.float32, device=dev) if ranges > 1 else None

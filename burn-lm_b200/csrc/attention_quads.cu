@@ -1,0 +1,713 @@
+// Attention without a softmax whose heads' weights are mixed before they meet the values (attention_sigmoid.cu states the
+// equations), bfloat16, up to four query heads a key/value head and up to eight key/value heads: scores, mix and values of a
+// tile of keys in one warp's registers.
+//
+// What bounds the form with shared memory between the three (attention_sigmoid.cu): every weight is written, read once a mixed
+// head and written again, and three barriers a chunk keep the tensor cores idle 95 % of the time.  Here the three products
+// are laid so that each leaves its result where the next one wants its operand:
+//   scores, transposed:  S^T = K Q^T.  A tile's sixteen rows are keys; its eight columns are (head of the key/value head, query),
+//     column 2 h + x.  Lane l then holds head l % 4 of every key/value head at key l / 4 - which is the B operand of
+//   the mix:  M = talk W, m16n8k8 in tf32: k runs over (key/value head pair, l % 4), the columns are keys.  Weights and talk are each
+//     the sum of two tf32 numbers (22 bits), three products of the four: the error is that of fp32 sums, not of tf32.
+//     Lane l gets head row l / 4 at keys 2 (l % 4), + 1 - which, packed to bfloat16, is the B operand of
+//   the values, transposed:  O^T += V^T M^T: rows are value lanes, k runs over keys, columns are eight head rows, of which four
+//     belong to the key/value head.  Two queries fill both halves: the second query's rows cross over by one shuffle.
+// Weights, their mix and the outputs never leave registers; shared memory holds keys, values, the queries' and talk's fragments.
+// 1,536 tokens of 32 heads of 64 on 8: 695 -> 163 us; 64 single tokens over 1,088 keys: 220 -> 38 us (3.7 TB/s).
+#include "common.cuh"
+
+BLM_API const char* blm_attention_quads_last_error() { return g_blm_error; }
+
+constexpr int kQuads = 8;          // key/value heads, four query heads (or fewer, the others' talk being zero) each
+
+struct QuadArgs {
+    const __nv_bfloat16* q;        // [N, H dk]
+    const __nv_bfloat16* pool;     // pages: keys [G][page][dk] then values [G][page][dv]
+    const int* block_table;
+    int table_stride;
+    const int *cu_seqlens, *slot_of_seq, *start_pos, *token_seq;
+    const float* talk;             // [H, H] or null
+    const float* head_bias;        // [H] or null
+    __nv_bfloat16* out;            // [N, H dv] (one range)
+    float* partial;                // [ranges][N][H dv] fp32 (several ranges)
+    int n_tokens, n_seqs, q_tiles, H, G, dk, dv, page, ranges;
+    float scale, softcap;
+};
+
+// Tiles of a range when a row's `tiles` are cut into `ranges` ranges of `least` tiles at least (fewer ranges then): 256 keys where
+// a block shares them among its queries, 64 for a single token.
+__host__ __device__ inline int tiles_of_range(int tiles, int ranges, int least) {
+    const int even = (tiles + ranges - 1) / ranges;
+    return even > least ? even : least;
+}
+constexpr int kLeastSingle = 64 / 16;
+
+__device__ __forceinline__ unsigned smem_at(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp16(unsigned dst, const void* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// A float as the sum of two tf32 numbers, 22 bits of it.
+__device__ __forceinline__ void split_tf32(float v, unsigned& hi, unsigned& lo) {
+    hi = __float_as_uint(v) & 0xffffe000u;
+    lo = __float_as_uint(v - __uint_as_float(hi)) & 0xffffe000u;
+}
+__device__ __forceinline__ unsigned pack_bf16(float a, float b) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<unsigned*>(&v);
+}
+
+// talk's fragments for the mix in shared memory: [row tile][k tile][hi, lo][lane] of 16 bytes.  Row r of row tile m is head
+// r % 4 of key/value head 4 m + r / 4; k of k tile t is head k % 4 of key/value head 2 t + k / 4.  Heads that are not there: zero.
+constexpr int kTalkBytes = 2 * 4 * 2 * 32 * 16;
+__device__ __forceinline__ void stage_talk(uint4* to, const QuadArgs& a, int tid, int threads) {
+    const int per = a.H / a.G;
+    for (int e = tid; e < 2 * 4 * 32; e += threads) {
+        const int lane = e % 32, t = e / 32 % 4, m = e / 128;
+        unsigned hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = (lane >> 2) + (i & 1) * 8, k = (lane & 3) + (i >> 1) * 4;
+            const int gr = 4 * m + r / 4, hr = r % 4, gk = 2 * t + k / 4, hk = k % 4;
+            float v = 0.f;
+            if (gr < a.G && hr < per && gk < a.G && hk < per)
+                v = a.talk ? a.talk[(size_t)(gr * per + hr) * a.H + gk * per + hk] : (gr == gk && hr == hk ? 1.f : 0.f);
+            split_tf32(v, hi[i], lo[i]);
+        }
+        to[((m * 4 + t) * 2 + 0) * 32 + lane] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        to[((m * 4 + t) * 2 + 1) * 32 + lane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
+// The queries' fragments of one pair of queries: [key/value head][32 lanes of a key][lane] of 16 bytes (two steps of sixteen; the
+// second one zero beyond the last); column n is head n / 2, query n % 2 (rows row0, row0 + 1; a query beyond `rows` is zero).
+__device__ __forceinline__ void stage_queries(uint4* to, const QuadArgs& a, size_t row0, int rows, int lane) {
+    const int per = a.H / a.G, steps = a.dk / 16, pairs = (steps + 1) / 2, n = lane >> 2, h = n >> 1, x = n & 1;
+    const bool live = h < per && x < rows;
+    const __nv_bfloat16* q = a.q + (row0 + (live ? x : 0)) * a.H * a.dk + (lane & 3) * 2;
+    for (int g = 0; g < a.G; ++g)
+        for (int s = 0; s < pairs; ++s) {
+            uint4 v = make_uint4(0, 0, 0, 0);
+            if (live) {
+                const __nv_bfloat16* p = q + (g * per + h) * a.dk + s * 32;
+                v.x = *reinterpret_cast<const unsigned*>(p);
+                v.y = *reinterpret_cast<const unsigned*>(p + 8);
+                if (2 * s + 1 < steps) {
+                    v.z = *reinterpret_cast<const unsigned*>(p + 16);
+                    v.w = *reinterpret_cast<const unsigned*>(p + 24);
+                }
+            }
+            to[(g * pairs + s) * 32 + lane] = v;
+        }
+}
+
+// Rows of keys and values in shared memory are 128 bytes (256 beyond 64 lanes); the 16-byte piece c of row r lies in place
+// c ^ (r % 8), so that the eight rows an ldmatrix reads at one piece lie in eight different groups of banks.
+//
+// Scores of a tile of sixteen keys (keys at `k`, rows of `row` bytes, a key/value head every `head` bytes) for the staged queries.
+template <int KS, bool FULL>
+__device__ __forceinline__ void score_tile(float (&c)[kQuads][4], unsigned k, int row, int head, const uint4* qf, int G, int steps, int lane) {
+    const unsigned at = k + ((lane & 7) + (lane >> 3 & 1) * 8) * row, turn = ((lane >> 4) ^ (lane & 7)) * 16;
+    const int pairs = FULL ? KS / 2 : (steps + 1) / 2;
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u) c[u][0] = c[u][1] = c[u][2] = c[u][3] = 0.f;
+#pragma unroll
+    for (int s = 0; s < KS / 2; ++s) {
+        if (FULL || s < pairs) {
+            // (four heads at a time: their products are independent, so that one's latency hides behind the others')
+#pragma unroll
+            for (int u0 = 0; u0 < kQuads; u0 += 4) {
+                if (FULL || u0 < G) {
+                    unsigned f[4][4];
+                    uint4 b[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int v = FULL || u0 + u < G ? u0 + u : 0;
+                        ldsm_x4(f[u], at + v * head + (turn ^ (s * 64)));
+                        b[u] = qf[(v * pairs + s) * 32 + lane];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) mma_bf16(c[u0 + u], f[u], b[u].x, b[u].y);
+                    if (FULL || 2 * s + 1 < steps) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) ldsm_x4(f[u], at + (FULL || u0 + u < G ? u0 + u : 0) * head + (turn ^ (s * 64 + 32)));
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) mma_bf16(c[u0 + u], f[u], b[u].z, b[u].w);
+                    }
+                }
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ float exp2_fast(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The numbers a score meets on its way to a weight 1 / (1 + exp(-(s' + bias))), s' = scale s or cap tanh(scale s / cap):
+// cap tanh(x) = cap - 2 cap / (1 + exp(2 x)), so that with a cap the exponent is one multiply-add of a reciprocal.
+struct WeighConsts {
+    float in, out;                 // exp2(s in); exponent: start + out / (1 + that), or start + s out without a cap
+    bool cap;
+};
+__device__ __forceinline__ WeighConsts weigh_consts(float scale, float cap) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    WeighConsts w;
+    w.cap = cap > 0.f;
+    w.in = w.cap ? 2.0f * scale / cap * kLog2e : 0.f;
+    w.out = w.cap ? 2.0f * cap * kLog2e : -scale * kLog2e;
+    return w;
+}
+__device__ __forceinline__ float weigh_start(float cap, float bias) { return -(cap > 0.f ? cap + bias : bias) * 1.4426950408889634f; }
+
+// Scores to weights, in place; key of c[.][2 r + x]: j + 8 r (j: the lane's first), query x at position p0 + x.
+template <int X>
+__device__ __forceinline__ void weigh(float (&c)[kQuads][4], const float (&start)[kQuads], int j, int p0, bool open, const WeighConsts& k) {
+    if (k.cap) {
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int x = 0; x < X; ++x) {
+                    const float t = rcp_fast(1.0f + exp2_fast(c[u][2 * r + x] * k.in));
+                    c[u][2 * r + x] = rcp_fast(1.0f + exp2_fast(fmaf(k.out, t, start[u])));
+                }
+    } else {
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int x = 0; x < X; ++x) c[u][2 * r + x] = rcp_fast(1.0f + exp2_fast(fmaf(k.out, c[u][2 * r + x], start[u])));
+    }
+    if (!open) {
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int x = 0; x < X; ++x)
+                    if (j + 8 * r > p0 + x) c[u][2 * r + x] = 0.f;
+    }
+}
+
+// The mix of X queries' weights, packed: p[query][row tile][row half][key half] is head row (lane / 4) + 8 half at keys
+// 2 (lane % 4), + 1.  A k tile's talk serves every query and key half, and their products do not wait for one another.
+template <int X, bool FULL>
+__device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[kQuads][4], const uint4* talk, int G, int lane) {
+    float c[X][2][2][4];
+#pragma unroll
+    for (int x = 0; x < X; ++x)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) c[x][m][r][0] = c[x][m][r][1] = c[x][m][r][2] = c[x][m][r][3] = 0.f;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        if (FULL || 2 * t < G) {
+            unsigned h0[X][2], l0[X][2], h1[X][2], l1[X][2];
+#pragma unroll
+            for (int x = 0; x < X; ++x)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    split_tf32(w[2 * t][2 * r + x], h0[x][r], l0[x][r]);
+                    split_tf32(w[2 * t + 1][2 * r + x], h1[x][r], l1[x][r]);
+                }
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (FULL || 4 * m < G) {
+                    const uint4 hi = talk[((m * 4 + t) * 2 + 0) * 32 + lane], lo = talk[((m * 4 + t) * 2 + 1) * 32 + lane];
+#pragma unroll
+                    for (int x = 0; x < X; ++x)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], lo, h0[x][r], h1[x][r]);
+#pragma unroll
+                    for (int x = 0; x < X; ++x)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], hi, l0[x][r], l1[x][r]);
+#pragma unroll
+                    for (int x = 0; x < X; ++x)
+#pragma unroll
+                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], hi, h0[x][r], h1[x][r]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < X; ++x)
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) p[x][m][half][r] = pack_bf16(c[x][m][r][2 * half], c[x][m][r][2 * half + 1]);
+}
+
+// ---------------------------------------------------------------------------------------------
+// portions: a block owns eight queries of a sequence and a range of its keys; a team of T warps owns two queries.
+// T = 1 (keys and values of up to 64 lanes): four warps, tiles of 16 keys in two buffers, two blocks a multiprocessor: the warps
+// of one block go through scores, exponentials, mix and values in step, so that one block's tensor cores idle while its special
+// function units work; a second one fills them (one block of eight warps: 206 us for 1,536 tokens of 32 heads on 8, two of
+// four 164).
+// T = 2: eight warps; two warps take 16 keys each up to the mix, hand the mixed weights to each other through shared memory, and
+// take 64 value lanes each.  Tiles of 32 keys, keys and values in one buffer each, the next tile's keys on their way from the
+// end of the scores, its values from the end of the value product.
+// ---------------------------------------------------------------------------------------------
+__host__ __device__ constexpr int portion_warps(int T) { return T == 1 ? 4 : 8; }
+
+struct PortionLayout {
+    int keys, krow, vrow, stages;             // keys of a tile; bytes of a row of keys and of values
+    size_t talk, q, swap, k, v, total;
+};
+__host__ __device__ inline PortionLayout portion_layout(int G, int dk, int T) {
+    PortionLayout l;
+    l.keys = 16 * T;
+    l.krow = l.vrow = 128 * T;
+    l.stages = T == 1 ? 2 : 1;
+    l.talk = 0;
+    l.q = kTalkBytes;
+    l.swap = l.q + (size_t)(portion_warps(T) / T) * G * ((dk + 16) / 32) * 32 * 16;
+    l.k = l.swap + (T == 1 ? 0 : (size_t)portion_warps(T) * 16 * 32 * 4);
+    l.v = l.k + (size_t)l.stages * G * l.keys * l.krow;
+    l.total = l.v + (size_t)l.stages * G * l.keys * l.vrow;
+    return l;
+}
+
+template <int KS, int T, bool FULL>
+__global__ void __launch_bounds__(portion_warps(T) * 32, T == 1 ? 2 : 1) quad_portions_kernel(const QuadArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int G = FULL ? kQuads : a.G;
+    const PortionLayout L = portion_layout(G, a.dk, T);
+    constexpr int kWarps = portion_warps(T), kBQ = 2 * kWarps / T, kKeys = 16 * T;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, team = warp / T, part = warp % T;
+    const int seq = blockIdx.x / a.q_tiles, tile = a.q_tiles - 1 - blockIdx.x % a.q_tiles;     // the rows with the most keys first
+    const int first = a.cu_seqlens[seq], n_new = a.cu_seqlens[seq + 1] - first, i0 = tile * kBQ;
+    if (i0 >= n_new) return;
+    const int start = a.start_pos[seq], kv_hi = start + min(i0 + kBQ, n_new);
+    const int tiles = (kv_hi + kKeys - 1) / kKeys, per = tiles_of_range(tiles, a.ranges, 256 / kKeys);
+    const int lo = blockIdx.y * per, hi = min(tiles, lo + per);
+    if (lo >= hi) return;
+    const int* table = a.block_table + (size_t)a.slot_of_seq[seq] * a.table_stride;
+    const uint4* talk = reinterpret_cast<const uint4*>(smem + L.talk);
+    const int steps = FULL ? KS : a.dk / 16, kp = 2 * steps, vp = FULL ? 8 * T : a.dv / 8;
+    uint4* qf = reinterpret_cast<uint4*>(smem + L.q) + (size_t)team * G * ((steps + 1) / 2) * 32;
+    const unsigned ks = smem_at(smem + L.k), vs = smem_at(smem + L.v);
+    const int khead = kKeys * L.krow, vhead = kKeys * L.vrow;
+    const size_t page_elems = (size_t)G * a.page * (a.dk + a.dv);
+    const int iq = i0 + 2 * team, p0 = start + iq;             // the team's queries: rows iq, iq + 1, positions p0, p0 + 1
+
+    auto load_keys = [&](int t, int stage, int pg) {
+        if (t < hi) {
+            const int j0 = t * kKeys, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)(j0 % a.page) * a.dk;
+            const unsigned to = ks + stage * G * khead;
+            for (int e = tid; e < G * kKeys * kp; e += kWarps * 32) {
+                const int c = e % kp, j = e / kp % kKeys, g = e / (kp * kKeys);
+                cp16(to + g * khead + j * L.krow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dk + c * 8, j < live);
+            }
+        }
+    };
+    auto load_values = [&](int t, int stage, int pg) {
+        if (t < hi) {
+            const int j0 = t * kKeys, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)G * a.page * a.dk + (size_t)(j0 % a.page) * a.dv;
+            const unsigned to = vs + stage * G * vhead;
+            for (int e = tid; e < G * kKeys * vp; e += kWarps * 32) {
+                const int c = e % vp, j = e / vp % kKeys, g = e / (vp * kKeys);
+                cp16(to + g * vhead + j * L.vrow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dv + c * 8, j < live);
+            }
+        }
+    };
+    auto page_of = [&](int t) { return t < hi ? table[t * kKeys / a.page] : 0; };
+
+    int ahead = 0;                                             // the page of the next tile to be asked for
+    if (T == 1) {
+        const int pg = page_of(lo);
+        load_keys(lo, 0, pg);
+        load_values(lo, 0, pg);
+        cp_commit();
+        ahead = page_of(lo + 1);
+    } else {
+        const int pg = page_of(lo);
+        load_keys(lo, 0, pg);
+        cp_commit();
+        load_values(lo, 0, pg);
+        cp_commit();
+        ahead = page_of(lo + 1);
+    }
+    stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, kWarps * 32);
+    if (part == 0) stage_queries(qf, a, (size_t)first + min(iq, n_new - 1), max(0, min(2, n_new - iq)), lane);
+    const WeighConsts consts = weigh_consts(a.scale, a.softcap);
+    float begin[kQuads];
+    {
+        const int per_kv = a.H / a.G;
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u)
+            begin[u] = weigh_start(a.softcap, a.head_bias && u < G && (lane & 3) < per_kv ? a.head_bias[u * per_kv + (lane & 3)] : 0.f);
+    }
+    float o[kQuads][4][4];
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) o[u][d][0] = o[u][d][1] = o[u][d][2] = o[u][d][3] = 0.f;
+
+    // one tile of sixteen keys of values (64 lanes from the address on) times the packed weights of both queries
+    auto values = [&](unsigned v, const unsigned (&b)[2][2][2][2]) {
+        const unsigned at = v + ((lane & 7) + (lane >> 4) * 8) * L.vrow, turn = ((lane >> 3 & 1) ^ (lane & 7)) * 16;
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u) {
+            if (FULL || u < G) {
+                const unsigned b0 = b[u & 1][u >> 2][u >> 1 & 1][0], b1 = b[u & 1][u >> 2][u >> 1 & 1][1];
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    unsigned f[4];
+                    ldsm_x4_trans(f, at + u * vhead + (turn ^ (d * 32)));
+                    mma_bf16(o[u][d], f, b0, b1);
+                }
+            }
+        }
+    };
+
+    for (int t = lo; t < hi; ++t) {
+        const int stage = T == 1 ? (t - lo) & 1 : 0;
+        cp_wait<T == 1 ? 0 : 1>();
+        __syncthreads();                                       // T 1: this tile is there, the one before done with; T 2: its keys
+        if (T == 1) {
+            load_keys(t + 1, stage ^ 1, ahead);
+            load_values(t + 1, stage ^ 1, ahead);
+            cp_commit();
+            ahead = page_of(t + 2);
+        }
+        const int j0 = t * kKeys + part * 16;
+        const bool some = j0 <= p0 + 1;                        // the warp's queries see some of its keys
+        float c[kQuads][4];
+        if (some) score_tile<KS, FULL>(c, ks + stage * G * khead + part * 16 * L.krow, L.krow, khead, qf, G, steps, lane);
+        if (T > 1) {
+            __syncthreads();                                   // the keys are done with
+            load_keys(t + 1, 0, ahead);
+            cp_commit();
+        }
+        // b[parity]: the weights of the even and the odd key/value heads of every pair, both queries in one operand
+        unsigned b[2][2][2][2];
+        if (some) {
+            weigh<2>(c, begin, j0 + (lane >> 2), p0, j0 + 15 <= p0, consts);
+            unsigned p[2][2][2][2];
+            mix<2, FULL>(p, c, talk, G, lane);
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const unsigned other = __shfl_xor_sync(0xffffffffu, p[1][m][half][r], 16);
+                        b[0][m][half][r] = lane < 16 ? p[0][m][half][r] : other;
+                        b[1][m][half][r] = lane < 16 ? other : p[0][m][half][r];
+                    }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = 0u;
+        }
+        if (T == 1) {
+            if (some) values(vs + stage * G * vhead, b);
+        } else {
+            unsigned* mine = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)warp * 16 * 32 + lane;
+            const unsigned* theirs = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)(warp ^ 1) * 16 * 32 + lane;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) mine[e * 32] = b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1];
+            cp_wait<1>();                                      // the values; the next keys may be on their way
+            __syncthreads();
+            const unsigned v = vs + part * 128;                // (a piece's place keeps its upper bit: 64 lanes are 8 pieces)
+            const bool own = FULL || part * 64 < a.dv;         // the warp has value lanes
+            if (own) values(v + part * 16 * L.vrow, b);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = theirs[e * 32];
+            if (own) values(v + (part ^ 1) * 16 * L.vrow, b);
+            __syncthreads();                                   // the values and the weights are done with
+            load_values(t + 1, 0, ahead);
+            cp_commit();
+            ahead = page_of(t + 2);
+        }
+    }
+    // column n of key/value head u: head n % 4; an even u's columns 0 .. 3 are query 0's, an odd one's query 1's
+    const int per_kv = a.H / a.G, HD = a.H * a.dv;
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = 2 * (lane & 3) + e, h = n & 3, x = (n >> 2) ^ (u & 1);
+            if (u >= G || h >= per_kv || iq + x >= n_new) continue;
+            const size_t at = (size_t)(first + iq + x) * HD + (u * per_kv + h) * a.dv;
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int lanev = part * 64 + d * 16 + (lane >> 2) + 8 * r;
+                    if (lanev < a.dv) {
+                        if (a.ranges > 1) a.partial[(size_t)blockIdx.y * a.n_tokens * HD + at + lanev] = o[u][d][2 * r + e];
+                        else a.out[at + lanev] = __float2bfloat16_rn(o[u][d][2 * r + e]);
+                    }
+                }
+        }
+}
+
+// ---------------------------------------------------------------------------------------------
+// single tokens: a block owns (sequence, range of keys); every warp walks tiles of sixteen keys of its own, with one buffer of
+// keys and one of values that are refilled as soon as their product is done, and no barrier between warps before the end.
+// The key/value heads 2 p and 2 p + 1 share an accumulator (columns 0 .. 3 and 4 .. 7), the second query's place being empty.
+// ---------------------------------------------------------------------------------------------
+struct SingleLayout {
+    int krow, vrow, warps;
+    size_t talk, q, bufs, warp_bytes, total;
+};
+__host__ __device__ inline SingleLayout single_layout(int G, int dk, int dv) {
+    SingleLayout l;
+    l.krow = dk > 64 ? 256 : 128;
+    l.vrow = dv > 64 ? 256 : 128;
+    l.talk = 0;
+    l.q = kTalkBytes;
+    l.bufs = l.q + (size_t)G * ((dk + 16) / 32) * 32 * 16;
+    l.warp_bytes = (size_t)G * 16 * (l.krow + l.vrow);
+    const size_t room = (227 * 1024 - l.bufs) / l.warp_bytes;
+    l.warps = room > 6 ? 6 : (int)room;
+    const size_t sums = 16 * 1024;             // a warp's sums pass through the buffers at the end
+    l.total = l.bufs + (l.warps * l.warp_bytes > sums ? l.warps * l.warp_bytes : sums);
+    return l;
+}
+
+template <int KS, int DT, bool FULL>
+__global__ void __launch_bounds__(192, 1) quad_singles_kernel(const QuadArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int G = FULL ? kQuads : a.G;
+    const SingleLayout L = single_layout(G, a.dk, a.dv);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = L.warps * 32;
+    const int seq = blockIdx.x, first = a.cu_seqlens[seq];
+    if (a.cu_seqlens[seq + 1] - first != 1) return;            // this kernel serves sequences that bring one token
+    const int pos = a.start_pos[seq], kv_hi = pos + 1;
+    const int tiles = (kv_hi + 15) / 16, per = tiles_of_range(tiles, a.ranges, kLeastSingle);
+    const int lo = blockIdx.y * per, hi = min(tiles, lo + per);
+    if (lo >= hi) return;
+    const int* table = a.block_table + (size_t)a.slot_of_seq[seq] * a.table_stride;
+    const uint4* talk = reinterpret_cast<const uint4*>(smem + L.talk);
+    uint4* qf = reinterpret_cast<uint4*>(smem + L.q);
+    const int steps = FULL ? KS : a.dk / 16, kp = 2 * steps, vp = FULL ? 2 * DT : a.dv / 8;
+    const unsigned ks = smem_at(smem + L.bufs + warp * L.warp_bytes), vs = ks + G * 16 * L.krow;
+    const int khead = 16 * L.krow, vhead = 16 * L.vrow;
+    const size_t page_elems = (size_t)G * a.page * (a.dk + a.dv);
+    auto load_keys = [&](int t, int pg) {
+        if (t < hi) {
+            const int j0 = t * 16, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)(j0 % a.page) * a.dk;
+#pragma unroll 8
+            for (int e = lane; e < G * 16 * kp; e += 32) {
+                const int c = e % kp, j = e / kp % 16, g = e / (kp * 16);
+                cp16(ks + g * khead + j * L.krow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dk + c * 8, j < live);
+            }
+        }
+        cp_commit();
+    };
+    auto load_values = [&](int t, int pg) {
+        if (t < hi) {
+            const int j0 = t * 16, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)G * a.page * a.dk + (size_t)(j0 % a.page) * a.dv;
+#pragma unroll 8
+            for (int e = lane; e < G * 16 * vp; e += 32) {
+                const int c = e % vp, j = e / vp % 16, g = e / (vp * 16);
+                cp16(vs + g * vhead + j * L.vrow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dv + c * 8, j < live);
+            }
+        }
+        cp_commit();
+    };
+    auto page_of = [&](int t) { return t < hi ? table[t * 16 / a.page] : 0; };
+    {
+        const int pg = page_of(lo + warp);
+        load_keys(lo + warp, pg);
+        load_values(lo + warp, pg);
+    }
+    int ahead = page_of(lo + warp + L.warps);
+    stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, threads);
+    if (warp == 0) stage_queries(qf, a, (size_t)first, 1, lane);
+    const int per_kv = a.H / a.G;
+    const WeighConsts consts = weigh_consts(a.scale, a.softcap);
+    float begin[kQuads];
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+        begin[u] = weigh_start(a.softcap, a.head_bias && u < G && (lane & 3) < per_kv ? a.head_bias[u * per_kv + (lane & 3)] : 0.f);
+    float o[kQuads / 2][DT][4];
+#pragma unroll
+    for (int p = 0; p < kQuads / 2; ++p)
+#pragma unroll
+        for (int d = 0; d < DT; ++d) o[p][d][0] = o[p][d][1] = o[p][d][2] = o[p][d][3] = 0.f;
+    __syncthreads();
+    for (int t = lo + warp; t < hi; t += L.warps) {
+        const int pg = ahead;
+        ahead = page_of(t + 2 * L.warps);
+        cp_wait<1>();
+        __syncwarp();
+        float c[kQuads][4];
+        score_tile<KS, FULL>(c, ks, L.krow, khead, qf, G, steps, lane);
+        __syncwarp();
+        load_keys(t + L.warps, pg);
+        weigh<1>(c, begin, t * 16 + (lane >> 2), pos, t * 16 + 15 <= pos, consts);
+        unsigned p[1][2][2][2];
+        mix<1, FULL>(p, c, talk, G, lane);
+        cp_wait<1>();
+        __syncwarp();
+        const unsigned at = vs + ((lane & 7) + (lane >> 4) * 8) * L.vrow, turn = ((lane >> 3 & 1) ^ (lane & 7)) * 16;
+#pragma unroll
+        for (int u = 0; u < kQuads; ++u) {
+            if (FULL || u < G) {
+                const bool mine = (lane >= 16) == (u & 1);
+                const unsigned b0 = mine ? p[0][u >> 2][u >> 1 & 1][0] : 0u, b1 = mine ? p[0][u >> 2][u >> 1 & 1][1] : 0u;
+#pragma unroll
+                for (int d = 0; d < DT; ++d) {
+                    if (FULL || d * 16 < a.dv) {
+                        unsigned f[4];
+                        ldsm_x4_trans(f, at + u * vhead + (turn ^ (d * 32)));
+                        mma_bf16(o[u >> 1][d], f, b0, b1);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        load_values(t + L.warps, pg);
+    }
+    cp_wait<0>();
+    __syncthreads();
+    // the warps' sums, in the order of the warps: through the buffers, which are done with
+    float* sums = reinterpret_cast<float*>(smem + L.bufs);
+    constexpr int kFloats = kQuads / 2 * DT * 4;               // a lane's
+    for (int w = 1; w < L.warps; ++w) {
+        if (warp == w) {
+#pragma unroll
+            for (int e = 0; e < kFloats; ++e) sums[e * 32 + lane] = o[e / 4 / DT][e / 4 % DT][e & 3];
+        }
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int e = 0; e < kFloats; ++e) o[e / 4 / DT][e / 4 % DT][e & 3] += sums[e * 32 + lane];
+        }
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    const int HD = a.H * a.dv;
+#pragma unroll
+    for (int p = 0; p < kQuads / 2; ++p)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int n = 2 * (lane & 3) + e, h = n & 3, g = 2 * p + (n >> 2);
+            if (g >= G || h >= per_kv) continue;
+            const size_t at = (size_t)first * HD + (g * per_kv + h) * a.dv;
+#pragma unroll
+            for (int d = 0; d < DT; ++d)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int lanev = d * 16 + (lane >> 2) + 8 * r;
+                    if (lanev < a.dv) {
+                        if (a.ranges > 1) a.partial[(size_t)blockIdx.y * a.n_tokens * HD + at + lanev] = o[p][d][2 * r + e];
+                        else a.out[at + lanev] = __float2bfloat16_rn(o[p][d][2 * r + e]);
+                    }
+                }
+        }
+}
+
+// out[n, :] = the ranges' partial outputs added in order: as many as the row's block of queries has; rows of no sequence get zeros
+__global__ void add_quad_ranges_kernel(const QuadArgs a, int bq, int keys, int least) {
+    const int n = blockIdx.x, HD = a.H * a.dv, seq = a.token_seq[n];
+    int used = 0;
+    if (seq >= 0) {
+        const int first = a.cu_seqlens[seq], n_new = a.cu_seqlens[seq + 1] - first, i0 = (n - first) / bq * bq;
+        const int tiles = (a.start_pos[seq] + min(i0 + bq, n_new) + keys - 1) / keys, per = tiles_of_range(tiles, a.ranges, least);
+        used = (tiles + per - 1) / per;
+    }
+    for (int e = threadIdx.x * 4; e < HD; e += blockDim.x * 4) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < used; ++r) {
+            const float4 v = *reinterpret_cast<const float4*>(a.partial + ((size_t)r * a.n_tokens + n) * HD + e);
+            s.x += v.x;
+            s.y += v.y;
+            s.z += v.z;
+            s.w += v.w;
+        }
+        *reinterpret_cast<uint2*>(a.out + (size_t)n * HD + e) = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+    }
+}
+
+// Whether these kernels take a shape (bfloat16 alone): at most eight key/value heads with at most four query heads each.
+BLM_API int blm_attention_quads_takes(int H, int G, int dk, int dv, int page) {
+    if (H < 1 || G < 1 || H % G || G > kQuads || H / G > 4) return 0;
+    return dk % 16 == 0 && dk >= 16 && dk <= 128 && dv % 8 == 0 && dv >= 8 && dv <= 128 && page % 32 == 0;
+}
+
+template <typename K>
+static int allow_smem(K kernel, size_t smem) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return e == cudaSuccess ? BLM_OK : blm_fail(BLM_CUDA_ERROR, "attention_quads: %s", cudaGetErrorString(e));
+}
+
+BLM_API int blm_attention_quads(const void* q, const void* pool, const int* block_table, int table_stride, const int* cu_seqlens,
+                                const int* slot_of_seq, const int* start_pos, const int* token_seq, const float* talk,
+                                const float* head_bias, void* out, float* partial, int n_tokens, int n_seqs, int max_q_len, int H, int G,
+                                int dk, int dv, int page, int ranges, float scale, float softcap, cudaStream_t stream) {
+    if (n_tokens == 0 || n_seqs == 0) return BLM_OK;
+    BLM_REQUIRE(blm_attention_quads_takes(H, G, dk, dv, page) && max_q_len > 0, "attention_quads: %d heads on %d, %d + %d lanes", H, G, dk, dv);
+    BLM_REQUIRE(ranges >= 1 && ranges <= 65535 && (ranges == 1 || partial != nullptr), "attention_quads: several key ranges need a workspace");
+    BLM_REQUIRE((((size_t)q | (size_t)pool | (size_t)out | (size_t)partial) & 15) == 0, "attention_quads: tensors start at multiples of 16 bytes");
+    QuadArgs a = {(const __nv_bfloat16*)q, (const __nv_bfloat16*)pool, block_table, table_stride, cu_seqlens, slot_of_seq, start_pos, token_seq,
+                  talk, head_bias, (__nv_bfloat16*)out, partial, n_tokens, n_seqs, 1, H, G, dk, dv, page, ranges, scale, softcap};
+    // the instances without tests of the sizes: eight key/value heads, 64 or 128 lanes
+    const bool full = G == kQuads && (dk == 64 || dk == 128) && (dv == 64 || dv == 128);
+    int bq = 1, keys = 16;
+    if (max_q_len == 1) {
+        const SingleLayout l = single_layout(G, dk, dv);
+        auto k = !full ? quad_singles_kernel<8, 8, false>
+                 : dk == 64 ? (dv == 64 ? quad_singles_kernel<4, 4, true> : quad_singles_kernel<4, 8, true>)
+                            : (dv == 64 ? quad_singles_kernel<8, 4, true> : quad_singles_kernel<8, 8, true>);
+        BLM_REQUIRE(l.warps >= 1, "attention_quads: shared memory");
+        if (int rc = allow_smem(k, l.total)) return rc;
+        k<<<dim3(n_seqs, ranges), l.warps * 32, l.total, stream>>>(a);
+    } else {
+        const int T = dv > 64 || dk > 64 ? 2 : 1;
+        bq = 2 * portion_warps(T) / T;
+        keys = 16 * T;
+        a.q_tiles = (max_q_len + bq - 1) / bq;
+        BLM_REQUIRE((long long)n_seqs * a.q_tiles <= 0x7fffffffLL, "attention_quads: grid too large");
+        const PortionLayout l = portion_layout(G, dk, T);
+        auto k = T == 1 ? (full ? quad_portions_kernel<4, 1, true> : quad_portions_kernel<4, 1, false>)
+                 : !full || dv == 64 ? quad_portions_kernel<8, 2, false>
+                                     : (dk == 64 ? quad_portions_kernel<4, 2, true> : quad_portions_kernel<8, 2, true>);
+        BLM_REQUIRE(l.total <= 227 * 1024, "attention_quads: shared memory");
+        if (int rc = allow_smem(k, l.total)) return rc;
+        k<<<dim3(n_seqs * a.q_tiles, ranges), portion_warps(T) * 32, l.total, stream>>>(a);
+    }
+    if (int rc = blm_check_launch("attention_quads")) return rc;
+    if (ranges == 1) return BLM_OK;
+    add_quad_ranges_kernel<<<n_tokens, 256, 0, stream>>>(a, bq, keys, max_q_len == 1 ? kLeastSingle : 256 / keys);
+    return blm_check_launch("attention_quads (ranges)");
+}

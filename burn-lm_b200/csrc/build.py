@@ -39,6 +39,7 @@ MODULES = {
     "scan_chunks": ["scan_chunks.cu"],
     "retention": ["retention.cu"],
     "attention_sigmoid": ["attention_sigmoid.cu"],
+    "attention_quads": ["attention_quads.cu"],
     "attention_latent": ["attention_latent.cu"],
     "gemm": ["gemm_f32.cu"],
     "gemv": ["gemv.cu"],

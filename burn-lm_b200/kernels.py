@@ -169,6 +169,11 @@ _protos = {
                                   c_float, c_float, c_int, c_void_p],
         "blm_sigmoid_attention_takes": [c_int, c_int, c_int, c_int, c_int, c_int],
     },
+    "attention_quads": {
+        "blm_attention_quads_takes": [c_int, c_int, c_int, c_int, c_int],
+        "blm_attention_quads": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
+    },
     "attention_latent": {
         "blm_latent_prepare": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p,
                                c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -1645,14 +1650,38 @@ def sigmoid_attention_takes(dtype, n_heads, n_kv, key_dim, value_dim) -> bool:
     return bool(_lib("attention_sigmoid").blm_sigmoid_attention_takes(_code(dtype), n_heads, n_kv, key_dim, value_dim, PAGE))
 
 
+def sigmoid_attention_in_registers(dtype, n_heads, n_kv, key_dim, value_dim) -> bool:
+    """Whether a shape runs the kernels that keep weights and mix in registers (attention_quads.cu)."""
+    return dtype == torch.bfloat16 and bool(_lib("attention_quads").blm_attention_quads_takes(n_heads, n_kv, key_dim, value_dim, PAGE))
+
+
+def sigmoid_attention_ranges(step, n_heads, n_kv, key_dim, value_dim, dtype, device) -> int:
+    """Over how many blocks a query's keys are cut: nothing is normalised over the keys, so partial outputs just add.  Few query
+    rows with long pasts would leave most multiprocessors idle otherwise."""
+    sms = sm_count(device)
+    if sigmoid_attention_in_registers(dtype, n_heads, n_kv, key_dim, value_dim):
+        # single tokens: one round of blocks, which fill a multiprocessor each (64 sequences of 1,088 keys, the whole mixer: 1 / 2 /
+        # 3 / 4 ranges 78 / 60 / 78 / 72 us).  Portions: blocks are of unequal length, so enough of them that the last round
+        # weighs little (1,536 tokens: 1 / 2 / 4 / 5 / 6 ranges 346 / 247 / 241 / 234 / 247 us)
+        if step.max_q_len == 1:
+            return max(1, min(sms // step.n_seqs, step.max_kv_len // PAGE, 64))
+        tiles = step.n_seqs * -(-step.max_q_len // 8)
+        return max(1, min(-(-6 * sms // tiles), step.max_kv_len // 256, 8))
+    tiles = step.n_seqs * ((step.max_q_len + 15) // 16)
+    want = (4 if step.max_q_len == 1 else 2) * sms                  # single rows: small blocks, four an SM
+    shortest = PAGE if step.max_q_len == 1 else 256                 # a single row's range may be one page
+    return max(1, min((want + tiles - 1) // tiles, step.max_kv_len // shortest, 64))
+
+
 def sigmoid_attention(q, pool, block_table, step, out, n_heads, n_kv, key_dim, value_dim, scale, softcap=0.0, talk=None,
                       head_bias=None, ranges=1, partial=None, scalar_only=False):
     """Causal attention whose weights are sigmoid(cap(scale q.k) + head_bias) without a normalisation over the keys, mixed
     across heads by talk [heads, heads] (row h: what head h takes of every head's weights) before they meet the values.
     q [N, heads * key_dim] and out [N, heads * value_dim] in the cache's dtype (out must hold zeros in rows of no
     sequence); `ranges` > 1 cuts every query's keys over that many blocks whose partial outputs (`partial`, float32
-    with room for ranges * N * heads * value_dim) are added in order.  Prompts in bfloat16 run the tensor-core kernel where
-    it takes the shape (key lanes in multiples of 16, value lanes of 8); `scalar_only` keeps them off it."""
+    with room for ranges * N * heads * value_dim) are added in order.  bfloat16 runs the tensor-core
+    kernels where they take the shape (key lanes in multiples of 16, value lanes of 8; up to eight key/value heads of up to
+    four query heads each: attention_quads.cu, others attention_sigmoid.cu); `scalar_only` keeps it off them."""
     _need_cuda(q, pool, block_table, out, talk, head_bias, partial)
     _f32(talk, head_bias, partial)
     n = step.n_tokens
@@ -1664,6 +1693,13 @@ def sigmoid_attention(q, pool, block_table, step, out, n_heads, n_kv, key_dim, v
         raise KernelError("sigmoid_attention: head_bias [heads]")
     if ranges > 1 and (partial is None or partial.numel() < ranges * n * n_heads * value_dim):
         raise KernelError("sigmoid_attention: the workspace is too small for the key ranges")
+    if not scalar_only and sigmoid_attention_in_registers(pool.dtype, n_heads, n_kv, key_dim, value_dim) and all(
+            t is None or t.data_ptr() % 16 == 0 for t in (q, pool, out, partial)):
+        _call("attention_quads", "blm_attention_quads", _ptr(q), _ptr(pool), _ptr(block_table), block_table.shape[1], _ptr(step.cu_seqlens),
+              _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias), _ptr(out),
+              _ptr(partial if ranges > 1 else None), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE, int(ranges),
+              c_float(scale), c_float(softcap), _stream(), kernels=2 if ranges > 1 else 1)
+        return
     _call("attention_sigmoid", "blm_sigmoid_attention", _ptr(q), _ptr(pool), _code(pool.dtype), _ptr(block_table), block_table.shape[1],
           _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias),
           _ptr(out), _ptr(partial), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE, int(ranges),

@@ -21,10 +21,6 @@ from .base import CacheNeed, Part
 from .linear import Linear
 from .mamba2 import f32
 
-BLOCKS_PER_SM = 2     # blocks a step should offer every multiprocessor before keys are cut into ranges
-RANGE_KEYS = 256      # a range of keys is not made shorter than this
-
-
 @dataclass(frozen=True)
 class SigmoidAttentionSpec:
     hidden_size: int
@@ -46,7 +42,7 @@ class SigmoidAttention(Part):
     family = "mixer"
     graph_safe = True
     roles = ("q", "k", "v", "o", "q_bias", "k_bias", "v_bias", "talk", "head_bias")
-    kernel_modules = ("attention_sigmoid",)
+    kernel_modules = ("attention_quads", "attention_sigmoid")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)
@@ -91,14 +87,6 @@ class SigmoidAttention(Part):
         s = self.spec
         return CacheNeed("kv", n_kv_heads=s.n_kv_heads, head_dim=s.head_dim, window=None, value_dim=s.value_dim)
 
-    def _ranges(self, step) -> int:
-        """Over how many blocks a query's keys are cut: nothing is normalised over the keys, so partial outputs just add.
-        Few query rows with long pasts (decoding) would leave most multiprocessors idle otherwise."""
-        tiles = step.n_seqs * ((step.max_q_len + 15) // 16)
-        want = (4 if step.max_q_len == 1 else BLOCKS_PER_SM) * K.sm_count(self.runtime.device)      # single rows: small blocks, four an SM
-        shortest = K.PAGE if step.max_q_len == 1 else RANGE_KEYS                  # a single row's range may be one page
-        return max(1, min((want + tiles - 1) // tiles, step.max_kv_len // shortest, 64))
-
     def forward(self, x, step, cache):
         s, rt = self.spec, self.runtime
         if not cache.writes:
@@ -109,7 +97,7 @@ class SigmoidAttention(Part):
         K.bias_rope_append(proj, self.bias, self.freq, s.rotary_dim, q, cache.pool, cache.block_table, step, s.n_heads,
                            s.n_kv_heads, s.head_dim, s.value_dim)
         out = torch.zeros((n, s.n_heads * s.value_dim), dtype=rt.dtype, device=proj.device)   # rows of no sequence stay zero
-        ranges = self._ranges(step)
+        ranges = K.sigmoid_attention_ranges(step, s.n_heads, s.n_kv_heads, s.head_dim, s.value_dim, rt.dtype, rt.device)
         partial = None
         if ranges > 1:
             partial = step.workspace.scratch("sigmoid_attention", ranges * n * s.n_heads * s.value_dim)
