@@ -68,6 +68,86 @@ __global__ void bias_rope_append_kernel(const float* __restrict__ proj, long lon
     else base[(size_t)G * page * dk + ((size_t)head * page + at) * dv + lane] = from_f32<T>(val);
 }
 
+// The same in pieces of four lanes, a block a token: the token's sines and cosines are worked out once (in fp64) for all heads
+// instead of once a lane of every head, and a piece turns together with its partner.  1,536 tokens of 40 heads of 64 + 8 of
+// 64: 34.8 -> 8.5 us.
+constexpr int kRopeThreads = 256;
+template <typename T>
+__device__ __forceinline__ void store4(T* to, const float (&v)[4]) {
+    if (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+        __nv_bfloat162 p[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+        *reinterpret_cast<uint2*>(to) = *reinterpret_cast<uint2*>(p);
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(kRopeThreads)
+    bias_rope_append_vec_kernel(const float* __restrict__ proj, long long stride, const float* __restrict__ bias, const double* __restrict__ freq,
+                                int rot, T* __restrict__ q_out, T* __restrict__ pool, const int* __restrict__ token_seq,
+                                const int* __restrict__ token_pos, const int* __restrict__ slot_of_seq, const int* __restrict__ block_table,
+                                int table_stride, int H, int G, int dk, int dv, int page) {
+    extern __shared__ __align__(16) float turns[];           // [half] cosines, [half] sines
+    const int n = blockIdx.x, half = rot / 2, pos = token_pos[n], seq = token_seq[n];
+    for (int i = threadIdx.x; i < half; i += kRopeThreads) {
+        double sd, cd;
+        sincos((double)pos * freq[i], &sd, &cd);
+        turns[i] = (float)cd;
+        turns[half + i] = (float)sd;
+    }
+    T* base = nullptr;                         // a row of no sequence: nothing of it reaches the cache
+    int at = 0;
+    if (seq >= 0) {
+        base = pool + (size_t)block_table[(size_t)slot_of_seq[seq] * table_stride + pos / page] * G * page * (dk + dv);
+        at = pos % page;
+    }
+    __syncthreads();
+    const float* row = proj + (size_t)n * stride;
+    auto read4 = [&](int e, float (&v)[4]) {
+        const float4 a = *reinterpret_cast<const float4*>(row + e);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+        if (bias) {
+            const float4 b = *reinterpret_cast<const float4*>(bias + e);
+            v[0] += b.x, v[1] += b.y, v[2] += b.z, v[3] += b.w;
+        }
+    };
+    // a head of q or k: half / 4 pieces that turn with their partners, then (dk - rot) / 4 that stay; then the values
+    const int turning = half / 4, per = turning + (dk - rot) / 4, qk_items = (H + G) * per, items = qk_items + G * (dv / 4);
+    for (int e = threadIdx.x; e < items; e += kRopeThreads) {
+        if (e >= qk_items) {
+            if (base == nullptr) continue;
+            const int head = (e - qk_items) / (dv / 4), d = (e - qk_items) % (dv / 4) * 4;
+            float v[4];
+            read4((H + G) * dk + head * dv + d, v);
+            store4(base + (size_t)G * page * dk + ((size_t)head * page + at) * dv + d, v);
+            continue;
+        }
+        const int head = e / per, p = e % per;
+        T* to = head < H ? q_out + ((size_t)n * H + head) * dk : (base ? base + ((size_t)(head - H) * page + at) * dk : nullptr);
+        if (to == nullptr) continue;
+        if (p < turning) {
+            const int d = p * 4;
+            float a[4], b[4], x[4], y[4];
+            read4(head * dk + d, a);
+            read4(head * dk + half + d, b);
+            const float4 c4 = *reinterpret_cast<const float4*>(turns + d), s4 = *reinterpret_cast<const float4*>(turns + half + d);
+            const float c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                x[i] = a[i] * c[i] - b[i] * s[i];
+                y[i] = b[i] * c[i] + a[i] * s[i];
+            }
+            store4(to + d, x);
+            store4(to + half + d, y);
+        } else {
+            const int d = rot + (p - turning) * 4;
+            float v[4];
+            read4(head * dk + d, v);
+            store4(to + d, v);
+        }
+    }
+}
+
 BLM_API int blm_bias_rope_append(const float* proj, long long stride, const float* bias, const double* freq, int rot, void* q_out,
                                  void* pool, int dtype, const int* token_seq, const int* token_pos, const int* slot_of_seq,
                                  const int* block_table, int table_stride, int n, int H, int G, int dk, int dv, int page,
@@ -77,6 +157,20 @@ BLM_API int blm_bias_rope_append(const float* proj, long long stride, const floa
     BLM_REQUIRE(rot >= 0 && rot <= dk && rot % 2 == 0 && (rot == 0 || freq != nullptr), "bias_rope_append: %d rotated lanes of %d", rot, dk);
     BLM_REQUIRE(n <= 65535, "bias_rope_append: a step of %d rows; this kernel takes 65,535", n);
     const int width = (H + G) * dk + G * dv;
+    // pieces of four lanes everywhere, none of which may straddle a head's end or the middle of its turning lanes
+    if (rot % 8 == 0 && dk % 4 == 0 && dv % 4 == 0 && stride % 4 == 0 && rot <= 4096 &&
+        (((size_t)proj | (size_t)bias | (size_t)q_out | (size_t)pool) & 15) == 0 && (dtype == BLM_F32 || dtype == BLM_BF16)) {
+        if (dtype == BLM_F32)
+            bias_rope_append_vec_kernel<float><<<n, kRopeThreads, rot * 4, stream>>>(proj, stride, bias, freq, rot, (float*)q_out, (float*)pool,
+                                                                                    token_seq, token_pos, slot_of_seq, block_table,
+                                                                                    table_stride, H, G, dk, dv, page);
+        else
+            bias_rope_append_vec_kernel<__nv_bfloat16><<<n, kRopeThreads, rot * 4, stream>>>(proj, stride, bias, freq, rot, (__nv_bfloat16*)q_out,
+                                                                                            (__nv_bfloat16*)pool, token_seq, token_pos,
+                                                                                            slot_of_seq, block_table, table_stride, H, G,
+                                                                                            dk, dv, page);
+        return blm_check_launch("bias_rope_append");
+    }
     dim3 grid((width + 255) / 256, n);
     if (dtype == BLM_F32)
         bias_rope_append_kernel<float><<<grid, 256, 0, stream>>>(proj, stride, bias, freq, rot, (float*)q_out, (float*)pool, token_seq,
