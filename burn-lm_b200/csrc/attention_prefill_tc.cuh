@@ -31,10 +31,15 @@
 // The kernel is a template of the keys' and the values' lanes (HDK, HDV: multiples of 64) and of GEN.  GEN false: keys and
 // values of one size, the dense decoder's use of it.  GEN true, the windowed family's: keys and values of any multiple of 8
 // lanes up to HDK and HDV (the TMA fills the lanes beyond with zeros: three-dimensional maps, lanes by rows by pages), a
-// window or chunks, two maps a head (a query head for each; their sums leave as shares for the kernel that forms the
+// window (beside it, kept first positions) or chunks, a sink in the denominator, two maps a head (a query head for each; their sums leave as shares for the kernel that forms the
 // difference), a gate per head or per lane, results scaled and written as columns of wider rows, values that are the keys (the
 // value map is then the keys' own: a page's tile of keys by lanes is the K-major operand of the scores and the MN-major one of
 // the second product).
+//
+// KEEP (with GEN): kept first positions and a sink.  The sink's score is the reference to begin with, and a reference that trails the
+// largest score means that the largest probability is not 1 but rounded as the others are; in the first two steps the
+// reference follows the largest score itself.  Error against 64 bits of a 2,048-token layer and time: never following 3.97e-3 and
+// 54 us, two steps 3.86e-3 and 59, five 3.85e-3 and 66, always 3.84e-3 (as the mma.sync kernel's) and 94.
 //
 // BIAS (with GEN): slope_h times the distance is taken off a score.  The pages are then walked from the diagonal back: the row's
 // largest score is mostly found in the first pages, where with a bias by distance it would otherwise move in every page, and with
@@ -66,6 +71,10 @@ struct AttnPrefillTcArgs {
     float out_scale;
     float* partial;              // null, or where a row's share goes: [N][n_heads][max, sum, dv lanes]
     const float* slope;          // BIAS: [n_heads]
+    int keep_first;              // > 0 (not with BIAS): the first positions of the sequence are seen beside the window
+    int sink;                    // the denominator has one more entry, of the score sink_logit[head] (null: 0), without a value
+    const float* sink_logit;
+    int n_tokens;                // rows behind the last sequence (padding up to a captured step's size) get zeros
     int shared;                  // the values are the keys, and a page holds the keys alone
 };
 
@@ -246,12 +255,15 @@ __device__ __forceinline__ void tmem_st32_bits(unsigned taddr, const unsigned (&
 constexpr float kLazy = 8.0f;     // the reference maximum of a row moves only when a block exceeds it by more than 2^kLazy
 }  // namespace attn_tc
 
-template <int HDK, int HDV, bool GEN, bool BIAS>
+enum { kPlain = 0, kBias = 1, kKeep = 2 };
+
+template <int HDK, int HDV, bool GEN, int OPT>
 __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
     attn_prefill_tc_kernel(const AttnPrefillTcArgs a, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap pool_map,
                            const __grid_constant__ CUtensorMap value_map) {
     // pool_map: the pool's rows (GEN: the keys of its pages); value_map: GEN only, the values of its pages
     using namespace attn_tc;
+    constexpr bool BIAS = OPT == kBias, KEEP = OPT == kKeep;
     constexpr int SUB = HDK / 64, SUBV = HDV / 64;       // 64-lane sub-tiles of a row
     constexpr int kKStages = key_stages(HDK, HDV), kSRing = score_ring(HDK, HDV);
     constexpr unsigned kTile = 128 * 128;                // bytes of a sub-tile: 128 rows of 128 bytes
@@ -281,6 +293,10 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
     const int qt = (int)gridDim.y - 1 - (int)blockIdx.y;
     const int tok0 = a.cu_seqlens[seq], q_len = a.cu_seqlens[seq + 1] - tok0;
     const int q0 = qt * BQ;
+    if (GEN && qt == 0 && seq == 0 && a.partial == nullptr) {
+        for (int n = a.cu_seqlens[gridDim.z]; n < a.n_tokens; ++n)
+            for (int d = threadIdx.x; d < a.dv; d += kThreads) a.out[(size_t)n * a.out_stride + (size_t)head * a.dv + d] = __float2bfloat16(0.f);
+    }
     if (q0 >= q_len) return;                                      // the whole block: nothing was set up yet
     pdl_launch_dependents();
     const int start = a.start_pos[seq];
@@ -292,8 +308,13 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
         return a.window > 0 ? max(0, pos - a.window + 1) : 0;
     };
     const int key_lo = first_key(start + q0);
-    const int kb_lo = key_lo / BKV, kb_hi = key_hi / BKV, n_blocks = kb_hi - kb_lo + 1;
-    auto page_at = [&](int step) -> int { return BIAS ? kb_hi - step : kb_lo + step; };      // the page of the sequence a step works on
+    const int kb_lo = key_lo / BKV, kb_hi = key_hi / BKV;
+    const int keep = KEEP ? a.keep_first : 0, n_kept = min((keep + BKV - 1) / BKV, kb_lo);      // kept pages before the window's
+    const int n_blocks = n_kept + kb_hi - kb_lo + 1;
+    auto page_at = [&](int step) -> int {                         // the page of the sequence a step works on
+        if (BIAS) return kb_hi - step;
+        return KEEP && step < n_kept ? step : kb_lo + step - n_kept;
+    };
     const int vh = GEN ? head / a.maps / (a.n_heads / a.n_kv) : 0;
     const int kvh = GEN ? vh * a.maps + head % a.maps : head / (a.n_heads / a.n_kv);
 
@@ -425,6 +446,10 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
         // moves when a block's maximum exceeds it by more than 2^kLazy: then the row of O is rescaled in tensor
         // memory (read, multiply, write back).  Otherwise probabilities may exceed one, by at most that factor.
         float m_run = -INFINITY, l_run = 0.f;
+        if (KEEP && a.sink) {                                    // the first entry of the sum, and the reference to begin with
+            m_run = a.sink_logit ? a.sink_logit[head] * 1.4426950408889634f : 0.f;
+            l_run = 1.f;
+        }
         const float slope = BIAS ? a.slope[head] * 1.4426950408889634f : 0.f;     // in units of log 2, like the scores
         bool ok = true;
         for (int j = 0; j < n_blocks && ok; ++j) {
@@ -437,9 +462,10 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
             // of zero without a look at the scores.
             const unsigned taddr = trow + (unsigned)(t * BKV);
             const int wpos_lo = start + q0 + quarter * 32, wpos_hi = wpos_lo + 31;
-            const bool open_block = key0 + BKV - 1 <= wpos_lo && key0 >= warp_hi_lo;
-            const bool dead = key0 > wpos_hi || key0 + BKV - 1 < warp_lo;
+            const bool open_block = key0 + BKV - 1 <= wpos_lo && (key0 >= warp_hi_lo || (KEEP && key0 + BKV <= keep));
+            const bool dead = key0 > wpos_hi || (key0 + BKV - 1 < warp_lo && !(KEEP && key0 < keep));
             unsigned buf[2][32];           // two loads of 32 columns: one in flight, one being worked on
+            const float lazy = KEEP && j < 2 ? 0.f : kLazy;      // (how far a score may outgrow the reference)
             float rs4[4] = {0.f, 0.f, 0.f, 0.f};
             // An open block of a row that has its reference maximum already: ONE pass over the scores.  The
             // exponentials are taken against the reference as it stands while the same pass finds the block's
@@ -469,13 +495,13 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
                         const float x1 = fmaf(s1, a.scale_log2e, BIAS ? fmaf(slope, (float)(c * 32 + i + 1), neg_ref) : neg_ref);
                         m4[(i >> 1) & 3] = fmaxf(m4[(i >> 1) & 3], BIAS ? fmaxf(x0, x1) : fmaxf(s0, s1));
                         const float p0 = ex2(x0), p1 = ex2(x1);
-                        rs4[(i >> 1) & 3] += p0 + p1;
                         const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+                        rs4[(i >> 1) & 3] += p0 + p1;
                         packed[c * 16 + (i >> 1)] = *reinterpret_cast<const unsigned*>(&pk);
                     }
                 }
                 const float m_one = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-                done = !__any_sync(0xffffffffu, BIAS ? m_one > kLazy : m_one * a.scale_log2e > m_run + kLazy);
+                done = !__any_sync(0xffffffffu, BIAS ? m_one > kLazy : m_one * a.scale_log2e > m_run + lazy);
                 if (!done) { rs4[0] = 0.f; rs4[1] = 0.f; rs4[2] = 0.f; rs4[3] = 0.f; }
             }
             if (!done) {
@@ -502,12 +528,12 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
                             const int key = key0 + c * 32 + i;
-                            if (live && key >= lo && key <= pos) mx = fmaxf(mx, v[i]);
+                            if (live && (key >= lo || (KEEP && key < keep)) && key <= pos) mx = fmaxf(mx, v[i]);
                         }
                     }
                 }
                 const float m_blk = BIAS ? mx : mx * a.scale_log2e;
-                const bool move = m_blk > m_run + kLazy;                     // also the first block that shows the row a key
+                const bool move = m_blk > m_run + lazy;                     // also the first block that shows the row a key
                 if (__any_sync(0xffffffffu, move)) {
                     const float alpha = move ? (m_run == -INFINITY ? 0.f : ex2(m_run - m_blk)) : 1.0f;
                     if (j > 0) {
@@ -544,18 +570,18 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
                             const float p0 = ex2(v[i]), p1 = ex2(v[i + 1]);
-                            rs4[(i >> 1) & 3] += p0 + p1;
                             const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+                            rs4[(i >> 1) & 3] += p0 + p1;
                             packed[c * 16 + (i >> 1)] = *reinterpret_cast<const unsigned*>(&pk);
                         }
                     } else {
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
                             const int key = key0 + c * 32 + i;
-                            const float p0 = (live && key >= lo && key <= pos) ? ex2(v[i]) : 0.f;
-                            const float p1 = (live && key + 1 >= lo && key + 1 <= pos) ? ex2(v[i + 1]) : 0.f;
-                            rs4[(i >> 1) & 3] += p0 + p1;
+                            const float p0 = (live && (key >= lo || (KEEP && key < keep)) && key <= pos) ? ex2(v[i]) : 0.f;
+                            const float p1 = (live && (key + 1 >= lo || (KEEP && key + 1 < keep)) && key + 1 <= pos) ? ex2(v[i + 1]) : 0.f;
                             const __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+                            rs4[(i >> 1) & 3] += p0 + p1;
                             packed[c * 16 + (i >> 1)] = *reinterpret_cast<const unsigned*>(&pk);
                         }
                     }
@@ -716,12 +742,12 @@ static bool attn_tc_map(const void* base, long long ld, long long rows, int widt
     return attn_tc_map_nd(base, 2, {(cuuint64_t)width, (cuuint64_t)rows, 1}, {(cuuint64_t)ld * 2, 0}, (cuuint32_t)box_rows, 1, out);
 }
 
-template <int HDK, int HDV, bool GEN, bool BIAS = false>
+template <int HDK, int HDV, bool GEN, int OPT = kPlain>
 static int attn_prefill_tc_launch(const AttnPrefillTcArgs& a, const CUtensorMap& qmap, const CUtensorMap& pmap, const CUtensorMap& vmap, dim3 grid,
                                   cudaStream_t stream) {
     const size_t smem = (size_t)(HDK / 64) * 128 * 128 + (size_t)attn_tc::key_stages(HDK, HDV) * (HDK / 64) * 64 * 128 +
                         (size_t)attn_tc::kVStages * (HDV / 64) * 64 * 128 + 24 * 8 + 16 + 1024;
-    auto kernel = attn_prefill_tc_kernel<HDK, HDV, GEN, BIAS>;
+    auto kernel = attn_prefill_tc_kernel<HDK, HDV, GEN, OPT>;
     static bool opted_in = false;
     if (!opted_in) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -752,6 +778,15 @@ static int launch_attn_prefill_tc(const AttnPrefillTcArgs& a, const void* q, lon
 // The windowed family's use of the kernel: whether it takes the sizes, and its launch (BLM_OK, or an error).  q [N, n_heads, dk]
 // contiguous; the pool's pages hold keys [n_kv, 64, dk], then (unless they are the keys) values [n_kv / maps, 64, dv], page_elems in all.
 static bool attn_prefill_tc_general_takes(int dk, int dv) { return dk >= 64 && dk <= 128 && dk % 8 == 0 && dv >= 64 && dv <= 256 && dv % 8 == 0; }
+template <int OPT>
+static int attn_prefill_tc_sized(const AttnPrefillTcArgs& a, const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap, dim3 grid,
+                                 int dk, cudaStream_t stream) {
+    if (dk <= 64 && a.dv <= 64) return attn_prefill_tc_launch<64, 64, true, OPT>(a, qmap, kmap, vmap, grid, stream);
+    if (dk <= 64 && a.dv <= 128) return attn_prefill_tc_launch<64, 128, true, OPT>(a, qmap, kmap, vmap, grid, stream);
+    if (a.dv <= 128) return attn_prefill_tc_launch<128, 128, true, OPT>(a, qmap, kmap, vmap, grid, stream);
+    if (a.dv <= 192) return attn_prefill_tc_launch<128, 192, true, OPT>(a, qmap, kmap, vmap, grid, stream);
+    return attn_prefill_tc_launch<128, 256, true, OPT>(a, qmap, kmap, vmap, grid, stream);
+}
 static int launch_attn_prefill_tc_general(const AttnPrefillTcArgs& a, const void* q, const void* pool, long long page_elems, int n_pages, int dk,
                                           int n_tokens, int n_seqs, int max_q_len, cudaStream_t stream) {
     const dim3 grid(a.n_heads, (max_q_len + attn_tc::BQ - 1) / attn_tc::BQ, n_seqs);
@@ -767,12 +802,9 @@ static int launch_attn_prefill_tc_general(const AttnPrefillTcArgs& a, const void
                         1, &vmap))
         return blm_fail(BLM_CUDA_ERROR, "attention prefill (tcgen05): cuTensorMapEncodeTiled failed");
     if (a.slope != nullptr)                              // (as many value lanes as key lanes: see the caller)
-        return dk <= 64 ? attn_prefill_tc_launch<64, 64, true, true>(a, qmap, kmap, vmap, grid, stream)
-                        : attn_prefill_tc_launch<128, 128, true, true>(a, qmap, kmap, vmap, grid, stream);
-    if (dk <= 64 && a.dv <= 64) return attn_prefill_tc_launch<64, 64, true>(a, qmap, kmap, vmap, grid, stream);
-    if (dk <= 64 && a.dv <= 128) return attn_prefill_tc_launch<64, 128, true>(a, qmap, kmap, vmap, grid, stream);
-    if (a.dv <= 128) return attn_prefill_tc_launch<128, 128, true>(a, qmap, kmap, vmap, grid, stream);
-    if (a.dv <= 192) return attn_prefill_tc_launch<128, 192, true>(a, qmap, kmap, vmap, grid, stream);
-    return attn_prefill_tc_launch<128, 256, true>(a, qmap, kmap, vmap, grid, stream);
+        return dk <= 64 ? attn_prefill_tc_launch<64, 64, true, kBias>(a, qmap, kmap, vmap, grid, stream)
+                        : attn_prefill_tc_launch<128, 128, true, kBias>(a, qmap, kmap, vmap, grid, stream);
+    if (a.sink || a.keep_first > 0) return attn_prefill_tc_sized<kKeep>(a, qmap, kmap, vmap, grid, dk, stream);
+    return attn_prefill_tc_sized<kPlain>(a, qmap, kmap, vmap, grid, dk, stream);
 }
 #endif

@@ -547,7 +547,7 @@ def attention_sink(q, step, pool, block_table, out, n_heads, n_kv, key_dim, valu
 
     `max_q_len`: the longest run of new tokens of one sequence (a bound is enough): bfloat16 steps of 8 or more run
     the tensor-core prompt kernel, 64 query rows a block (it reads step.cu_seqlens and step.start_pos), and steps of 64 or
-    more without options of the scores the tcgen05 kernel (keys of 64 to 128 lanes, values of 64 to 256); shorter ones
+    more without a cap or head numbers the tcgen05 kernel (keys of 64 to 128 lanes, values of 64 to 256); shorter ones
     the tensor-core decode kernel (bfloat16, up to 16 query heads a kv head) or else the row kernel, a block per (row,
     kv head) either, whose keys `n_splits` > 1 cuts over that many blocks (it then needs `scratch`:
     attention_sink_scratch_floats(...) float32)."""
