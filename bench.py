@@ -545,7 +545,7 @@ def ridopel_kernels(z, pk):
         # the key shares the mixer takes at this size (parts.latent_attention.LatentAttention._splits)
         tile = K.latent_attention_tile_rows(bf, H, R, dr, new)
         tiles = (new * H + tile - 1) // tile * n_seqs
-        splits = max(1, min(2 * K.sm_count() // tiles, total // (2 * K.PAGE), 32))
+        splits = max(1, min(K.sm_count() // tiles, total // (2 * K.PAGE), 32))
         pool = torch.randn((n_seqs * pages_each, K.PAGE, R + dr), dtype=bf, device=dev)
         q_lat = torch.randn((H, n, R), dtype=torch.float32, device=dev) * 0.1
         q_rot = torch.randn((n, H, dr), dtype=torch.float32, device=dev)
@@ -706,7 +706,7 @@ def marinex_kernels(z, pk):
         tile = K.latent_attention_tile_rows(bf, H, R, dr, new)
         tiles = (new * H + tile - 1) // tile * n_seqs
         seen = min(total, W + new)
-        splits = max(1, min(2 * K.sm_count() // tiles, seen // (2 * K.PAGE), 32))
+        splits = max(1, min(K.sm_count() // tiles, seen // (2 * K.PAGE), 32))
         lpool = torch.randn((n_seqs * pages_each, K.PAGE, R + dr), dtype=bf, device=dev)
         if new < 16:
             q_lat = torch.randn((H, n, R), dtype=torch.float32, device=dev) * 0.1

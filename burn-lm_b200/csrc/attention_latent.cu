@@ -270,14 +270,19 @@ __global__ void __launch_bounds__(kLatThreads)
 // ---------------------------------------------------------------------------------------------
 // The same attention with both products on the tensor cores (mma.sync m16n8k16, bfloat16 operands, fp32 sums), for a
 // bfloat16 cache whose latent and rotated part are multiples of 16 lanes.  A block owns 16 MT rows and a share of the
-// keys; a chunk of 32 keys lies in shared memory once, as it is cached, and serves as B operand of both products:
-// as it lies for the scores (lanes are the contraction), read transposed for the sums (keys are).  Eight warps:
-//   scores  warp = (8 keys of the chunk, one half of the lanes), all row tiles; the halves meet in the softmax
-//   softmax a warp takes 2 MT rows, a lane a key; weights go to shared memory as bfloat16, sums stay fp32
+// keys; a chunk of KC keys lies in shared memory once, as it is cached, and serves as B operand of both products:
+// as it lies for the scores (lanes are the contraction), read transposed for the sums (keys are).  Sixteen warps:
+//   scores  warp = (16 keys of the chunk, a share of the lanes), all row tiles; the shares meet in the softmax
+//   softmax a warp takes MT rows, a lane KC / 32 keys; weights go to shared memory as bfloat16, sums stay fp32
 //   sums    a warp owns 8 NT output columns of all rows, in registers
+// What bounds it is the chain of a chunk (three barriers, a warp's products one after another, two reductions over a warp) and, next,
+// reads of shared memory (the rows are read again for every 16 keys).  So a block is one multiprocessor's, its sixteen warps make
+// every link short, a chunk is 64 keys where two fit (half the links a key), and the next one is on its way meanwhile.  32 sequences
+// of 2,501 keys, 32 heads on 512 + 64 lanes: two blocks of eight warps and a chunk of 32 copied and waited for between barriers
+// 99 us; sixteen warps, three buffers of 32 keys 78; two of 64 keys 69; 16 instead of 8 keys a warp of the scores 61 (1.5 TB/s).
 // ---------------------------------------------------------------------------------------------
 namespace lat {
-constexpr int KC = 32, THREADS = 256, SS = KC + 8, PS = KC + 8;
+constexpr int THREADS = 512, WARPS = THREADS / 32;
 __device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], const void* p) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
@@ -297,24 +302,30 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+// `on` false: zeros (a weight of 0 silences no NaN)
+__device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__host__ __device__ inline size_t smem_bytes(int rows, int D) {
-    return ((size_t)rows * (D + 8) + (size_t)KC * (D + 8) + (size_t)rows * PS) * sizeof(__nv_bfloat16) + (size_t)2 * rows * SS * sizeof(float);
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+__host__ __device__ constexpr int parts(int kc) { return WARPS / (kc / 16); }        // shares of the lanes in the scores
+__host__ __device__ inline size_t smem_bytes(int rows, int D, int kc, int bufs) {
+    return ((size_t)rows * (D + 8) + (size_t)bufs * kc * (D + 8) + (size_t)rows * (kc + 8)) * sizeof(__nv_bfloat16) +
+           (size_t)parts(kc) * rows * (kc + 8) * sizeof(float);
 }
+constexpr size_t kRoom = 226 * 1024;       // of the 227 KB a block can have, the rest being the kernel's own arrays
 }  // namespace lat
 
-template <typename TO, int MT, int NT>
-__global__ void __launch_bounds__(lat::THREADS, 2)
+template <typename TO, int MT, int NT, int KC, int BUFS>
+__global__ void __launch_bounds__(lat::THREADS, 1)
     latent_attention_mma_kernel(const float* __restrict__ q_lat, const float* __restrict__ q_rot, const __nv_bfloat16* __restrict__ pool,
                                 const int* __restrict__ block_table, int table_stride, const int* __restrict__ cu_seqlens,
                                 const int* __restrict__ slot_of_seq, const int* __restrict__ start_pos, TO* __restrict__ out,
                                 float* __restrict__ partial, int n_tokens, int H, int R, int dr, int page_size, float scale,
                                 int n_splits, int window, const float* __restrict__ sink) {
     using namespace lat;
-    constexpr int ROWS = 16 * MT;
+    constexpr int ROWS = 16 * MT, PARTS = parts(KC), SS = KC + 8, PS = KC + 8, LK = KC / 32;
     const int seq = blockIdx.y, split = blockIdx.z;
     const int first = cu_seqlens[seq];
     const int n_new = cu_seqlens[seq + 1] - first;
@@ -332,18 +343,41 @@ __global__ void __launch_bounds__(lat::THREADS, 2)
     const int D = R + dr, LD = D + 8;
     extern __shared__ __align__(16) unsigned char lat_mma_smem[];
     __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(lat_mma_smem);      // [ROWS][LD]
-    __nv_bfloat16* Ks = Qs + ROWS * LD;                                      // [KC][LD]
-    __nv_bfloat16* Ps = Ks + KC * LD;                                        // [ROWS][PS]
-    float* Ss = reinterpret_cast<float*>(Ps + ROWS * PS);                    // [2][ROWS][SS]: the two halves of the lanes
+    __nv_bfloat16* Kall = Qs + ROWS * LD;                                    // [BUFS][KC][LD]
+    __nv_bfloat16* Ps = Kall + BUFS * KC * LD;                               // [ROWS][PS]
+    float* Ss = reinterpret_cast<float*>(Ps + ROWS * PS);                    // [PARTS][ROWS][SS]: the shares of the lanes
     __shared__ float m_s[ROWS], l_s[ROWS], alpha_s[ROWS];
-    __shared__ int page_of[KC];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int* table = block_table + (size_t)slot_of_seq[seq] * table_stride;
-    for (int row = warp; row < ROWS; row += THREADS / 32) {      // a warp a row: no division an element, loads side by side
+    const int vecs = D / 8, ksteps = D / 16, chunks = (key_hi - key_lo + KC - 1) / KC;
+    // A chunk lies in one page (shares begin at pages, and a page is whole chunks), whose number was fetched a chunk before: the
+    // copies are issued without a wait for it.
+    int next_page = chunks > 0 ? table[key_lo / page_size] : 0, page_at = key_lo / page_size, in_page = 0, loaded = 0;
+    auto load = [&]() {                      // the next chunk, if there is one: a warp takes two keys, its lanes their pieces
+        if (loaded < chunks) {
+            const int nk = key_hi - key_lo - loaded * KC;
+            const __nv_bfloat16* src = pool + ((size_t)next_page * page_size + in_page) * D;
+            __nv_bfloat16* dst = Kall + loaded % BUFS * KC * LD;
+            in_page += KC;
+            if (in_page == page_size) { in_page = 0; ++page_at; }
+            if (loaded + 1 < chunks) next_page = table[page_at];
+            ++loaded;
+#pragma unroll
+            for (int i = 0; i < KC / WARPS; ++i) {
+                const int j = warp + i * WARPS;
+#pragma unroll 3
+                for (int c = lane; c < vecs; c += 32) cp_async_16(dst + j * LD + c * 8, src + (size_t)j * D + c * 8, j < nk);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < BUFS - 1; ++i) load();
+    for (int row = warp; row < ROWS; row += WARPS) {      // a warp a row: no division an element, loads side by side
         const int r = r0 + row, n = first + r / H, h = r % H;
         const float* lat_row = q_lat + ((size_t)h * n_tokens + n) * R;
         const float* rot_row = q_rot + ((size_t)n * H + h) * dr;
-#pragma unroll 4
+#pragma unroll 9
         for (int d = lane; d < D; d += 32) {
             float v = 0.f;
             if (row < n_rows) v = d < R ? lat_row[d] : rot_row[d - R];
@@ -362,61 +396,81 @@ __global__ void __launch_bounds__(lat::THREADS, 2)
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
-    const int vecs = D / 8, ksteps = D / 16;
-    for (int k0 = key_lo; k0 < key_hi; k0 += KC) {
-        const int nk = min(KC, key_hi - k0);
-        __syncthreads();                     // the chunk before is used up (and Qs, m_s, l_s are written)
-        if (tid < KC) page_of[tid] = tid < nk ? table[(k0 + tid) / page_size] : 0;
-        __syncthreads();
-        for (int idx = tid; idx < KC * vecs; idx += THREADS) {   // asynchronous copies: all of a thread's pieces are on their way at once
-            const int j = idx / vecs, c = idx - j * vecs;
-            __nv_bfloat16* dst = Ks + j * LD + c * 8;
-            if (j < nk)
-                cp_async_16(dst, pool + ((size_t)page_of[j] * page_size + (k0 + j) % page_size) * D + c * 8);
-            else
-                *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);   // keys beyond the share are zeros: a weight of 0 silences no NaN
-        }
-        cp_async_wait_all();
-        __syncthreads();
-        {                                    // scores
-            const int nt = warp & 3, half = warp >> 2;
-            const int ks_lo = half ? (ksteps + 1) / 2 : 0, ks_hi = half ? ksteps : (ksteps + 1) / 2;
-            float c[MT][4];
+    int limits[MT];                          // the last keys this warp's rows of the softmax see (none: behind the last row)
 #pragma unroll
-            for (int m = 0; m < MT; ++m) c[m][0] = c[m][1] = c[m][2] = c[m][3] = 0.f;
+    for (int rr = 0; rr < MT; ++rr) limits[rr] = MT * warp + rr < n_rows ? start + (r0 + MT * warp + rr) / H : -1;
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+        const int k0 = key_lo + chunk * KC, nk = min(KC, key_hi - k0);
+        const __nv_bfloat16* Ks = Kall + chunk % BUFS * KC * LD;
+        if (BUFS > 1) {
+            cp_async_wait<(BUFS > 1 ? BUFS - 2 : 0)>();
+            __syncthreads();                 // this chunk is there, the one before is used up (and Qs, m_s, l_s are written)
+            load();
+        } else {
+            __syncthreads();
+            load();
+            cp_async_wait<0>();
+            __syncthreads();
+        }
+        {                                    // scores
+            const int nt = warp % (KC / 16), part = warp / (KC / 16);
+            const int ks_lo = part * ksteps / PARTS, ks_hi = (part + 1) * ksteps / PARTS;
+            float c[MT][2][4];
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) c[m][0][i] = c[m][1][i] = 0.f;
+            const __nv_bfloat16* kp = Ks + (nt * 16 + (lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8;
+            const __nv_bfloat16* qp = Qs + (lane & 15) * LD + (lane >> 4) * 8;
+#pragma unroll 3
             for (int ks = ks_lo; ks < ks_hi; ++ks) {
-                unsigned b0, b1;
-                ldsm_x2(b0, b1, Ks + (nt * 8 + (lane & 7)) * LD + ks * 16 + ((lane >> 3) & 1) * 8);
+                unsigned b[4];
+                ldsm_x4(b, kp + ks * 16);
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     unsigned a[4];
-                    ldsm_x4(a, Qs + (m * 16 + (lane & 15)) * LD + ks * 16 + (lane >> 4) * 8);
-                    mma_bf16(c[m], a, b0, b1);
+                    ldsm_x4(a, qp + m * 16 * LD + ks * 16);
+                    mma_bf16(c[m][0], a, b[0], b[1]);
+                    mma_bf16(c[m][1], a, b[2], b[3]);
                 }
             }
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                float* dst = Ss + ((size_t)half * ROWS + m * 16 + g) * SS + nt * 8 + 2 * t;
-                *reinterpret_cast<float2*>(dst) = make_float2(c[m][0], c[m][1]);
-                *reinterpret_cast<float2*>(dst + 8 * SS) = make_float2(c[m][2], c[m][3]);
-            }
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float* dst = Ss + (part * ROWS + m * 16 + g) * SS + nt * 16 + i * 8 + 2 * t;
+                    *reinterpret_cast<float2*>(dst) = make_float2(c[m][i][0], c[m][i][1]);
+                    *reinterpret_cast<float2*>(dst + 8 * SS) = make_float2(c[m][i][2], c[m][i][3]);
+                }
         }
         __syncthreads();
 #pragma unroll
-        for (int rr = 0; rr < 2 * MT; ++rr) {     // running softmax: a warp takes 2 MT rows, a lane a key
-            const int row = 2 * MT * warp + rr;
-            const int limit = start + (r0 + row) / H;
-            const bool seen = row < n_rows && lane < nk && k0 + lane <= limit && (window <= 0 || k0 + lane > limit - window);
-            const float s = seen ? (Ss[row * SS + lane] + Ss[(ROWS + row) * SS + lane]) * scale : -INFINITY;
-            const float m_old = m_s[row];
-            const float m_new = fmaxf(m_old, warp_max(s));
-            float p = 0.f, alpha = 1.f;
-            if (m_new > -INFINITY) {
-                p = s > -INFINITY ? expf(s - m_new) : 0.f;
-                alpha = m_old > -INFINITY ? expf(m_old - m_new) : 0.f;
+        for (int rr = 0; rr < MT; ++rr) {         // running softmax: a warp takes MT rows, a lane LK keys
+            const int row = MT * warp + rr;
+            const int limit = limits[rr];
+            float s[LK];
+            float top = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < LK; ++i) {
+                const int j = lane + 32 * i;
+                const bool seen = j < nk && k0 + j <= limit && (window <= 0 || k0 + j > limit - window);
+                float sum_s = Ss[row * SS + j];
+#pragma unroll
+                for (int part = 1; part < PARTS; ++part) sum_s += Ss[(part * ROWS + row) * SS + j];
+                s[i] = seen ? sum_s * scale : -INFINITY;
+                top = fmaxf(top, s[i]);
             }
-            const float sum = warp_sum(p);
-            Ps[row * PS + lane] = __float2bfloat16(p);
+            const float m_old = m_s[row];
+            const float m_new = fmaxf(m_old, warp_max(top));
+            float sum = 0.f, alpha = 1.f;
+#pragma unroll
+            for (int i = 0; i < LK; ++i) {
+                const float p = s[i] > -INFINITY ? expf(s[i] - m_new) : 0.f;
+                Ps[row * PS + lane + 32 * i] = __float2bfloat16(p);
+                sum += p;
+            }
+            if (m_new > -INFINITY) alpha = m_old > -INFINITY ? expf(m_old - m_new) : 0.f;
+            sum = warp_sum(sum);
             if (lane == 0) {
                 m_s[row] = m_new;
                 l_s[row] = l_s[row] * alpha + sum;
@@ -493,7 +547,7 @@ __global__ void __launch_bounds__(lat::THREADS, 2)
 static bool latent_takes_mma(int dtype, int R, int dr) { return dtype == BLM_BF16 && R % 16 == 0 && dr % 16 == 0 && R <= 512; }
 BLM_API int blm_latent_attention_tile_rows(int dtype, int H, int R, int dr, int max_q_len) {
     if (!latent_takes_mma(dtype, R, dr)) return kTM;
-    return (long long)max_q_len * H > 16 ? 32 : 16;
+    return (long long)max_q_len * H > 16 && lat::smem_bytes(32, R + dr, 32, 1) <= lat::kRoom ? 32 : 16;
 }
 
 // the shares of a row's keys, merged in the order of the shares
@@ -540,16 +594,22 @@ BLM_API int blm_latent_attention(const float* q_lat, const float* q_rot, const v
     BLM_REQUIRE(n_splits == 1 || partial != nullptr, "latent_attention: key shares need their scratch");
     BLM_REQUIRE(window >= 0, "latent_attention: a window of %d", window);
     const int D = R + dr;
-    if (latent_takes_mma(dtype, R, dr) && (out_dtype == BLM_BF16 || out_dtype == BLM_F32) && ((size_t)pool & 15) == 0) {
-        const int rows = blm_latent_attention_tile_rows(dtype, H, R, dr, max_q_len);
-        const size_t smem = lat::smem_bytes(rows, D);
+    const int rows = blm_latent_attention_tile_rows(dtype, H, R, dr, max_q_len);
+    if (latent_takes_mma(dtype, R, dr) && (out_dtype == BLM_BF16 || out_dtype == BLM_F32) && ((size_t)pool & 15) == 0 && page_size % 64 == 0 &&
+        lat::smem_bytes(rows, D, 32, 1) <= lat::kRoom) {
+        // 64 keys a chunk wherever two fit (the kernel's figures), else 32: copies under the arithmetic are worth more than length
+        const int kc = lat::smem_bytes(rows, D, 64, 2) <= lat::kRoom ? 64 : 32;
+        const int bufs = lat::smem_bytes(rows, D, kc, 2) <= lat::kRoom ? 2 : 1;
+        const size_t smem = lat::smem_bytes(rows, D, kc, bufs);
         const long long tiles = ((long long)max_q_len * H + rows - 1) / rows;
         BLM_REQUIRE(tiles < (1ll << 31) && n_seqs <= 65535 && n_splits <= 65535, "latent_attention: too many blocks");
         const dim3 grid((unsigned)tiles, (unsigned)n_seqs, (unsigned)n_splits);
-        const int nt = R <= 128 ? 2 : R <= 256 ? 4 : 8;
+        const int nt = R <= 256 ? 2 : 4;
 #define BLM_LAT_MMA(TO, MT, NT)                                                                                          \
     {                                                                                                                    \
-        auto kern = latent_attention_mma_kernel<TO, MT, NT>;                                                             \
+        auto kern = kc == 64    ? latent_attention_mma_kernel<TO, MT, NT, 64, 2>                                         \
+                    : bufs == 2 ? latent_attention_mma_kernel<TO, MT, NT, 32, 2>                                         \
+                                : latent_attention_mma_kernel<TO, MT, NT, 32, 1>;                                        \
         if (smem > 48 * 1024) {                                                                                          \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
             if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "latent_attention: %s", cudaGetErrorString(e));        \
@@ -560,8 +620,7 @@ BLM_API int blm_latent_attention(const float* q_lat, const float* q_rot, const v
     }
 #define BLM_LAT_MMA_N(TO, MT)                                            \
     if (nt == 2) BLM_LAT_MMA(TO, MT, 2)                                  \
-    else if (nt == 4) BLM_LAT_MMA(TO, MT, 4)                             \
-    else BLM_LAT_MMA(TO, MT, 8)
+    else BLM_LAT_MMA(TO, MT, 4)
         if (out_dtype == BLM_BF16) {
             if (rows == 32) { BLM_LAT_MMA_N(__nv_bfloat16, 2) } else { BLM_LAT_MMA_N(__nv_bfloat16, 1) }
         } else {

@@ -40,7 +40,7 @@ from ..weights.loader import TensorSpec
 from .base import CacheNeed, Part
 from .linear import Linear
 
-BLOCKS_PER_SM = 2     # blocks of the attention kernel a step should offer every multiprocessor
+BLOCKS_PER_SM = 1     # blocks of the attention kernel a step should offer every multiprocessor (a block fills one)
 EXPAND_TOKENS = 16    # from this many new tokens of a sequence on, a bfloat16 step writes out keys and values of the heads
 EXPAND_SPAN = 4       # ... with a window only while the longest sequence is at most this many times (new tokens + window) long
 NO_WINDOW = 1 << 30   # what the windowed family's kernels take for "every earlier key"
