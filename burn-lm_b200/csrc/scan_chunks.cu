@@ -287,7 +287,8 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         float s = 0.f;
         if (i < kQ) {
 #pragma unroll
-            for (int y = 0; y < kQ; ++y) s += As[j][y] * Ts[y][i];
+            for (int y = 0; y < kQ; ++y)
+                if (y <= j) s += As[j][y] * Ts[y][i];           // (nothing of a later token, not even times zero)
         }
         m[e] = s;
         m[kMat + e] = i < kQ ? Ts[j][i] : 0.f;
@@ -473,6 +474,29 @@ __device__ __forceinline__ void dots(const float* src, const f32x2 (&s)[NP / RG 
         for (int c = 0; c < CK; ++c) res[t][c] = RG == 32 ? v[t * TG][c] + __shfl_xor_sync(0xffffffffu, v[t * TG][CK + c], 16) : v[t * TG][c];
 }
 
+// sum += row[i] x[i] over the tokens i <= j.  The later ones are left out and not multiplied by the matrix's zeros: a zero does not
+// silence a value that is not finite, and a token's output must not depend on the tokens behind it.  (The predicate costs no
+// instruction beside its comparison; one chain of sums for the even and one for the odd tokens.)
+template <int C, int CK>
+__device__ __forceinline__ void apply_up_to(const float* row, int j, const float (&x)[kQ][C], float (&sum)[CK]) {
+    float odd[CK];
+#pragma unroll
+    for (int c = 0; c < CK; ++c) odd[c] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kQ; i += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(row + i);
+#pragma unroll
+        for (int c = 0; c < CK; ++c) {
+            if (i <= j) sum[c] = fmaf(m.x, x[i][c], sum[c]);
+            if (i + 1 <= j) odd[c] = fmaf(m.y, x[i + 1][c], odd[c]);
+            if (i + 2 <= j) sum[c] = fmaf(m.z, x[i + 2][c], sum[c]);
+            if (i + 3 <= j) odd[c] = fmaf(m.w, x[i + 3][c], odd[c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < CK; ++c) sum[c] += odd[c];
+}
+
 template <int NP, int C, int RG, int CT, int KIND>
 __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArgs a) {
     constexpr int kWalkers = RG * CT / C;      // threads that compute; one more warp loads
@@ -615,18 +639,12 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
         float u[TL][CK];
 #pragma unroll
         for (int t = 0; t < TL; ++t) {
+            const int j = t * TG + tg;
+            apply_up_to<C, CK>(M + j * kMs, j, x, o[t]);
+            if (KIND == kDelta) {
 #pragma unroll
-            for (int c = 0; c < CK; ++c) u[t][c] = 0.f;
-#pragma unroll
-            for (int i = 0; i < kQ; i += 4) {
-                const float4 mm = *reinterpret_cast<const float4*>(M + (t * TG + tg) * kMs + i);
-#pragma unroll
-                for (int c = 0; c < CK; ++c) o[t][c] += (mm.x * x[i][c] + mm.y * x[i + 1][c]) + (mm.z * x[i + 2][c] + mm.w * x[i + 3][c]);
-                if (KIND == kDelta) {
-                    const float4 tt = *reinterpret_cast<const float4*>(M + kMat + (t * TG + tg) * kMs + i);
-#pragma unroll
-                    for (int c = 0; c < CK; ++c) u[t][c] += (tt.x * x[i][c] + tt.y * x[i + 1][c]) + (tt.z * x[i + 2][c] + tt.w * x[i + 3][c]);
-                }
+                for (int c = 0; c < CK; ++c) u[t][c] = 0.f;
+                apply_up_to<C, CK>(M + kMat + j * kMs, j, x, u[t]);
             }
         }
         if (KIND == kDelta) {

@@ -122,3 +122,38 @@ def test_chunks_against_the_walk_in_float64(kind, heads, rows, dv, lens, starts)
         at += m
     for slot in set(range(state.shape[0])) - set(step.slot_of_seq.tolist()):
         assert torch.equal(state[slot], before[slot].float())
+
+
+@pytest.mark.parametrize("heads,rows,dv", [(2, 20, 5), (3, 64, 64), (2, 128, 100)])      # 8, 16 and 32 row groups
+@pytest.mark.parametrize("kind,where", [("ssm", "value"), ("ssm", "key"), ("wkv", "value"), ("wkv", "key"), ("lower", "value"), ("delta", "value"),
+                                        ("delta", "key"), ("delta", "beta")])
+def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(kind, where, heads, rows, dv):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(heads + rows)
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    lens, starts, bad = [40, 35], [0, 3], 40 + 22                             # (in the middle of a chunk of the second sequence)
+    step, n = step_of(lens, starts), sum(lens)
+    state = state_of(step, heads, rows, dv, 0, gen)
+    q, k, v, a, b = rnd(n, heads * rows), rnd(n, heads * rows), rnd(n, heads * dv), rnd(n, heads * rows), rnd(n, heads)
+    bias, extra, per_head = rnd(heads * rows), torch.rand(heads * rows, generator=gen, device="cuda"), [rnd(heads) for _ in range(3)]
+
+    def run(value, key, beta):
+        out, own = torch.zeros((n, heads * dv), device="cuda"), state.clone()
+        if kind == "ssm":
+            x = torch.cat([value, key, q], 1)
+            K.ssm_scan(x, 0, heads * dv, heads * (dv + rows), b, 0, *per_head, out, heads, heads, rows, dv, step, own, 0)
+        elif kind == "delta":
+            K.delta_scan(q, 0, key, 0, value, 0, beta, 0, a, 0, bias, per_head[0], out, heads, heads, rows, dv, step, own, 0)
+        else:
+            K.decay_scan(q, 0, key if kind == "wkv" else None, 0, value, 0, a, 0, bias, extra, out, heads, rows, dv,
+                         K.DECAY_EXP_EXP if kind == "wkv" else K.DECAY_LOWER_BOUND, kind == "wkv", step, own, 0)
+        return out, own
+
+    clean, _ = run(v, k, b)
+    for wrong in (float("nan"), float("inf"), float("-inf")):
+        spoilt = dict(value=v.clone(), key=k.clone(), beta=b.clone())
+        spoilt[where][bad] = float("nan") if where == "beta" else wrong      # (beta passes through a sigmoid)
+        out, own = run(spoilt["value"], spoilt["key"], spoilt["beta"])
+        assert torch.equal(out[:bad], clean[:bad])
+        assert not torch.isfinite(out[bad]).any()
+        assert torch.isfinite(own[int(step.slot_of_seq[0])]).all() and not torch.isfinite(own[int(step.slot_of_seq[1]), (3 + 35) & 1]).all()
