@@ -7,8 +7,9 @@
 // are laid so that each leaves its result where the next one wants its operand:
 //   scores, transposed:  S^T = K Q^T.  A tile's sixteen rows are keys; its eight columns are (head of the key/value head, query),
 //     column 2 h + x.  Lane l then holds head l % 4 of every key/value head at key l / 4 - which is the B operand of
-//   the mix:  M = talk W, m16n8k8 in tf32: k runs over (key/value head pair, l % 4), the columns are keys.  Weights and talk are each
-//     the sum of two tf32 numbers (22 bits), three products of the four: the error is that of fp32 sums, not of tf32.
+//   the mix:  M = talk W, m16n8k16: k runs over (four key/value heads, l % 4), the columns are keys.  Weights and talk are each
+//     the sum of three bfloat16 numbers, which hold all 24 bits of a float; of their nine products the six that reach 2^-24 of
+//     a product are formed.  (Two tf32 numbers each hold 22 bits: 24-bit weights of heads that cancel came out wrong.)
 //     Lane l gets head row l / 4 at keys 2 (l % 4), + 1 - which, packed to bfloat16, is the B operand of
 //   the values, transposed:  O^T += V^T M^T: rows are value lanes, k runs over keys, columns are eight head rows, of which four
 //     belong to the key/value head.  Two queries fill both halves: the second query's rows cross over by one shuffle.
@@ -54,10 +55,9 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
+    const unsigned v[4] = {a.x, a.y, a.z, a.w};
+    mma_bf16(c, v, b0, b1);
 }
 __device__ __forceinline__ void cp16(unsigned dst, const void* src, bool on) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
@@ -66,35 +66,53 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// A float as the sum of two tf32 numbers, 22 bits of it.
-__device__ __forceinline__ void split_tf32(float v, unsigned& hi, unsigned& lo) {
-    hi = __float_as_uint(v) & 0xffffe000u;
-    lo = __float_as_uint(v - __uint_as_float(hi)) & 0xffffe000u;
-}
 __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
     __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<unsigned*>(&v);
 }
 
-// talk's fragments for the mix in shared memory: [row tile][k tile][hi, lo][lane] of 16 bytes.  Row r of row tile m is head
-// r % 4 of key/value head 4 m + r / 4; k of k tile t is head k % 4 of key/value head 2 t + k / 4.  Heads that are not there: zero.
-constexpr int kTalkBytes = 2 * 4 * 2 * 32 * 16;
+// Two floats as the sums of three bfloat16 numbers each: eight bits a number, so all 24 of a float.
+struct Limbs {
+    unsigned hi, mid, lo;          // pairs, the first float in the lower half
+};
+__device__ __forceinline__ Limbs split_bf16(float a, float b) {
+    Limbs l;
+    l.hi = pack_bf16(a, b);
+    a -= __uint_as_float(l.hi << 16);
+    b -= __uint_as_float(l.hi & 0xffff0000u);
+    l.mid = pack_bf16(a, b);
+    l.lo = pack_bf16(a - __uint_as_float(l.mid << 16), b - __uint_as_float(l.mid & 0xffff0000u));
+    return l;
+}
+
+// talk's fragments for the mix in shared memory: [row tile][k tile][hi, mid, lo][lane] of 16 bytes.  Row r of row tile m is head
+// r % 4 of key/value head 4 m + r / 4; k = 2 h + e + 8 half of k tile t is head h of key/value head 4 t + 2 half + e.  Heads that
+// are not there: zero.
+constexpr int kTalkBytes = 2 * 2 * 3 * 32 * 16;
 __device__ __forceinline__ void stage_talk(uint4* to, const QuadArgs& a, int tid, int threads) {
     const int per = a.H / a.G;
-    for (int e = tid; e < 2 * 4 * 32; e += threads) {
-        const int lane = e % 32, t = e / 32 % 4, m = e / 128;
-        unsigned hi[4], lo[4];
+    for (int e = tid; e < 2 * 2 * 32; e += threads) {
+        const int lane = e % 32, t = e / 32 % 2, m = e / 64;
+        unsigned hi[4], mid[4], lo[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int r = (lane >> 2) + (i & 1) * 8, k = (lane & 3) + (i >> 1) * 4;
-            const int gr = 4 * m + r / 4, hr = r % 4, gk = 2 * t + k / 4, hk = k % 4;
-            float v = 0.f;
-            if (gr < a.G && hr < per && gk < a.G && hk < per)
-                v = a.talk ? a.talk[(size_t)(gr * per + hr) * a.H + gk * per + hk] : (gr == gk && hr == hk ? 1.f : 0.f);
-            split_tf32(v, hi[i], lo[i]);
+            const int r = (lane >> 2) + (i & 1) * 8, gr = 4 * m + r / 4, hr = r % 4, hk = lane & 3;
+            float v[2] = {0.f, 0.f};
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int gk = 4 * t + 2 * (i >> 1) + x;
+                if (gr < a.G && hr < per && gk < a.G && hk < per)
+                    v[x] = a.talk ? a.talk[(size_t)(gr * per + hr) * a.H + gk * per + hk] : (gr == gk && hr == hk ? 1.f : 0.f);
+            }
+            const Limbs l = split_bf16(v[0], v[1]);
+            hi[i] = l.hi;
+            mid[i] = l.mid;
+            lo[i] = l.lo;
         }
-        to[((m * 4 + t) * 2 + 0) * 32 + lane] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        to[((m * 4 + t) * 2 + 1) * 32 + lane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        uint4* at = to + (m * 2 + t) * 3 * 32 + lane;
+        at[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        at[32] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+        at[64] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
 }
 
@@ -219,7 +237,8 @@ __device__ __forceinline__ void weigh(float (&c)[kQuads][4], const float (&start
 }
 
 // The mix of X queries' weights, packed: p[query][row tile][row half][key half] is head row (lane / 4) + 8 half at keys
-// 2 (lane % 4), + 1.  A k tile's talk serves every query and key half, and their products do not wait for one another.
+// 2 (lane % 4), + 1.  A k tile's talk serves every query and key half, and their products do not wait for one another.  Of the
+// nine products of limbs the three below 2^-24 of a product are left out; the smallest are added first.
 template <int X, bool FULL>
 __device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[kQuads][4], const uint4* talk, int G, int lane) {
     float c[X][2][2][4];
@@ -230,32 +249,30 @@ __device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[
 #pragma unroll
             for (int r = 0; r < 2; ++r) c[x][m][r][0] = c[x][m][r][1] = c[x][m][r][2] = c[x][m][r][3] = 0.f;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-        if (FULL || 2 * t < G) {
-            unsigned h0[X][2], l0[X][2], h1[X][2], l1[X][2];
+    for (int t = 0; t < 2; ++t) {
+        if (FULL || 4 * t < G) {
+            Limbs b[X][2][2];
 #pragma unroll
             for (int x = 0; x < X; ++x)
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    split_tf32(w[2 * t][2 * r + x], h0[x][r], l0[x][r]);
-                    split_tf32(w[2 * t + 1][2 * r + x], h1[x][r], l1[x][r]);
-                }
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) b[x][r][half] = split_bf16(w[4 * t + 2 * half][2 * r + x], w[4 * t + 2 * half + 1][2 * r + x]);
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 if (FULL || 4 * m < G) {
-                    const uint4 hi = talk[((m * 4 + t) * 2 + 0) * 32 + lane], lo = talk[((m * 4 + t) * 2 + 1) * 32 + lane];
-#pragma unroll
-                    for (int x = 0; x < X; ++x)
-#pragma unroll
-                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], lo, h0[x][r], h1[x][r]);
-#pragma unroll
-                    for (int x = 0; x < X; ++x)
-#pragma unroll
-                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], hi, l0[x][r], l1[x][r]);
-#pragma unroll
-                    for (int x = 0; x < X; ++x)
-#pragma unroll
-                        for (int r = 0; r < 2; ++r) mma_tf32(c[x][m][r], hi, h0[x][r], h1[x][r]);
+                    const uint4* at = talk + (m * 2 + t) * 3 * 32 + lane;
+                    const uint4 hi = at[0], mid = at[32], lo = at[64];
+#define BLM_MIX(A, B)                                                                            \
+    _Pragma("unroll") for (int x = 0; x < X; ++x) _Pragma("unroll") for (int r = 0; r < 2; ++r) \
+        mma_bf16(c[x][m][r], A, b[x][r][0].B, b[x][r][1].B)
+                    BLM_MIX(lo, hi);
+                    BLM_MIX(hi, lo);
+                    BLM_MIX(mid, mid);
+                    BLM_MIX(mid, hi);
+                    BLM_MIX(hi, mid);
+                    BLM_MIX(hi, hi);
+#undef BLM_MIX
                 }
             }
         }

@@ -66,3 +66,34 @@ def test_weights_mix_and_values(H, G, dk, dv, lens, starts, ranges):
             room = 2.0 ** -7 * torch.einsum("hnt,thd->nhd", w.abs(), v.abs()) + 2.0 ** -17 * torch.einsum("hnt,thd->nhd", terms, v.abs())
             assert ((out[sl].double().view(m, H, dv) - want).abs() <= room).all()
         assert not out[n:].any()
+
+
+@pytest.mark.parametrize("lens", [[1], [2, 1]])                               # the kernel of single tokens, and that of portions
+@pytest.mark.parametrize("H,G,dk,dv", [(32, 8, 64, 64), (20, 5, 48, 72), (6, 2, 16, 8)])
+def test_the_mix_keeps_every_bit_of_the_weights(H, G, dk, dv, lens):
+    """Scores of zero give weights of exactly a half; every head takes two others' weights with factors that differ in their last
+    bits, so that what is left of the two is those bits."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(H)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu = [0]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    n = cu[-1]
+    step = SimpleNamespace(n_tokens=n, n_seqs=len(lens), max_q_len=max(lens), max_kv_len=max(lens), cu_seqlens=i32(cu),
+                           token_seq=i32([s for s, m in enumerate(lens) for _ in range(m)]), slot_of_seq=i32(list(range(len(lens)))),
+                           start_pos=i32([0] * len(lens)))
+    assert K.sigmoid_attention_in_registers(torch.bfloat16, H, G, dk, dv)
+    pool = torch.zeros((len(lens), G * K.PAGE * (dk + dv)), dtype=torch.bfloat16, device="cuda")
+    pool[:, G * K.PAGE * dk:].view(-1, G, K.PAGE, dv)[:, :, 0] = 1.0          # the first position's values: one
+    talk = torch.zeros((H, H), device="cuda")
+    for h in range(H):
+        a, b = torch.randperm(H, generator=torch.Generator().manual_seed(h))[:2].tolist()
+        bits = int(torch.randint(1 << 23, (1,), generator=torch.Generator().manual_seed(h + 100)))
+        talk[h, a] = (1 << 23 | bits) * 2.0 ** -23                            # (24 bits, between one and two)
+        talk[h, b] = -((1 << 23 | bits) - 1 - h % 7) * 2.0 ** -23
+    out = torch.zeros((n, H * dv), dtype=torch.bfloat16, device="cuda")
+    K.sigmoid_attention(torch.zeros((n, H * dk), dtype=torch.bfloat16, device="cuda"), pool, i32([[s] for s in range(len(lens))]), step, out,
+                        H, G, dk, dv, 1.0, talk=talk)
+    want = (talk.double().sum(1) * 0.5)[:, None].expand(H, dv).reshape(-1)     # every position sees the first one's value; the others' are zero
+    assert ((out.double() - want).abs() <= 2.0 ** -7 * want.abs()).all()      # (bfloat16 rounds what is left, twice)
