@@ -37,9 +37,10 @@
 // the second product).
 //
 // KEEP (with GEN): kept first positions and a sink.  The sink's score is the reference to begin with, and a reference that trails the
-// largest score means that the largest probability is not 1 but rounded as the others are; in the first two steps the
-// reference follows the largest score itself.  Error against 64 bits of a 2,048-token layer and time: never following 3.97e-3 and
-// 54 us, two steps 3.86e-3 and 59, five 3.85e-3 and 66, always 3.84e-3 (as the mma.sync kernel's) and 94.
+// largest score means that the largest probability is not 1 but rounded as the others are: here the reference follows the largest
+// score itself in every step, and a step finds its maximum first (some row of the warp moves in most steps, so that the single
+// pass would mostly be done twice).  Error against 64 bits of a 2,048-token layer and time: trailing by up to 2^8 3.97e-3 and 54 us,
+// from the third step on 3.86e-3 and 59, never 3.84e-3 (as the mma.sync kernel's) and 72 (with the single pass first 90).
 //
 // BIAS (with GEN): slope_h times the distance is taken off a score.  The pages are then walked from the diagonal back: the row's
 // largest score is mostly found in the first pages, where with a bias by distance it would otherwise move in every page, and with
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
             const bool open_block = key0 + BKV - 1 <= wpos_lo && (key0 >= warp_hi_lo || (KEEP && key0 + BKV <= keep));
             const bool dead = key0 > wpos_hi || (key0 + BKV - 1 < warp_lo && !(KEEP && key0 < keep));
             unsigned buf[2][32];           // two loads of 32 columns: one in flight, one being worked on
-            const float lazy = KEEP && j < 2 ? 0.f : kLazy;      // (how far a score may outgrow the reference)
+            constexpr float lazy = KEEP ? 0.f : kLazy;           // how far a score may outgrow the reference
             float rs4[4] = {0.f, 0.f, 0.f, 0.f};
             // An open block of a row that has its reference maximum already: ONE pass over the scores.  The
             // exponentials are taken against the reference as it stands while the same pass finds the block's
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
             if (dead) {
 #pragma unroll
                 for (int i = 0; i < BKV / 2; ++i) packed[i] = 0u;
-            } else if (open_block && __all_sync(0xffffffffu, m_run != -INFINITY)) {
+            } else if (!KEEP && open_block && __all_sync(0xffffffffu, m_run != -INFINITY)) {
                 const float neg_ref = BIAS ? slope * (float)(key0 - pos) - m_run : -m_run;
                 float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 tmem_ld32_issue(taddr, buf[0]);
@@ -501,7 +502,7 @@ __global__ void __launch_bounds__(attn_tc::kThreads, attn_tc::blocks_an_sm(HDV))
                     }
                 }
                 const float m_one = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-                done = !__any_sync(0xffffffffu, BIAS ? m_one > kLazy : m_one * a.scale_log2e > m_run + lazy);
+                done = !__any_sync(0xffffffffu, BIAS ? m_one > lazy : m_one * a.scale_log2e > m_run + lazy);
                 if (!done) { rs4[0] = 0.f; rs4[1] = 0.f; rs4[2] = 0.f; rs4[3] = 0.f; }
             }
             if (!done) {

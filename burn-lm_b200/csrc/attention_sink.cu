@@ -1536,7 +1536,7 @@ BLM_API int blm_attention_sink(const void* q, const void* pool, int dtype, long 
     if (is_prompt && max_q_len >= 64 && status != nullptr && n_pages > 0 && attn_prefill_tc_general_takes(dk, dv) && softcap == 0.f &&
         head_scale == nullptr && ((!sink && keep_first == 0) || (maps == 1 && slope == nullptr && chunk == 0)) && (scale > 0.f || slope != nullptr) && (slope == nullptr || dk == dv) && out_stride % 8 == 0 && (((size_t)out | (size_t)q | (size_t)pool) & 15) == 0) {
         // long portions without a cap or head numbers: the products on tcgen05, accumulators in tensor memory (2,048 tokens of 32
-        // heads of 128 on 8, a window of 1,024, 64 kept first, a sink: 59 us; the mma.sync kernel 177)
+        // heads of 128 on 8, a window of 1,024, 64 kept first, a sink: 72 us; the mma.sync kernel 177)
         AttnPrefillTcArgs t = {};
         t.block_table = block_table; t.table_stride = table_stride; t.cu_seqlens = cu_seqlens; t.slot_of_seq = slot_of_seq;
         t.start_pos = start_pos; t.out = (__nv_bfloat16*)out; t.n_heads = n_heads; t.n_kv = n_kv; t.window = window < kNoWindow ? window : 0;

@@ -61,3 +61,35 @@ def test_window_kept_positions_and_sink(H, G, dk, dv, window, keep, sink, lens, 
         assert ((out[sl].double().view(m, H, dv) - want).abs() <= room).all()
     assert not out[n:].any()                                                  # rows of no sequence hold zeros
     K.check_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 64), (128, 128), (64, 200)])
+def test_the_largest_probability_is_not_rounded(dk, dv):
+    """Rows whose largest score comes late and exceeds what came before by less than 2^8: their probabilities are taken against that
+    score itself, so that it enters the sum over the values as exactly one."""
+    tops = torch.linspace(0.5, 5.4, 24).bfloat16()
+    n_seqs, m, at = len(tops), 256, 200
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    step = SimpleNamespace(n_tokens=n_seqs * m, n_seqs=n_seqs, max_q_len=m, max_kv_len=m, cu_seqlens=i32([m * s for s in range(n_seqs + 1)]),
+                           token_seq=i32([s for s in range(n_seqs) for _ in range(m)]), token_pos=i32(list(range(m)) * n_seqs),
+                           slot_of_seq=i32(list(range(n_seqs))), start_pos=i32([0] * n_seqs))
+    pages = m // K.PAGE
+    pool = torch.zeros((n_seqs * pages, K.PAGE * (dk + dv)), dtype=torch.bfloat16, device="cuda")
+    of_top = pool.view(n_seqs, pages, -1)[:, at // K.PAGE]                    # the page of the one key that is not zero
+    of_top[:, : K.PAGE * dk].view(n_seqs, K.PAGE, dk)[:, at % K.PAGE, 0] = tops.cuda()
+    of_top[:, K.PAGE * dk:].view(n_seqs, K.PAGE, dv)[:, at % K.PAGE] = 1.0     # ... nor its values
+    if dk == dv:
+        pool = pool.view(-1, 2, 1, K.PAGE, dk)
+    q = torch.zeros((n_seqs * m, dk), dtype=torch.bfloat16, device="cuda")
+    q[:, 0] = 1.0
+    out = torch.zeros((n_seqs * m, dv), dtype=torch.bfloat16, device="cuda")
+    K.attention_sink(q, step, pool, i32(list(range(n_seqs * pages))).view(n_seqs, pages), out, 1, 1, dk, dv, 1.0, 4000, 3, sink=True,
+                     max_q_len=m)
+    e = torch.exp(tops.double().cuda())[:, None]
+    others = torch.arange(at, m, device="cuda", dtype=torch.float64)[None] + 1.0      # the keys before and after it, and the sink: exp(0) each
+    want = (e / (e + others))[:, :, None]
+    got = out.double().view(n_seqs, m, dv)
+    assert not got[:, :at].any()
+    # half a place of a bfloat16 output, and 2^-14 for the fp32 sums of some two hundred exponentials
+    assert ((got[:, at:] - want).abs() <= 2.0 ** (torch.floor(torch.log2(want)) - 8) + 2.0 ** -14 * want).all()
+    K.check_status(torch.device("cuda"))
