@@ -273,13 +273,15 @@ __global__ void __launch_bounds__(kLatThreads)
 // keys; a chunk of KC keys lies in shared memory once, as it is cached, and serves as B operand of both products:
 // as it lies for the scores (lanes are the contraction), read transposed for the sums (keys are).  Sixteen warps:
 //   scores  warp = (16 keys of the chunk, a share of the lanes), all row tiles; the shares meet in the softmax
-//   softmax a warp takes MT rows, a lane KC / 32 keys; weights go to shared memory as bfloat16, sums stay fp32
+//   softmax a warp takes MT rows, a lane KC / 32 keys; weights go to shared memory as two bfloat16 numbers each, sums stay fp32
 //   sums    a warp owns 8 NT output columns of all rows, in registers
 // What bounds it is the chain of a chunk (three barriers, a warp's products one after another, two reductions over a warp) and, next,
 // reads of shared memory (the rows are read again for every 16 keys).  So a block is one multiprocessor's, its sixteen warps make
 // every link short, a chunk is 64 keys where two fit (half the links a key), and the next one is on its way meanwhile.  32 sequences
 // of 2,501 keys, 32 heads on 512 + 64 lanes: two blocks of eight warps and a chunk of 32 copied and waited for between barriers
 // 99 us; sixteen warps, three buffers of 32 keys 78; two of 64 keys 69; 16 instead of 8 keys a warp of the scores 61 (1.5 TB/s).
+// Longer chunks meet fewer running maxima, whose weights are exactly one, and as single bfloat16 numbers the weights of 64 keys
+// were 0.3 to 1.5 % further from 64 bits than those of 32; as two (16 bits: 70 us) 0.5 to 5 % nearer.
 // ---------------------------------------------------------------------------------------------
 namespace lat {
 constexpr int THREADS = 512, WARPS = THREADS / 32;
@@ -346,6 +348,9 @@ __global__ void __launch_bounds__(lat::THREADS, 1)
     __nv_bfloat16* Kall = Qs + ROWS * LD;                                    // [BUFS][KC][LD]
     __nv_bfloat16* Ps = Kall + BUFS * KC * LD;                               // [ROWS][PS]
     float* Ss = reinterpret_cast<float*>(Ps + ROWS * PS);                    // [PARTS][ROWS][SS]: the shares of the lanes
+    // over the first share, a row over its own; four rows of eight start 16 bytes later, so that the eight start in different banks
+    __nv_bfloat16* Ls = reinterpret_cast<__nv_bfloat16*>(Ss);
+    auto second_half = [&](int row) { return row * 2 * SS + (row & 4) * 2; };
     __shared__ float m_s[ROWS], l_s[ROWS], alpha_s[ROWS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int* table = block_table + (size_t)slot_of_seq[seq] * table_stride;
@@ -463,10 +468,13 @@ __global__ void __launch_bounds__(lat::THREADS, 1)
             const float m_old = m_s[row];
             const float m_new = fmaxf(m_old, warp_max(top));
             float sum = 0.f, alpha = 1.f;
+            __syncwarp();                    // the row's scores are read: the weights' second halves take the place of their first share
 #pragma unroll
             for (int i = 0; i < LK; ++i) {
                 const float p = s[i] > -INFINITY ? expf(s[i] - m_new) : 0.f;
-                Ps[row * PS + lane + 32 * i] = __float2bfloat16(p);
+                const __nv_bfloat16 first_half = __float2bfloat16(p);
+                Ps[row * PS + lane + 32 * i] = first_half;
+                Ls[second_half(row) + lane + 32 * i] = __float2bfloat16(p - __bfloat162float(first_half));
                 sum += p;
             }
             if (m_new > -INFINITY) alpha = m_old > -INFINITY ? expf(m_old - m_new) : 0.f;
@@ -488,15 +496,23 @@ __global__ void __launch_bounds__(lat::THREADS, 1)
         }
 #pragma unroll
         for (int kk = 0; kk < KC / 16; ++kk) {
-            unsigned a[MT][4];
+            unsigned a[MT][4], al[MT][4];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) ldsm_x4(a[m], Ps + (m * 16 + (lane & 15)) * PS + kk * 16 + (lane >> 4) * 8);
+            for (int m = 0; m < MT; ++m) {
+                ldsm_x4(a[m], Ps + (m * 16 + (lane & 15)) * PS + kk * 16 + (lane >> 4) * 8);
+                ldsm_x4(al[m], Ls + second_half(m * 16 + (lane & 15)) + kk * 16 + (lane >> 4) * 8);
+            }
 #pragma unroll
             for (int np = 0; np < NT / 2; ++np) {
                 const int n0 = (warp * NT + 2 * np) * 8;
                 if (n0 < R) {                // R is a multiple of 16: a pair of column tiles is inside or outside
                     unsigned b[4];
                     ldsm_x4_trans(b, Ks + (kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + n0 + (lane >> 4) * 8);
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        mma_bf16(acc[m][2 * np], al[m], b[0], b[1]);
+                        mma_bf16(acc[m][2 * np + 1], al[m], b[2], b[3]);
+                    }
 #pragma unroll
                     for (int m = 0; m < MT; ++m) {
                         mma_bf16(acc[m][2 * np], a[m], b[0], b[1]);

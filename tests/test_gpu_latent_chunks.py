@@ -56,3 +56,29 @@ def test_latent_attention_in_chunks(H, R, dr, splits, window, sink, lens, starts
             # the weights are rounded to bfloat16 (2^-8), bfloat16 outputs once more; the rest is float32
             room = 2.0 ** -8 * (p @ keys[:, :R].abs()) + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0) + 1e-4
             assert ((out[:, sl].double() - want).abs() <= room).all()
+
+
+@pytest.mark.parametrize("H,R,dr", [(16, 256, 32), (32, 512, 64), (20, 512, 512)])           # 64 keys twice, and 32
+@pytest.mark.parametrize("splits", [1, 4])
+def test_weights_are_kept_to_sixteen_bits(H, R, dr, splits):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(R + dr)
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    n, keys, D = 3, 700, R + dr
+    pages = -(-keys // K.PAGE)
+    step = SimpleNamespace(n_tokens=n, n_seqs=n, max_q_len=1, max_kv_len=keys, cu_seqlens=i32(list(range(n + 1))), token_seq=i32(list(range(n))),
+                           token_pos=i32([keys - 1] * n), slot_of_seq=i32(list(range(n))), start_pos=i32([keys - 1] * n))
+    latents = rnd(n, pages * K.PAGE, D).bfloat16()
+    q_lat, q_rot = rnd(H, n, R).bfloat16().float(), rnd(n, H, dr).bfloat16().float()
+    out = torch.empty((H, n, R), device="cuda")
+    partial = torch.empty((max(1, K.latent_attention_scratch_floats(n, H, R, splits)),), device="cuda")
+    scale = 2.0 * D ** -0.5
+    K.latent_attention(q_lat, q_rot, latents.view(n * pages, K.PAGE, D), i32(list(range(n * pages))).view(n, pages), step, out, H, R, dr, scale,
+                       n_splits=splits, partial=partial)
+    seen = latents[:, :keys].double()
+    p = torch.softmax(torch.einsum("nhd,ntd->nht", torch.cat([q_lat.transpose(0, 1), q_rot], -1).double(), seen) * scale, -1)
+    want = torch.einsum("nht,ntd->nhd", p, seen[..., :R]).transpose(0, 1)
+    terms = torch.einsum("nht,ntd->nhd", p, seen[..., :R].abs()).transpose(0, 1)
+    # two bfloat16 numbers round a weight by 2^-17; fp32 scores of up to 10 and their exponentials by some 2^-19
+    assert ((out.double() - want).abs() <= 2.0 ** -15 * terms).all()
