@@ -9,7 +9,8 @@
 //
 // A scan block owns (sequence, head, some value columns): 256 threads = columns x row groups; thread (col, rg) keeps rows
 // rg, rg + RG, rg + 2 RG, ... of its column in registers.  A sum over rows is a thread's partial sum and then shuffles
-// over the row groups (adjacent lanes): the same order whatever the step's size or batch.  RG = 8 (32 columns a block).
+// over the row groups (adjacent lanes): the same order whatever the step's size or batch.  Sequences that bring many new tokens
+// run in chunks instead (scan_chunks.cu; `below` says from which length on they are left alone).  RG = 8 (32 columns a block).
 // More lanes a column were measured and left out.  RG = 32 (a warp a column, four times the warps): a 2,048-token scan of
 // 64 heads x 128 rows x 64 lanes 0.97 against 0.86 ms, 64 single tokens 0.117 against 0.067 ms.  RG = 16: that scan 0.86
 // against 0.79 ms (with the unrolled loop), the delta rule of 16 heads x 128 x 128 1.15 against 1.34 ms (its 64 blocks
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kScanThreads)
                     const float* __restrict__ A_log, const float* __restrict__ D, float* __restrict__ y, long long y_stride,
                     int heads, int groups, int N, int dv, const int* __restrict__ cu_seqlens, const int* __restrict__ slot_of_seq,
                     const int* __restrict__ start_pos, float* __restrict__ state, long long slot_stride, long long copy_stride,
-                    long long state_off) {
+                    long long state_off, int below) {
     constexpr int NP = RN * RG, kCols = kScanThreads / RG, kRowGroups = RG;
     extern __shared__ __align__(16) float sm[];
     float* Bs = sm;                         // [kChunk][NP]
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(kScanThreads)
     AT* decs = dts + kChunk;                                    // [kChunk]
     const int seq = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kCols;
     const ScanSeq sq = scan_seq(seq, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off);
-    if (sq.n_new <= 0) return;
+    if (sq.n_new <= 0 || sq.n_new >= below) return;
     const int tid = threadIdx.x, col = tid / kRowGroups, rg = tid % kRowGroups;
     const int g = h / (heads / groups);
     const bool live = col0 + col < dv;
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(kScanThreads)
                       const float* __restrict__ dt_bias, const float* __restrict__ A_log, float* __restrict__ o, long long o_stride,
                       int heads, int qk_heads, int dk, int dv, const int* __restrict__ cu_seqlens,
                       const int* __restrict__ slot_of_seq, const int* __restrict__ start_pos, float* __restrict__ state,
-                      long long slot_stride, long long copy_stride, long long state_off) {
+                      long long slot_stride, long long copy_stride, long long state_off, int below) {
     constexpr int NP = RN * RG, kCols = kScanThreads / RG, kRowGroups = RG;
     extern __shared__ __align__(16) float sm[];
     float* ks = sm;                          // [kChunk][NP]
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(kScanThreads)
     float* betas = vs + kChunk * kCols;      // [kChunk]
     const int seq = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kCols;
     const ScanSeq sq = scan_seq(seq, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off);
-    if (sq.n_new <= 0) return;
+    if (sq.n_new <= 0 || sq.n_new >= below) return;
     const int tid = threadIdx.x, col = tid / kRowGroups, rg = tid % kRowGroups;
     const int lane = tid & 31, warp = tid >> 5;
     const int c = h / (heads / qk_heads);
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(kScanThreads)
                       long long a_stride, int a_col0, const float* __restrict__ bias, const float* __restrict__ extra,
                       float* __restrict__ o, long long o_stride, int heads, int dk, int dv, int kind,
                       const int* __restrict__ cu_seqlens, const int* __restrict__ slot_of_seq, const int* __restrict__ start_pos,
-                      float* __restrict__ state, long long slot_stride, long long copy_stride, long long state_off) {
+                      float* __restrict__ state, long long slot_stride, long long copy_stride, long long state_off, int below) {
     constexpr int NP = RN * RG, kCols = kScanThreads / RG, kRowGroups = RG;
     extern __shared__ __align__(16) float sm[];
     float* ks = sm;                          // [kChunk][NP]
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(kScanThreads)
     float* vs = ws + kChunk * NP;            // [kChunk][kCols]
     const int seq = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kCols;
     const ScanSeq sq = scan_seq(seq, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off);
-    if (sq.n_new <= 0) return;
+    if (sq.n_new <= 0 || sq.n_new >= below) return;
     const int tid = threadIdx.x, col = tid / kRowGroups, rg = tid % kRowGroups;
     const bool live = col0 + col < dv;
     const size_t head_off = (size_t)h * RN * dv * kRowGroups;
@@ -644,11 +645,12 @@ static int allow_smem(Kern k, size_t smem, const char* what) {
     return BLM_OK;
 }
 
+// below: sequences of so many new tokens or more are left alone (scan_chunks.cu runs them)
 BLM_API int blm_ssm_scan(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
                          long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                          long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens, const int* slot_of_seq,
                          const int* start_pos, int n_seqs, float* state, long long slot_stride, long long copy_stride,
-                         long long state_off, int wide_sums, cudaStream_t stream) {
+                         long long state_off, int wide_sums, int below, cudaStream_t stream) {
     if (n_seqs == 0) return BLM_OK;
     const int rn = rows_per_thread(N);
     BLM_REQUIRE(rn > 0, "ssm_scan: a state of %d rows; this kernel takes up to %d", N, 32 * 8);
@@ -657,7 +659,7 @@ BLM_API int blm_ssm_scan(const float* xbc, long long xbc_stride, int x_col0, int
     const int rg = row_groups(N), cols = kScanThreads / rg;
     dim3 grid(n_seqs, heads, (dv + cols - 1) / cols);
     const size_t smem = ((size_t)2 * kChunk * rn * rg + kChunk * cols) * sizeof(float) + 2 * kChunk * sizeof(double);
-#define SSM_ARGS xbc, xbc_stride, x_col0, b_col0, c_col0, dt_raw, dt_stride, dt_col0, dt_bias, A_log, D, y, y_stride, heads, groups, N, dv, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off
+#define SSM_ARGS xbc, xbc_stride, x_col0, b_col0, c_col0, dt_raw, dt_stride, dt_col0, dt_bias, A_log, D, y, y_stride, heads, groups, N, dv, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off, below
 #define BLM_SCAN(RN, RG)                                                                                 \
     if (rn == RN && rg == RG && wide_sums) {                                                             \
         int rc = allow_smem(ssm_scan_kernel<RN, RG, double>, smem, "ssm_scan_kernel");                   \
@@ -667,7 +669,7 @@ BLM_API int blm_ssm_scan(const float* xbc, long long xbc_stride, int x_col0, int
     if (rn == RN && rg == RG && !wide_sums) {                                                            \
         int rc = allow_smem(ssm_scan_kernel<RN, RG, float>, smem, "ssm_scan_kernel");                    \
         if (rc != BLM_OK) return rc;                                                                     \
-        ssm_scan_kernel<RN, RG, float><<<grid, kScanThreads, smem, stream>>>(xbc, xbc_stride, x_col0, b_col0, c_col0, dt_raw, dt_stride, dt_col0, dt_bias, A_log, D, y, y_stride, heads, groups, N, dv, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off); \
+        ssm_scan_kernel<RN, RG, float><<<grid, kScanThreads, smem, stream>>>(SSM_ARGS);                  \
     }
     BLM_SCAN(1, 8) BLM_SCAN(2, 8) BLM_SCAN(4, 8) BLM_SCAN(8, 8) BLM_SCAN(16, 8) BLM_SCAN(32, 8)
 #undef BLM_SCAN
@@ -680,7 +682,7 @@ BLM_API int blm_delta_scan(const float* q, long long q_stride, int q_col0, const
                            const float* a_raw, long long a_stride, int a_col0, const float* dt_bias, const float* A_log, float* o,
                            long long o_stride, int heads, int qk_heads, int dk, int dv, const int* cu_seqlens,
                            const int* slot_of_seq, const int* start_pos, int n_seqs, float* state, long long slot_stride,
-                           long long copy_stride, long long state_off, cudaStream_t stream) {
+                           long long copy_stride, long long state_off, int below, cudaStream_t stream) {
     if (n_seqs == 0) return BLM_OK;
     const int rn = rows_per_thread(dk);
     BLM_REQUIRE(rn > 0, "delta_scan: keys of %d lanes; this kernel takes up to %d", dk, 32 * 8);
@@ -693,7 +695,7 @@ BLM_API int blm_delta_scan(const float* q, long long q_stride, int q_col0, const
     if (rn == RN && rg == RG) {                                                                          \
         int rc = allow_smem(delta_scan_kernel<RN, RG>, smem, "delta_scan_kernel");                                   \
         if (rc != BLM_OK) return rc;                                                                     \
-        delta_scan_kernel<RN, RG><<<grid, kScanThreads, smem, stream>>>(q, q_stride, q_col0, k, k_stride, k_col0, v, v_stride, v_col0, b_raw, b_stride, b_col0, a_raw, a_stride, a_col0, dt_bias, A_log, o, o_stride, heads, qk_heads, dk, dv, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off); \
+        delta_scan_kernel<RN, RG><<<grid, kScanThreads, smem, stream>>>(q, q_stride, q_col0, k, k_stride, k_col0, v, v_stride, v_col0, b_raw, b_stride, b_col0, a_raw, a_stride, a_col0, dt_bias, A_log, o, o_stride, heads, qk_heads, dk, dv, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off, below); \
     }
     BLM_SCAN(1, 8) BLM_SCAN(2, 8) BLM_SCAN(4, 8) BLM_SCAN(8, 8) BLM_SCAN(16, 8) BLM_SCAN(32, 8)
 #undef BLM_SCAN
@@ -705,7 +707,7 @@ BLM_API int blm_decay_scan(const float* q, long long q_stride, int q_col0, const
                            const float* bias, const float* extra, float* o, long long o_stride, int heads, int dk, int dv, int kind,
                            int read_first, const int* cu_seqlens, const int* slot_of_seq, const int* start_pos, int n_seqs,
                            float* state, long long slot_stride, long long copy_stride, long long state_off, int wide_sums,
-                           cudaStream_t stream) {
+                           int below, cudaStream_t stream) {
     if (n_seqs == 0) return BLM_OK;
     const int rn = rows_per_thread(dk);
     BLM_REQUIRE(rn > 0, "decay_scan: keys of %d lanes; this kernel takes up to %d", dk, 32 * 8);
@@ -716,7 +718,7 @@ BLM_API int blm_decay_scan(const float* q, long long q_stride, int q_col0, const
     const int rg = row_groups(dk), cols = kScanThreads / rg;
     dim3 grid(n_seqs, heads, (dv + cols - 1) / cols);
     const size_t smem = ((size_t)3 * kChunk * rn * rg + kChunk * cols) * sizeof(float);
-#define DECAY_ARGS q, q_stride, q_col0, k, k_stride, k_col0, v, v_stride, v_col0, a_raw, a_stride, a_col0, bias, extra, o, o_stride, heads, dk, dv, kind, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off
+#define DECAY_ARGS q, q_stride, q_col0, k, k_stride, k_col0, v, v_stride, v_col0, a_raw, a_stride, a_col0, bias, extra, o, o_stride, heads, dk, dv, kind, cu_seqlens, slot_of_seq, start_pos, state, slot_stride, copy_stride, state_off, below
 #define BLM_ONE(RN, RG, FIRST, AT)                                                                       \
     {                                                                                                    \
         int rc = allow_smem(decay_scan_kernel<RN, RG, FIRST, AT>, smem, "decay_scan_kernel");            \

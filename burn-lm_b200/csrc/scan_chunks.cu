@@ -29,9 +29,18 @@ __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v));
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
-// Chunk c of sequence s has the index cu[s] / 16 + s + c: distinct for all chunks, below n_tokens / 16 + n_seqs.
-__host__ __device__ inline int chunk_bound(int n_tokens, int n_seqs) { return n_tokens / kQ + n_seqs; }
-__device__ __forceinline__ int chunk_base(int cu, int seq) { return cu / kQ + seq; }
+// Only sequences of `least` or more new tokens are run (the others are walked token by token: recurrent.cu).  Chunk c of sequence
+// s has the index cu[s] / 16 + s + c, which are distinct and below n_tokens / 16 + n_seqs; beside many short sequences 3 cu[s] /
+// 32 + c, which is below 3 n_tokens / 32: the ceil(n / 16) chunks of n >= 32 tokens are no more than 3 n / 32, rounded down.
+struct Chunks {
+    const int* cu;
+    int n_seqs, least, packed;
+};
+static bool chunks_packed(int n_tokens, int n_seqs, int least) { return least >= 2 * kQ && 3LL * n_tokens / (2 * kQ) < (long long)n_tokens / kQ + n_seqs; }
+static long long chunk_bound(int n_tokens, int n_seqs, int least) {
+    return chunks_packed(n_tokens, n_seqs, least) ? 3LL * n_tokens / (2 * kQ) : (long long)n_tokens / kQ + n_seqs;
+}
+__device__ __forceinline__ int chunk_base(int cu, int seq, int packed) { return packed ? (int)(3LL * cu / (2 * kQ)) : cu / kQ + seq; }
 
 // Floats of one (chunk, head) in scratch: [decayed k for the correction (delta)] [decayed q] [k decayed to the chunk's end]
 // [the chunk's decay], rows of NP (not for the state-space scan, whose rows are shared by heads and read where they lie);
@@ -41,12 +50,12 @@ __host__ __device__ constexpr int small_floats(int kind) { return kMat * (kind =
 __host__ __device__ constexpr int part_floats(int kind, int np) { return rows_floats(kind, np) + small_floats(kind); }
 
 // Which sequence and chunk a chunk index names; false when none.  All threads of the block call it.
-__device__ __forceinline__ bool find_chunk(int idx, const int* __restrict__ cu, int n_seqs, int* found, int& seq, int& chunk) {
+__device__ __forceinline__ bool find_chunk(int idx, const Chunks& ch, int* found, int& seq, int& chunk) {
     if (threadIdx.x == 0) found[0] = -1;
     __syncthreads();
-    for (int s = threadIdx.x; s < n_seqs; s += blockDim.x) {
-        const int lo = cu[s], n = cu[s + 1] - lo, base = chunk_base(lo, s);
-        if (n > 0 && idx >= base && idx < base + (n + kQ - 1) / kQ) {
+    for (int s = threadIdx.x; s < ch.n_seqs; s += blockDim.x) {
+        const int lo = ch.cu[s], n = ch.cu[s + 1] - lo, base = chunk_base(lo, s, ch.packed);
+        if (n >= ch.least && idx >= base && idx < base + (n + kQ - 1) / kQ) {
             found[0] = s;
             found[1] = idx - base;
         }
@@ -91,8 +100,8 @@ struct RowsIn {                    // a column range of a float32 [N, *] tensor
 struct PrepArgs {
     RowsIn q, k, a, b;
     const float *bias, *extra, *A_log;
-    const int* cu;
-    int n_seqs, heads, qk_heads, dk;
+    Chunks ch;
+    int heads, qk_heads, dk;
     float* scratch;
 };
 
@@ -113,8 +122,8 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
     __shared__ float As[kQ][kMs], Cs[kQ][kMs], Ts[kQ][kMs], betas[kQ];
     const int h = blockIdx.y, r = threadIdx.x, lane = r & 31, warp = r >> 5;
     int seq, chunk;
-    if (!find_chunk(blockIdx.x, a.cu, a.n_seqs, found, seq, chunk)) return;
-    const int first = a.cu[seq] + chunk * kQ, nt = min(kQ, a.cu[seq + 1] - first);
+    if (!find_chunk(blockIdx.x, a.ch, found, seq, chunk)) return;
+    const int first = a.ch.cu[seq] + chunk * kQ, nt = min(kQ, a.ch.cu[seq + 1] - first);
     const int c = h / (a.heads / a.qk_heads);
     float w[kQ], kk[kQ], qq[kQ];
     const bool live = r < a.dk;
@@ -305,8 +314,8 @@ struct SsmPrepArgs {
     RowsIn x, dt;                  // x names the tensor; B at b_col0, C at c_col0
     int b_col0, c_col0;
     const float *dt_bias, *A_log, *D;
-    const int* cu;
-    int n_seqs, heads, groups, N;
+    Chunks ch;
+    int heads, groups, N;
     float* scratch;
 };
 
@@ -318,8 +327,8 @@ __global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
     const int g = blockIdx.y / tiles, h0 = g * per + blockIdx.y % tiles * kSsmHeads, nh = min(kSsmHeads, (g + 1) * per - h0);
     const int tid = threadIdx.x, j = tid >> 4, i = tid & 15;
     int seq, chunk;
-    if (!find_chunk(blockIdx.x, a.cu, a.n_seqs, found, seq, chunk)) return;
-    const int first = a.cu[seq] + chunk * kQ, nt = min(kQ, a.cu[seq + 1] - first);
+    if (!find_chunk(blockIdx.x, a.ch, found, seq, chunk)) return;
+    const int first = a.ch.cu[seq] + chunk * kQ, nt = min(kQ, a.ch.cu[seq + 1] - first);
     if (tid < kSsmHeads * kQ) {
         const int hh = tid >> 4, t = tid & 15;
         float dt = 0.f, dec = 1.f;             // a token beyond the chunk's end changes nothing
@@ -391,7 +400,8 @@ struct WalkArgs {
     float* y;
     long long y_stride;
     int heads, dv, vec;            // vec: B and C can be copied in 16-byte pieces
-    const int *cu, *slot_of_seq, *start_pos;
+    Chunks ch;
+    const int *slot_of_seq, *start_pos;
     float* state;
     long long slot_stride, copy_stride, state_off;
 };
@@ -506,9 +516,9 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
     extern __shared__ __align__(16) float sm[];
     float* Ws = sm + kStages * kStage;               // delta: v - acc, then the corrected values, [2][16][CT]
     const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
-    const int first = a.cu[seq], n_new = a.cu[seq + 1] - first;
-    if (n_new <= 0) return;
-    const int chunks = (n_new + kQ - 1) / kQ, base = chunk_base(first, seq), start = a.start_pos[seq];
+    const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
+    if (n_new < a.ch.least) return;
+    const int chunks = (n_new + kQ - 1) / kQ, base = chunk_base(first, seq, a.ch.packed), start = a.start_pos[seq];
     const int tid = threadIdx.x;
 
     if (tid >= kWalkers) {                     // the loading warp, two chunks ahead of the others
@@ -754,29 +764,30 @@ static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
 }
 
 // Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows).
-BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs) {
+BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
     const int np = padded_rows(rows);
     if (np < 32 || np > 256 || kind < kSsm || kind > kDelta) return 0;
-    return (long long)chunk_bound(n_tokens, n_seqs) * heads * part_floats(kind, np);
+    return chunk_bound(n_tokens, n_seqs, least) * heads * part_floats(kind, np);
 }
 
-static int check_step(int n_tokens, int n_seqs, int heads) {
-    BLM_REQUIRE(heads > 0 && heads <= 65535 && n_seqs <= 65535 && n_tokens > 0, "scan_chunks: %d heads, %d sequences", heads, n_seqs);
+static int check_step(int n_tokens, int n_seqs, int heads, int least) {
+    BLM_REQUIRE(heads > 0 && heads <= 65535 && n_seqs <= 65535 && n_tokens > 0 && least > 0, "scan_chunks: %d heads, %d sequences", heads, n_seqs);
     return BLM_OK;
 }
 
 BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
                                 long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                                 long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
-                                const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, float* state,
+                                const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, float* state,
                                 long long slot_stride, long long copy_stride, long long state_off, float* scratch, cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0 && dv > 0, "scan_chunks: bad head counts");
-    if (int rc = check_step(n_tokens, n_seqs, heads)) return rc;
+    if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
+    const Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least)};
     const int np = padded_rows(N), per = heads / groups;
-    SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, cu_seqlens, n_seqs, heads,
-                     groups, N, scratch};
-    prep_ssm_kernel<<<dim3(chunk_bound(n_tokens, n_seqs), groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
+    SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
+                     scratch};
+    prep_ssm_kernel<<<dim3(chunk_bound(n_tokens, n_seqs, least), groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
     if (int rc = blm_check_launch("scan_chunks (state-space scan)")) return rc;
     WalkArgs a = {};
     a.v = {xbc, xbc_stride, x_col0};
@@ -792,7 +803,7 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
     a.heads = heads;
     a.dv = dv;
     a.vec = ((size_t)xbc & 15) == 0 && xbc_stride % 4 == 0 && b_col0 % 4 == 0 && c_col0 % 4 == 0 && N % 4 == 0;
-    a.cu = cu_seqlens;
+    a.ch = ch;
     a.slot_of_seq = slot_of_seq;
     a.start_pos = start_pos;
     a.state = state;
@@ -824,19 +835,20 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
                                  const float* a_raw, long long a_stride, int a_col0, const float* bias, const float* extra,
                                  const float* A_log, float* o, long long o_stride, int heads, int qk_heads, int dk, int dv,
                                  int lower_bound, int read_first, const int* cu_seqlens, const int* slot_of_seq, const int* start_pos,
-                                 int n_tokens, int n_seqs, float* state, long long slot_stride, long long copy_stride,
+                                 int n_tokens, int n_seqs, int least, float* state, long long slot_stride, long long copy_stride,
                                  long long state_off, float* scratch, cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(qk_heads > 0 && heads % qk_heads == 0 && dk > 0 && dv > 0, "scan_chunks: bad head counts");
-    if (int rc = check_step(n_tokens, n_seqs, heads)) return rc;
+    if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
+    const Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least)};
     const bool delta = b_raw != nullptr;
     BLM_REQUIRE(delta ? k != nullptr && A_log != nullptr && !read_first && !lower_bound : (k != nullptr || lower_bound), "scan_chunks: no keys");
     BLM_REQUIRE(!lower_bound || (extra != nullptr && !read_first), "scan_chunks: a lower bound, and the state read last");
     const int np = padded_rows(dk);
     PrepArgs p = {{q, q_stride, q_col0}, {k, k_stride, k_col0}, {a_raw, a_stride, a_col0}, {b_raw, b_stride, b_col0}, bias, extra, A_log,
-                  cu_seqlens, n_seqs, heads, qk_heads, dk, scratch};
+                  ch, heads, qk_heads, dk, scratch};
     const int mode = delta ? kModeDelta : (lower_bound ? kModeLower : (read_first ? kModeExpFirst : kModeExp));
-    const dim3 grid(chunk_bound(n_tokens, n_seqs), heads);
+    const dim3 grid(chunk_bound(n_tokens, n_seqs, least), heads);
     int rc = BLM_OK;
     switch (np) {
         case 32: rc = prep<32>(p, mode, grid, stream); break;
@@ -853,7 +865,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     a.y_stride = o_stride;
     a.heads = heads;
     a.dv = dv;
-    a.cu = cu_seqlens;
+    a.ch = ch;
     a.slot_of_seq = slot_of_seq;
     a.start_pos = start_pos;
     a.state = state;

@@ -76,6 +76,7 @@ class Engine:
         # decode steps (one token each, its logits wanted) replay a CUDA graph when every part allows it
         self.use_graphs = (all(getattr(p, "graph_safe", False) for p in model.parts())
                            and all(getattr(layer.block, "graph_safe", False) for layer in model.layers))
+        self._scans = "scan_chunks" in model.kernel_modules()       # some part carries a matrix state
         self._staging_free = None
         self.decode_ahead = False           # decode_greedy(more=True) may enqueue the following step at once
         self._ahead = None                  # decode_graph.StepInFlight: a greedy step enqueued before it was asked for
@@ -324,13 +325,14 @@ class Engine:
             for slot, new_len in growth:
                 self.cache.set_length(slot, new_len)
             return logits
+        scan_runs = K.scan_runs([b - a for a, b in zip(cu, cu[1:])]) if self._scans else None
         if self.use_graphs:
             # short prompt steps: the same launches at a bucket's sizes, replayed as a graph from its second use
             from .prefill_graph import bucket_of
             bucket = bucket_of(len(tokens), len(entries), max_q, len(want_rows))
             if bucket is not None:
                 graphs = self._prefill_graphs
-                logits = graphs.get(bucket).run(tokens, token_seq, token_pos, cu, slots, starts, want_rows, graphs.pool)
+                logits = graphs.get(bucket, scan_runs).run(tokens, token_seq, token_pos, cu, slots, starts, want_rows, graphs.pool)
                 for slot, new_len in growth:
                     self.cache.set_length(slot, new_len)
                 return logits
@@ -340,7 +342,7 @@ class Engine:
             n_tokens=len(tokens), n_seqs=len(entries), max_q_len=max_q, max_kv_len=max_kv,
             tokens=d_tokens, token_seq=d_seq, token_pos=d_pos, cu_seqlens=d_cu, slot_of_seq=d_slots,
             start_pos=d_starts, want_rows=d_want if want_rows else None, n_want=len(want_rows),
-            workspace=self.workspace,
+            workspace=self.workspace, scan_runs=scan_runs,
             host={"cu_seqlens": cu, "slots": slots, "start_pos": starts})
         logits = self.model.forward(ctx, self.cache)
         for slot, new_len in growth:

@@ -14,6 +14,9 @@ and what the rounding adds changes no result:
     attention kernels finds a query row in them;
   * wanted rows after the last repeat the last one and are cut from the result.
 
+The matrix-state scans run every sequence by its own length, which they read on the device; whether a step has long ones, short
+ones or both is part of a graph's key for models that have such scans, so that no step launches a kernel without work.
+
 What a step brings goes through one pinned buffer and one copy into device buffers with fixed
 addresses, as for the decode graphs.  A bucket's first step runs the same padded launches plainly
 (which also loads every kernel it needs); its second step captures them; from then on a step is
@@ -65,7 +68,7 @@ def bucket_of(n_tokens: int, n_seqs: int, max_q_len: int, n_want: int) -> Option
 class PrefillGraph:
     """The launches of one bucket's step, with the device buffers they read."""
 
-    def __init__(self, engine, bucket: tuple):
+    def __init__(self, engine, bucket: tuple, scan_runs: Optional[tuple] = None):
         self._engine = weakref.ref(engine)
         self.bucket = bucket
         t, s, q, w = bucket
@@ -84,6 +87,7 @@ class PrefillGraph:
             tokens=views[0], token_seq=views[1], token_pos=views[2], cu_seqlens=views[3], slot_of_seq=views[4],
             start_pos=views[5], want_rows=views[6] if w else None, n_want=w,
             workspace=Workspace(dev),       # its own: a captured graph keeps the addresses it saw
+            scan_runs=scan_runs,
             host={"cu_seqlens": None, "slots": None, "start_pos": None})
         self._graph = None
         self._captured = None
@@ -132,16 +136,19 @@ class PrefillGraphs:
         self._graphs: "OrderedDict[tuple, PrefillGraph]" = OrderedDict()
         self._pool = None
 
-    def get(self, bucket: tuple) -> PrefillGraph:
-        g = self._graphs.get(bucket)
+    def get(self, bucket: tuple, scan_runs: Optional[tuple] = None) -> PrefillGraph:
+        """`scan_runs`: which of the two ways of a matrix-state scan the step has work for; a graph holds the launches of
+        those alone (a model without such scans: None)."""
+        key = (bucket, scan_runs)
+        g = self._graphs.get(key)
         if g is None:
             if self._pool is None:
                 # one memory pool for all of them: they run one after another and keep nothing between steps
                 self._pool = torch.cuda.graph_pool_handle()
-            g = self._graphs[bucket] = PrefillGraph(self._engine(), bucket)
+            g = self._graphs[key] = PrefillGraph(self._engine(), bucket, scan_runs)
             while len(self._graphs) > MAX_GRAPHS:
                 self._graphs.popitem(last=False)
-        self._graphs.move_to_end(bucket)
+        self._graphs.move_to_end(key)
         return g
 
     @property

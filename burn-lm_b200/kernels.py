@@ -127,14 +127,14 @@ _protos = {
                           c_int, c_void_p, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
         "blm_decay_scan": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong,
                            c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                           c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
+                           c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p],
         "blm_ssm_scan": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                         c_longlong, c_longlong, c_longlong, c_int, c_void_p],
+                         c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p],
         "blm_delta_scan": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p,
                            c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int,
                            c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong, c_longlong,
-                           c_void_p],
+                           c_int, c_void_p],
         "blm_selective_scan": [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p, c_int, c_int,
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_longlong, c_float, c_int, c_int,
                                c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_longlong, c_longlong, c_longlong, c_void_p],
@@ -143,14 +143,14 @@ _protos = {
                                  c_float, c_void_p, c_int, c_longlong, c_int, c_void_p],
     },
     "scan_chunks": {
-        "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int],
+        "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int, c_int],
         "blm_scan_chunks_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
-                                c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+                                c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
         "blm_scan_chunks_rows": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p,
                                  c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong,
-                                 c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p,
-                                 c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+                                 c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                 c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     },
     "retention": {
         "blm_retention_scan": _RETENTION + [c_void_p, c_longlong, c_void_p],
@@ -1364,22 +1364,37 @@ def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, sta
           kernels=2 if k > 1 and not single else 1)
 
 
-# From this many new tokens of a sequence on, a step's recurrences run in chunks of sixteen tokens (scan_chunks.cu): the two
-# launches cost what walking some 24 tokens does (a part of 2,048 lanes, chunks against the walk: 16 tokens 56 / 51 us for the
-# state-space scan, 32 / 33 for the lower-bounded decay; 32 tokens 52 / 52 and 28 / 38; 64 tokens 61 / 73 and 30 / 57).  A single
-# token costs a chunk all the same (64 of them: 241 / 121 and 104 / 53 us), so steps that are mostly single tokens are walked.
+# From this many new tokens on, a sequence's recurrence runs in chunks of sixteen tokens (scan_chunks.cu), below it token by token
+# (recurrent.cu), each by its own length, whatever shares the step.  Chunks against the walk, us on the device, sequences of
+# 24 / 32 / 64 tokens: state-space scan of 64 heads of 128 x 64, one 17 / 12, 16 / 15, 20 / 27, sixteen 88 / 77, 88 / 98, 133 / 188;
+# delta rule of 16 heads of 128 x 128, one 15 / 19, 15 / 24, 18 / 45, sixteen 78 / 64, 78 / 83, 128 / 159; WKV of 32 heads of 128 x
+# 128, one 13 / 18, 13 / 23, 17 / 43, sixteen 83 / 106, 85 / 139, 133 / 290.  A single token costs a chunk all the same (255 of them
+# beside 64 tokens 899 / 260 for the state-space scan), and beside many of them the chunks of a long prompt are still the faster
+# way for that prompt.
 SCAN_CHUNK_TOKENS = 32
-SCAN_CHUNK_MEAN = 4
 _SCAN_SSM, _SCAN_DECAY, _SCAN_DELTA = 0, 1, 2
+_NO_LIMIT = (1 << 31) - 1
 
 
-def _scan_chunks_scratch(kind, heads, rows, step, device):
-    """Scratch for a step whose recurrence runs in chunks, or None where it is walked token by token: single tokens and
-    short portions, states of up to 16 rows."""
-    if getattr(step, "max_q_len", 0) < SCAN_CHUNK_TOKENS or step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs:
-        return None
-    floats = int(_lib("scan_chunks").blm_scan_chunks_scratch(kind, heads, rows, step.n_tokens, step.n_seqs))
-    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
+def scan_runs(lengths) -> tuple:
+    """What a step's new tokens by sequence bring the matrix-state scans: (some sequence is run in chunks, some is walked)."""
+    return max(lengths, default=0) >= SCAN_CHUNK_TOKENS, min(lengths, default=0) < SCAN_CHUNK_TOKENS
+
+
+def _scan_route(kind, heads, rows, step, device):
+    """How a step's recurrence runs: (scratch of the chunk kernels, or None without them; the length from which they run a
+    sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
+    its own length, which the kernels read; step.scan_runs says which of the two have work (the engine's steps know)."""
+    longest = getattr(step, "max_q_len", 0)
+    # (a step that does not know and brings 64 tokens a sequence and more on average: short ones are few if any, and cost a chunk each)
+    known = getattr(step, "scan_runs", None)
+    in_chunks, walked = known or (True, step.n_tokens < 2 * SCAN_CHUNK_TOKENS * step.n_seqs and (step.n_seqs > 1 or step.n_tokens != longest))
+    if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
+        least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
+        floats = int(_lib("scan_chunks").blm_scan_chunks_scratch(kind, heads, rows, step.n_tokens, step.n_seqs, least))
+        if floats:
+            return torch.empty(floats, dtype=torch.float32, device=device), least, SCAN_CHUNK_TOKENS if walked else 0
+    return None, 0, _NO_LIMIT
 
 
 def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y, heads, groups, n_state, value_dim, step, state,
@@ -1397,15 +1412,16 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     dp, ds, dc = _cols(dt, dt_col0, heads)
     if tuple(y.shape) != (step.n_tokens, heads * value_dim) or not y.is_contiguous():
         raise KernelError("ssm_scan: y float32 [N, heads * value_dim]")
-    scratch = None if wide_sums else _scan_chunks_scratch(_SCAN_SSM, heads, n_state, step, y.device)
+    scratch, least, below = (None, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+    if below == 0:
         return
     _call("recurrent", "blm_ssm_scan", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
           _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-          _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, _stream())
+          _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, below, _stream())
 
 
 def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a_log, out, heads, qk_heads, key_dim, value_dim,
@@ -1423,15 +1439,16 @@ def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a
     aa = _cols(a, a_col0, heads * key_dim)
     if tuple(out.shape) != (step.n_tokens, heads * value_dim) or not out.is_contiguous() or dt_bias.numel() != heads * key_dim:
         raise KernelError("delta_scan: out float32 [N, heads * value_dim], dt_bias [heads * key_dim]")
-    scratch = _scan_chunks_scratch(_SCAN_DELTA, heads, key_dim, step, out.device)
+    scratch, least, below = _scan_route(_SCAN_DELTA, heads, key_dim, step, out.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(None), _ptr(a_log), _ptr(out),
               c_longlong(out.stride(0)), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+    if below == 0:
         return
     _call("recurrent", "blm_delta_scan", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(a_log), _ptr(out), c_longlong(out.stride(0)),
           heads, qk_heads, key_dim, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_seqs,
-          *_state_args(state, state_offset), _stream())
+          *_state_args(state, state_offset), below, _stream())
 
 
 def shift_mix(x, mu, out, step, state, state_offset):
@@ -1472,16 +1489,17 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
         raise KernelError("decay_scan: out float32 [N, heads * value_dim], bias [heads * key_dim]")
     if extra is not None and extra.numel() != heads * key_dim:
         raise KernelError("decay_scan: extra [heads * key_dim]")
-    scratch = None if wide_sums else _scan_chunks_scratch(_SCAN_DECAY, heads, key_dim, step, out.device)
+    scratch, least, below = (None, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_DECAY, heads, key_dim, step, out.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, c_void_p(0), c_longlong(0), 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
               _ptr(out), c_longlong(out.stride(0)), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
-              1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs,
+              1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs, least,
               *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+    if below == 0:
         return
     _call("recurrent", "blm_decay_scan", *qa, *ka, *va, *aa, _ptr(bias), _ptr(extra), _ptr(out), c_longlong(out.stride(0)), heads,
           key_dim, value_dim, int(kind), 1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos),
-          step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, _stream())
+          step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, below, _stream())
 
 
 GATE_FIRST, GATE_LAST, GATE_SILU_LAST, GATE_NONE = 0, 1, 2, 3

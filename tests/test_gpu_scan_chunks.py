@@ -157,3 +157,79 @@ def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(kind, where, hea
         assert torch.equal(out[:bad], clean[:bad])
         assert not torch.isfinite(out[bad]).any()
         assert torch.isfinite(own[int(step.slot_of_seq[0])]).all() and not torch.isfinite(own[int(step.slot_of_seq[1]), (3 + 35) & 1]).all()
+
+
+def scan_of(kind, heads, rows, dv, n, gen):
+    """run(rows of the inputs, out, step, state) of a recurrence on drawn inputs of n tokens."""
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    q, k, v, a, b = rnd(n, heads * rows), rnd(n, heads * rows), rnd(n, heads * dv), rnd(n, heads * rows), rnd(n, heads)
+    bias, extra, per_head = rnd(heads * rows), torch.rand(heads * rows, generator=gen, device="cuda"), [rnd(heads) for _ in range(3)]
+    x = torch.cat([v, k, q], 1)
+    if kind == "ssm":
+        return lambda sl, out, step, state: K.ssm_scan(x[sl], 0, heads * dv, heads * (dv + rows), b[sl], 0, *per_head, out, heads, heads, rows,
+                                                       dv, step, state, 0)
+    if kind == "delta":
+        return lambda sl, out, step, state: K.delta_scan(q[sl], 0, k[sl], 0, v[sl], 0, b[sl], 0, a[sl], 0, bias, per_head[0], out, heads, heads,
+                                                         rows, dv, step, state, 0)
+    exp = kind == "wkv"
+    return lambda sl, out, step, state: K.decay_scan(q[sl], 0, k[sl] if exp else None, 0, v[sl], 0, a[sl], 0, bias, extra, out, heads, rows, dv,
+                                                     K.DECAY_EXP_EXP if exp else K.DECAY_LOWER_BOUND, exp, step, state, 0)
+
+
+@pytest.mark.parametrize("lens", [[1, 1, 1, 40, 1, 20, 0, 35, 0], [31, 32, 33], [1] * 15 + [4], [0, 64, 1]])
+@pytest.mark.parametrize("heads,rows,dv", [(3, 64, 64), (2, 128, 100)])
+@pytest.mark.parametrize("kind", ["ssm", "wkv", "lower", "delta"])
+def test_a_sequence_runs_by_its_own_length_whatever_shares_the_step(kind, heads, rows, dv, lens):
+    """In a step of a captured size (rows and sequences behind the real ones, a longest run that is rounded up), every sequence's
+    outputs and state are the bits that it has alone: short ones walked, long ones in chunks."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(len(lens) + rows)
+    starts = [(5 * s) % 7 for s in range(len(lens))]
+    real, n = step_of(lens, starts), -(-sum(lens) // 64) * 64
+    run = scan_of(kind, heads, rows, dv, n, gen)
+    state = state_of(real, heads, rows, dv, 0, gen)
+    pad = lambda t, m, v: torch.cat([t, torch.full((m,), v, dtype=torch.int32, device="cuda")])
+    more = 16 - len(lens)
+    step = SimpleNamespace(cu_seqlens=pad(real.cu_seqlens, more, sum(lens)), slot_of_seq=pad(real.slot_of_seq, more, int(real.slot_of_seq[-1])),
+                           start_pos=pad(real.start_pos, more, starts[-1]), n_tokens=n, n_seqs=16, max_q_len=min(n, 128))
+    scratch, least, below = K._scan_route(K._SCAN_SSM, heads, rows, step, "cuda")
+    assert scratch is not None and least == below == K.SCAN_CHUNK_TOKENS
+    got, got_state = torch.full((n, heads * dv), 7.0, device="cuda"), state.clone()
+    run(slice(0, n), got, step, got_state)
+    want_state, at = state.clone(), 0
+    for s, m in enumerate(lens):
+        if m == 0:
+            continue
+        own = step_of([m], [starts[s]])
+        own.slot_of_seq = real.slot_of_seq[s:s + 1]
+        assert (K._scan_route(K._SCAN_SSM, heads, rows, own, "cuda")[0] is not None) == (m >= K.SCAN_CHUNK_TOKENS)
+        out = torch.empty((m, heads * dv), device="cuda")
+        run(slice(at, at + m), out, own, want_state)
+        assert torch.equal(got[at:at + m], out), s
+        at += m
+    assert torch.equal(got_state, want_state)
+    assert (got[at:] == 7.0).all()                                            # rows of no sequence are left alone
+
+
+def test_the_engine_launches_the_scans_that_have_work(tmp_path, monkeypatch):
+    from burn_lm_b200 import StepEntry
+    from nufolix_tiny import NUF_D, make_folder
+    from burn_lm_b200.engine.engine import Engine
+    folder, calls, plain = make_folder(tmp_path, "nuf_d"), [], K._call
+
+    def watching(module, name, *args, **kw):
+        calls.append(name)
+        return plain(module, name, *args, **kw)
+
+    monkeypatch.setattr(K, "_call", watching)
+    engine = Engine.from_folder(folder, "bfloat16", max_tokens=64 * 64, max_seqs=20)
+    slots = [engine.acquire() for _ in range(16)]
+    engine.step([StepEntry(s, [1, 2, 3, 4, 5], [0]) for s in slots])          # (another bucket than those below)
+    chunked = lambda: [n for n in calls if n.startswith("blm_scan_chunks_")]
+    walked = lambda: [n for n in calls if n in ("blm_ssm_scan", "blm_delta_scan")]
+    for lengths, in_chunks, by_walk in (([1] * 15 + [4], False, True), ([20], False, True), ([1] * 15 + [300], True, True), ([40, 33], True, False),
+                                        ([1] * 15 + [4], False, True)):
+        calls.clear()
+        logits = engine.step([StepEntry(s, [t % NUF_D["vocab"] for t in range(m)], [m - 1]) for s, m in zip(slots, lengths)])
+        assert bool(chunked()) == in_chunks and bool(walked()) == by_walk, lengths
+        assert bool(torch.isfinite(logits).all())
