@@ -542,10 +542,7 @@ def ridopel_kernels(z, pk):
         o = torch.empty_like(q)
         ms_llama = _time(lambda: K.attention(q, q.shape[1], pool5, bt, st.cu_seqlens, st.slot_of_seq, st.start_pos, o, n, n_seqs, new,
                                              H, G, hd, hd ** -0.5, window=0, n_splits=1, max_kv_len=total))
-        # the key shares the mixer takes at this size (parts.latent_attention.LatentAttention._splits)
-        tile = K.latent_attention_tile_rows(bf, H, R, dr, new)
-        tiles = (new * H + tile - 1) // tile * n_seqs
-        splits = max(1, min(K.sm_count() // tiles, total // (2 * K.PAGE), 32))
+        splits = K.latent_attention_splits(bf, H, R, dr, n_seqs, new, total, torch.device(dev))      # the key shares the mixer takes at this size
         pool = torch.randn((n_seqs * pages_each, K.PAGE, R + dr), dtype=bf, device=dev)
         q_lat = torch.randn((H, n, R), dtype=torch.float32, device=dev) * 0.1
         q_rot = torch.randn((n, H, dr), dtype=torch.float32, device=dev)
@@ -703,10 +700,7 @@ def marinex_kernels(z, pk):
                                                 head_scale=temp, softcap=30.0))
         ms_plain = _time(lambda: K.attention_sink(q, st, pool, bt, o, H, G, hd, hd, hd ** -0.5, 1 << 30, 0, sink=True, max_q_len=new))
         # over the latent, with the window: single tokens on the latent itself, portions on keys and values written out
-        tile = K.latent_attention_tile_rows(bf, H, R, dr, new)
-        tiles = (new * H + tile - 1) // tile * n_seqs
-        seen = min(total, W + new)
-        splits = max(1, min(K.sm_count() // tiles, seen // (2 * K.PAGE), 32))
+        splits = K.latent_attention_splits(bf, H, R, dr, n_seqs, new, min(total, W + new), torch.device(dev))
         lpool = torch.randn((n_seqs * pages_each, K.PAGE, R + dr), dtype=bf, device=dev)
         if new < 16:
             q_lat = torch.randn((H, n, R), dtype=torch.float32, device=dev) * 0.1

@@ -565,6 +565,11 @@ BLM_API int blm_latent_attention_tile_rows(int dtype, int H, int R, int dr, int 
     if (!latent_takes_mma(dtype, R, dr)) return kTM;
     return (long long)max_q_len * H > 16 && lat::smem_bytes(32, R + dr, 32, 1) <= lat::kRoom ? 32 : 16;
 }
+// blocks that fit a multiprocessor, and that a step should offer it: one of the tensor cores' sixteen warps, which take its shared
+// memory, or two of the CUDA cores' eight
+BLM_API int blm_latent_attention_blocks(int dtype, int R, int dr) {
+    return latent_takes_mma(dtype, R, dr) && lat::smem_bytes(16, R + dr, 32, 1) <= lat::kRoom ? 1 : 2;
+}
 
 // the shares of a row's keys, merged in the order of the shares
 template <typename TO>

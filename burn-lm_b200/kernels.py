@@ -186,6 +186,7 @@ _protos = {
                                  c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p,
                                  c_void_p],
         "blm_latent_attention_tile_rows": [c_int, c_int, c_int, c_int, c_int],
+        "blm_latent_attention_blocks": [c_int, c_int, c_int],
         "blm_sigmoid_gate": [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p],
     },
     "moe": {
@@ -1800,6 +1801,15 @@ def latent_attention_tile_rows(dtype, n_heads, rank, rot_dim, max_q_len) -> int:
     """How many rows (new token x head) a block of latent_attention owns at these sizes: 16 on the CUDA cores, 16 or 32
     on the tensor cores (a bfloat16 cache whose latent and rotated part are multiples of 16 lanes, up to 512)."""
     return int(_lib("attention_latent").blm_latent_attention_tile_rows(_code(dtype), n_heads, rank, rot_dim, max_q_len))
+
+
+def latent_attention_splits(dtype, n_heads, rank, rot_dim, n_seqs, max_q_len, keys, device) -> int:
+    """Over how many blocks a row's keys are cut: a few tokens with many keys leave most multiprocessors idle otherwise.  No more
+    than one round of blocks, and every block should still have a few pages of the longest sequence's `keys`."""
+    rows = latent_attention_tile_rows(dtype, n_heads, rank, rot_dim, max_q_len)
+    tiles = (max_q_len * n_heads + rows - 1) // rows * n_seqs
+    blocks = int(_lib("attention_latent").blm_latent_attention_blocks(_code(dtype), rank, rot_dim)) * sm_count(device)
+    return max(1, min(blocks // tiles, keys // (2 * PAGE), 32))
 
 
 def latent_attention(q_lat, q_rot, pool, block_table, step, out, n_heads, rank, rot_dim, scale, n_splits=1, partial=None,

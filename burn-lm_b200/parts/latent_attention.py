@@ -40,7 +40,6 @@ from ..weights.loader import TensorSpec
 from .base import CacheNeed, Part
 from .linear import Linear
 
-BLOCKS_PER_SM = 1     # blocks of the attention kernel a step should offer every multiprocessor (a block fills one)
 EXPAND_TOKENS = 16    # from this many new tokens of a sequence on, a bfloat16 step writes out keys and values of the heads
 EXPAND_SPAN = 4       # ... with a window only while the longest sequence is at most this many times (new tokens + window) long
 NO_WINDOW = 1 << 30   # what the windowed family's kernels take for "every earlier key"
@@ -156,14 +155,10 @@ class LatentAttention(Part):
             K.sigmoid_gate(heads, gate, heads, share=self.spec.value_dim if self.spec.gate_per_head else 1)
 
     def _splits(self, step) -> int:
-        """Over how many blocks a row's keys are cut: a few tokens with many keys leave most multiprocessors idle
-        otherwise.  Every block should still have a few pages."""
-        s = self.spec
-        rows = K.latent_attention_tile_rows(self.runtime.dtype, s.n_heads, s.rank, s.rot_dim, step.max_q_len)
-        tiles = (step.max_q_len * s.n_heads + rows - 1) // rows * step.n_seqs
-        want = BLOCKS_PER_SM * K.sm_count(self.runtime.device)
+        """Over how many blocks a row's keys are cut."""
+        s, rt = self.spec, self.runtime
         seen = step.max_kv_len if s.window is None else min(step.max_kv_len, s.window + step.max_q_len)
-        return max(1, min(want // tiles, seen // (2 * K.PAGE), 32))                # no block left over for a second round
+        return K.latent_attention_splits(rt.dtype, s.n_heads, s.rank, s.rot_dim, step.n_seqs, step.max_q_len, seen, rt.device)
 
     def forward(self, x, step, cache):
         s, rt = self.spec, self.runtime

@@ -82,3 +82,16 @@ def test_weights_are_kept_to_sixteen_bits(H, R, dr, splits):
     terms = torch.einsum("nht,ntd->nhd", p, seen[..., :R].abs()).transpose(0, 1)
     # two bfloat16 numbers round a weight by 2^-17; fp32 scores of up to 10 and their exponentials by some 2^-19
     assert ((out.double() - want).abs() <= 2.0 ** -15 * terms).all()
+
+
+@pytest.mark.parametrize("dtype,rank,rot,blocks", [(torch.bfloat16, 512, 64, 1), (torch.float32, 512, 64, 2), (torch.bfloat16, 500, 64, 2),
+                                                   (torch.bfloat16, 640, 64, 2)])
+@pytest.mark.parametrize("n_seqs", [1, 7, 32])
+def test_shares_offer_every_multiprocessor_the_blocks_it_holds(dtype, rank, rot, blocks, n_seqs):
+    """One block of the tensor-core kernel fills a multiprocessor, two of the CUDA-core kernel do (32-bit caches, ranks that are no
+    multiples of 16 lanes or too long)."""
+    heads, dev = 32, torch.device("cuda")
+    splits = K.latent_attention_splits(dtype, heads, rank, rot, n_seqs, 1, 1 << 20, dev)
+    tiles = -(-heads // K.latent_attention_tile_rows(dtype, heads, rank, rot, 1)) * n_seqs
+    most = blocks * K.sm_count(dev)
+    assert splits == 32 and tiles * splits <= most or most - tiles < tiles * splits <= most
