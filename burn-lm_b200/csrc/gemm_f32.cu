@@ -55,14 +55,14 @@ __global__ void __launch_bounds__(TN * TM) gemm_f32_kernel(const GemmArgs a) {
     const int r0 = tid / kPer, c = tid % kPer * P;
     const float* xt = x + (size_t)n0 * a.ldx + k_lo + c;
     const float* wt = w + (size_t)m0 * a.ldw + k_lo + c;
-    int off[VEC ? kPieces : 1];
+    int off[VEC ? kPieces : 1];                // (VEC: a tile's rows lie within 2^31 places, which the caller makes sure of)
     auto offset = [&](int i) {
         const int r = r0 + i * kStep;
-        return (int)(r < BN ? min(r, a.N - 1 - n0) * a.ldx : min(r - BN, a.M - 1 - m0) * a.ldw);
+        return r < BN ? min(r, a.N - 1 - n0) * a.ldx : min(r - BN, a.M - 1 - m0) * a.ldw;
     };
     if (VEC) {
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) off[VEC ? i : 0] = offset(i);
+        for (int i = 0; i < kPieces; ++i) off[VEC ? i : 0] = (int)offset(i);
     }
     auto load = [&](int slice) {
         if (slice < slices) {
@@ -175,7 +175,8 @@ BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int b
     const int shares = shares_of(K);
     BLM_REQUIRE((long long)batch * shares <= 65535 && (long long)batch * N <= 0x7fffffffLL && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
     BLM_REQUIRE(shares == 1 || scratch != nullptr, "gemm_f32: a sum over %d places needs scratch", K);
-    const bool vec = (((size_t)x | (size_t)w) & 15) == 0 && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bx % 4 == 0 && bw % 4 == 0;
+    // 16-byte pieces where every row starts at a multiple of 16 bytes, and 64 rows lie within what an int can tell
+    const bool vec = (((size_t)x | (size_t)w) & 15) == 0 && ldx < (1 << 25) && ldw < (1 << 25) && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bx % 4 == 0 && bw % 4 == 0;
     const GemmArgs a = {x, w, shares > 1 ? scratch : y, N, M, K, shares, batch, ldx, ldw, ldy, bx, bw, by};
     // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights 49 us,
     // with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)

@@ -25,3 +25,15 @@ def test_product_at_the_edges(n, m, k):
     wide[:, 1, :k] = x
     both = K.batched_product(wide[:, :, :k].transpose(0, 1), torch.stack([w, w]), out=torch.empty((n, 2, m), device="cuda").transpose(0, 1))
     assert torch.equal(both[1], y) and not both[0].any()
+
+
+@pytest.mark.parametrize("of", ["x", "w"])
+def test_rows_further_apart_than_an_int_can_tell(of):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    apart = (1 << 31) // 63 // 4 * 4 + 4                                      # the 64th row of a tile lies 2^31 places behind the first
+    wide = torch.empty(63 * apart + 8, device="cuda").as_strided((1, 64, 8), (0, apart, 1))
+    wide.copy_(torch.randn((1, 64, 8), generator=gen, device="cuda"))
+    near = torch.randn((1, 60, 8), generator=gen, device="cuda")
+    x, w = (wide, near) if of == "x" else (near, wide)
+    assert torch.equal(K.batched_product(x, w), K.batched_product(x.contiguous(), w.contiguous()))
