@@ -10,6 +10,8 @@
 // (317 x 2,048 x 8,192: 160 tiles, 1,280 blocks).  Two places of K an instruction (fma.rn.f32x2) ran at the same rate, 8 x 8
 // outputs a thread too (four blocks a multiprocessor hide the loads, two do not).  With 16,384 x 2,048 / 2,048 x 8,192 weights,
 // us: 1 row 189 / 381 -> 48 / 30, 16 rows 189 / 383 -> 49 / 31, 48 rows 192 / 437 -> 101 / 58, 317 rows 703 / 671 -> 497 / 254.
+#include <algorithm>
+
 #include "common.cuh"
 
 BLM_API const char* blm_gemm_last_error() { return g_blm_error; }
@@ -162,35 +164,46 @@ static int launch(const GemmArgs& a, bool vec, cudaStream_t stream) {
 
 static int shares_of(int K) { return (K + kShare - 1) / kShare; }
 
+// Products that one launch takes: the grid's third dimension holds their shares.
+static int products_at_once(int batch, int K) { return std::max(1, std::min(batch, 65535 / std::max(1, shares_of(K)))); }
+
 // Floats of scratch a product needs: a plane of sums a share, none for a single share.
 BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
-    return shares_of(K) > 1 ? (long long)shares_of(K) * batch * N * M : 0;
+    return shares_of(K) > 1 ? (long long)shares_of(K) * products_at_once(batch, K) * N * M : 0;
 }
 
-// `batch` products y[b] = x[b] . W[b]^T of one shape in one launch; the operands of product b lie b * (bx, bw, by) elements on.
+// `batch` products y[b] = x[b] . W[b]^T of one shape; the operands of product b lie b * (bx, bw, by) elements on.
 BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int batch, int N, int M, int K, long long ldx, long long ldw,
                                  long long ldy, long long bx, long long bw, long long by, float* scratch, cudaStream_t stream) {
     if (N == 0 || M == 0 || batch == 0) return BLM_OK;
     BLM_REQUIRE(N > 0 && M > 0 && K > 0 && batch > 0, "gemm_f32: bad sizes %d x %d %d %d", batch, N, M, K);
     const int shares = shares_of(K);
-    BLM_REQUIRE((long long)batch * shares <= 65535 && (long long)batch * N <= 0x7fffffffLL && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
+    BLM_REQUIRE(batch <= 65535 && shares <= 65535 && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
+    const int at_once = products_at_once(batch, K);
+    BLM_REQUIRE(shares == 1 || (long long)at_once * N <= 0x7fffffffLL, "gemm_f32: too many rows or products (%d x %d)", batch, N);
     BLM_REQUIRE(shares == 1 || scratch != nullptr, "gemm_f32: a sum over %d places needs scratch", K);
     // 16-byte pieces where every row starts at a multiple of 16 bytes, and 64 rows lie within what an int can tell
     const bool vec = (((size_t)x | (size_t)w) & 15) == 0 && ldx < (1 << 25) && ldw < (1 << 25) && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bx % 4 == 0 && bw % 4 == 0;
-    const GemmArgs a = {x, w, shares > 1 ? scratch : y, N, M, K, shares, batch, ldx, ldw, ldy, bx, bw, by};
-    // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights 49 us,
-    // with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
-    const int rc = N <= 16   ? launch<4, 16, 4, 2>(a, vec, stream)
-                   : N <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
-                   : N <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
-                             : launch<8, 16, 8, 4>(a, vec, stream);
-    if (rc != BLM_OK || shares == 1) return rc;
     const bool vec4 = (((size_t)y | (size_t)scratch) & 15) == 0 && M % 4 == 0 && ldy % 4 == 0 && by % 4 == 0;
-    const int per = 256 * (vec4 ? 4 : 1);
-    const dim3 grid(batch * N, (M + per - 1) / per);
-    if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(scratch, y, N, M, shares, batch, ldy, by);
-    else add_shares_kernel<1><<<grid, 256, 0, stream>>>(scratch, y, N, M, shares, batch, ldy, by);
-    return blm_check_launch("gemm_f32 (shares)");
+    for (int b0 = 0; b0 < batch; b0 += at_once) {
+        const int products = std::min(at_once, batch - b0);
+        float* to = y + (size_t)b0 * by;
+        const GemmArgs a = {x + (size_t)b0 * bx, w + (size_t)b0 * bw, shares > 1 ? scratch : to, N, M, K, shares, products, ldx, ldw, ldy, bx, bw, by};
+        // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights 49 us,
+        // with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
+        const int rc = N <= 16   ? launch<4, 16, 4, 2>(a, vec, stream)
+                       : N <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
+                       : N <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
+                                 : launch<8, 16, 8, 4>(a, vec, stream);
+        if (rc != BLM_OK) return rc;
+        if (shares == 1) continue;
+        const int per = 256 * (vec4 ? 4 : 1);
+        const dim3 grid(products * N, (M + per - 1) / per);
+        if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(scratch, to, N, M, shares, products, ldy, by);
+        else add_shares_kernel<1><<<grid, 256, 0, stream>>>(scratch, to, N, M, shares, products, ldy, by);
+        if (int added = blm_check_launch("gemm_f32 (shares)")) return added;
+    }
+    return BLM_OK;
 }
 
 BLM_API int blm_gemm_f32(const float* x, const float* w, float* y, int N, int M, int K,

@@ -37,3 +37,14 @@ def test_rows_further_apart_than_an_int_can_tell(of):
     near = torch.randn((1, 60, 8), generator=gen, device="cuda")
     x, w = (wide, near) if of == "x" else (near, wide)
     assert torch.equal(K.batched_product(x, w), K.batched_product(x.contiguous(), w.contiguous()))
+
+
+def test_batches_whose_shares_fill_more_than_one_grid():
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    x, w = (torch.randn(shape, generator=gen, device="cuda") for shape in ((40000, 1, 1030), (40000, 3, 1030)))
+    y = K.batched_product(x, w)                                               # two shares each: 80,000 blocks deep
+    for b in (0, 1, 32766, 32767, 32768, 39999):
+        assert torch.equal(y[b], K.gemm_f32(x[b], w[b])), b
+    want = torch.einsum("bnk,bmk->bnm", x.double(), w.double())
+    assert (y.double() - want).abs().max() <= 4 * 1030 * 2.0 ** -24
