@@ -164,12 +164,46 @@ static int launch(const GemmArgs& a, bool vec, cudaStream_t stream) {
 
 static int shares_of(int K) { return (K + kShare - 1) / kShare; }
 
-// Products that one launch takes: the grid's third dimension holds their shares.
-static int products_at_once(int batch, int K) { return std::max(1, std::min(batch, 65535 / std::max(1, shares_of(K)))); }
+// What one pass of a product takes: products (the grid's third dimension holds their shares), rows, columns.  With several shares a
+// pass is cut so that its planes of sums stay within kPlanes floats (256 MB), in even parts of whole tiles along the longer side
+// (every pass reads the shorter side's operand again): a large product would otherwise hold K / 1,024 times its result (2,048 rows
+// of logits over 128,256 columns and K 4,096: 4.2 GB).  Every pass ends in a round of blocks that
+// is not full: 600 x 32,768 x 4,096 in two passes 3,731 -> 3,776 us, 2,048 x 4,096 x 14,336 5,198 -> 5,229 (in six and eight: 3,842, 5,492).
+constexpr long long kPlanes = 64 << 20;
+struct Pass {
+    int products, rows, cols;
+};
+static Pass pass_of(int batch, int N, int M, int K) {
+    const int shares = shares_of(K);
+    Pass p = {std::max(1, std::min(batch, 65535 / std::max(1, shares))), std::max(1, N), std::max(1, M)};
+    if (shares <= 1) return p;
+    const long long one = (long long)shares * p.rows * p.cols;
+    if (one <= kPlanes) {
+        p.products = (int)std::min<long long>(p.products, kPlanes / one);
+        return p;
+    }
+    p.products = 1;
+    auto cut = [&](int& side, int other) {     // in even parts, as many as it takes, none below a tile
+        const long long parts = ((long long)shares * side * other + kPlanes - 1) / kPlanes;
+        side = (int)std::min<long long>(side, ((side + parts - 1) / parts + 63) / 64 * 64);
+        while (side > 64 && (long long)shares * side * other > kPlanes) side = (side - 1) / 64 * 64;
+    };
+    int &longer = p.cols >= p.rows ? p.cols : p.rows, &other = p.cols >= p.rows ? p.rows : p.cols;
+    cut(longer, other);
+    if ((long long)shares * longer * other > kPlanes) cut(other, longer);
+    return p;
+}
 
-// Floats of scratch a product needs: a plane of sums a share, none for a single share.
+// Floats of scratch a product needs: a plane of sums a share, none for a single share; and how many kernels it launches.
 BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
-    return shares_of(K) > 1 ? (long long)shares_of(K) * products_at_once(batch, K) * N * M : 0;
+    if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
+    const Pass p = pass_of(batch, N, M, K);
+    return shares_of(K) > 1 ? (long long)shares_of(K) * p.products * p.rows * p.cols : 0;
+}
+BLM_API int blm_gemm_f32_launches(int batch, int N, int M, int K) {
+    if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
+    const Pass p = pass_of(batch, N, M, K);
+    return ((batch - 1) / p.products + 1) * ((N - 1) / p.rows + 1) * ((M - 1) / p.cols + 1) * (shares_of(K) > 1 ? 2 : 1);
 }
 
 // `batch` products y[b] = x[b] . W[b]^T of one shape; the operands of product b lie b * (bx, bw, by) elements on.
@@ -179,30 +213,32 @@ BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int b
     BLM_REQUIRE(N > 0 && M > 0 && K > 0 && batch > 0, "gemm_f32: bad sizes %d x %d %d %d", batch, N, M, K);
     const int shares = shares_of(K);
     BLM_REQUIRE(batch <= 65535 && shares <= 65535 && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
-    const int at_once = products_at_once(batch, K);
-    BLM_REQUIRE(shares == 1 || (long long)at_once * N <= 0x7fffffffLL, "gemm_f32: too many rows or products (%d x %d)", batch, N);
     BLM_REQUIRE(shares == 1 || scratch != nullptr, "gemm_f32: a sum over %d places needs scratch", K);
     // 16-byte pieces where every row starts at a multiple of 16 bytes, and 64 rows lie within what an int can tell
     const bool vec = (((size_t)x | (size_t)w) & 15) == 0 && ldx < (1 << 25) && ldw < (1 << 25) && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bx % 4 == 0 && bw % 4 == 0;
     const bool vec4 = (((size_t)y | (size_t)scratch) & 15) == 0 && M % 4 == 0 && ldy % 4 == 0 && by % 4 == 0;
-    for (int b0 = 0; b0 < batch; b0 += at_once) {
-        const int products = std::min(at_once, batch - b0);
-        float* to = y + (size_t)b0 * by;
-        const GemmArgs a = {x + (size_t)b0 * bx, w + (size_t)b0 * bw, shares > 1 ? scratch : to, N, M, K, shares, products, ldx, ldw, ldy, bx, bw, by};
-        // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights 49 us,
-        // with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
-        const int rc = N <= 16   ? launch<4, 16, 4, 2>(a, vec, stream)
-                       : N <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
-                       : N <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
-                                 : launch<8, 16, 8, 4>(a, vec, stream);
-        if (rc != BLM_OK) return rc;
-        if (shares == 1) continue;
-        const int per = 256 * (vec4 ? 4 : 1);
-        const dim3 grid(products * N, (M + per - 1) / per);
-        if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(scratch, to, N, M, shares, products, ldy, by);
-        else add_shares_kernel<1><<<grid, 256, 0, stream>>>(scratch, to, N, M, shares, products, ldy, by);
-        if (int added = blm_check_launch("gemm_f32 (shares)")) return added;
-    }
+    const Pass pass = pass_of(batch, N, M, K);
+    for (int b0 = 0; b0 < batch; b0 += pass.products)
+        for (int n0 = 0; n0 < N; n0 += pass.rows)
+            for (int m0 = 0; m0 < M; m0 += pass.cols) {
+                const int products = std::min(pass.products, batch - b0), rows = std::min(pass.rows, N - n0), cols = std::min(pass.cols, M - m0);
+                float* to = y + (size_t)b0 * by + (size_t)n0 * ldy + m0;
+                const GemmArgs a = {x + (size_t)b0 * bx + (size_t)n0 * ldx, w + (size_t)b0 * bw + (size_t)m0 * ldw, shares > 1 ? scratch : to,
+                                    rows, cols, K, shares, products, ldx, ldw, ldy, bx, bw, by};
+                // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights
+                // 49 us, with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
+                const int rc = rows <= 16   ? launch<4, 16, 4, 2>(a, vec, stream)
+                               : rows <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
+                               : rows <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
+                                            : launch<8, 16, 8, 4>(a, vec, stream);
+                if (rc != BLM_OK) return rc;
+                if (shares == 1) continue;
+                const int per = 256 * (vec4 ? 4 : 1);
+                const dim3 grid(products * rows, (cols + per - 1) / per);
+                if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(scratch, to, rows, cols, shares, products, ldy, by);
+                else add_shares_kernel<1><<<grid, 256, 0, stream>>>(scratch, to, rows, cols, shares, products, ldy, by);
+                if (int added = blm_check_launch("gemm_f32 (shares)")) return added;
+            }
     return BLM_OK;
 }
 

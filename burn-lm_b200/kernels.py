@@ -212,6 +212,7 @@ _protos = {
         "blm_gemm_f32_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                  c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
         "blm_gemm_f32_scratch": [c_int, c_int, c_int, c_int],
+        "blm_gemm_f32_launches": [c_int, c_int, c_int, c_int],
     },
     "gemv": {
         "blm_gemv": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
@@ -857,15 +858,17 @@ def gemm_f32(x, w, out=None):
         out = torch.empty((n, m), dtype=torch.float32, device=x.device)
     elif tuple(out.shape) != (n, m) or out.dtype != torch.float32:
         raise KernelError("gemm_f32: out must be float32 [N, M]")
-    scratch = _gemm_f32_scratch(1, n, m, k, x.device)
-    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _stream(), kernels=2 if scratch is not None else 1)
+    scratch, launches = _gemm_f32_scratch(1, n, m, k, x.device)
+    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _stream(), kernels=launches)
     return out
 
 
 def _gemm_f32_scratch(batch, n, m, k, device):
-    """A plane of sums for every share of K that the float32 product cuts its sums into; None where there is one share."""
-    floats = int(_lib("gemm").blm_gemm_f32_scratch(batch, n, m, k))
-    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
+    """(a plane of sums for every share of K that the float32 product cuts its sums into, None where there is one share; the
+    kernels it launches: products whose planes would take more than 256 MB run in several passes)"""
+    lib = _lib("gemm")
+    floats = int(lib.blm_gemm_f32_scratch(batch, n, m, k))
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, int(lib.blm_gemm_f32_launches(batch, n, m, k))
 
 
 def batched_product(x, w, out=None, out_dtype=None):
@@ -886,10 +889,10 @@ def batched_product(x, w, out=None, out_dtype=None):
             out = torch.empty((b, n, m), dtype=torch.float32, device=x.device)
         if out.dtype != torch.float32 or tuple(out.shape) != (b, n, m) or any(t.stride(2) != 1 for t in (x, w, out)):
             raise KernelError("batched_product: float32 out [B, N, M]; unit stride along the last axis")
-        scratch = _gemm_f32_scratch(b, n, m, k, x.device)
+        scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device)
         _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, c_longlong(x.stride(1)), c_longlong(w.stride(1)),
               c_longlong(out.stride(1)), c_longlong(x.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)), _ptr(scratch),
-              _stream(), kernels=2 if scratch is not None else 1)
+              _stream(), kernels=launches)
         return out
     if out is not None:
         return torch.bmm(x, w.transpose(1, 2), out=out)

@@ -48,3 +48,23 @@ def test_batches_whose_shares_fill_more_than_one_grid():
         assert torch.equal(y[b], K.gemm_f32(x[b], w[b])), b
     want = torch.einsum("bnk,bmk->bnm", x.double(), w.double())
     assert (y.double() - want).abs().max() <= 4 * 1030 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n,m,k", [(1030, 20000, 4096), (9000, 300, 30000), (270, 20000, 16384)])
+def test_passes_change_no_bit(n, m, k):
+    """Products whose planes of sums would be larger than one pass may take, cut along their columns and along their rows."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    x, w = (torch.randn(shape, generator=gen, device="cuda") for shape in ((n, k), (m, k)))
+    scratch, launches = K._gemm_f32_scratch(1, n, m, k, "cuda")
+    assert scratch.numel() <= 64 << 20 and launches > 2
+    y = K.gemm_f32(x, w)
+    rows, cols = [0, n // 2, n - 1], slice(m // 2 - 20, m // 2 + 20)
+    assert torch.equal(y[rows], K.gemm_f32(x[rows].contiguous(), w))
+    assert torch.equal(y[:, cols], K.gemm_f32(x, w[cols].contiguous()))
+    assert torch.equal(y[:, -1:], K.gemm_f32(x, w[-1:].contiguous()))
+
+
+@pytest.mark.parametrize("batch,n,m,k", [(1, 2048, 128256, 4096), (1, 128256, 2048, 14336), (32, 2048, 512, 2048), (1, 4000000, 3, 4096)])
+def test_scratch_is_bounded(batch, n, m, k):
+    assert 0 < int(K._lib("gemm").blm_gemm_f32_scratch(batch, n, m, k)) <= 64 << 20
