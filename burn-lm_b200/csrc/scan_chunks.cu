@@ -35,12 +35,18 @@ __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + lo
 struct Chunks {
     const int* cu;
     int n_seqs, least, packed;
+    int from, count;               // the chunk indexes of this pass
 };
 static bool chunks_packed(int n_tokens, int n_seqs, int least) { return least >= 2 * kQ && 3LL * n_tokens / (2 * kQ) < (long long)n_tokens / kQ + n_seqs; }
 static long long chunk_bound(int n_tokens, int n_seqs, int least) {
     return chunks_packed(n_tokens, n_seqs, least) ? 3LL * n_tokens / (2 * kQ) : (long long)n_tokens / kQ + n_seqs;
 }
 __device__ __forceinline__ int chunk_base(int cu, int seq, int packed) { return packed ? (int)(3LL * cu / (2 * kQ)) : cu / kQ + seq; }
+
+// A step's chunks are run in passes whose scratch stays within kScratch floats (128 MB: some 3,700 tokens of a decay of 32 heads of
+// 128 rows), or a 32,768-token prompt would hold 1.2 GB.  Between two passes a sequence's state lies where it is written in the
+// end, as it would lie in registers: the passes change no bit.
+constexpr long long kScratch = 32 << 20;
 
 // Floats of one (chunk, head) in scratch: [decayed k for the correction (delta)] [decayed q] [k decayed to the chunk's end]
 // [the chunk's decay], rows of NP (not for the state-space scan, whose rows are shared by heads and read where they lie);
@@ -51,6 +57,7 @@ __host__ __device__ constexpr int part_floats(int kind, int np) { return rows_fl
 
 // Which sequence and chunk a chunk index names; false when none.  All threads of the block call it.
 __device__ __forceinline__ bool find_chunk(int idx, const Chunks& ch, int* found, int& seq, int& chunk) {
+    idx += ch.from;
     if (threadIdx.x == 0) found[0] = -1;
     __syncthreads();
     for (int s = threadIdx.x; s < ch.n_seqs; s += blockDim.x) {
@@ -518,13 +525,16 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
     const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
     const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
     if (n_new < a.ch.least) return;
-    const int chunks = (n_new + kQ - 1) / kQ, base = chunk_base(first, seq, a.ch.packed), start = a.start_pos[seq];
+    // the sequence's chunks of this pass: from `lo` up to `hi`; `base`: where its first one lies, or would lie, in scratch
+    const int base = chunk_base(first, seq, a.ch.packed) - a.ch.from, start = a.start_pos[seq];
+    const int lo = max(0, -base), hi = min((n_new + kQ - 1) / kQ, a.ch.count - base);
+    if (lo >= hi) return;
     const int tid = threadIdx.x;
 
     if (tid >= kWalkers) {                     // the loading warp, two chunks ahead of the others
         const int lane = tid - kWalkers;
-        for (int chunk = 0; chunk < chunks + 2; ++chunk) {
-            if (chunk < chunks) {
+        for (int chunk = lo; chunk < hi + 2; ++chunk) {
+            if (chunk < hi) {
                 float* st = sm + chunk % kStages * kStage;
                 const float* src = a.scratch + ((size_t)(base + chunk) * a.heads + h) * kPart;
                 const int at = first + chunk * kQ, nt = min(kQ, n_new - chunk * kQ);
@@ -571,7 +581,7 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
                 }
             }
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 2;\n" ::: "memory");
-            if (chunk >= 2) __syncthreads();   // chunk - 2 is there, and the others are done with the one before it
+            if (chunk >= lo + 2) __syncthreads();   // chunk - 2 is there, and the others are done with the one before it
         }
         return;
     }
@@ -580,8 +590,8 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
     const int turn = RG == 32 && g >= 16 ? C / 2 : 0;           // column p of the thread is cl + (p ^ turn)
     // the state as it lies: [head][row / 8][column][row % 8]; the thread's rows are m * 4 RG + 4 g .. + 3
     float* both = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off + (size_t)h * NP * a.dv;
-    const float* old = both + (size_t)(start & 1) * a.copy_stride;
     float* fresh = both + (size_t)((start + n_new) & 1) * a.copy_stride;
+    const float* old = lo > 0 ? fresh : both + (size_t)(start & 1) * a.copy_stride;      // (behind an earlier pass: what that wrote)
     f32x2 s[2 * P4][C];
 #pragma unroll
     for (int m = 0; m < P4; ++m)
@@ -589,7 +599,7 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
         for (int c = 0; c < C; ++c) {
             const int col = col0 + cl + (c ^ turn);
             float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (start > 0 && col < a.dv) {
+            if ((start > 0 || lo > 0) && col < a.dv) {
                 const float* p = old + ((size_t)(m * (RG / 2) + (g >> 1)) * a.dv + col) * 8 + (g & 1) * 4;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) v[e] = p[e];
@@ -614,7 +624,7 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
         }
     };
 
-    for (int chunk = 0; chunk < chunks; ++chunk) {
+    for (int chunk = lo; chunk < hi; ++chunk) {
         __syncthreads();
         const float* st = sm + chunk % kStages * kStage;
         const float* q = st + (KIND == kDelta ? kQ * NP : 0);
@@ -763,11 +773,23 @@ static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
     return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
 }
 
-// Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows).
+// Chunks of a pass.
+static int chunks_at_once(int kind, int heads, int np, int n_tokens, int n_seqs, int least) {
+    const long long most = kScratch / ((long long)heads * part_floats(kind, np)), all = chunk_bound(n_tokens, n_seqs, least);
+    return (int)(all < most ? all : (most > 1 ? most : 1));
+}
+
+// Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows).  And the
+// number of kernels it launches.
 BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
     const int np = padded_rows(rows);
-    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta) return 0;
-    return chunk_bound(n_tokens, n_seqs, least) * heads * part_floats(kind, np);
+    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta || heads < 1) return 0;
+    return (long long)chunks_at_once(kind, heads, np, n_tokens, n_seqs, least) * heads * part_floats(kind, np);
+}
+BLM_API int blm_scan_chunks_launches(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
+    if (blm_scan_chunks_scratch(kind, heads, rows, n_tokens, n_seqs, least) == 0) return 0;
+    const int at_once = chunks_at_once(kind, heads, padded_rows(rows), n_tokens, n_seqs, least);
+    return 2 * (int)((chunk_bound(n_tokens, n_seqs, least) + at_once - 1) / at_once);
 }
 
 static int check_step(int n_tokens, int n_seqs, int heads, int least) {
@@ -783,12 +805,10 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
-    const Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least)};
+    Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least), 0, 0};
     const int np = padded_rows(N), per = heads / groups;
     SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
                      scratch};
-    prep_ssm_kernel<<<dim3(chunk_bound(n_tokens, n_seqs, least), groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
-    if (int rc = blm_check_launch("scan_chunks (state-space scan)")) return rc;
     WalkArgs a = {};
     a.v = {xbc, xbc_stride, x_col0};
     a.scratch = scratch;
@@ -803,14 +823,21 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
     a.heads = heads;
     a.dv = dv;
     a.vec = ((size_t)xbc & 15) == 0 && xbc_stride % 4 == 0 && b_col0 % 4 == 0 && c_col0 % 4 == 0 && N % 4 == 0;
-    a.ch = ch;
     a.slot_of_seq = slot_of_seq;
     a.start_pos = start_pos;
     a.state = state;
     a.slot_stride = slot_stride;
     a.copy_stride = copy_stride;
     a.state_off = state_off;
-    return walk<kSsm>(a, np, n_seqs, stream);
+    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(kSsm, heads, np, n_tokens, n_seqs, least);
+    for (ch.from = 0; ch.from < all; ch.from += at_once) {
+        ch.count = all - ch.from < at_once ? all - ch.from : at_once;
+        p.ch = a.ch = ch;
+        prep_ssm_kernel<<<dim3(ch.count, groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
+        if (int rc = blm_check_launch("scan_chunks (state-space scan)")) return rc;
+        if (int rc = walk<kSsm>(a, np, n_seqs, stream)) return rc;
+    }
+    return BLM_OK;
 }
 
 template <int NP, int MODE>
@@ -840,7 +867,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(qk_heads > 0 && heads % qk_heads == 0 && dk > 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
-    const Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least)};
+    Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least), 0, 0};
     const bool delta = b_raw != nullptr;
     BLM_REQUIRE(delta ? k != nullptr && A_log != nullptr && !read_first && !lower_bound : (k != nullptr || lower_bound), "scan_chunks: no keys");
     BLM_REQUIRE(!lower_bound || (extra != nullptr && !read_first), "scan_chunks: a lower bound, and the state read last");
@@ -848,16 +875,6 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     PrepArgs p = {{q, q_stride, q_col0}, {k, k_stride, k_col0}, {a_raw, a_stride, a_col0}, {b_raw, b_stride, b_col0}, bias, extra, A_log,
                   ch, heads, qk_heads, dk, scratch};
     const int mode = delta ? kModeDelta : (lower_bound ? kModeLower : (read_first ? kModeExpFirst : kModeExp));
-    const dim3 grid(chunk_bound(n_tokens, n_seqs, least), heads);
-    int rc = BLM_OK;
-    switch (np) {
-        case 32: rc = prep<32>(p, mode, grid, stream); break;
-        case 64: rc = prep<64>(p, mode, grid, stream); break;
-        case 128: rc = prep<128>(p, mode, grid, stream); break;
-        case 256: rc = prep<256>(p, mode, grid, stream); break;
-        default: return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
-    }
-    if (rc != BLM_OK) return rc;
     WalkArgs a = {};
     a.v = {v, v_stride, v_col0};
     a.scratch = scratch;
@@ -865,12 +882,27 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     a.y_stride = o_stride;
     a.heads = heads;
     a.dv = dv;
-    a.ch = ch;
     a.slot_of_seq = slot_of_seq;
     a.start_pos = start_pos;
     a.state = state;
     a.slot_stride = slot_stride;
     a.copy_stride = copy_stride;
     a.state_off = state_off;
-    return delta ? walk<kDelta>(a, np, n_seqs, stream) : walk<kDecay>(a, np, n_seqs, stream);
+    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(delta ? kDelta : kDecay, heads, np, n_tokens, n_seqs, least);
+    for (ch.from = 0; ch.from < all; ch.from += at_once) {
+        ch.count = all - ch.from < at_once ? all - ch.from : at_once;
+        p.ch = a.ch = ch;
+        const dim3 grid(ch.count, heads);
+        int rc = BLM_OK;
+        switch (np) {
+            case 32: rc = prep<32>(p, mode, grid, stream); break;
+            case 64: rc = prep<64>(p, mode, grid, stream); break;
+            case 128: rc = prep<128>(p, mode, grid, stream); break;
+            case 256: rc = prep<256>(p, mode, grid, stream); break;
+            default: return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
+        }
+        if (rc == BLM_OK) rc = delta ? walk<kDelta>(a, np, n_seqs, stream) : walk<kDecay>(a, np, n_seqs, stream);
+        if (rc != BLM_OK) return rc;
+    }
+    return BLM_OK;
 }

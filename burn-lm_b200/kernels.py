@@ -144,6 +144,7 @@ _protos = {
     },
     "scan_chunks": {
         "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int, c_int],
+        "blm_scan_chunks_launches": [c_int, c_int, c_int, c_int, c_int, c_int],
         "blm_scan_chunks_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
@@ -1386,8 +1387,8 @@ def scan_runs(lengths) -> tuple:
 
 
 def _scan_route(kind, heads, rows, step, device):
-    """How a step's recurrence runs: (scratch of the chunk kernels, or None without them; the length from which they run a
-    sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
+    """How a step's recurrence runs: (scratch of the chunk kernels, or None without them; how many of them are launched; the length
+    from which they run a sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
     its own length, which the kernels read; step.scan_runs says which of the two have work (the engine's steps know)."""
     longest = getattr(step, "max_q_len", 0)
     # (a step that does not know and brings 64 tokens a sequence and more on average: short ones are few if any, and cost a chunk each)
@@ -1395,10 +1396,12 @@ def _scan_route(kind, heads, rows, step, device):
     in_chunks, walked = known or (True, step.n_tokens < 2 * SCAN_CHUNK_TOKENS * step.n_seqs and (step.n_seqs > 1 or step.n_tokens != longest))
     if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
         least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
-        floats = int(_lib("scan_chunks").blm_scan_chunks_scratch(kind, heads, rows, step.n_tokens, step.n_seqs, least))
+        lib, sizes = _lib("scan_chunks"), (kind, heads, rows, step.n_tokens, step.n_seqs, least)
+        floats = int(lib.blm_scan_chunks_scratch(*sizes))
         if floats:
-            return torch.empty(floats, dtype=torch.float32, device=device), least, SCAN_CHUNK_TOKENS if walked else 0
-    return None, 0, _NO_LIMIT
+            return (torch.empty(floats, dtype=torch.float32, device=device), int(lib.blm_scan_chunks_launches(*sizes)), least,
+                    SCAN_CHUNK_TOKENS if walked else 0)
+    return None, 0, 0, _NO_LIMIT
 
 
 def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y, heads, groups, n_state, value_dim, step, state,
@@ -1416,11 +1419,12 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     dp, ds, dc = _cols(dt, dt_col0, heads)
     if tuple(y.shape) != (step.n_tokens, heads * value_dim) or not y.is_contiguous():
         raise KernelError("ssm_scan: y float32 [N, heads * value_dim]")
-    scratch, least, below = (None, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
+    scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              kernels=launches)
     if below == 0:
         return
     _call("recurrent", "blm_ssm_scan", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
@@ -1443,11 +1447,12 @@ def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a
     aa = _cols(a, a_col0, heads * key_dim)
     if tuple(out.shape) != (step.n_tokens, heads * value_dim) or not out.is_contiguous() or dt_bias.numel() != heads * key_dim:
         raise KernelError("delta_scan: out float32 [N, heads * value_dim], dt_bias [heads * key_dim]")
-    scratch, least, below = _scan_route(_SCAN_DELTA, heads, key_dim, step, out.device)
+    scratch, launches, least, below = _scan_route(_SCAN_DELTA, heads, key_dim, step, out.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(None), _ptr(a_log), _ptr(out),
               c_longlong(out.stride(0)), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              kernels=launches)
     if below == 0:
         return
     _call("recurrent", "blm_delta_scan", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(a_log), _ptr(out), c_longlong(out.stride(0)),
@@ -1493,12 +1498,13 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
         raise KernelError("decay_scan: out float32 [N, heads * value_dim], bias [heads * key_dim]")
     if extra is not None and extra.numel() != heads * key_dim:
         raise KernelError("decay_scan: extra [heads * key_dim]")
-    scratch, least, below = (None, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_DECAY, heads, key_dim, step, out.device)
+    scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_DECAY, heads, key_dim, step, out.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, c_void_p(0), c_longlong(0), 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
               _ptr(out), c_longlong(out.stride(0)), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
               1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs, least,
-              *_state_args(state, state_offset), _ptr(scratch), _stream(), kernels=2)
+              *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              kernels=launches)
     if below == 0:
         return
     _call("recurrent", "blm_decay_scan", *qa, *ka, *va, *aa, _ptr(bias), _ptr(extra), _ptr(out), c_longlong(out.stride(0)), heads,

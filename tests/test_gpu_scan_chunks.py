@@ -192,7 +192,7 @@ def test_a_sequence_runs_by_its_own_length_whatever_shares_the_step(kind, heads,
     more = 16 - len(lens)
     step = SimpleNamespace(cu_seqlens=pad(real.cu_seqlens, more, sum(lens)), slot_of_seq=pad(real.slot_of_seq, more, int(real.slot_of_seq[-1])),
                            start_pos=pad(real.start_pos, more, starts[-1]), n_tokens=n, n_seqs=16, max_q_len=min(n, 128))
-    scratch, least, below = K._scan_route(K._SCAN_SSM, heads, rows, step, "cuda")
+    scratch, _, least, below = K._scan_route(K._SCAN_SSM, heads, rows, step, "cuda")
     assert scratch is not None and least == below == K.SCAN_CHUNK_TOKENS
     got, got_state = torch.full((n, heads * dv), 7.0, device="cuda"), state.clone()
     run(slice(0, n), got, step, got_state)
@@ -233,3 +233,38 @@ def test_the_engine_launches_the_scans_that_have_work(tmp_path, monkeypatch):
         logits = engine.step([StepEntry(s, [t % NUF_D["vocab"] for t in range(m)], [m - 1]) for s, m in zip(slots, lengths)])
         assert bool(chunked()) == in_chunks and bool(walked()) == by_walk, lengths
         assert bool(torch.isfinite(logits).all())
+
+
+@pytest.mark.parametrize("kind,heads,rows,dv,lens", [("wkv", 32, 128, 16, [2100, 1700]), ("delta", 32, 128, 16, [900, 1800]),
+                                                     ("ssm", 2048, 32, 1, [500, 33, 400])])
+def test_passes_change_no_bit(kind, heads, rows, dv, lens):
+    """Steps whose scratch would be larger than one pass may take: the bits of two of the heads are those of a step of the two."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(heads + rows)
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    starts, n, few = list(range(len(lens))), sum(lens), 2
+    step = step_of(lens, starts)
+    route = lambda h: K._scan_route({"wkv": K._SCAN_DECAY, "delta": K._SCAN_DELTA, "ssm": K._SCAN_SSM}[kind], h, rows, step, "cuda")
+    assert route(heads)[0].numel() <= 32 << 20 and route(heads)[1] > 2 and route(few)[1] == 2
+    state = state_of(step, heads, rows, dv, 0, gen)
+    own = state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(state.shape[0], 2, -1).contiguous()
+    b, bias, extra, per_head = rnd(n, heads), rnd(heads * rows), rnd(heads * rows), [rnd(heads) for _ in range(3)]
+    v = rnd(n, heads * dv)
+    if kind == "ssm":
+        x = torch.cat([v, rnd(n, 2 * rows)], 1)
+        run = lambda h, out, st: K.ssm_scan(x, 0, heads * dv, heads * dv + rows, b, 0, *[t[:h].contiguous() for t in per_head], out, h, 1, rows, dv,
+                                            step, st, 0)
+    else:
+        q, k, a = rnd(n, heads * rows), rnd(n, heads * rows), rnd(n, heads * rows)
+        part = lambda t, h: t[:h * rows].contiguous()
+        if kind == "delta":
+            run = lambda h, out, st: K.delta_scan(q, 0, k, 0, v, 0, b, 0, a, 0, part(bias, h), per_head[0][:h].contiguous(), out, h, h, rows, dv,
+                                                  step, st, 0)
+        else:
+            run = lambda h, out, st: K.decay_scan(q, 0, k, 0, v, 0, a, 0, part(bias, h), part(extra, h), out, h, rows, dv, K.DECAY_EXP_EXP, True,
+                                                  step, st, 0)
+    out, two = torch.empty((n, heads * dv), device="cuda"), torch.empty((n, few * dv), device="cuda")
+    run(heads, out, state)
+    run(few, two, own)
+    assert torch.equal(out[:, :few * dv], two)
+    assert torch.equal(state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(own.shape), own)
