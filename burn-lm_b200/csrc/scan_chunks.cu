@@ -779,11 +779,11 @@ static int chunks_at_once(int kind, int heads, int np, int n_tokens, int n_seqs,
     return (int)(all < most ? all : (most > 1 ? most : 1));
 }
 
-// Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows).  And the
-// number of kernels it launches.
+// Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows, more
+// sequences than a grid's third dimension holds).  And the number of kernels it launches.
 BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
     const int np = padded_rows(rows);
-    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta || heads < 1) return 0;
+    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta || heads < 1 || n_seqs > 65535) return 0;
     return (long long)chunks_at_once(kind, heads, np, n_tokens, n_seqs, least) * heads * part_floats(kind, np);
 }
 BLM_API int blm_scan_chunks_launches(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {

@@ -268,3 +268,8 @@ def test_passes_change_no_bit(kind, heads, rows, dv, lens):
     run(few, two, own)
     assert torch.equal(out[:, :few * dv], two)
     assert torch.equal(state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(own.shape), own)
+
+
+def test_more_sequences_than_a_grid_holds_are_walked():
+    step = SimpleNamespace(n_tokens=300000, n_seqs=70000, max_q_len=64)
+    assert K._scan_route(K._SCAN_SSM, 2, 64, step, "cuda") == (None, 0, 0, K._NO_LIMIT)
