@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(TN * TM) gemm_f32_kernel(const GemmArgs a) {
     const int k_lo = share * kShare, k_hi = min(a.K, k_lo + kShare);
     const int slices = (k_hi - k_lo + kBK - 1) / kBK;
 
-    // the thread's pieces of a slice: places c .. of the rows r0 + i kStep, x's rows first.  A row beyond the end is read as the
-    // last one (its outputs are not stored), so that only the last places of a share need a test.
+    // the thread's pieces of a slice: places c .. of the rows r0 + i kStep, x's rows first.  A row of W beyond the
+    // end is read as the last one (its outputs are not stored), one of x comes as zeros, from the last one's address.
     constexpr int P = VEC ? 4 : 1, kPer = kBK / P, kStep = T / kPer, kPieces = (BN + BM) / kStep;
     static_assert(T % kPer == 0 && BN % kStep == 0 && BM % kStep == 0, "a piece of every row falls to one thread");
     const int r0 = tid / kPer, c = tid % kPer * P;
