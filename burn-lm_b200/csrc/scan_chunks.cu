@@ -30,18 +30,18 @@ __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf
 __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // Only sequences of `least` or more new tokens are run (the others are walked token by token: recurrent.cu).  Chunk c of sequence
-// s has the index cu[s] / 16 + s + c, which are distinct and below n_tokens / 16 + n_seqs; beside many short sequences 3 cu[s] /
-// 32 + c, which is below 3 n_tokens / 32: the ceil(n / 16) chunks of n >= 32 tokens are no more than 3 n / 32, rounded down.
+// s has the index cu[s] / 16 + s + c, which are distinct and below n_tokens / 16 + n_seqs; beside many short sequences cu[s] / 8 + c,
+// which is below n_tokens / 8: the ceil(n / 16) chunks of n >= 16 tokens are no more than n / 8, rounded down.
 struct Chunks {
     const int* cu;
     int n_seqs, least, packed;
     int from, count;               // the chunk indexes of this pass
 };
-static bool chunks_packed(int n_tokens, int n_seqs, int least) { return least >= 2 * kQ && 3LL * n_tokens / (2 * kQ) < (long long)n_tokens / kQ + n_seqs; }
+static bool chunks_packed(int n_tokens, int n_seqs, int least) { return least >= kQ && n_tokens / (kQ / 2) < (long long)n_tokens / kQ + n_seqs; }
 static long long chunk_bound(int n_tokens, int n_seqs, int least) {
-    return chunks_packed(n_tokens, n_seqs, least) ? 3LL * n_tokens / (2 * kQ) : (long long)n_tokens / kQ + n_seqs;
+    return chunks_packed(n_tokens, n_seqs, least) ? n_tokens / (kQ / 2) : (long long)n_tokens / kQ + n_seqs;
 }
-__device__ __forceinline__ int chunk_base(int cu, int seq, int packed) { return packed ? (int)(3LL * cu / (2 * kQ)) : cu / kQ + seq; }
+__device__ __forceinline__ int chunk_base(int cu, int seq, int packed) { return packed ? cu / (kQ / 2) : cu / kQ + seq; }
 
 // A step's chunks are run in passes whose scratch stays within kScratch floats (128 MB: some 3,700 tokens of a decay of 32 heads of
 // 128 rows), or a 32,768-token prompt would hold 1.2 GB.  Between two passes a sequence's state lies where it is written in the

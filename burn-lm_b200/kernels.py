@@ -1371,12 +1371,15 @@ def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, sta
 
 # From this many new tokens on, a sequence's recurrence runs in chunks of sixteen tokens (scan_chunks.cu), below it token by token
 # (recurrent.cu), each by its own length, whatever shares the step.  Chunks against the walk, us on the device, sequences of
-# 24 / 32 / 64 tokens: state-space scan of 64 heads of 128 x 64, one 17 / 12, 16 / 15, 20 / 27, sixteen 88 / 77, 88 / 98, 133 / 188;
-# delta rule of 16 heads of 128 x 128, one 15 / 19, 15 / 24, 18 / 45, sixteen 78 / 64, 78 / 83, 128 / 159; WKV of 32 heads of 128 x
-# 128, one 13 / 18, 13 / 23, 17 / 43, sixteen 83 / 106, 85 / 139, 133 / 290.  A single token costs a chunk all the same (255 of them
-# beside 64 tokens 899 / 260 for the state-space scan), and beside many of them the chunks of a long prompt are still the faster
-# way for that prompt.
-SCAN_CHUNK_TOKENS = 32
+# 16 / 24 / 32 / 64 tokens: state-space scan of 64 heads of 128 x 64, one 15 / 9, 17 / 12, 16 / 15, 20 / 27, sixteen 67 / 55, 88 / 77,
+# 88 / 98, 133 / 188; delta rule of 16 heads of 128 x 128, one 13 / 14, 15 / 19, 15 / 24, 18 / 45, sixteen 60 / 46, 78 / 64, 78 / 83,
+# 128 / 159; WKV of 32 heads of 128 x 128, one 12 / 13, 13 / 18, 13 / 23, 17 / 43, sixteen 61 / 72, 83 / 106, 85 / 139, 133 / 290.  The line
+# lies at the lower end because a walk beside chunks comes on top of them, up to a microsecond a token of its longest sequence.  A
+# single token costs a chunk all the same (255 of them beside 64 tokens 899 / 260 for the state-space scan).
+SCAN_CHUNK_TOKENS = 16
+# A step that does not know its lengths (`scan_runs`; the engine's steps know) runs in chunks throughout from this longest run and this
+# many tokens a sequence on average on; with fewer tokens a sequence both are launched.
+SCAN_CHUNK_RUN, SCAN_CHUNK_MEAN = 32, 4
 _SCAN_SSM, _SCAN_DECAY, _SCAN_DELTA = 0, 1, 2
 _NO_LIMIT = (1 << 31) - 1
 
@@ -1391,9 +1394,7 @@ def _scan_route(kind, heads, rows, step, device):
     from which they run a sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
     its own length, which the kernels read; step.scan_runs says which of the two have work (the engine's steps know)."""
     longest = getattr(step, "max_q_len", 0)
-    # (a step that does not know and brings 64 tokens a sequence and more on average: short ones are few if any, and cost a chunk each)
-    known = getattr(step, "scan_runs", None)
-    in_chunks, walked = known or (True, step.n_tokens < 2 * SCAN_CHUNK_TOKENS * step.n_seqs and (step.n_seqs > 1 or step.n_tokens != longest))
+    in_chunks, walked = getattr(step, "scan_runs", None) or (longest >= SCAN_CHUNK_RUN, step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs)
     if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
         least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
         lib, sizes = _lib("scan_chunks"), (kind, heads, rows, step.n_tokens, step.n_seqs, least)

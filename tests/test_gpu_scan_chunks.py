@@ -63,6 +63,7 @@ def test_chunks_against_the_walk_in_float64(kind, heads, rows, dv, lens, starts)
     gen.manual_seed(heads * 1000 + rows + len(lens))
     rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
     step, n, offset = step_of(lens, starts), sum(lens), 7                    # (an odd offset: the state is not 16-byte aligned)
+    assert K._scan_route(K._SCAN_SSM, heads, rows, step, "cuda")[2] == 1      # every sequence in chunks
     state = state_of(step, heads, rows, dv, offset, gen)
     before = state.double()
     out = torch.zeros((n, heads * dv), device="cuda")
@@ -176,7 +177,7 @@ def scan_of(kind, heads, rows, dv, n, gen):
                                                      K.DECAY_EXP_EXP if exp else K.DECAY_LOWER_BOUND, exp, step, state, 0)
 
 
-@pytest.mark.parametrize("lens", [[1, 1, 1, 40, 1, 20, 0, 35, 0], [31, 32, 33], [1] * 15 + [4], [0, 64, 1]])
+@pytest.mark.parametrize("lens", [[1, 1, 1, 40, 1, 13, 0, 35, 0], [15, 16, 17, 31], [1] * 15 + [4], [0, 64, 1]])
 @pytest.mark.parametrize("heads,rows,dv", [(3, 64, 64), (2, 128, 100)])
 @pytest.mark.parametrize("kind", ["ssm", "wkv", "lower", "delta"])
 def test_a_sequence_runs_by_its_own_length_whatever_shares_the_step(kind, heads, rows, dv, lens):
@@ -191,7 +192,8 @@ def test_a_sequence_runs_by_its_own_length_whatever_shares_the_step(kind, heads,
     pad = lambda t, m, v: torch.cat([t, torch.full((m,), v, dtype=torch.int32, device="cuda")])
     more = 16 - len(lens)
     step = SimpleNamespace(cu_seqlens=pad(real.cu_seqlens, more, sum(lens)), slot_of_seq=pad(real.slot_of_seq, more, int(real.slot_of_seq[-1])),
-                           start_pos=pad(real.start_pos, more, starts[-1]), n_tokens=n, n_seqs=16, max_q_len=min(n, 128))
+                           start_pos=pad(real.start_pos, more, starts[-1]), n_tokens=n, n_seqs=16, max_q_len=min(n, 128),
+                           scan_runs=(True, True))
     scratch, _, least, below = K._scan_route(K._SCAN_SSM, heads, rows, step, "cuda")
     assert scratch is not None and least == below == K.SCAN_CHUNK_TOKENS
     got, got_state = torch.full((n, heads * dv), 7.0, device="cuda"), state.clone()
@@ -201,7 +203,7 @@ def test_a_sequence_runs_by_its_own_length_whatever_shares_the_step(kind, heads,
         if m == 0:
             continue
         own = step_of([m], [starts[s]])
-        own.slot_of_seq = real.slot_of_seq[s:s + 1]
+        own.slot_of_seq, own.scan_runs = real.slot_of_seq[s:s + 1], K.scan_runs([m])
         assert (K._scan_route(K._SCAN_SSM, heads, rows, own, "cuda")[0] is not None) == (m >= K.SCAN_CHUNK_TOKENS)
         out = torch.empty((m, heads * dv), device="cuda")
         run(slice(at, at + m), out, own, want_state)
@@ -227,7 +229,7 @@ def test_the_engine_launches_the_scans_that_have_work(tmp_path, monkeypatch):
     engine.step([StepEntry(s, [1, 2, 3, 4, 5], [0]) for s in slots])          # (another bucket than those below)
     chunked = lambda: [n for n in calls if n.startswith("blm_scan_chunks_")]
     walked = lambda: [n for n in calls if n in ("blm_ssm_scan", "blm_delta_scan")]
-    for lengths, in_chunks, by_walk in (([1] * 15 + [4], False, True), ([20], False, True), ([1] * 15 + [300], True, True), ([40, 33], True, False),
+    for lengths, in_chunks, by_walk in (([1] * 15 + [4], False, True), ([15], False, True), ([1] * 15 + [300], True, True), ([40, 16], True, False),
                                         ([1] * 15 + [4], False, True)):
         calls.clear()
         logits = engine.step([StepEntry(s, [t % NUF_D["vocab"] for t in range(m)], [m - 1]) for s, m in zip(slots, lengths)])
