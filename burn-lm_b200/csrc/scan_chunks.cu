@@ -610,18 +610,13 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
     // the thread's columns of sixteen rows [16][CT]
     auto columns = [&](const float* from, float (&x)[kQ][C]) {
 #pragma unroll
-        for (int i = 0; i < kQ; ++i) {
-            if (C == 1) {
-                x[i][0] = from[i * CT + cl];
-            } else {
+        for (int i = 0; i < kQ; ++i)
 #pragma unroll
-                for (int c = 0; c < C; c += 2) {
-                    const float2 f = *reinterpret_cast<const float2*>(from + i * CT + cl + (c ^ turn));
-                    x[i][c] = f.x;
-                    x[i][C > 1 ? c + 1 : 0] = f.y;
-                }
+            for (int c = 0; c < C; c += 2) {
+                const float2 f = *reinterpret_cast<const float2*>(from + i * CT + cl + (c ^ turn));
+                x[i][c] = f.x;
+                x[i][c + 1] = f.y;
             }
-        }
     };
 
     for (int chunk = lo; chunk < hi; ++chunk) {
