@@ -14,7 +14,7 @@
 //   the values, transposed:  O^T += V^T M^T: rows are value lanes, k runs over keys, columns are eight head rows, of which four
 //     belong to the key/value head.  Two queries fill both halves: the second query's rows cross over by one shuffle.
 // Weights, their mix and the outputs never leave registers; shared memory holds keys, values, the queries' and talk's fragments.
-// 1,536 tokens of 32 heads of 64 on 8: 695 -> 163 us; 64 single tokens over 1,088 keys: 220 -> 38 us (3.7 TB/s).
+// 1,536 tokens of 32 heads of 64 on 8: 695 -> 167 us; 64 single tokens over 1,088 keys: 220 -> 38 us (3.7 TB/s).
 #include "common.cuh"
 
 BLM_API const char* blm_attention_quads_last_error() { return g_blm_error; }
