@@ -48,7 +48,7 @@ MODULES = {
     "sampling": ["sampling.cu"],
     "runtime": ["runtime.cu"],
 }
-HEADERS = ["common.cuh", "attention_decode.cuh", "attention_prefill.cuh", "attention_prefill_tc.cuh", "sampling_no_alloc.h"]
+HEADERS = ["common.cuh", "attention_decode.cuh", "attention_prefill.cuh", "attention_prefill_tc.cuh", "sampling_no_alloc.h", "tcgen05.cuh"]
 
 _lock = threading.Lock()
 _loaded: dict[str, ctypes.CDLL] = {}

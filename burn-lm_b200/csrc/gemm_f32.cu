@@ -1,18 +1,19 @@
-// y[N, M] = x[N, K] . W[M, K]^T in true fp32: FFMA on CUDA cores, no tensor-core mode of any kind.
+// y[N, M] = x[N, K] . W[M, K]^T in 32 bits: all 24 bits of both operands, float32 sums.
 // This is the matrix product of the 32-bit path.  The sum over K runs in one fixed order that depends on neither N nor M, so a
-// token's result is the same whatever else is in the batch: K is cut into shares of 1,024, each is summed in order, and the
-// shares' sums are added in order by a second kernel.
+// token's result is the same whatever else is in the batch: K is cut into shares, each is summed in order, and the shares' sums are
+// added in order.  Two kernels: on the tensor cores (further down) where K and W's rows come in 16-byte pieces, and FFMA for
+// everything else.
 //
-// What bounds it: fp32 multiply-adds from some 50 rows on (74 TFLOP/s on this chip at best), the weights' way in below.  Both
+// FFMA: what bounds it is fp32 multiply-adds from some 50 rows on (74 TFLOP/s on this chip at best), the weights' way in below.  Both
 // operands lie along K and stay so in shared memory (rows padded by a 16-byte piece, so that eight rows start in eight different
 // groups of banks): a slice comes by cp.async two slices ahead, nothing is transposed, and twelve 16-byte loads feed 128
-// multiply-adds of a thread with 8 x 4 outputs.  The shares give a product of few columns as many blocks as one of many
-// (317 x 2,048 x 8,192: 160 tiles, 1,280 blocks).  Two places of K an instruction (fma.rn.f32x2) ran at the same rate, 8 x 8
-// outputs a thread too (four blocks a multiprocessor hide the loads, two do not).  With 16,384 x 2,048 / 2,048 x 8,192 weights,
-// us: 1 row 189 / 381 -> 48 / 30, 16 rows 189 / 383 -> 49 / 31, 48 rows 192 / 437 -> 101 / 58, 317 rows 703 / 671 -> 497 / 254.
+// multiply-adds of a thread with 8 x 4 outputs.  The shares of 1,024 give a product of few columns as many blocks as one of many
+// (317 x 2,048 x 8,192: 160 tiles, 1,280 blocks); a second kernel adds their sums.  Two places of K an instruction (fma.rn.f32x2) ran at the
+// same rate, 8 x 8 outputs a thread too (four blocks a multiprocessor hide the loads, two do not).  With 16,384 x 2,048 / 2,048 x 8,192 weights,
+// us: 1 row 50 / 36, 16 rows 58 / 36, 64 rows 128 / 77, 317 rows 507 / 263.
 #include <algorithm>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 BLM_API const char* blm_gemm_last_error() { return g_blm_error; }
 
@@ -148,6 +149,343 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The product on the tensor cores, for K a multiple of 4 from kTcLeast on and rows of W at multiples of 16 bytes: a choice by K and
+// W's layout alone, so that a row's bits depend on neither N nor M.
+//
+// Both operands as three bfloat16 numbers a float (tcgen05.cuh): 24 bits and six products, 282 TFLOP/s of the chip's 1,692 against
+// 74 of FFMA.  x is split once by a launch of its own (it is read by every tile of W's rows); W, which is read once or a few times,
+// comes as it lies and is split on its way, so no weight is kept twice.  A block: 128 rows of W x nt rows of x, K in steps of 64.
+// One warp brings W by TMA, one x's parts; four warps split W's floats, a lane a row, into tensor memory, from where the tensor
+// core takes its 128-row operand (through shared memory that operand's reads took its whole bandwidth: 317 rows below 142 us);
+// two threads in turn issue the 24 tcgen05.mma of a step, the small products first; eight warps add the finished step to their sums.  The
+// tensor core's additions cut bits off, so no more than a step is left to it (four additions of the large products); the sums over
+// the steps are float32 additions in order, and so are those over shares of 1,024 places of K.  The shares of a tile are a
+// block's, which adds them up in y, or where there are few tiles a block each and planes of sums: the same additions.
+// Infinities: an infinite x1 makes x2 not a number, and a zero x2 times an infinity is not one either, so an output that is not
+// finite is formed again with fmaf from the floats themselves.  Operands below 2^-109 lose their last bits (x3 would be below
+// the smallest bfloat16 number).
+// With 16,384 x 2,048 / 2,048 x 8,192 weights, us (FFMA above): 1 row 40 / 30, 16 rows 40 / 30, 64 rows 44 / 32, 160 rows 62 / 44, 317 rows
+// 110 / 69, 2,000 rows 603 / 390 (3,000 / 1,513); the error against 64 bits 1.5e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
+// of which the tensor core works 1,920: x's parts have room for two steps only.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTcLeast = 64;
+constexpr int kTcShare = 1024;    // places of K of a share at most
+constexpr int kTcK = 32;          // of a slice; two slices are a step
+constexpr int kTcRows = 128;      // rows of W of a tile
+constexpr int kTcMost = 160;      // rows of x of a tile at most
+constexpr int kTcFew = 64;        // up to so many rows of x a tile, W's way through the converting warps is what takes the time
+constexpr int kTcW = 2 * kTcRows * kTcK * 4;          // bytes of a step of W's floats
+constexpr int kTcCols = 512, kTcPart = kTcK / 2;      // columns of tensor memory: all, of a part of a slice of W
+constexpr int kTcSmem = 227 * 1024 - 1024;
+constexpr int kTcThreads = 16 * 32;
+
+struct TcArgs {
+    const float *x, *w;
+    float* y;                     // as GemmArgs
+    int N, M, K, shares, share_len, batch;
+    long long ldx, ldw, ldy, bx, bw, by;
+    int nt, n_tiles, m_tiles, w_stages, x_stages, w_batches;
+    int planes;                   // every share by a block of its own, its sums a plane of y; else a block adds a tile's shares up in y
+    int* status;
+};
+
+struct RingAt {                    // a place of a ring and the parity of its phase
+    int at = 0;
+    unsigned phase = 0;
+    __device__ __forceinline__ void next(int n) {
+        if (++at == n) {
+            at = 0;
+            phase ^= 1;
+        }
+    }
+};
+
+// one output that is not finite, formed again by the whole warp
+__device__ __noinline__ float tc_again(const float* x, const float* w, int k) {
+    const int lane = threadIdx.x & 31;
+    float s = 0.f;
+    for (int c0 = 0; c0 < k; c0 += 128) {
+        const int c = c0 + 4 * lane;
+        if (c < k) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s = fmaf(x[c + e], w[c + e], s);
+        }
+        if (__any_sync(0xffffffffu, isnan(s))) break;      // (stays so)
+    }
+    return warp_sum(s);
+}
+
+template <bool FEW>
+__global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap xmap,
+                                                                    const __grid_constant__ CUtensorMap wmap) {
+    using namespace tc5;
+    constexpr int kConverters = FEW ? 8 : 4, kAdders = FEW ? 4 : 8, kMine = FEW ? kTcFew : kTcMost / 2;      // rows of x a warp adds
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int x_part = a.nt * 2 * kTcK * 2, x_bytes = 3 * x_part;
+    unsigned char* w_ring = smem;                              // [w_stages][2][128][32] floats
+    unsigned char* x_ring = smem + a.w_stages * kTcW;          // [x_stages][3][nt][128 bytes]
+    unsigned long long* w_full = reinterpret_cast<unsigned long long*>(x_ring + a.x_stages * x_bytes);
+    unsigned long long* w_empty = w_full + a.w_stages;
+    unsigned long long* x_full = w_empty + a.w_stages;
+    unsigned long long* split = x_full + a.x_stages;           // W's parts are there
+    unsigned long long* done = split + a.x_stages;             // a step's products are in tensor memory, x's and W's parts free
+    unsigned long long* added = done + a.x_stages;             // [2] and have been added to the sums
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(added + 2);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned parts0 = 2 * a.nt;          // tensor memory: two accumulators, then W's parts [x_stages][2][3][16 columns]
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < a.w_stages; ++s) {
+            mbar_init(w_full + s, 1);
+            mbar_init(w_empty + s, kConverters);
+        }
+        for (int s = 0; s < a.x_stages; ++s) {
+            mbar_init(x_full + s, 1);
+            mbar_init(split + s, kConverters);
+            mbar_init(done + s, 1);
+        }
+        for (int b = 0; b < 2; ++b) mbar_init(added + b, kAdders);
+        mbar_init_fence();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, kTcCols);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const unsigned tmem_base = *tmem_slot;
+
+    // unit t: a tile's share.  The rows of x beside one another (they share W's slices in L2), then W's rows, the planes, the
+    // products; a block that adds a tile's shares up takes them one after the other
+    const int at_once = a.planes ? 1 : a.shares;
+    const long long units = (long long)a.n_tiles * a.m_tiles * (a.planes ? a.shares : 1) * a.batch * at_once;
+    auto next_unit = [&](long long t) { return (t + 1) % at_once ? t + 1 : t + 1 + (long long)(gridDim.x - 1) * at_once; };
+    const long long first_unit = (long long)blockIdx.x * at_once;
+    struct Unit {
+        int n0, m0, k0, steps, share, b;
+    };
+    auto unit_at = [&](long long t) {
+        Unit r;
+        r.share = (int)(t % at_once);
+        t /= at_once;
+        r.n0 = (int)(t % a.n_tiles) * a.nt;
+        t /= a.n_tiles;
+        r.m0 = (int)(t % a.m_tiles) * kTcRows;
+        t /= a.m_tiles;
+        if (a.planes) {
+            r.share = (int)(t % a.shares);
+            t /= a.shares;
+        }
+        r.b = (int)t;
+        r.k0 = r.share * a.share_len;
+        r.steps = (min(a.share_len, a.K - r.k0) + 2 * kTcK - 1) / (2 * kTcK);      // (places beyond K come as zeros)
+        return r;
+    };
+    bool ok = true;
+    auto wait = [&](unsigned long long* bar, unsigned phase) {
+        if (ok && !mbar_wait(bar, phase)) {
+            ok = false;
+            if (lane == 0) atomicCAS(a.status, TC5_OK, TC5_TIMEOUT);
+        }
+        return ok;
+    };
+
+    if (warp == 0 || warp == 15) {
+        // ---------------- the loads: warp 0 W's floats, warp 15 x's parts as soon as the kernel before has written them ----------------
+        const bool of_w = warp == 0;
+        const int stages = of_w ? a.w_stages : a.x_stages;
+        unsigned long long *full = of_w ? w_full : x_full, *empty = of_w ? w_empty : done;
+        RingAt r;
+        unsigned free = stages;                // stages that nothing was in yet
+        if (!of_w) pdl_wait();
+        for (long long t = first_unit; t < units && ok; t = next_unit(t)) {
+            const Unit u = unit_at(t);
+            for (int k = 0; k < u.steps; ++k) {
+                if (free) --free;
+                else if (!wait(empty + r.at, r.phase ^ 1)) break;
+                if (elect()) {
+                    const int c = u.k0 + k * 2 * kTcK;
+                    if (of_w) {
+                        unsigned char* to = w_ring + r.at * kTcW;
+                        mbar_expect_tx(full + r.at, kTcW);
+                        tma_load_3d(to, &wmap, c, u.m0, min(u.b, a.w_batches - 1), full + r.at);
+                        tma_load_3d(to + kTcW / 2, &wmap, c + kTcK, u.m0, min(u.b, a.w_batches - 1), full + r.at);
+                    } else {
+                        mbar_expect_tx(full + r.at, x_bytes);
+                        tma_load_3d(x_ring + r.at * x_bytes, &xmap, c, u.n0, u.b * 3, full + r.at);
+                    }
+                }
+                __syncwarp();
+                r.next(stages);
+            }
+        }
+    } else if (warp < 3) {
+        // ---------------- the tensor core: a warp the even steps, one the odd ones (one warp for all: 64 rows of x 128 us instead of 114) ----------------
+        const int b = warp - 1;
+        const unsigned idesc = instruction(a.nt), d = tmem_base + (unsigned)(b * a.nt);
+        const unsigned long long x_desc = operand(x_ring, 2, 1024);
+        RingAt r;
+        unsigned turn = 0;
+        for (long long t = first_unit; t < units && ok; t = next_unit(t)) {
+            const int steps = unit_at(t).steps;
+            for (int k = 0; k < steps; ++k, ++turn, r.next(a.x_stages)) {
+                if ((int)(turn & 1) != b) continue;
+                if (turn >= 2) wait(added + b, ((turn >> 1) - 1) & 1);
+                wait(x_full + r.at, r.phase);
+                if (!wait(split + r.at, r.phase)) break;
+                fence_after();
+                if (elect()) {
+                    // (part of W, part of x): the smallest products first
+                    constexpr int of_w[6] = {2, 0, 1, 1, 0, 0}, of_x[6] = {0, 2, 1, 0, 1, 0};
+                    const unsigned wd = tmem_base + parts0 + r.at * 6 * kTcPart;
+                    const unsigned long long xd = x_desc + (unsigned)(r.at * (x_bytes >> 4));
+#pragma unroll
+                    for (int p = 0; p < 6; ++p)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ts(d, wd + (kk >> 1) * 3 * kTcPart + of_w[p] * kTcPart + 8 * (kk & 1),
+                                   xd + (unsigned)(of_x[p] * (x_part >> 4) + 2 * kk), idesc, p > 0 || kk > 0);
+                    commit(done + r.at);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp < 3 + kConverters) {
+        // ---------------- W's floats into parts: a lane a row; four warps both slices of a step, or eight one each ----------------
+        const int row = (warp & 3) * 32 + lane, only = (warp - 3) >> 2;
+        const unsigned to = tmem_base + ((unsigned)((warp & 3) * 32) << 16) + parts0;
+        RingAt r, o;                           // where W comes from, and where its parts go
+        unsigned free = a.x_stages;
+        for (long long t = first_unit; t < units && ok; t = next_unit(t)) {
+            const int steps = unit_at(t).steps;
+            for (int k = 0; k < steps; ++k) {
+                if (free) --free;
+                else wait(done + o.at, o.phase ^ 1);
+                if (!wait(w_full + r.at, r.phase)) break;
+                fence_after();
+#pragma unroll 1
+                for (int half = FEW ? only : 0; half < (FEW ? only + 1 : 2); ++half) {
+                    const unsigned char* w = w_ring + r.at * kTcW + half * (kTcW / 2) + row * (kTcK * 4);
+                    float4 v[kTcK / 4];
+#pragma unroll
+                    for (int c = 0; c < kTcK / 4; ++c) v[c] = *reinterpret_cast<const float4*>(w + ((c ^ (row & 7)) << 4));      // 128-byte swizzle
+                    unsigned p[3][kTcPart];
+#pragma unroll
+                    for (int c = 0; c < kTcK / 4; ++c) {
+                        split3(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+                        split3(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) tmem_st16(to + ((o.at * 2 + half) * 3 + i) * kTcPart, p[i]);
+                }
+                wait_st();
+                fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(w_empty + r.at);
+                    mbar_arrive(split + o.at);
+                }
+                r.next(a.w_stages);
+                o.next(a.x_stages);
+            }
+        }
+    } else {
+        // ---------------- the sums: a lane a row of W, all or half of the tile's rows of x a warp ----------------
+        const int quarter = warp & 3, half = FEW ? a.nt : a.nt >> 1, c0 = warp >= 3 + kConverters + 4 ? half : 0;
+        RingAt r;
+        unsigned turn = 0;
+        for (long long t = first_unit; t < units && ok; t = next_unit(t)) {
+            const Unit u = unit_at(t);
+            float sum[kMine];
+#pragma unroll
+            for (int j = 0; j < kMine; ++j) sum[j] = 0.f;
+            for (int k = 0; k < u.steps; ++k, ++turn, r.next(a.x_stages)) {
+                const int b = turn & 1;
+                if (!wait(done + r.at, r.phase)) break;
+                fence_after();
+                const unsigned at = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(b * a.nt + c0);
+#pragma unroll
+                for (int j = 0; j < kMine; j += 16) {
+                    if (j < half) {
+                        float v[16];
+                        tmem_ld16(at + j, v);
+                        wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) sum[j + e] += v[e];
+                    }
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(added + b);
+            }
+            if (!ok) break;
+            const int m = u.m0 + quarter * 32 + lane, n0 = u.n0 + c0;
+            float bad = 0.f;
+#pragma unroll
+            for (int j = 0; j < kMine; ++j) bad += j < half ? sum[j] * 0.f : 0.f;      // not zero if one is not finite
+            if (__any_sync(0xffffffffu, bad != 0.f)) {
+                const float* x = a.x + (size_t)u.b * a.bx + u.k0;
+                const float* w = a.w + (size_t)u.b * a.bw + u.k0;
+#pragma unroll
+                for (int j = 0; j < kMine; ++j) {
+                    const bool mine = j < half && n0 + j < a.N && m < a.M && !isfinite(sum[j]);
+                    unsigned rows = __ballot_sync(0xffffffffu, mine);
+                    while (rows) {
+                        const int l = __ffs(rows) - 1;
+                        rows &= rows - 1;
+                        const float v = tc_again(x + (size_t)(n0 + j) * a.ldx, w + (size_t)(u.m0 + quarter * 32 + l) * a.ldw, min(a.share_len, a.K - u.k0));
+                        if (lane == l) sum[j] = v;
+                    }
+                }
+            }
+            const long long ldy = a.planes ? a.M : a.ldy;
+            float* y = (a.planes ? a.y + ((size_t)u.share * a.batch + u.b) * a.N * a.M : a.y + (size_t)u.b * a.by) + (size_t)n0 * ldy + m;
+            const bool more = !a.planes && u.share > 0;        // (the same thread wrote the shares before)
+#pragma unroll
+            for (int j = 0; j < kMine; j += 8) {
+                if (j >= half || m >= a.M) continue;
+                if (more) {
+                    float before[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) before[e] = n0 + j + e < a.N ? y[(size_t)e * ldy] : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) sum[j + e] += before[e];
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (n0 + j + e < a.N) y[(size_t)e * ldy] = sum[j + e];
+                y += 8 * ldy;
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        fence_after();
+        tmem_free(tmem_base, kTcCols);
+    }
+}
+
+// x's rows as three bfloat16 numbers a float: planes [batch][3][N][pitch]
+template <bool VEC>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, int N, int K, int pitch,
+                                                         long long ldx, long long bx) {
+    pdl_launch_dependents();
+    const int n = blockIdx.x, b = blockIdx.z;
+    const float* row = x + (size_t)b * bx + (size_t)n * ldx;
+    __nv_bfloat16* to = out + ((size_t)b * 3 * N + n) * pitch;
+    const size_t plane = (size_t)N * pitch;
+    for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4; c < K; c += gridDim.y * blockDim.x * 4) {
+        const float4 v = VEC ? *reinterpret_cast<const float4*>(row + c) : make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
+        uint2 p1, p2, p3;
+        tc5::split3(v.x, v.y, p1.x, p2.x, p3.x);
+        tc5::split3(v.z, v.w, p1.y, p2.y, p3.y);
+        *reinterpret_cast<uint2*>(to + c) = p1;
+        *reinterpret_cast<uint2*>(to + plane + c) = p2;
+        *reinterpret_cast<uint2*>(to + 2 * plane + c) = p3;
+    }
+}
+
 template <int TN, int TM, int AN, int AM>
 static int launch(const GemmArgs& a, bool vec, cudaStream_t stream) {
     constexpr int BN = TN * AN, BM = TM * AM;
@@ -162,87 +500,176 @@ static int launch(const GemmArgs& a, bool vec, cudaStream_t stream) {
     return blm_check_launch("gemm_f32");
 }
 
-static int shares_of(int K) { return (K + kShare - 1) / kShare; }
+// Rows of x of a tile, and whether every share of K is a block's own: the ones with the least time by this count.  A slice of a tile
+// takes what was measured for its rows of x (a block alone, 256 slices after one another: 87, 114, 132, 169, 202 us), the end of a
+// share some 1.5 us; planes of sums are a launch more and are written and read.
+struct Plan {
+    int nt, planes;
+};
+static Plan tc_plan(int batch, int N, int M, int K, int sms) {
+    constexpr double slice_us[kTcMost / 32] = {0.32, 0.405, 0.49, 0.63, 0.76};
+    Plan best = {32, 0};
+    double least = -1;
+    const int shares = (K + kTcShare - 1) / kTcShare;
+    for (int nt = 32; nt <= kTcMost; nt += 32)
+        for (int planes = 0; planes <= (shares > 1 ? 1 : 0); ++planes) {
+            const long long units = (long long)((N + nt - 1) / nt) * ((M + kTcRows - 1) / kTcRows) * batch * (planes ? shares : 1);
+            const long long rounds = (units + sms - 1) / sms;
+            const double share = (double)K / shares / kTcK * slice_us[nt / 32 - 1] + 1.5;
+            const double cost = rounds * share * (planes ? 1 : shares) + (planes ? 3 + 1.6e-6 * batch * shares * N * M : 0);
+            if (least < 0 || cost < least) {
+                least = cost;
+                best = {nt, planes};
+            }
+        }
+    return best;
+}
+
+// The tensor cores take it: by K and how W lies, never by N or M.
+static bool tc_takes(const float* w, int K, long long ldw, long long bw) {
+    return K >= kTcLeast && K % 4 == 0 && ((size_t)w & 15) == 0 && ldw > 0 && ldw % 4 == 0 && ldw < (1ll << 37) && bw >= 0 && bw % 4 == 0 &&
+           bw < (1ll << 37) && tc5::encode_tiled() != nullptr;
+}
+
+// x's parts go to `scratch`
+static int launch_tc(const GemmArgs& g, const Plan& plan, float* scratch, int* status, cudaStream_t stream) {
+    const int pitch = (g.K + 7) / 8 * 8;
+    __nv_bfloat16* parts = reinterpret_cast<__nv_bfloat16*>(scratch);
+    TcArgs a = {g.x, g.w, g.y, g.N, g.M, g.K, g.shares, ((g.K + g.shares - 1) / g.shares + 63) / 64 * 64, g.batch, g.ldx, g.ldw, g.ldy, g.bx, g.bw, g.by};
+    a.m_tiles = (g.M + kTcRows - 1) / kTcRows;
+    a.nt = plan.nt;
+    a.planes = plan.planes;
+    a.n_tiles = (g.N + a.nt - 1) / a.nt;
+    a.w_batches = g.batch > 1 && g.bw > 0 ? g.batch : 1;
+    a.status = status;
+    constexpr int kBarriers = 256;
+    const int x_step = 2 * a.nt * kTcK * 6;
+    a.x_stages = std::min(4, (kTcCols - 2 * a.nt) / (6 * kTcPart));
+    a.w_stages = std::min(6, (kTcSmem - kBarriers - a.x_stages * x_step) / kTcW);
+    const int smem = a.w_stages * kTcW + a.x_stages * x_step + kBarriers + 1024;
+    CUtensorMap xmap, wmap;
+    if (!tc5::make_map_3d(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, parts, {g.K, g.N, 3ll * g.batch}, {2ll * pitch, 2ll * pitch * g.N}, {2 * kTcK, a.nt, 3},
+                          CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !tc5::make_map_3d(&wmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, g.w, {g.K, g.M, a.w_batches}, {4 * g.ldw, a.w_batches > 1 ? 4 * g.bw : 4 * g.ldw},
+                          {kTcK, kTcRows, 1}, CU_TENSOR_MAP_SWIZZLE_128B))
+        return blm_fail(BLM_CUDA_ERROR, "gemm_f32: cuTensorMapEncodeTiled refused %d x %d x %d", g.N, g.M, g.K);
+    auto kernel = a.nt <= kTcFew ? gemm_f32_tc_kernel<true> : gemm_f32_tc_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem + 1024);
+    if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "gemm_f32: %s", cudaGetErrorString(e));
+    const bool vec = ((size_t)g.x & 15) == 0 && g.ldx % 4 == 0 && g.bx % 4 == 0;
+    const dim3 grid(g.N, std::min(8, (g.K + 1023) / 1024), g.batch);
+    if (vec) split_rows_kernel<true><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
+    else split_rows_kernel<false><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
+    if (int rc = blm_check_launch("gemm_f32 (parts)")) return rc;
+    const long long tiles = (long long)a.n_tiles * a.m_tiles * (a.planes ? g.shares : 1) * g.batch;
+    e = blm_launch_dependent(kernel, dim3((unsigned)std::min<long long>(tiles, blm_sm_count())), dim3(kTcThreads), smem, stream, a, xmap, wmap);
+    if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "gemm_f32: %s", cudaGetErrorString(e));
+    return blm_check_launch("gemm_f32 (tensor cores)");
+}
+
+static int shares_of(bool tc, int K) { return tc ? (K + kTcShare - 1) / kTcShare : (K + kShare - 1) / kShare; }
 
 // What one pass of a product takes: products (the grid's third dimension holds their shares), rows, columns.  With several shares a
-// pass is cut so that its planes of sums stay within kPlanes floats (256 MB), in even parts of whole tiles along the longer side
-// (every pass reads the shorter side's operand again): a large product would otherwise hold K / 1,024 times its result (2,048 rows
-// of logits over 128,256 columns and K 4,096: 4.2 GB).  Every pass ends in a round of blocks that
-// is not full: 600 x 32,768 x 4,096 in two passes 3,731 -> 3,776 us, 2,048 x 4,096 x 14,336 5,198 -> 5,229 (in six and eight: 3,842, 5,492).
-constexpr long long kPlanes = 64 << 20;
+// pass is cut so that its planes of sums stay within kPlanes floats (256 MB; on the tensor cores 192 MB, beside 24 MB for x's parts, which stay in L2), in
+// even parts of whole tiles along the longer side (every pass reads the shorter side's operand again): a large product would
+// otherwise hold K / 1,024 times its result (2,048 rows of logits over 128,256 columns and K 4,096: 4.2 GB).  Every pass ends in a
+// round of blocks that is not full: FFMA, 600 x 32,768 x 4,096 in two passes 3,731 -> 3,776 us, 2,048 x 4,096 x 14,336
+// 5,198 -> 5,229 (in six and eight: 3,842, 5,492).
+constexpr long long kPlanes = 64 << 20, kTcPlanes = 48 << 20, kTcParts = 6 << 20;
 struct Pass {
     int products, rows, cols;
 };
-static Pass pass_of(int batch, int N, int M, int K) {
-    const int shares = shares_of(K);
+static long long tc_parts(int products, int rows, int K) { return (long long)products * rows * ((K + 7) / 8 * 8) * 3 / 2; }      // floats
+static Pass pass_of(bool tc, int batch, int N, int M, int K) {
+    const int shares = shares_of(tc, K);
+    const long long planes = tc ? kTcPlanes : kPlanes;
     Pass p = {std::max(1, std::min(batch, 65535 / std::max(1, shares))), std::max(1, N), std::max(1, M)};
-    if (shares <= 1) return p;
+    if (tc && tc_parts(1, p.rows, K) > kTcParts) {
+        const long long parts = (tc_parts(1, p.rows, K) + kTcParts - 1) / kTcParts;
+        p.rows = (int)std::min<long long>(p.rows, ((p.rows + parts - 1) / parts + 63) / 64 * 64);
+        while (p.rows > 64 && tc_parts(1, p.rows, K) > kTcParts) p.rows = (p.rows - 1) / 64 * 64;
+    }
+    if (tc) p.products = (int)std::max(1ll, std::min<long long>(p.products, kTcParts / tc_parts(1, p.rows, K)));
+    if (shares <= 1 || (tc && !tc_plan(p.products, p.rows, p.cols, K, blm_sm_count()).planes)) return p;
     const long long one = (long long)shares * p.rows * p.cols;
-    if (one <= kPlanes) {
-        p.products = (int)std::min<long long>(p.products, kPlanes / one);
+    if (one <= planes) {
+        p.products = (int)std::min<long long>(p.products, planes / one);
         return p;
     }
     p.products = 1;
     auto cut = [&](int& side, int other) {     // in even parts, as many as it takes, none below a tile
-        const long long parts = ((long long)shares * side * other + kPlanes - 1) / kPlanes;
+        const long long parts = ((long long)shares * side * other + planes - 1) / planes;
         side = (int)std::min<long long>(side, ((side + parts - 1) / parts + 63) / 64 * 64);
-        while (side > 64 && (long long)shares * side * other > kPlanes) side = (side - 1) / 64 * 64;
+        while (side > 64 && (long long)shares * side * other > planes) side = (side - 1) / 64 * 64;
     };
     int &longer = p.cols >= p.rows ? p.cols : p.rows, &other = p.cols >= p.rows ? p.rows : p.cols;
     cut(longer, other);
-    if ((long long)shares * longer * other > kPlanes) cut(other, longer);
+    if ((long long)shares * longer * other > planes) cut(other, longer);
     return p;
 }
+static bool planes_of(bool tc, const Pass& p, int K) {
+    return shares_of(tc, K) > 1 && (!tc || tc_plan(p.products, p.rows, p.cols, K, blm_sm_count()).planes);
+}
+static long long scratch_of(bool tc, int batch, int N, int M, int K) {
+    const Pass p = pass_of(tc, batch, N, M, K);
+    return (planes_of(tc, p, K) ? (long long)shares_of(tc, K) * p.products * p.rows * p.cols : 0) + (tc ? tc_parts(p.products, p.rows, K) : 0);
+}
 
-// Floats of scratch a product needs: a plane of sums a share, none for a single share; and how many kernels it launches.
+// Floats of scratch a product needs, however W lies (planes of sums, x's parts);
 BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
     if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
-    const Pass p = pass_of(batch, N, M, K);
-    return shares_of(K) > 1 ? (long long)shares_of(K) * p.products * p.rows * p.cols : 0;
+    const long long ffma = scratch_of(false, batch, N, M, K);
+    return K >= kTcLeast && K % 4 == 0 ? std::max(ffma, scratch_of(true, batch, N, M, K)) : ffma;
 }
-BLM_API int blm_gemm_f32_launches(int batch, int N, int M, int K) {
+// whether the tensor cores form it, and how many kernels it launches.
+BLM_API int blm_gemm_f32_tensor(const float* w, int K, long long ldw, long long bw) { return tc_takes(w, K, ldw, bw); }
+BLM_API int blm_gemm_f32_launches(int tensor, int batch, int N, int M, int K) {
     if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
-    const Pass p = pass_of(batch, N, M, K);
-    return ((batch - 1) / p.products + 1) * ((N - 1) / p.rows + 1) * ((M - 1) / p.cols + 1) * (shares_of(K) > 1 ? 2 : 1);
+    const Pass p = pass_of(tensor, batch, N, M, K);
+    return ((batch - 1) / p.products + 1) * ((N - 1) / p.rows + 1) * ((M - 1) / p.cols + 1) * (1 + (tensor ? 1 : 0) + (planes_of(tensor, p, K) ? 1 : 0));
 }
 
 // `batch` products y[b] = x[b] . W[b]^T of one shape; the operands of product b lie b * (bx, bw, by) elements on.
 BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int batch, int N, int M, int K, long long ldx, long long ldw,
-                                 long long ldy, long long bx, long long bw, long long by, float* scratch, cudaStream_t stream) {
+                                 long long ldy, long long bx, long long bw, long long by, float* scratch, int* status, cudaStream_t stream) {
     if (N == 0 || M == 0 || batch == 0) return BLM_OK;
     BLM_REQUIRE(N > 0 && M > 0 && K > 0 && batch > 0, "gemm_f32: bad sizes %d x %d %d %d", batch, N, M, K);
-    const int shares = shares_of(K);
+    const bool tc = tc_takes(w, K, ldw, batch > 1 ? bw : 0);
+    const int shares = shares_of(tc, K);
     BLM_REQUIRE(batch <= 65535 && shares <= 65535 && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
-    BLM_REQUIRE(shares == 1 || scratch != nullptr, "gemm_f32: a sum over %d places needs scratch", K);
+    BLM_REQUIRE((shares == 1 && !tc) || (scratch != nullptr && status != nullptr), "gemm_f32: a sum over %d places needs scratch and a status word", K);
     // 16-byte pieces where every row starts at a multiple of 16 bytes, and 64 rows lie within what an int can tell
     const bool vec = (((size_t)x | (size_t)w) & 15) == 0 && ldx < (1 << 25) && ldw < (1 << 25) && K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bx % 4 == 0 && bw % 4 == 0;
     const bool vec4 = (((size_t)y | (size_t)scratch) & 15) == 0 && M % 4 == 0 && ldy % 4 == 0 && by % 4 == 0;
-    const Pass pass = pass_of(batch, N, M, K);
+    const Pass pass = pass_of(tc, batch, N, M, K);
+    const bool planes = planes_of(tc, pass, K);      // (a last, smaller pass as the others)
     for (int b0 = 0; b0 < batch; b0 += pass.products)
         for (int n0 = 0; n0 < N; n0 += pass.rows)
             for (int m0 = 0; m0 < M; m0 += pass.cols) {
                 const int products = std::min(pass.products, batch - b0), rows = std::min(pass.rows, N - n0), cols = std::min(pass.cols, M - m0);
                 float* to = y + (size_t)b0 * by + (size_t)n0 * ldy + m0;
-                const GemmArgs a = {x + (size_t)b0 * bx + (size_t)n0 * ldx, w + (size_t)b0 * bw + (size_t)m0 * ldw, shares > 1 ? scratch : to,
+                float* sums = tc ? scratch + tc_parts(products, rows, K) : scratch;
+                const GemmArgs a = {x + (size_t)b0 * bx + (size_t)n0 * ldx, w + (size_t)b0 * bw + (size_t)m0 * ldw, planes ? sums : to,
                                     rows, cols, K, shares, products, ldx, ldw, ldy, bx, bw, by};
                 // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights
                 // 49 us, with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
-                const int rc = rows <= 16   ? launch<4, 16, 4, 2>(a, vec, stream)
+                const int rc = tc           ? launch_tc(a, {tc_plan(products, rows, cols, K, blm_sm_count()).nt, planes}, scratch, status, stream)
+                               : rows <= 16 ? launch<4, 16, 4, 2>(a, vec, stream)
                                : rows <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
                                : rows <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
                                             : launch<8, 16, 8, 4>(a, vec, stream);
                 if (rc != BLM_OK) return rc;
-                if (shares == 1) continue;
+                if (!planes) continue;
                 const int per = 256 * (vec4 ? 4 : 1);
                 const dim3 grid(products * rows, (cols + per - 1) / per);
-                if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(scratch, to, rows, cols, shares, products, ldy, by);
-                else add_shares_kernel<1><<<grid, 256, 0, stream>>>(scratch, to, rows, cols, shares, products, ldy, by);
+                if (vec4) add_shares_kernel<4><<<grid, 256, 0, stream>>>(sums, to, rows, cols, shares, products, ldy, by);
+                else add_shares_kernel<1><<<grid, 256, 0, stream>>>(sums, to, rows, cols, shares, products, ldy, by);
                 if (int added = blm_check_launch("gemm_f32 (shares)")) return added;
             }
     return BLM_OK;
 }
 
 BLM_API int blm_gemm_f32(const float* x, const float* w, float* y, int N, int M, int K,
-                         long long ldx, long long ldw, long long ldy, float* scratch, cudaStream_t stream) {
-    return blm_gemm_f32_batched(x, w, y, 1, N, M, K, ldx, ldw, ldy, 0, 0, 0, scratch, stream);
+                         long long ldx, long long ldw, long long ldy, float* scratch, int* status, cudaStream_t stream) {
+    return blm_gemm_f32_batched(x, w, y, 1, N, M, K, ldx, ldw, ldy, 0, 0, 0, scratch, status, stream);
 }

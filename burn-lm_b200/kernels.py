@@ -209,11 +209,12 @@ _protos = {
     },
     "gemm": {
         "blm_gemm_f32": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
-                         c_longlong, c_void_p, c_void_p],
+                         c_longlong, c_void_p, c_void_p, c_void_p],
         "blm_gemm_f32_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
-                                 c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+                                 c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
         "blm_gemm_f32_scratch": [c_int, c_int, c_int, c_int],
-        "blm_gemm_f32_launches": [c_int, c_int, c_int, c_int],
+        "blm_gemm_f32_tensor": [c_void_p, c_int, c_longlong, c_longlong],
+        "blm_gemm_f32_launches": [c_int, c_int, c_int, c_int, c_int],
     },
     "gemv": {
         "blm_gemv": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
@@ -849,7 +850,7 @@ def attention(q, q_stride, pool, block_table, cu_seqlens, slot_of_seq, start_pos
 
 
 def gemm_f32(x, w, out=None):
-    """x [N, K] times w [M, K] transposed, in true fp32 (no tensor-core mode)."""
+    """x [N, K] times w [M, K] transposed in 32 bits: all 24 bits of both operands, float32 sums."""
     _need_cuda(x, w, out)
     if x.dtype != torch.float32 or w.dtype != torch.float32 or x.shape[1] != w.shape[1]:
         raise KernelError("gemm_f32: float32 x [N, K] and w [M, K]")
@@ -859,23 +860,29 @@ def gemm_f32(x, w, out=None):
         out = torch.empty((n, m), dtype=torch.float32, device=x.device)
     elif tuple(out.shape) != (n, m) or out.dtype != torch.float32:
         raise KernelError("gemm_f32: out must be float32 [N, M]")
-    scratch, launches = _gemm_f32_scratch(1, n, m, k, x.device)
-    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _stream(), kernels=launches)
+    scratch, launches = _gemm_f32_scratch(1, n, m, k, x.device, w)
+    _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _ptr(status_word(x.device)), _stream(),
+          kernels=launches)
     return out
 
 
-def _gemm_f32_scratch(batch, n, m, k, device):
-    """(a plane of sums for every share of K that the float32 product cuts its sums into, None where there is one share; the
-    kernels it launches: products whose planes would take more than 256 MB run in several passes)"""
+def _gemm_f32_scratch(batch, n, m, k, device, w=None):
+    """(scratch of a float32 product, None where it needs none: a plane of sums for every share of K that it cuts its sums into, and x
+    in three bfloat16 numbers a float where the tensor cores form it; the kernels it launches: products that would need more than
+    256 MB run in several passes).  `w` [M, K] or [B, M, K]: the weights; without them, rows at multiples of 16 bytes."""
     lib = _lib("gemm")
     floats = int(lib.blm_gemm_f32_scratch(batch, n, m, k))
-    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, int(lib.blm_gemm_f32_launches(batch, n, m, k))
+    if w is None:
+        tensor = lib.blm_gemm_f32_tensor(None, k, 4, 0)
+    else:
+        tensor = lib.blm_gemm_f32_tensor(_ptr(w), k, w.stride(-2), w.stride(0) if w.dim() == 3 and batch > 1 else 0)
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, int(lib.blm_gemm_f32_launches(tensor, batch, n, m, k))
 
 
 def batched_product(x, w, out=None, out_dtype=None):
     """out[b] = x[b] w[b]^T for a batch of small products of one shape: x [B, N, K], w [B, M, K], out [B, N, M]; the
     operands may be strided views (rows a fixed distance apart, unit stride along K and M).  float32 operands run this
-    package's FFMA product, true 32-bit; bfloat16 operands the library's batched product, as the plain products of a
+    package's 32-bit product; bfloat16 operands the library's batched product, as the plain products of a
     prompt do, with a bfloat16 or (`out_dtype`) float32 result."""
     _need = [t for t in (x, w, out) if t is not None]
     for t in _need:
@@ -890,10 +897,10 @@ def batched_product(x, w, out=None, out_dtype=None):
             out = torch.empty((b, n, m), dtype=torch.float32, device=x.device)
         if out.dtype != torch.float32 or tuple(out.shape) != (b, n, m) or any(t.stride(2) != 1 for t in (x, w, out)):
             raise KernelError("batched_product: float32 out [B, N, M]; unit stride along the last axis")
-        scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device)
+        scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device, w)
         _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, c_longlong(x.stride(1)), c_longlong(w.stride(1)),
               c_longlong(out.stride(1)), c_longlong(x.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)), _ptr(scratch),
-              _stream(), kernels=launches)
+              _ptr(status_word(x.device)), _stream(), kernels=launches)
         return out
     if out is not None:
         return torch.bmm(x, w.transpose(1, 2), out=out)
@@ -1068,7 +1075,7 @@ def check_status(device) -> None:
                 33: "prompt attention: a value tile did not arrive", 34: "prompt attention: the scores did not arrive",
                 35: "prompt attention: the probabilities were not written", 36: "prompt attention: the product with the values did not arrive",
                 37: "prompt attention: the producer waited in vain for a free stage",
-                11: "gemm_tc: the tensor-core thread waited in vain for a stage", 12: "gemm_tc: the producer waited in vain for a free stage",
+                15: "float32 product: a wait on an mbarrier ran out", 11: "gemm_tc: the tensor-core thread waited in vain for a stage", 12: "gemm_tc: the producer waited in vain for a free stage",
                 13: "gemm_tc: the epilogue waited in vain for the accumulator",
                 41: "gemm_sk: the tensor-core thread waited in vain for a stage", 42: "gemm_sk: the producer waited in vain for a free stage",
                 43: "gemm_sk: the epilogue waited in vain for the accumulator"}
