@@ -9,11 +9,14 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -160,7 +163,46 @@ def build_many(modules, verbose: bool = True) -> list[str]:
 
 
 def build_all(verbose: bool = True) -> list[str]:
-    return [build(m, verbose) for m in MODULES]
+    host = build_entry()
+    return [build(m, verbose) for m in MODULES] + ([host] if host else [])
+
+
+def build_entry() -> str | None:
+    """Compile entry.c, the native way to call an entry point, for this interpreter; None where that cannot be done (no C compiler, no
+    headers of the interpreter, another processor): ctypes calls them then."""
+    src = os.path.join(HERE, "entry.c")
+    with open(src, "rb") as f:
+        tag = hashlib.sha256(f.read() + sys.implementation.cache_tag.encode()).hexdigest()[:12]
+    out = os.path.join(_build_dir(), f"blm_entry_{tag}.so")
+    if os.path.exists(out):
+        return out
+    cc = shutil.which("gcc") or shutil.which("cc")
+    if cc is None:
+        return None
+    tmp = f"{out}.{os.getpid()}.tmp"
+    cmd = [cc, "-O2", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", tmp, src]
+    if subprocess.run(cmd, stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL).returncode != 0:
+        if os.path.exists(tmp):
+            os.remove(tmp)
+        return None
+    os.replace(tmp, out)
+    return out
+
+
+_entry_type: list = []
+
+
+def entry_type():
+    """The class of native callers (entry.c), or None."""
+    with _lock:
+        if not _entry_type:
+            path, made = build_entry(), None
+            if path:
+                loader = importlib.machinery.ExtensionFileLoader("blm_entry", path)
+                made = importlib.util.module_from_spec(importlib.util.spec_from_file_location("blm_entry", path, loader=loader))
+                loader.exec_module(made)
+            _entry_type.append(made.Entry if made else None)
+        return _entry_type[0]
 
 
 def load(module: str) -> ctypes.CDLL:

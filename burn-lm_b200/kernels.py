@@ -46,20 +46,20 @@ def _code(dtype: torch.dtype) -> int:
     raise KernelError(f"kernels take float32 or bfloat16, not {dtype}")
 
 
-def _ptr(t):
-    return c_void_p(t.data_ptr()) if t is not None else c_void_p(0)
+def _ptr(t) -> int:
+    return t.data_ptr() if t is not None else 0
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 _current_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
-def _stream():
+def _stream() -> int:
     """torch's current stream on the current device, as a raw handle.  Asked once per launch: the short way
     (two calls into torch's C module) costs a tenth of building a torch.cuda.Stream object each time."""
     if _raw_stream is not None and _current_device is not None:
-        return c_void_p(_raw_stream(_current_device()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _need_cuda(*tensors):
@@ -289,17 +289,38 @@ def launch_count() -> int:
 
 def stream_handle() -> int:
     """torch's current stream as an integer."""
-    return _stream().value or 0
+    return _stream()
+
+
+_entries: dict = {}
+
+
+def _entry(module: str, name: str):
+    """The entry point as a callable of plain numbers: native where that could be built (csrc/entry.c), else ctypes' own."""
+    lib = _lib(module)
+    fn, native = getattr(lib, name), _build.entry_type()
+    kinds = "".join("f" if t is c_float else "i" for t in fn.argtypes)
+    if native is not None and kinds.count("f") <= 8 and kinds.count("i") <= 64 and set(fn.argtypes) <= _NUMBERS:
+        fn = native(ctypes.cast(fn, c_void_p).value, kinds, fn.restype is c_longlong)
+    _entries[name] = fn
+    return fn
+
+
+_NUMBERS = {c_float, c_int, c_longlong, c_size_t, c_void_p}
 
 
 def _call(module: str, name: str, *args, kernels: int = 1):
     global _launches
-    lib = _lib(module)
-    rc = getattr(lib, name)(*args)
+    rc = (_entries.get(name) or _entry(module, name))(*args)
     _launches += kernels
     if rc != 0:
-        msg = getattr(lib, f"blm_{module}_last_error")().decode(errors="replace")
+        msg = getattr(_lib(module), f"blm_{module}_last_error")().decode(errors="replace")
         raise KernelError(f"{name}: {msg}")
+
+
+def _ask(module: str, name: str, *args) -> int:
+    """A question that launches nothing."""
+    return (_entries.get(name) or _entry(module, name))(*args)
 
 
 def loaded_modules():
@@ -346,7 +367,7 @@ def add_rmsnorm(resid, delta, gamma, eps, out, rows=None):
         raise KernelError("add_rmsnorm: rows must be int32")
     _call("elementwise", "blm_add_rmsnorm", _ptr(resid), _ptr(delta), _code(delta.dtype) if delta is not None else _code(out.dtype),
           _ptr(gamma), _code(gamma.dtype), _ptr(out),
-          _code(out.dtype), _ptr(rows), n_out, d, c_float(eps), _stream())
+          _code(out.dtype), _ptr(rows), n_out, d, eps, _stream())
 
 
 def add_rmsnorm_parts(resid, outputs, biases, gamma, eps, out, rows=None):
@@ -367,7 +388,7 @@ def add_rmsnorm_parts(resid, outputs, biases, gamma, eps, out, rows=None):
     os_, bs = outputs + [None] * (2 - len(outputs)), biases + [None] * (2 - len(biases))
     code = lambda t: _code(t.dtype) if t is not None else F32
     _call("elementwise", "blm_add_rmsnorm_parts", _ptr(resid), _ptr(os_[0]), code(os_[0]), _ptr(os_[1]), code(os_[1]), _ptr(bs[0]), _ptr(bs[1]),
-          _ptr(gamma), code(gamma), _ptr(out), code(out), _ptr(rows), n_out, d, c_float(eps), _stream())
+          _ptr(gamma), code(gamma), _ptr(out), code(out), _ptr(rows), n_out, d, eps, _stream())
 
 
 def embed_pairs(tokens, table, pairs, out, step, ids_pool, block_table, buckets, mul_prev, mul_cur, norm=None):
@@ -455,7 +476,7 @@ def qk_norm_append(proj, step, pool, block_table, q_out, n_heads, n_kv, key_dim,
         if t is not None and (t.dtype != torch.float32 or t.numel() != size):
             raise KernelError("qk_norm_append: weights, blend and values are float32 of the sizes the head counts give")
     _call("attention_sink", "blm_qk_norm_append", _ptr(proj), proj.stride(0), n, n_heads, n_kv, key_dim, value_dim, _ptr(q_weight),
-          _ptr(k_weight), c_float(eps), _ptr(blend), _ptr(values_in), _ptr(values_out), _ptr(q_out), _ptr(pool), _code(pool.dtype),
+          _ptr(k_weight), eps, _ptr(blend), _ptr(values_in), _ptr(values_out), _ptr(q_out), _ptr(pool), _code(pool.dtype),
           _flat_pool(pool, n_kv, key_dim, value_dim), PAGE, _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq),
           _ptr(block_table), block_table.shape[1], _stream())
 
@@ -494,16 +515,16 @@ def head_norm_rope_append(proj, step, pool, block_table, q_out, n_heads, n_kv, k
             raise KernelError("head_norm_rope_append: the norms' weights are float32 [key_dim]")
     if rotary_dims and (freq is None or freq.dtype != torch.float64 or freq.numel() != rotary_dims // 2):
         raise KernelError("head_norm_rope_append: freq must be float64 [rotary_dims / 2]")
-    _call("attention_sink", "blm_head_norm_rope_append", _ptr(proj), c_longlong(proj.stride(0)), n, n_heads, n_kv, int(maps), key_dim,
-          value_dim, _ptr(q_weight), _ptr(k_weight), c_float(eps), 1 if value_norm else 0, _ptr(freq), int(rotary_dims), 1 if halves else 0,
-          c_float(turn_scale), _ptr(table), table.shape[0] if table is not None else 0, _ptr(q_out), _ptr(pool), _code(pool.dtype), c_longlong(_flat_pool(pool, n_kv, key_dim, value_dim, maps, shared)), PAGE,
-          _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq), _ptr(block_table), block_table.shape[1], _ptr(bias), c_float(coef),
+    _call("attention_sink", "blm_head_norm_rope_append", _ptr(proj), proj.stride(0), n, n_heads, n_kv, int(maps), key_dim,
+          value_dim, _ptr(q_weight), _ptr(k_weight), eps, 1 if value_norm else 0, _ptr(freq), int(rotary_dims), 1 if halves else 0,
+          turn_scale, _ptr(table), table.shape[0] if table is not None else 0, _ptr(q_out), _ptr(pool), _code(pool.dtype), _flat_pool(pool, n_kv, key_dim, value_dim, maps, shared), PAGE,
+          _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq), _ptr(block_table), block_table.shape[1], _ptr(bias), coef,
           int(every), 1 if shared else 0, _stream())
 
 
 def attention_sink_pairs(dtype, key_dim, value_dim, n_heads, n_kv, maps) -> bool:
     """Whether the decode kernel takes both maps of a head in one block and, without splits, forms their difference itself."""
-    return bool(_lib("attention_sink").blm_attention_sink_pairs(_code(dtype), key_dim, value_dim, PAGE, n_heads, n_kv, maps))
+    return bool(_ask("attention_sink", "blm_attention_sink_pairs", _code(dtype), key_dim, value_dim, PAGE, n_heads, n_kv, maps))
 
 
 def attention_sink_scratch_floats(n_tokens, n_heads, value_dim, n_splits, maps=1, inside=False) -> int:
@@ -514,19 +535,19 @@ def attention_sink_scratch_floats(n_tokens, n_heads, value_dim, n_splits, maps=1
 
 def attention_sink_prompt_takes(dtype, key_dim, value_dim, max_q_len, n_heads) -> bool:
     """Whether a step of this shape runs the tensor-core prompt kernel (else the row kernel, which takes every shape)."""
-    return bool(_lib("attention_sink").blm_attention_sink_prompt_takes(_code(dtype), key_dim, value_dim, PAGE, max_q_len, n_heads))
+    return bool(_ask("attention_sink", "blm_attention_sink_prompt_takes", _code(dtype), key_dim, value_dim, PAGE, max_q_len, n_heads))
 
 
 def attention_sink_decode_takes(dtype, key_dim, value_dim, n_heads, n_kv) -> bool:
     """Whether single tokens and short portions of this shape run the tensor-core decode kernel, whose splits are cut by
     pages (else the row kernel, which takes every shape and cuts its splits by chunks of 32 keys)."""
-    return bool(_lib("attention_sink").blm_attention_sink_decode_takes(_code(dtype), key_dim, value_dim, PAGE, n_heads, n_kv))
+    return bool(_ask("attention_sink", "blm_attention_sink_decode_takes", _code(dtype), key_dim, value_dim, PAGE, n_heads, n_kv))
 
 
 def attention_sink_streams(dtype, key_dim, n_heads, n_kv) -> bool:
     """Whether single tokens whose values are the keys run the dense decoder's streaming kernel (with no other option than a window
     and slopes); its splits are then cut as that mixer's are."""
-    return bool(_lib("attention_sink").blm_attention_sink_streams(_code(dtype), key_dim, PAGE, n_heads, n_kv))
+    return bool(_ask("attention_sink", "blm_attention_sink_streams", _code(dtype), key_dim, PAGE, n_heads, n_kv))
 
 
 def attention_sink(q, step, pool, block_table, out, n_heads, n_kv, key_dim, value_dim, scale, window, keep_first=0, sink=True,
@@ -582,10 +603,10 @@ def attention_sink(q, step, pool, block_table, out, n_heads, n_kv, key_dim, valu
     _call("attention_sink", "blm_attention_sink", _ptr(q), _ptr(pool), _code(pool.dtype), _flat_pool(pool, n_kv, key_dim, value_dim, maps, shared),
           _ptr(block_table), block_table.shape[1], _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq), _ptr(cu),
           _ptr(step.start_pos if cu is not None else None), (cu.numel() - 1) if cu is not None else 0, int(max_q_len), _ptr(gate), int(gate_stride),
-          int(gate_lanes), _ptr(out), c_longlong(out.stride(0)), c_float(out_scale), _ptr(scratch if need else None), int(n_splits), n, n_heads,
-          n_kv, int(maps), key_dim, value_dim, PAGE, int(window), int(chunk), int(keep_first), c_float(scale), 1 if sink else 0,
-          _ptr(head_scale), _ptr(sink_logit if sink else None), c_float(softcap or 0.0), _ptr(slope), 1 if shared else 0,
-          *(c_float(v) for v in difference),
+          int(gate_lanes), _ptr(out), out.stride(0), out_scale, _ptr(scratch if need else None), int(n_splits), n, n_heads,
+          n_kv, int(maps), key_dim, value_dim, PAGE, int(window), int(chunk), int(keep_first), scale, 1 if sink else 0,
+          _ptr(head_scale), _ptr(sink_logit if sink else None), softcap or 0.0, _ptr(slope), 1 if shared else 0,
+          *difference,
           pool.shape[0] if cu is not None else 0, int(getattr(step, "max_kv_len", 0)), _ptr(status_word(q.device)) if cu is not None else None, _stream(),
           kernels=2 if need else 1)
 
@@ -655,13 +676,13 @@ def moe_experts(h, ids, weights, gate_up, down, extra=None, weight_on_input=True
     place_of = torch.empty(pairs, dtype=torch.int32, device=dev)
     act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
     # steps that bring an expert a few tokens cut the second product's reduction over several blocks: a plane of sums each
-    planes = int(_lib("moe").blm_moe_down_splits(_code(h.dtype), n, d, ff, e, top))
+    planes = _ask("moe", "blm_moe_down_splits", _code(h.dtype), n, d, ff, e, top)
     y = torch.empty((planes, pairs, d), dtype=torch.float32, device=dev)
     out = torch.empty((n, d), dtype=out_dtype or h.dtype, device=dev)
     stream = _stream()
     _call("moe", "blm_moe_group", _ptr(ids), pairs, e, _ptr(offsets), _ptr(order), _ptr(place_of), stream)
     _call("moe", "blm_moe_experts", _ptr(h), _code(h.dtype), _ptr(weights), _ptr(order), _ptr(offsets), _ptr(gate_up), _ptr(down),
-          _ptr(act), _ptr(y), n, d, ff, e, top, 1 if weight_on_input else 0, c_float(clamp_limit), c_float(clamp_alpha), int(unit), planes, stream, kernels=2)
+          _ptr(act), _ptr(y), n, d, ff, e, top, 1 if weight_on_input else 0, clamp_limit, clamp_alpha, int(unit), planes, stream, kernels=2)
     _call("moe", "blm_moe_combine", _ptr(y), _ptr(place_of), _ptr(weights), _ptr(extra), _ptr(out), _code(h.dtype), n, d, top,
           0 if weight_on_input else 1, _code(out.dtype), planes, stream)
     return out
@@ -684,7 +705,7 @@ def _moe_experts_tc(h, ids, weights, up, down, extra, out_dtype, unit=UNIT_GELU,
     ff = down.shape[2]
     top = ids.shape[1]
     pairs, dev, stream = n * top, h.device, _stream()
-    tiles = int(_lib("moe").blm_moe_padded_tiles(pairs, e, MOE_TC_ROWS))
+    tiles = _ask("moe", "blm_moe_padded_tiles", pairs, e, MOE_TC_ROWS)
     places = tiles * MOE_TC_ROWS
     place_of = torch.empty(pairs, dtype=torch.int32, device=dev)
     pair_of_place = torch.empty(places, dtype=torch.int32, device=dev)
@@ -696,10 +717,10 @@ def _moe_experts_tc(h, ids, weights, up, down, extra, out_dtype, unit=UNIT_GELU,
     status = status_word(dev)
     _call("moe", "blm_moe_group_padded", _ptr(ids), pairs, e, MOE_TC_ROWS, _ptr(place_of), _ptr(pair_of_place), _ptr(tile_expert), stream)
     _call("moe", "blm_moe_gather_rows", _ptr(h), _ptr(pair_of_place), _ptr(xs), places, d, top, stream)
-    _call("gemm_tc", "blm_gemm_tc_grouped", _ptr(xs), c_longlong(d), _ptr(up), c_longlong(d), _ptr(act), c_longlong(ff), places, rows, d, e,
-          _ptr(tile_expert), MOE_TC_UNITS[unit], c_float(clamp_limit), c_float(clamp_alpha), _ptr(status), stream)
-    _call("gemm_tc", "blm_gemm_tc_grouped", _ptr(act), c_longlong(ff), _ptr(down), c_longlong(ff), _ptr(y), c_longlong(d), places, d, ff, e,
-          _ptr(tile_expert), 4, c_float(0.0), c_float(0.0), _ptr(status), stream)
+    _call("gemm_tc", "blm_gemm_tc_grouped", _ptr(xs), d, _ptr(up), d, _ptr(act), ff, places, rows, d, e,
+          _ptr(tile_expert), MOE_TC_UNITS[unit], clamp_limit, clamp_alpha, _ptr(status), stream)
+    _call("gemm_tc", "blm_gemm_tc_grouped", _ptr(act), ff, _ptr(down), ff, _ptr(y), d, places, d, ff, e,
+          _ptr(tile_expert), 4, 0.0, 0.0, _ptr(status), stream)
     _call("moe", "blm_moe_combine", _ptr(y), _ptr(place_of), _ptr(weights), _ptr(extra), _ptr(out), _code(h.dtype), n, d, top,
           1, _code(out.dtype), 1, stream)
     return out
@@ -712,7 +733,7 @@ def rope_table(inv_freq, n_positions, turn_scale=1.0):
     _need_cuda(inv_freq)
     half = inv_freq.numel()
     table = torch.empty((n_positions, half, 2), dtype=torch.float32, device=inv_freq.device)
-    _call("elementwise", "blm_rope_table", _ptr(inv_freq), _ptr(table), n_positions, half, c_float(turn_scale), _stream())
+    _call("elementwise", "blm_rope_table", _ptr(inv_freq), _ptr(table), n_positions, half, turn_scale, _stream())
     return table
 
 
@@ -748,7 +769,7 @@ def rope_append(qkv, token_seq, token_pos, slot_of_seq, block_table, inv_freq, r
           _ptr(slot_of_seq), _ptr(block_table), block_table.shape[1], _ptr(inv_freq), rotary_dim,
           int(interleaved), _ptr(pool), n, n_heads, n_kv, head_dim, PAGE, 1 if write_cache else 0,
           _ptr(table), table.shape[0] if table is not None else 0,
-          1 if (table is not None and max_position is not None and max_position < table.shape[0]) else 0, c_float(turn_scale), _stream())
+          1 if (table is not None and max_position is not None and max_position < table.shape[0]) else 0, turn_scale, _stream())
 
 
 def tiled_pair_order(head_dim: int) -> list:
@@ -770,7 +791,7 @@ def swiglu(gate_up, out, tile=0):
     n, two_i = gate_up.shape
     if tuple(out.shape) != (n, two_i // 2) or out.dtype != gate_up.dtype or two_i % 2:
         raise KernelError("swiglu: out must be [N, I] for gate_up [N, 2 I], same dtype")
-    _call("elementwise", "blm_swiglu", _ptr(gate_up), _ptr(out), c_longlong(out.stride(0)), _code(out.dtype), n, two_i // 2, tile, _stream())
+    _call("elementwise", "blm_swiglu", _ptr(gate_up), _ptr(out), out.stride(0), _code(out.dtype), n, two_i // 2, tile, _stream())
 
 
 def convert(src, dst):
@@ -779,7 +800,7 @@ def convert(src, dst):
     if src.numel() != dst.numel():
         raise KernelError("convert: sizes differ")
     _call("elementwise", "blm_convert", _ptr(src), _code(src.dtype), _ptr(dst), _code(dst.dtype),
-          c_size_t(src.numel()), _stream())
+          src.numel(), _stream())
 
 
 def decode_advance(tokens, pos, sampled, history, step_no, counters=None):
@@ -845,7 +866,7 @@ def attention(q, q_stride, pool, block_table, cu_seqlens, slot_of_seq, start_pos
     _call("attention", "blm_attention", _ptr(q), q_stride, _ptr(pool), _code(q.dtype), _ptr(block_table),
           block_table.shape[1], _ptr(cu_seqlens), _ptr(slot_of_seq), _ptr(start_pos), _ptr(out), _ptr(scratch),
           n_tokens, n_seqs, max_q_len, n_heads, n_kv, head_dim, PAGE, int(window or 0), n_splits,
-          c_float(scale), 1 if general_only else 0, _ptr(status_word(q.device)), pool.shape[0], int(max_kv_len), _ptr(seq_table),
+          scale, 1 if general_only else 0, _ptr(status_word(q.device)), pool.shape[0], int(max_kv_len), _ptr(seq_table),
           1 if ahead else 0, _stream(), kernels=2 if n_splits > 1 else 1)
 
 
@@ -898,8 +919,8 @@ def batched_product(x, w, out=None, out_dtype=None):
         if out.dtype != torch.float32 or tuple(out.shape) != (b, n, m) or any(t.stride(2) != 1 for t in (x, w, out)):
             raise KernelError("batched_product: float32 out [B, N, M]; unit stride along the last axis")
         scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device, w)
-        _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, c_longlong(x.stride(1)), c_longlong(w.stride(1)),
-              c_longlong(out.stride(1)), c_longlong(x.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)), _ptr(scratch),
+        _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, x.stride(1), w.stride(1),
+              out.stride(1), x.stride(0), w.stride(0), out.stride(0), _ptr(scratch),
               _ptr(status_word(x.device)), _stream(), kernels=launches)
         return out
     if out is not None:
@@ -921,11 +942,11 @@ class _GemvRope(ctypes.Structure):
 def gemv_supported(n_tokens, m, k, plain_tokens=False) -> bool:
     """Whether gemv() takes the shape.  `plain_tokens`: the input is a bfloat16 [N, K] tensor used row by row
     (no stream to normalise, no gathered rows): then a very wide K is taken too."""
-    return bool(_lib("gemv").blm_gemv_supported(n_tokens, m, k, 1 if plain_tokens else 0))
+    return bool(_ask("gemv", "blm_gemv_supported", n_tokens, m, k, 1 if plain_tokens else 0))
 
 
 def gemm_tc_supported(m, n, k) -> bool:
-    return bool(_lib("gemm_tc").blm_gemm_tc_supported(m, n, k))
+    return bool(_ask("gemm_tc", "blm_gemm_tc_supported", m, n, k))
 
 
 def gemm_tc(x, w, out=None, swiglu=False, add_into=None, relu2=False):
@@ -958,7 +979,7 @@ SK_TOKENS = 128          # gemm_sk takes up to this many tokens
 
 
 def gemm_sk_supported(n_tokens, m, k) -> bool:
-    return bool(_lib("gemm_sk").blm_gemm_sk_supported(n_tokens, m, k))
+    return bool(_ask("gemm_sk", "blm_gemm_sk_supported", n_tokens, m, k))
 
 
 def gemm_sk(w, x, out=None, add_into=None, swiglu=False, squares=None, eps=0.0, hand_over=None, rope=None):
@@ -1015,9 +1036,9 @@ def gemm_sk(w, x, out=None, add_into=None, swiglu=False, squares=None, eps=0.0, 
         raise KernelError("gemm_sk: out must be [N, M] bfloat16 (or float32 for a plain store)")
     _call("gemm_sk", "blm_gemm_sk", _ptr(w), w.stride(0), m_rows, k, _ptr(x), x.stride(0), n, _ptr(out),
           out.stride(0) if out is not None else 0, 1 if (out is not None and out.dtype == torch.float32) else 0, _ptr(add_into), epi,
-          _ptr(squares), squares.shape[0] if squares is not None else 0, c_float(eps), _ptr(next_gamma),
+          _ptr(squares), squares.shape[0] if squares is not None else 0, eps, _ptr(next_gamma),
           1 if (next_gamma is not None and next_gamma.dtype == torch.float32) else 0, _ptr(scaled), _ptr(squares_out),
-          ctypes.byref(rope_arg) if rope_arg is not None else None, _ptr(status_word(w.device)), _stream())
+          ctypes.addressof(rope_arg) if rope_arg is not None else None, _ptr(status_word(w.device)), _stream())
 
 
 def graph_step(graph_exec: int, dev_in, host_in, host_out, dev_out, dev_in2=None, host_in2=None, written_by_graph=False):
@@ -1031,7 +1052,7 @@ def graph_step(graph_exec: int, dev_in, host_in, host_out, dev_out, dev_in2=None
     nbytes = lambda t: t.numel() * t.element_size() if t is not None else 0
     fn = getattr(_lib("runtime"), "blm_graph_step")
     args = (c_void_p(graph_exec), _ptr(dev_in), c_void_p(host_in.data_ptr()), nbytes(host_in),
-            _ptr(dev_in2), c_void_p(host_in2.data_ptr()) if host_in2 is not None else c_void_p(0), nbytes(host_in2),
+            _ptr(dev_in2), c_void_p(host_in2.data_ptr()) if host_in2 is not None else 0, nbytes(host_in2),
             c_void_p(host_out.data_ptr()), _ptr(dev_out), nbytes(host_out), 1 if written_by_graph else 0, _stream())
 
     def again():
@@ -1046,7 +1067,7 @@ def host_device_pointer(pinned) -> int:
     if not pinned.is_pinned():
         raise KernelError("host_device_pointer: the tensor is not in pinned host memory")
     dev = c_void_p(0)
-    _call("runtime", "blm_host_device_pointer", c_void_p(pinned.data_ptr()), ctypes.byref(dev), kernels=0)
+    _call("runtime", "blm_host_device_pointer", pinned.data_ptr(), ctypes.addressof(dev), kernels=0)
     return int(dev.value or 0)
 
 
@@ -1055,11 +1076,12 @@ _status: dict = {}
 
 def status_word(device) -> torch.Tensor:
     """The device word in which kernels with bounded waits record that a wait ran out (0: all well)."""
-    dev = torch.device(device)
-    key = (dev.type, dev.index if dev.index is not None else torch.cuda.current_device())
-    w = _status.get(key)
+    w = _status.get(device)                    # (a tensor's device names its index)
     if w is None:
-        w = _status[key] = torch.zeros(1, dtype=torch.int32, device=dev)
+        dev = torch.device(device)
+        if dev.index is None:
+            return status_word(torch.device(dev.type, torch.cuda.current_device()))
+        w = _status[dev] = torch.zeros(1, dtype=torch.int32, device=dev)
     return w
 
 
@@ -1165,12 +1187,12 @@ def gemv(w, n_tokens, x=None, stream_rows=None, gamma=None, eps=0.0, rows=None, 
             or (swiglu and out.dtype != torch.bfloat16):
         raise KernelError("gemv: out must be [N, M] bfloat16 (or float32 for a plain store)")
     _call("gemv", "blm_gemv", _ptr(w), w.stride(0), m, k, _ptr(x), x.stride(0) if x is not None else 0,
-          _ptr(stream_rows), _ptr(gamma), 1 if (gamma is not None and gamma.dtype == torch.float32) else 0, c_float(eps),
+          _ptr(stream_rows), _ptr(gamma), 1 if (gamma is not None and gamma.dtype == torch.float32) else 0, eps,
           _ptr(rows), n_tokens, _ptr(out), out.stride(0) if out is not None else 0,
           1 if (out is not None and out.dtype == torch.float32) else 0, _ptr(add_into), _ptr(add_bias), epi,
           _ptr(squares), squares.shape[0] if squares is not None else 0,
           _ptr(next_gamma), 1 if (next_gamma is not None and next_gamma.dtype == torch.float32) else 0,
-          _ptr(scaled), _ptr(squares_out), ctypes.byref(rope_arg) if rope_arg is not None else None,
+          _ptr(scaled), _ptr(squares_out), ctypes.addressof(rope_arg) if rope_arg is not None else None,
           _ptr(status_word(w.device)), _stream())
 
 
@@ -1208,7 +1230,7 @@ def argmax(logits, out, mirror=None, tickets=None, advance=None):
     tokens, pos, history, step_no = fed if fed is not None else (None, None, None, None)
     _call("sampling", "blm_argmax", _ptr(logits), logits.stride(0), b, v, _ptr(out),
           c_void_p(host_device_pointer(mirror) if mirror is not None else 0), _ptr(scratch), _ptr(tickets),
-          _ptr(tokens), _ptr(pos), _ptr(history), _ptr(step_no), c_void_p(0), history.shape[0] if history is not None else 0,
+          _ptr(tokens), _ptr(pos), _ptr(history), _ptr(step_no), 0, history.shape[0] if history is not None else 0,
           _stream(), kernels=(1 if tickets is not None else 2) if need else 1)
     if advance is not None and fed is None:
         decode_advance(advance[0], advance[1], out, advance[2], advance[3])
@@ -1263,7 +1285,7 @@ def embed_scaled(tokens, table, out, scale: float):
     n, (v, d) = tokens.numel(), table.shape
     if tokens.dtype != torch.int32 or out.dtype != torch.float32 or tuple(out.shape) != (n, d):
         raise KernelError("embed_scaled: tokens int32 [N], out float32 [N, D]")
-    _call("stream_ops", "blm_embed_scaled", _ptr(tokens), _ptr(table), _code(table.dtype), _ptr(out), n, d, v, c_float(scale), _stream())
+    _call("stream_ops", "blm_embed_scaled", _ptr(tokens), _ptr(table), _code(table.dtype), _ptr(out), n, d, v, scale, _stream())
 
 
 def sandwich_norm(resid, delta, post_weight, mult, eps_post, pre_weight, eps_pre, out, rows=None, delta_bias=None, second=None):
@@ -1291,10 +1313,10 @@ def sandwich_norm(resid, delta, post_weight, mult, eps_post, pre_weight, eps_pre
     _need_cuda(delta_b)
     if delta_b is not None and (delta is None or delta_b.shape != delta.shape or delta_b.dtype != delta.dtype):
         raise KernelError("sandwich_norm: the second output must match the first in shape and dtype")
-    _call("stream_ops", "blm_sandwich_norm", _ptr(resid), _ptr(delta), _ptr(delta_b), c_float(sa), c_float(sb),
+    _call("stream_ops", "blm_sandwich_norm", _ptr(resid), _ptr(delta), _ptr(delta_b), sa, sb,
           _code(delta.dtype) if delta is not None else F32,
-          _ptr(delta_bias), _ptr(post_weight), _ptr(pre_weight if out is not None else None), c_float(mult), c_float(eps_post),
-          c_float(eps_pre), _ptr(out), _code(out.dtype) if out is not None else F32, _ptr(rows), n_out, d, _stream())
+          _ptr(delta_bias), _ptr(post_weight), _ptr(pre_weight if out is not None else None), mult, eps_post,
+          eps_pre, _ptr(out), _code(out.dtype) if out is not None else F32, _ptr(rows), n_out, d, _stream())
 
 
 
@@ -1320,7 +1342,7 @@ def weighted_sum(a, scale_a, b, scale_b, out):
     _f32(a, b, out)
     if a.shape != b.shape or a.shape != out.shape:
         raise KernelError("weighted_sum: shapes differ")
-    _call("stream_ops", "blm_weighted_sum", _ptr(a), _ptr(b), _ptr(out), c_float(scale_a), c_float(scale_b), c_size_t(a.numel()), _stream())
+    _call("stream_ops", "blm_weighted_sum", _ptr(a), _ptr(b), _ptr(out), scale_a, scale_b, a.numel(), _stream())
 
 
 # ------------------------------------------------------------------------------------------------
@@ -1340,13 +1362,13 @@ def _state_args(state, offset):
     """state float32 [slots, 2, floats]: (pointer, floats a slot, floats a copy, this piece's offset in a copy)."""
     if state.dtype != torch.float32 or state.dim() != 3 or state.shape[1] != 2 or not state.is_contiguous():
         raise KernelError("a recurrent state is float32 [slots, 2, floats]")
-    return _ptr(state), c_longlong(2 * state.shape[2]), c_longlong(state.shape[2]), c_longlong(offset)
+    return _ptr(state), 2 * state.shape[2], state.shape[2], offset
 
 
 def _cols(t, col0, width):
     if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1 or col0 < 0 or col0 + width > t.shape[1]:
         raise KernelError("a column range must lie inside a float32 [N, *] tensor with unit stride along its rows")
-    return _ptr(t), c_longlong(t.stride(0)), int(col0)
+    return _ptr(t), t.stride(0), int(col0)
 
 
 def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, state_offset, silu=True, out_bf16=None, residual=False):
@@ -1372,7 +1394,7 @@ def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, sta
     single = getattr(step, "max_q_len", 0) == 1
     _call("recurrent", "blm_causal_conv", xp, xs, xc, channels, _ptr(taps), _ptr(bias), k, 2 if residual else (1 if silu else 0), op, os_, oc,
           _ptr(step.token_seq), _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs,
-          *_state_args(state, state_offset), 1 if single else 0, _ptr(out_bf16), c_longlong(channels), _stream(),
+          *_state_args(state, state_offset), 1 if single else 0, _ptr(out_bf16), channels, _stream(),
           kernels=2 if k > 1 and not single else 1)
 
 
@@ -1430,13 +1452,13 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
-              _ptr(d_skip), _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+              _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
               _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
               kernels=launches)
     if below == 0:
         return
     _call("recurrent", "blm_ssm_scan", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-          _ptr(y), c_longlong(y.stride(0)), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+          _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
           _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, below, _stream())
 
 
@@ -1458,12 +1480,12 @@ def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a
     scratch, launches, least, below = _scan_route(_SCAN_DELTA, heads, key_dim, step, out.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(None), _ptr(a_log), _ptr(out),
-              c_longlong(out.stride(0)), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+              out.stride(0), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
               _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
               kernels=launches)
     if below == 0:
         return
-    _call("recurrent", "blm_delta_scan", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(a_log), _ptr(out), c_longlong(out.stride(0)),
+    _call("recurrent", "blm_delta_scan", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(a_log), _ptr(out), out.stride(0),
           heads, qk_heads, key_dim, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_seqs,
           *_state_args(state, state_offset), below, _stream())
 
@@ -1479,7 +1501,7 @@ def shift_mix(x, mu, out, step, state, state_offset):
     if n != step.n_tokens or tuple(mu.shape) != (s, c) or tuple(out.shape) != (s, n, c):
         raise KernelError("shift_mix: x [N, C], mu [S, C], out [S, N, C]")
     single = getattr(step, "max_q_len", 0) == 1
-    _call("recurrent", "blm_shift_mix", _ptr(x), c_longlong(x.stride(0)), c, _ptr(mu), s, _ptr(out), _code(out.dtype),
+    _call("recurrent", "blm_shift_mix", _ptr(x), x.stride(0), c, _ptr(mu), s, _ptr(out), _code(out.dtype),
           _ptr(step.token_seq), _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), n, step.n_seqs,
           *_state_args(state, state_offset), 1 if single else 0, _stream(), kernels=1 if single else 2)
 
@@ -1499,7 +1521,7 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
     _need_cuda(bias, extra, out, state)
     _f32(bias, extra, out)
     qa = _cols(q, q_col0, heads * key_dim)
-    ka = _cols(k, k_col0, heads * key_dim) if k is not None else (c_void_p(0), c_longlong(0), 0)
+    ka = _cols(k, k_col0, heads * key_dim) if k is not None else (0, 0, 0)
     va = _cols(v, v_col0, heads * value_dim)
     aa = _cols(a, a_col0, heads * key_dim)
     if tuple(out.shape) != (step.n_tokens, heads * value_dim) or not out.is_contiguous() or bias.numel() != heads * key_dim:
@@ -1508,14 +1530,14 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
         raise KernelError("decay_scan: extra [heads * key_dim]")
     scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_DECAY, heads, key_dim, step, out.device)
     if scratch is not None:
-        _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, c_void_p(0), c_longlong(0), 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
-              _ptr(out), c_longlong(out.stride(0)), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
+        _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, 0, 0, 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
+              _ptr(out), out.stride(0), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
               1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs, least,
               *_state_args(state, state_offset), _ptr(scratch), _stream(),
               kernels=launches)
     if below == 0:
         return
-    _call("recurrent", "blm_decay_scan", *qa, *ka, *va, *aa, _ptr(bias), _ptr(extra), _ptr(out), c_longlong(out.stride(0)), heads,
+    _call("recurrent", "blm_decay_scan", *qa, *ka, *va, *aa, _ptr(bias), _ptr(extra), _ptr(out), out.stride(0), heads,
           key_dim, value_dim, int(kind), 1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos),
           step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, below, _stream())
 
@@ -1555,10 +1577,10 @@ def selective_scan(x, low, rank, n_state, dt_bias, a_log, d_skip, z, out, step, 
     for t in (z, out):
         if not t.is_cuda or tuple(t.shape) != (n, channels) or t.stride(1) != 1:
             raise KernelError("selective_scan: z and out are CUDA tensors [N, C] with unit stride along their rows")
-    _call("recurrent", "blm_selective_scan", _ptr(x), c_longlong(x.stride(0)), _ptr(low), c_longlong(low.stride(0)), int(rank),
-          int(rank + n_state), _ptr(dt), c_longlong(channels), _ptr(dt_weight), _code(dt_weight.dtype) if dt_weight is not None else F32,
-          int(rank), _ptr(dt_bias), _ptr(a_log), _ptr(rates), _ptr(d_skip), _ptr(z), c_longlong(z.stride(0)), _ptr(out), _code(out.dtype),
-          c_longlong(out.stride(0)), c_float(scale), channels, int(n_state), _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+    _call("recurrent", "blm_selective_scan", _ptr(x), x.stride(0), _ptr(low), low.stride(0), int(rank),
+          int(rank + n_state), _ptr(dt), channels, _ptr(dt_weight), _code(dt_weight.dtype) if dt_weight is not None else F32,
+          int(rank), _ptr(dt_bias), _ptr(a_log), _ptr(rates), _ptr(d_skip), _ptr(z), z.stride(0), _ptr(out), _code(out.dtype),
+          out.stride(0), scale, channels, int(n_state), _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
           _ptr(step.start_pos), step.n_seqs, 1 if getattr(step, "max_q_len", 0) == 1 else 0, *_state_args(state, state_offset), _stream())
 
 
@@ -1581,9 +1603,9 @@ def gated_group_norm(y, gate, gate_col0, weight, group, mode, eps, out):
     n, c = y.shape
     if c % group or weight.numel() not in (c, group) or tuple(out.shape) != (n, c) or not y.is_contiguous() or not out.is_cuda or out.stride(1) != 1:
         raise KernelError("gated_group_norm: groups must divide the row; weight of a row's or a group's size")
-    gp, gs, gc = _cols(gate, gate_col0, c) if gate is not None else (c_void_p(0), c_longlong(0), 0)
-    _call("recurrent", "blm_gated_group_norm", _ptr(y), c_longlong(y.stride(0)), gp, gs, gc, _ptr(weight), weight.numel(), group,
-          c // group, int(mode), c_float(eps), _ptr(out), _code(out.dtype), c_longlong(out.stride(0)), n, _stream())
+    gp, gs, gc = _cols(gate, gate_col0, c) if gate is not None else (0, 0, 0)
+    _call("recurrent", "blm_gated_group_norm", _ptr(y), y.stride(0), gp, gs, gc, _ptr(weight), weight.numel(), group,
+          c // group, int(mode), eps, _ptr(out), _code(out.dtype), out.stride(0), n, _stream())
 
 
 # ------------------------------------------------------------------------------------------------
@@ -1612,18 +1634,18 @@ def _retention_args(what, proj, step, state, state_offset, heads, key_dim, value
     ptr, slot_stride, copy_stride, offset = _state_args(state, state_offset)
     if state_offset + heads * key_dim * value_dim > state.shape[2]:
         raise KernelError(f"{what}: a state copy of {state.shape[2]} floats is too small")
-    return [_ptr(proj), c_longlong(proj.stride(0)), heads, key_dim, value_dim, c_float(k_scale), _ptr(freq), int(rotary_dims), _ptr(table),
+    return [_ptr(proj), proj.stride(0), heads, key_dim, value_dim, k_scale, _ptr(freq), int(rotary_dims), _ptr(table),
             table.shape[0] if table is not None else 0, _ptr(powers), _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos),
             step.n_seqs, ptr, slot_stride, copy_stride, offset]
 
 
 def retention_chunks_take(key_dim, value_dim) -> bool:
     """Whether portions with heads of these sizes run by chunks on the tensor cores (bfloat16; else the scan)."""
-    return bool(_lib("retention").blm_retention_chunks_take(key_dim, value_dim))
+    return bool(_ask("retention", "blm_retention_chunks_take", key_dim, value_dim))
 
 
 def retention_step_takes(key_dim, value_dim) -> bool:
-    return bool(_lib("retention").blm_retention_step_takes(key_dim, value_dim))
+    return bool(_ask("retention", "blm_retention_step_takes", key_dim, value_dim))
 
 
 def retention_scan(proj, step, state, state_offset, heads, key_dim, value_dim, k_scale, powers, o, freq=None, rotary_dims=0, table=None):
@@ -1635,7 +1657,7 @@ def retention_scan(proj, step, state, state_offset, heads, key_dim, value_dim, k
     _need_cuda(o)
     if o.dtype != torch.float32 or tuple(o.shape) != (proj.shape[0], heads * value_dim):
         raise KernelError("retention_scan: o is float32 [N, heads * value_dim]")
-    _call("retention", "blm_retention_scan", *args, _ptr(o), c_longlong(o.stride(0)), _stream())
+    _call("retention", "blm_retention_scan", *args, _ptr(o), o.stride(0), _stream())
 
 
 def retention(proj, step, state, state_offset, heads, key_dim, value_dim, k_scale, powers, eps, out, freq=None, rotary_dims=0, table=None):
@@ -1647,14 +1669,14 @@ def retention(proj, step, state, state_offset, heads, key_dim, value_dim, k_scal
     if not out.is_cuda or tuple(out.shape) != (n, heads * value_dim) or out.stride(1) != 1:
         raise KernelError("retention: out is a CUDA tensor [N, heads * value_dim] with unit stride along its rows")
     if step.max_q_len == 1:
-        _call("retention", "blm_retention_step", *args, _ptr(step.token_seq), _ptr(step.token_pos), n, c_float(eps), _ptr(out), _code(out.dtype),
-              c_longlong(out.stride(0)), _stream())
+        _call("retention", "blm_retention_step", *args, _ptr(step.token_seq), _ptr(step.token_pos), n, eps, _ptr(out), _code(out.dtype),
+              out.stride(0), _stream())
         return
     if out.dtype != torch.bfloat16:
         raise KernelError("retention: portions by chunks write bfloat16")
-    chunks = int(_lib("retention").blm_retention_chunks(n, step.n_seqs))
+    chunks = _ask("retention", "blm_retention_chunks", n, step.n_seqs)
     kv = torch.empty(chunks * heads * key_dim * value_dim, dtype=torch.float32, device=proj.device)
-    _call("retention", "blm_retention_portions", *args, n, c_float(eps), _ptr(kv), _ptr(out), c_longlong(out.stride(0)), _stream(), kernels=3)
+    _call("retention", "blm_retention_portions", *args, n, eps, _ptr(kv), _ptr(out), out.stride(0), _stream(), kernels=3)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -1677,18 +1699,18 @@ def bias_rope_append(proj, bias, freq, rotary_dim, q_out, pool, block_table, ste
         raise KernelError("bias_rope_append: the pool does not consist of pages of keys [kv, PAGE, key_dim] and values [kv, PAGE, value_dim]")
     if rotary_dim and (freq is None or freq.dtype != torch.float64 or freq.numel() != rotary_dim // 2):
         raise KernelError("bias_rope_append: freq must be float64 [rotary_dim / 2]")
-    _call("attention_sigmoid", "blm_bias_rope_append", _ptr(proj), c_longlong(proj.stride(0)), _ptr(bias), _ptr(freq), int(rotary_dim),
+    _call("attention_sigmoid", "blm_bias_rope_append", _ptr(proj), proj.stride(0), _ptr(bias), _ptr(freq), int(rotary_dim),
           _ptr(q_out), _ptr(pool), _code(pool.dtype), _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq),
           _ptr(block_table), block_table.shape[1], n, n_heads, n_kv, key_dim, value_dim, PAGE, _stream())
 
 
 def sigmoid_attention_takes(dtype, n_heads, n_kv, key_dim, value_dim) -> bool:
-    return bool(_lib("attention_sigmoid").blm_sigmoid_attention_takes(_code(dtype), n_heads, n_kv, key_dim, value_dim, PAGE))
+    return bool(_ask("attention_sigmoid", "blm_sigmoid_attention_takes", _code(dtype), n_heads, n_kv, key_dim, value_dim, PAGE))
 
 
 def sigmoid_attention_in_registers(dtype, n_heads, n_kv, key_dim, value_dim) -> bool:
     """Whether a shape runs the kernels that keep weights and mix in registers (attention_quads.cu)."""
-    return dtype == torch.bfloat16 and bool(_lib("attention_quads").blm_attention_quads_takes(n_heads, n_kv, key_dim, value_dim, PAGE))
+    return dtype == torch.bfloat16 and bool(_ask("attention_quads", "blm_attention_quads_takes", n_heads, n_kv, key_dim, value_dim, PAGE))
 
 
 def sigmoid_attention_ranges(step, n_heads, n_kv, key_dim, value_dim, dtype, device) -> int:
@@ -1734,12 +1756,12 @@ def sigmoid_attention(q, pool, block_table, step, out, n_heads, n_kv, key_dim, v
         _call("attention_quads", "blm_attention_quads", _ptr(q), _ptr(pool), _ptr(block_table), block_table.shape[1], _ptr(step.cu_seqlens),
               _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias), _ptr(out),
               _ptr(partial if ranges > 1 else None), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE, int(ranges),
-              c_float(scale), c_float(softcap), _stream(), kernels=2 if ranges > 1 else 1)
+              scale, softcap, _stream(), kernels=2 if ranges > 1 else 1)
         return
     _call("attention_sigmoid", "blm_sigmoid_attention", _ptr(q), _ptr(pool), _code(pool.dtype), _ptr(block_table), block_table.shape[1],
           _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias),
           _ptr(out), _ptr(partial), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE, int(ranges),
-          c_float(scale), c_float(softcap), 1 if scalar_only else 0, _stream(), kernels=2 if ranges > 1 else 1)
+          scale, softcap, 1 if scalar_only else 0, _stream(), kernels=2 if ranges > 1 else 1)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -1774,8 +1796,8 @@ def latent_prepare(q_proj, down, c_weight, eps, freq, rot_dims, q_nope, q_rot, p
         raise KernelError("latent_prepare: the pool does not consist of pages [PAGE, rank + rot_dim]")
     if rot_dims and (freq is None or freq.dtype != torch.float64 or freq.numel() != rot_dims // 2):
         raise KernelError("latent_prepare: freq must be float64 [rot_dims / 2]")
-    _call("attention_latent", "blm_latent_prepare", _ptr(q_proj), c_longlong(q_proj.stride(0)), _ptr(down), c_longlong(down.stride(0)),
-          _ptr(c_weight), c_float(eps), _ptr(freq), int(rot_dims), _ptr(q_nope), _ptr(q_rot), _ptr(q_full), int(hd_full), _ptr(pool),
+    _call("attention_latent", "blm_latent_prepare", _ptr(q_proj), q_proj.stride(0), _ptr(down), down.stride(0),
+          _ptr(c_weight), eps, _ptr(freq), int(rot_dims), _ptr(q_nope), _ptr(q_rot), _ptr(q_full), int(hd_full), _ptr(pool),
           _code(pool.dtype), _ptr(step.token_seq), _ptr(step.token_pos), _ptr(step.slot_of_seq), _ptr(block_table), block_table.shape[1],
           n, n_heads, key_dim, rot_dim, rank, PAGE, 1 if halves else 0, _stream())
 
@@ -1806,7 +1828,7 @@ def latent_expand(kv, gathered, out, n_heads, key_dim, rot_dim, value_dim, rank)
             or tuple(out.shape) != (rows // PAGE, 2, n_heads, PAGE, hd) or hd < max(key_dim + rot_dim, value_dim)):
         raise KernelError("latent_expand: kv [rows, heads * (key_dim + value_dim)], gathered [rows, rank + rot_dim], "
                           "out [rows / PAGE, 2, heads, PAGE, hd]")
-    _call("attention_latent", "blm_latent_expand", _ptr(kv), c_longlong(kv.stride(0)), _ptr(gathered), _ptr(out), _code(out.dtype),
+    _call("attention_latent", "blm_latent_expand", _ptr(kv), kv.stride(0), _ptr(gathered), _ptr(out), _code(out.dtype),
           rows // PAGE, n_heads, key_dim, rot_dim, value_dim, rank, hd, PAGE, _stream())
 
 
@@ -1817,7 +1839,7 @@ def latent_attention_scratch_floats(n_tokens, n_heads, rank, n_splits) -> int:
 def latent_attention_tile_rows(dtype, n_heads, rank, rot_dim, max_q_len) -> int:
     """How many rows (new token x head) a block of latent_attention owns at these sizes: 16 on the CUDA cores, 16 or 32
     on the tensor cores (a bfloat16 cache whose latent and rotated part are multiples of 16 lanes, up to 512)."""
-    return int(_lib("attention_latent").blm_latent_attention_tile_rows(_code(dtype), n_heads, rank, rot_dim, max_q_len))
+    return _ask("attention_latent", "blm_latent_attention_tile_rows", _code(dtype), n_heads, rank, rot_dim, max_q_len)
 
 
 def latent_attention_splits(dtype, n_heads, rank, rot_dim, n_seqs, max_q_len, keys, device) -> int:
@@ -1825,7 +1847,7 @@ def latent_attention_splits(dtype, n_heads, rank, rot_dim, n_seqs, max_q_len, ke
     than one round of blocks, and every block should still have a few pages of the longest sequence's `keys`."""
     rows = latent_attention_tile_rows(dtype, n_heads, rank, rot_dim, max_q_len)
     tiles = (max_q_len * n_heads + rows - 1) // rows * n_seqs
-    blocks = int(_lib("attention_latent").blm_latent_attention_blocks(_code(dtype), rank, rot_dim)) * sm_count(device)
+    blocks = _ask("attention_latent", "blm_latent_attention_blocks", _code(dtype), rank, rot_dim) * sm_count(device)
     return max(1, min(blocks // tiles, keys // (2 * PAGE), 32))
 
 
@@ -1849,7 +1871,7 @@ def latent_attention(q_lat, q_rot, pool, block_table, step, out, n_heads, rank, 
         raise KernelError("latent_attention: the workspace is too small for the key shares")
     _call("attention_latent", "blm_latent_attention", _ptr(q_lat), _ptr(q_rot), _ptr(pool), _code(pool.dtype), _ptr(block_table),
           block_table.shape[1], _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(out),
-          _code(out.dtype), _ptr(partial), n, step.n_seqs, step.max_q_len, n_heads, rank, rot_dim, PAGE, c_float(scale), int(n_splits),
+          _code(out.dtype), _ptr(partial), n, step.n_seqs, step.max_q_len, n_heads, rank, rot_dim, PAGE, scale, int(n_splits),
           int(window or 0), _ptr(sink), _stream(), kernels=2 if n_splits > 1 else 1)
 
 
@@ -1863,7 +1885,7 @@ def sigmoid_gate(o, gate, out, share=1):
     if (o.dim() != 2 or share < 1 or o.shape[1] % share or tuple(gate.shape) != (o.shape[0], o.shape[1] // share) or o.shape != out.shape
             or o.dtype != out.dtype):
         raise KernelError("sigmoid_gate: o and out [N, C], gate [N, C / share]; out in o's dtype")
-    _call("attention_latent", "blm_sigmoid_gate", _ptr(o), _code(o.dtype), _ptr(gate), _code(gate.dtype), c_longlong(gate.stride(0)),
+    _call("attention_latent", "blm_sigmoid_gate", _ptr(o), _code(o.dtype), _ptr(gate), _code(gate.dtype), gate.stride(0),
           _ptr(out), o.shape[0], o.shape[1], int(share), _stream())
 
 
@@ -1879,14 +1901,14 @@ def pack_cols(src, delta, dst, col0):
     if dst.dim() != 2 or dst.shape[0] != n or col0 < 0 or col0 + d > dst.shape[1] or (delta is not None and delta.shape != src.shape):
         raise KernelError("pack_cols: src [N, D], dst [N, W] with room for D columns at col0")
     _call("stream_ops", "blm_pack_cols", _ptr(src), _ptr(delta), _code(delta.dtype) if delta is not None else F32, _ptr(dst),
-          _code(dst.dtype), c_longlong(dst.stride(0)), int(col0), n, d, _stream())
+          _code(dst.dtype), dst.stride(0), int(col0), n, d, _stream())
 
 
 def softcap(x, cap: float = 0.0, scale: float = 1.0):
     """x <- cap * tanh(scale * x / cap) in place (cap 0: scale * x); x float32."""
     _need_cuda(x)
     _f32(x)
-    _call("stream_ops", "blm_softcap", _ptr(x), c_float(scale), c_float(cap), c_size_t(x.numel()), _stream())
+    _call("stream_ops", "blm_softcap", _ptr(x), scale, cap, x.numel(), _stream())
 
 
 def pass_entry(resid, delta, embedded, step):
