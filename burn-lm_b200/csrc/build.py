@@ -40,6 +40,7 @@ MODULES = {
     "stream_ops": ["stream_ops.cu"],
     "recurrent": ["recurrent.cu"],
     "scan_chunks": ["scan_chunks.cu"],
+    "scan_long": ["scan_long.cu"],
     "retention": ["retention.cu"],
     "attention_sigmoid": ["attention_sigmoid.cu"],
     "attention_quads": ["attention_quads.cu"],

@@ -15,6 +15,8 @@
 // Two launches.  What does not depend on the state (decayed rows, A, T) is formed for all chunks at once; then a block owns
 // (sequence, head, 16 or 32 value columns), holds its part of S in registers, and walks the sequence's chunks, while one more
 // warp brings the next chunk into shared memory (cp.async).
+#include <limits.h>
+
 #include "common.cuh"
 
 BLM_API const char* blm_scan_chunks_last_error() { return g_blm_error; }
@@ -34,7 +36,7 @@ __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + lo
 // which is below n_tokens / 8: the ceil(n / 16) chunks of n >= 16 tokens are no more than n / 8, rounded down.
 struct Chunks {
     const int* cu;
-    int n_seqs, least, packed;
+    int n_seqs, least, most, packed;   // (sequences of `most` or more tokens are run by scan_long.cu)
     int from, count;               // the chunk indexes of this pass
 };
 static bool chunks_packed(int n_tokens, int n_seqs, int least) { return least >= kQ && n_tokens / (kQ / 2) < (long long)n_tokens / kQ + n_seqs; }
@@ -62,7 +64,7 @@ __device__ __forceinline__ bool find_chunk(int idx, const Chunks& ch, int* found
     __syncthreads();
     for (int s = threadIdx.x; s < ch.n_seqs; s += blockDim.x) {
         const int lo = ch.cu[s], n = ch.cu[s + 1] - lo, base = chunk_base(lo, s, ch.packed);
-        if (n >= ch.least && idx >= base && idx < base + (n + kQ - 1) / kQ) {
+        if (n >= ch.least && n < ch.most && idx >= base && idx < base + (n + kQ - 1) / kQ) {
             found[0] = s;
             found[1] = idx - base;
         }
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
     float* Ws = sm + kStages * kStage;               // delta: v - acc, then the corrected values, [2][16][CT]
     const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
     const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
-    if (n_new < a.ch.least) return;
+    if (n_new < a.ch.least || n_new >= a.ch.most) return;
     // the sequence's chunks of this pass: from `lo` up to `hi`; `base`: where its first one lies, or would lie, in scratch
     const int base = chunk_base(first, seq, a.ch.packed) - a.ch.from, start = a.start_pos[seq];
     const int lo = max(0, -base), hi = min((n_new + kQ - 1) / kQ, a.ch.count - base);
@@ -795,12 +797,12 @@ static int check_step(int n_tokens, int n_seqs, int heads, int least) {
 BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
                                 long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                                 long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
-                                const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, float* state,
+                                const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, int most, float* state,
                                 long long slot_stride, long long copy_stride, long long state_off, float* scratch, cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
-    Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least), 0, 0};
+    Chunks ch = {cu_seqlens, n_seqs, least, most, chunks_packed(n_tokens, n_seqs, least), 0, 0};
     const int np = padded_rows(N), per = heads / groups;
     SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
                      scratch};
@@ -862,7 +864,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(qk_heads > 0 && heads % qk_heads == 0 && dk > 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
-    Chunks ch = {cu_seqlens, n_seqs, least, chunks_packed(n_tokens, n_seqs, least), 0, 0};
+    Chunks ch = {cu_seqlens, n_seqs, least, INT_MAX, chunks_packed(n_tokens, n_seqs, least), 0, 0};
     const bool delta = b_raw != nullptr;
     BLM_REQUIRE(delta ? k != nullptr && A_log != nullptr && !read_first && !lower_bound : (k != nullptr || lower_bound), "scan_chunks: no keys");
     BLM_REQUIRE(!lower_bound || (extra != nullptr && !read_first), "scan_chunks: a lower bound, and the state read last");

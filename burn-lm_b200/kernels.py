@@ -146,12 +146,19 @@ _protos = {
         "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int, c_int],
         "blm_scan_chunks_launches": [c_int, c_int, c_int, c_int, c_int, c_int],
         "blm_scan_chunks_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                 c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
         "blm_scan_chunks_rows": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p,
                                  c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong,
                                  c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                  c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+    },
+    "scan_long": {
+        "blm_scan_long_scratch": [c_int] * 7,
+        "blm_scan_long_launches": [c_int] * 7,
+        "blm_scan_chunks_long_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
+                                     c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                     c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
     },
     "retention": {
         "blm_retention_scan": _RETENTION + [c_void_p, c_longlong, c_void_p],
@@ -252,7 +259,7 @@ _protos = {
 _bound: dict[str, ctypes.CDLL] = {}
 
 
-_LONG_RESULTS = ("blm_scan_chunks_scratch", "blm_gemm_f32_scratch")     # entry points that return a number of floats instead of a status
+_LONG_RESULTS = ("blm_scan_chunks_scratch", "blm_scan_long_scratch", "blm_gemm_f32_scratch")     # entry points that return a number of floats instead of a status
 
 
 def _lib(module: str) -> ctypes.CDLL:
@@ -1414,8 +1421,10 @@ _NO_LIMIT = (1 << 31) - 1
 
 
 def scan_runs(lengths) -> tuple:
-    """What a step's new tokens by sequence bring the matrix-state scans: (some sequence is run in chunks, some is walked)."""
-    return max(lengths, default=0) >= SCAN_CHUNK_TOKENS, min(lengths, default=0) < SCAN_CHUNK_TOKENS
+    """What a step's new tokens by sequence bring the matrix-state scans: (some sequence is run in chunks, some is
+    walked, some may be run as a long one, all are)."""
+    least, most = min(lengths, default=0), max(lengths, default=0)
+    return most >= SCAN_CHUNK_TOKENS, least < SCAN_CHUNK_TOKENS, most >= SCAN_LONG_TOKENS, least >= SCAN_LONG_TOKENS_FEW_HEADS
 
 
 def _scan_route(kind, heads, rows, step, device):
@@ -1423,7 +1432,7 @@ def _scan_route(kind, heads, rows, step, device):
     from which they run a sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
     its own length, which the kernels read; step.scan_runs says which of the two have work (the engine's steps know)."""
     longest = getattr(step, "max_q_len", 0)
-    in_chunks, walked = getattr(step, "scan_runs", None) or (longest >= SCAN_CHUNK_RUN, step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs)
+    in_chunks, walked = (getattr(step, "scan_runs", None) or ())[:2] or (longest >= SCAN_CHUNK_RUN, step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs)
     if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
         least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
         lib, sizes = _lib("scan_chunks"), (kind, heads, rows, step.n_tokens, step.n_seqs, least)
@@ -1432,6 +1441,28 @@ def _scan_route(kind, heads, rows, step, device):
             return (torch.empty(floats, dtype=torch.float32, device=device), int(lib.blm_scan_chunks_launches(*sizes)), least,
                     SCAN_CHUNK_TOKENS if walked else 0)
     return None, 0, 0, _NO_LIMIT
+
+
+# From this many new tokens on, a sequence's state-space scan runs in chunks of 64 tokens on the tensor cores (scan_long.cu) where that
+# kernel takes the size: where the blocks of the chunks of sixteen tokens (16 columns of a head each) fill the multiprocessors
+# more than once, and where they do not.  One prompt of 1,024 / 2,048 / 2,700 tokens, states of 128 x 64, us by chunks of sixteen and here: 64
+# heads 126 / 230 / 300 and 106 / 124 / 208, 24 heads 79 / 136 / 173 and 103 / 108 / 114; 512 tokens of 64 heads 75 and 73, 600 85 and 97.
+SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1024, 2048
+
+
+def _long_route(heads, groups, n_state, value_dim, step, device):
+    """How a step's long sequences run: (scratch of scan_long.cu, how many of its kernels are launched, the length from which they run
+    a sequence, whether every sequence is as long), or None where they run none."""
+    longest, runs = min(getattr(step, "max_q_len", 0), step.n_tokens), getattr(step, "scan_runs", None)
+    if longest < SCAN_LONG_TOKENS or (runs is not None and len(runs) > 2 and not runs[2]):
+        return None
+    least = SCAN_LONG_TOKENS if heads * -(-value_dim // 16) > sm_count(device) else SCAN_LONG_TOKENS_FEW_HEADS
+    sizes = (heads, heads // groups, n_state, value_dim, step.n_tokens, step.n_seqs, longest)
+    floats = -(-_ask("scan_long", "blm_scan_long_scratch", *sizes) // 4) if longest >= least else 0
+    if floats == 0:
+        return None
+    alone = runs[3] if runs is not None and len(runs) > 3 else runs is None and step.n_seqs == 1 and longest == step.n_tokens
+    return torch.empty(floats, dtype=torch.float32, device=device), _ask("scan_long", "blm_scan_long_launches", *sizes), least, alone
 
 
 def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y, heads, groups, n_state, value_dim, step, state,
@@ -1449,17 +1480,26 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     dp, ds, dc = _cols(dt, dt_col0, heads)
     if tuple(y.shape) != (step.n_tokens, heads * value_dim) or not y.is_contiguous():
         raise KernelError("ssm_scan: y float32 [N, heads * value_dim]")
+    long = None if wide_sums else _long_route(heads, groups, n_state, value_dim, step, y.device)
+    if long is not None:
+        _call("scan_long", "blm_scan_chunks_long_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
+              _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, min(step.max_q_len, step.n_tokens), long[2], *_state_args(state, state_offset),
+              _ptr(long[0]), _ptr(status_word(y.device)), _stream(), kernels=long[1])
+        if long[3]:
+            return
+    most = long[2] if long is not None else _NO_LIMIT
     scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, most, *_state_args(state, state_offset), _ptr(scratch), _stream(),
               kernels=launches)
     if below == 0:
         return
     _call("recurrent", "blm_ssm_scan", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
           _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-          _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, below, _stream())
+          _ptr(step.start_pos), step.n_seqs, *_state_args(state, state_offset), 1 if wide_sums else 0, min(below, most), _stream())
 
 
 def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a_log, out, heads, qk_heads, key_dim, value_dim,

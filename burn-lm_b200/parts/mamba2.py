@@ -40,7 +40,7 @@ class Mamba2(Part):
     family = "mixer"
     graph_safe = True
     roles = ("in", "conv", "conv_bias", "dt_bias", "A_log", "D", "norm", "o")
-    kernel_modules = ("recurrent", "scan_chunks")
+    kernel_modules = ("recurrent", "scan_chunks", "scan_long")
 
     def __init__(self, spec, tensors, runtime):
         super().__init__(spec, tensors, runtime)

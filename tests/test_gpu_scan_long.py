@@ -1,0 +1,128 @@
+"""The state-space scan in chunks of 64 tokens on the tensor cores (scan_long.cu) against the walk in float64, at the edges of its chunks
+and groups of chunks, beside shorter sequences, with rows that cannot be copied in 16-byte pieces, and with values that are not finite."""
+import pytest
+import torch
+
+from burn_lm_b200 import kernels as K
+from test_gpu_scan_chunks import read_state, state_of, step_of, walk
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def from_64_tokens_on(monkeypatch):
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", 64)
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS_FEW_HEADS", 64)
+
+
+def inputs(heads, groups, rows, dv, n, gen, odd=0):
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    b0 = (heads * dv + 3) // 4 * 4 + odd
+    return rnd(n, b0 + 2 * groups * rows), b0, rnd(n, heads), rnd(heads) - 2, rnd(heads), rnd(heads)
+
+
+def scan(x, b0, dt, dt_bias, a_log, skip, heads, groups, rows, dv, step, state, offset):
+    out = torch.zeros((step.n_tokens, heads * dv), device="cuda")
+    K.ssm_scan(x, 0, b0, b0 + groups * rows, dt, 0, dt_bias, a_log, skip, out, heads, groups, rows, dv, step, state, offset)
+    return out
+
+
+@pytest.mark.parametrize("lens,starts", [([64], [0]), ([65], [5]), ([127, 40, 1, 576], [2, 0, 9, 1]), ([512, 513], [0, 3]), ([1153], [1])])
+@pytest.mark.parametrize("heads,groups,rows,dv", [(2, 1, 128, 64), (8, 2, 100, 36), (12, 3, 66, 63), (36, 1, 128, 64)])
+def test_long_sequences_against_the_walk_in_float64(heads, groups, rows, dv, lens, starts):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(heads + rows + sum(lens))
+    step, n, offset = step_of(lens, starts), sum(lens), 7
+    route = K._long_route(heads, groups, rows, dv, step, "cuda")
+    assert route is not None and route[2] == 64 and route[3] == (len(lens) == 1)
+    state = state_of(step, heads, rows, dv, offset, gen)
+    before = state.double()
+    x, b0, dt, dt_bias, a_log, skip = args = inputs(heads, groups, rows, dv, n, gen, odd=heads % 8 == 2)
+    out = scan(*args, heads, groups, rows, dv, step, state, offset)
+    f64 = lambda t, *shape: t.double().reshape(n, *shape)
+    d = torch.nn.functional.softplus(dt.double() + dt_bias.double())
+    v = f64(x[:, :heads * dv], heads, dv)
+    k = f64(x[:, b0:b0 + groups * rows], groups, rows).repeat_interleave(heads // groups, 1) * d[..., None]
+    q = f64(x[:, b0 + groups * rows:], groups, rows).repeat_interleave(heads // groups, 1)
+    w = torch.exp(-torch.exp(a_log.double()) * d)[..., None].expand(n, heads, rows)
+    at = 0
+    for s, (m, start) in enumerate(zip(lens, starts)):
+        slot, sl = int(step.slot_of_seq[s]), slice(at, at + m)
+        S = read_state(before, slot, start & 1, offset, heads, dv)[:, :rows]
+        want, S = walk(q[sl], k[sl], v[sl], w[sl], None, None, torch.zeros_like(S) if start == 0 else S)
+        want = want + skip.double()[:, None] * v[sl]
+        got = read_state(state, slot, (start + m) & 1, offset, heads, dv).double()
+        # as for the chunks of sixteen tokens: fp32 sums, decays of at most 64 factors, operands with all 24 bits
+        assert (out[sl].double().view(m, heads, dv) - want).abs().max() <= 1e-5 * want.abs().max()
+        assert (got[:, :rows] - S).abs().max() <= 1e-5 * S.abs().max()
+        assert not got[:, rows:].any()
+        at += m
+    assert torch.equal(state[:, :, :offset], before[:, :, :offset].float())
+    assert K.check_status("cuda") is None
+
+
+def test_a_sequence_has_the_bits_it_has_alone():
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    heads, groups, rows, dv, lens = 8, 2, 128, 64, [70, 30, 700, 64]
+    step = step_of(lens, [0, 0, 4, 1])
+    step.scan_runs = K.scan_runs(lens)
+    state = state_of(step, heads, rows, dv, 0, gen)
+    args = x, b0, dt, dt_bias, a_log, skip = inputs(heads, groups, rows, dv, sum(lens), gen)
+    together, own, at = state.clone(), state.clone(), 0
+    out = scan(*args, heads, groups, rows, dv, step, together, 0)
+    for s, m in enumerate(lens):
+        alone = step_of([m], [[0, 0, 4, 1][s]])
+        alone.slot_of_seq, alone.scan_runs = step.slot_of_seq[s:s + 1], K.scan_runs([m])
+        got = scan(x[at:at + m], b0, dt[at:at + m], dt_bias, a_log, skip, heads, groups, rows, dv, alone, own, 0)
+        assert torch.equal(got, out[at:at + m]), s
+        at += m
+    assert torch.equal(own, together)
+
+
+def test_scratch_is_bounded_and_heads_in_passes_change_no_bit():
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(4)
+    heads, groups, rows, dv, n = 64, 4, 128, 64, 12000
+    step = step_of([n], [0])
+    scratch, launches, _, _ = K._long_route(heads, groups, rows, dv, step, "cuda")
+    assert scratch.numel() <= 64 << 20 and launches > 3
+    state = state_of(step, heads, rows, dv, 0, gen)
+    x, b0, dt, dt_bias, a_log, skip = inputs(heads, groups, rows, dv, n, gen)
+    few = heads // groups                                                     # the heads of the first group, in one pass
+    part = torch.cat([x[:, :few * dv], x[:, b0:b0 + rows], x[:, b0 + groups * rows:b0 + (groups + 1) * rows]], 1).contiguous()
+    own = state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(state.shape[0], 2, -1).contiguous()
+    out = scan(x, b0, dt, dt_bias, a_log, skip, heads, groups, rows, dv, step, state, 0)
+    got = scan(part, few * dv, dt[:, :few].contiguous(), dt_bias[:few].contiguous(), a_log[:few].contiguous(), skip[:few].contiguous(), few, 1, rows, dv,
+               step, own, 0)
+    assert torch.equal(out[:, :few * dv], got)
+    assert torch.equal(state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(own.shape), own)
+
+
+@pytest.mark.parametrize("where", ["value", "key", "dt"])
+def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(where):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    heads, rows, dv, lens, bad = 4, 128, 64, [70, 640], 70 + 100              # (in the second chunk of the second sequence's first group)
+    step = step_of(lens, [0, 3])
+    state = state_of(step, heads, rows, dv, 0, gen)
+    x, b0, dt, *per_head = inputs(heads, 1, rows, dv, sum(lens), gen)
+    clean = scan(x, b0, dt, *per_head, heads, 1, rows, dv, step, state.clone(), 0)
+    for wrong in (float("nan"), float("inf"), float("-inf")):
+        x2, dt2, own = x.clone(), dt.clone(), state.clone()
+        if where == "value":
+            x2[bad, 5] = wrong                                                # one column of one head
+        elif where == "key":
+            x2[bad, b0:b0 + rows] = wrong
+        else:
+            dt2[bad] = float("nan")
+        out = scan(x2, b0, dt2, *per_head, heads, 1, rows, dv, step, own, 0)
+        assert torch.equal(out[:bad], clean[:bad])
+        last = own[int(step.slot_of_seq[1]), (3 + 640) & 1]
+        assert torch.isfinite(own[int(step.slot_of_seq[0])]).all() and not torch.isfinite(last).all()
+        if where == "value":
+            assert not torch.isfinite(out[bad, 5])
+            others = [c for c in range(heads * dv) if c != 5]
+            assert torch.equal(out[:, others], clean[:, others])
+        else:
+            assert not torch.isfinite(out[bad]).any()
