@@ -2,22 +2,24 @@
 //
 // Walked token by token (recurrent.cu) a prompt is a chain: every token waits for the sums over a state's rows of the one
 // before it, and a 2,048-token prompt took 1.1 to 1.8 ms for work that the multiprocessors' fp32 units can do in 0.07.  Here
-// a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 228, state-space scan
-// of 64 heads of 128 x 64 1,116 -> 218, delta rule of 16 heads of 128 x 128 over 1,501 + 500 tokens 1,224 -> 214).  With P(i..j) the product of the decays of the tokens i..j (per row, or
+// a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 182, state-space scan
+// of 64 heads of 128 x 64 1,116 -> 218, and 124 in chunks of 64 (scan_long.cu), delta rule of 16 heads of 128 x 128 over 1,501 + 500
+// tokens 1,224 -> 214).  With P(i..j) the product of the decays of the tokens i..j (per row, or
 // one number per head) and S the state in front of the chunk:
 //     out_j  = (P(0..j) q_j)^T S + sum_(i <= j) A_ji x_i,     A_ji = sum_rows q_j P(i+1..j) k_i
 //     S'     = P(0..15) S + sum_j (P(j+1..15) k_j) x_j^T
 // x is the value, or for the delta rule the corrected value: x = T (v - (P(0..j) k_j)^T S), T = (I + beta C)^-1 beta with
 // C_ji = k_j . P(i+1..j) k_i below the diagonal, so that the sixteen corrections, each of which waits for the one before it,
 // are one small triangular product.  Every factor is a product of at most 16 decays, never a quotient of two: nothing
-// overflows however strong a decay is, and all of it is fp32 multiply-adds, as in the walk.
+// overflows however strong a decay is, and all of it is float32 sums of products of whole floats, as in the walk: multiply-adds, or
+// six tensor-core products of bfloat16 parts.
 //
 // Two launches.  What does not depend on the state (decayed rows, A, T) is formed for all chunks at once; then a block owns
 // (sequence, head, 16 or 32 value columns), holds its part of S in registers, and walks the sequence's chunks, while one more
-// warp brings the next chunk into shared memory (cp.async).
+// warp brings the next chunks into shared memory.
 #include <limits.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 BLM_API const char* blm_scan_chunks_last_error() { return g_blm_error; }
 
@@ -56,6 +58,27 @@ constexpr long long kScratch = 32 << 20;
 __host__ __device__ constexpr int rows_floats(int kind, int np) { return kind == kSsm ? 0 : (kind == kDelta ? 3 : 2) * kQ * np + np; }
 __host__ __device__ constexpr int small_floats(int kind) { return kMat * (kind == kDelta ? 2 : 1) + (kind == kSsm ? 48 : 0); }
 __host__ __device__ constexpr int part_floats(int kind, int np) { return rows_floats(kind, np) + small_floats(kind); }
+
+// Where the walk runs on the tensor cores (states of 64 and 128 rows that decay), floats as three bfloat16 numbers: a (chunk, head) has
+// [q][k] [3][16][NP] (the state-space scan once a group of heads, behind all chunks' and heads'), [the chunk's decay], A [3][16][16],
+// and for the state-space scan the 48 numbers.  Rows of tokens lie in 16-byte pieces, piece c of token t at c ^ (t % 8); rows of A,
+// two pieces, at c ^ (j / 4 % 2).
+__host__ __device__ constexpr bool on_tensor_cores(int kind, int np) { return kind != kDelta && (np == 64 || np == 128); }
+__host__ __device__ constexpr int limb_rows(int np) { return 2 * 3 * kQ * np / 2; }      // floats
+constexpr int kLimbMat = 3 * kQ * kQ / 2;
+__host__ __device__ constexpr int limb_part(int kind, int np) { return kind == kSsm ? kLimbMat + 48 : limb_rows(np) + np + kLimbMat; }
+__device__ __forceinline__ int limb_at(int t, int r, int np) { return (t * np + (((r >> 3) ^ (t & 7)) << 3) + (r & 7)) * 2; }      // bytes
+__device__ __forceinline__ int limb_mat_at(int j, int i) { return j * 32 + (((i >> 3) ^ (j >> 2 & 1)) << 4) + (i & 7) * 2; }
+// the 16 x 16 matrix A as parts: a thread two neighbouring i
+__device__ __forceinline__ void store_limb_mat(float* to, const float (&As)[kQ][kMs], int tid) {
+    for (int e = tid; e < kQ * kQ / 2; e += blockDim.x) {
+        const int j = e >> 3, i = (e & 7) * 2;
+        unsigned p[3];
+        tc5::split3(As[j][i], As[j][i + 1], p[0], p[1], p[2]);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) *reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(to) + l * kQ * kQ * 2 + limb_mat_at(j, i)) = p[l];
+    }
+}
 
 // Which sequence and chunk a chunk index names; false when none.  All threads of the block call it.
 __device__ __forceinline__ bool find_chunk(int idx, const Chunks& ch, int* found, int& seq, int& chunk) {
@@ -199,28 +222,62 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         const float s = sum_sixteen(v);
         if (!(lane & 1)) sums[2][warp][lane >> 1] = s;
     }
-    float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h) * part_floats(DELTA ? kDelta : kDecay, NP);
-    if (r < NP) {
-        float p = 1.f;
+    constexpr bool kLimbs = !DELTA && on_tensor_cores(kDecay, NP);
+    float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h) * (kLimbs ? limb_part(kDecay, NP) : part_floats(DELTA ? kDelta : kDecay, NP));
+    if (kLimbs && r < NP) {
+        // an even lane writes its row and the next one's first eight tokens, an odd one the last eight of the row before and its own
+        const bool up = lane & 1;
+        unsigned char* rows = reinterpret_cast<unsigned char*>(out);
+        float qd[kQ], kd[kQ], p = 1.f;
 #pragma unroll
         for (int t = 0; t < kQ; ++t) {
-            if (kFirst) out[t * NP + r] = qq[t] * p;
+            if (kFirst) qd[t] = qq[t] * p;
             p *= w[t];
-            if (DELTA) {
-                out[t * NP + r] = kk[t] * p;
-                out[(kQ + t) * NP + r] = qq[t] * p;
-            } else if (!kFirst) {
-                out[t * NP + r] = qq[t] * p;
-            }
+            if (!kFirst) qd[t] = qq[t] * p;
         }
-        float* kd = out + (DELTA ? 2 : 1) * kQ * NP;
         p = 1.f;
 #pragma unroll
         for (int t = kQ - 1; t >= 0; --t) {
-            kd[t * NP + r] = kk[t] * p;
+            kd[t] = kk[t] * p;
             p *= w[t];
         }
-        kd[kQ * NP + r] = p;
+        out[limb_rows(NP) + r] = p;
+#pragma unroll
+        for (int which = 0; which < 2; ++which)
+#pragma unroll
+            for (int t = 0; t < kQ / 2; ++t) {
+                const float low = which ? kd[t] : qd[t], high = which ? kd[t + 8] : qd[t + 8];
+                const float other = __shfl_xor_sync(0xffffffffu, up ? low : high, 1);
+                unsigned l[3];
+                tc5::split3(up ? other : low, up ? high : other, l[0], l[1], l[2]);
+                const int at = limb_at(up ? t + 8 : t, r & ~1, NP);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) *reinterpret_cast<unsigned*>(rows + (which * 3 + x) * kQ * NP * 2 + at) = l[x];
+            }
+    }
+    if (r < NP) {
+        float p = 1.f;
+        if (!kLimbs) {
+#pragma unroll
+            for (int t = 0; t < kQ; ++t) {
+                if (kFirst) out[t * NP + r] = qq[t] * p;
+                p *= w[t];
+                if (DELTA) {
+                    out[t * NP + r] = kk[t] * p;
+                    out[(kQ + t) * NP + r] = qq[t] * p;
+                } else if (!kFirst) {
+                    out[t * NP + r] = qq[t] * p;
+                }
+            }
+            float* kd = out + (DELTA ? 2 : 1) * kQ * NP;
+            p = 1.f;
+#pragma unroll
+            for (int t = kQ - 1; t >= 0; --t) {
+                kd[t * NP + r] = kk[t] * p;
+                p *= w[t];
+            }
+            kd[kQ * NP + r] = p;
+        }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             constexpr int kAll = kQ;
@@ -281,6 +338,10 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         As[r][r] = s;
     }
     __syncthreads();
+    if (kLimbs) {
+        store_limb_mat(out + limb_rows(NP) + NP, As, r);
+        return;
+    }
     float* m = out + rows_floats(DELTA ? kDelta : kDecay, NP);
     if (!DELTA) {
         for (int e = r; e < kMat; e += T) m[e] = (&As[0][0])[e];
@@ -324,13 +385,15 @@ struct SsmPrepArgs {
     int b_col0, c_col0;
     const float *dt_bias, *A_log, *D;
     Chunks ch;
-    int heads, groups, N;
+    int heads, groups, N, np;
     float* scratch;
+    float* limbs;                  // the groups' rows as parts, or null
 };
 
 __global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
     __shared__ int found[2];
     __shared__ float Bs[kQ][65], Cs[kQ][65];   // 64 rows of the state at a time
+    __shared__ float As[kQ][kMs];
     __shared__ float dts[kSsmHeads][kQ], decs[kSsmHeads][kQ], run[kSsmHeads][kQ][kQ + 1];
     const int per = a.heads / a.groups, tiles = (per + kSsmHeads - 1) / kSsmHeads;
     const int g = blockIdx.y / tiles, h0 = g * per + blockIdx.y % tiles * kSsmHeads, nh = min(kSsmHeads, (g + 1) * per - h0);
@@ -359,6 +422,17 @@ __global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
             Cs[t][n] = on ? row[a.c_col0] : 0.f;
         }
         __syncthreads();
+        if (a.limbs && blockIdx.y % tiles == 0) {
+            unsigned char* rows = reinterpret_cast<unsigned char*>(a.limbs + ((size_t)blockIdx.x * a.groups + g) * limb_rows(a.np));
+            for (int e = tid; e < 2 * kQ * 32; e += 256) {
+                const int n = (e & 31) * 2, t = e >> 5 & 15, which = e >> 9;
+                const float(*from)[65] = which ? Bs : Cs;
+                unsigned l[3];
+                tc5::split3(from[t][n], from[t][n + 1], l[0], l[1], l[2]);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) *reinterpret_cast<unsigned*>(rows + (which * 3 + x) * kQ * a.np * 2 + limb_at(t, n0 + n, a.np)) = l[x];
+            }
+        }
         float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int n = 0; n < 64; ++n) s[n & 3] += Cs[j][n] * Bs[i][n];
@@ -377,15 +451,23 @@ __global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
     }
     __syncthreads();
     for (int hh = 0; hh < nh; ++hh) {
-        const float p = run[hh][j][i];
-        float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h0 + hh) * part_floats(kSsm, 0);
-        out[j * kMs + i] = i > j ? 0.f : cb * p * dts[hh][i] + (i == j ? a.D[h0 + hh] : 0.f);
-        if (i < kMs - kQ) out[j * kMs + kQ + i] = 0.f;
-        if (i == 0) {                          // token j's factor of the read-out
-            out[kMat + j] = p * decs[hh][0];
-            if (j == kQ - 1) out[kMat + 32] = p * decs[hh][0];
+        const float p = run[hh][j][i], aji = i > j ? 0.f : cb * p * dts[hh][i] + (i == j ? a.D[h0 + hh] : 0.f);
+        float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h0 + hh) * (a.limbs ? limb_part(kSsm, 0) : part_floats(kSsm, 0));
+        float* nums = out + (a.limbs ? kLimbMat : kMat);
+        if (a.limbs) {
+            __syncthreads();                   // (the matrix of the head before has left)
+            As[j][i] = aji;
+            __syncthreads();
+            store_limb_mat(out, As, tid);
+        } else {
+            out[j * kMs + i] = aji;
+            if (i < kMs - kQ) out[j * kMs + kQ + i] = 0.f;
         }
-        if (j == kQ - 1) out[kMat + kQ + i] = p * dts[hh][i];       // and of what it writes
+        if (i == 0) {                          // token j's factor of the read-out
+            nums[j] = p * decs[hh][0];
+            if (j == kQ - 1) nums[32] = p * decs[hh][0];
+        }
+        if (j == kQ - 1) nums[kQ + i] = p * dts[hh][i];             // and of what it writes
     }
 }
 
@@ -403,6 +485,8 @@ constexpr int kStages = 4;                     // chunks in shared memory: the o
 struct WalkArgs {
     RowsIn v;
     const float* scratch;
+    int* status;
+    const float* limbs;            // state-space scan on the tensor cores: the groups' B and C as parts
     const float* rows;             // state-space scan: B and C where they lie
     long long rows_stride;
     int b_col0, c_col0, per_group, N;
@@ -730,6 +814,298 @@ __global__ void __launch_bounds__(RG * CT / C + 32, 1) walk_kernel(const WalkArg
         }
 }
 
+// ---------------------------------------------------------------------------------------------
+// the walk on the tensor cores, for states of 64 and 128 rows that decay
+//
+// What bounds the walk above is the issue of instructions: 700 a warp and chunk, of which 256 multiply-add.  Here a block of four warps
+// keeps 16 columns of the state, transposed, as accumulators of mma.sync (m16n8k16: 16 columns x 8 rows), a quarter of the rows a
+// warp, which are at once the first operand of the read-out: q S is columns x tokens, k summed over the rows.  All operands are
+// floats as three bfloat16 numbers (tcgen05.cuh: 24 bits, six products, float32 sums); what a chunk adds to the state is summed by
+// itself and joins it by a float32 multiply-add, since the tensor core's additions cut bits off.  The warps' shares of the
+// read-out meet in shared memory, and are added and stored a chunk later, so that a chunk has one barrier.  What a chunk's tokens
+// read of one another is formed by a warp of its own, which stores too; another one loads: a bulk copy a chunk (52 cp.async of a
+// warp took longer than the products), x by cp.async.
+// Both launches, us, FFMA and so: decay of 32 heads of 128 x 128, 512 / 2,048 tokens 73 / 237 and 60 / 188 (the rows' parts are 111 MB
+// instead of 74, so the first one takes 61 instead of 52); state-space scan of 64 heads of 128 x 64, 512 tokens 75 and 54, four times
+// 500 206 and 155; decay of 16 heads of 64 x 128, 2,048 tokens 109 and 107.  A chunk takes 1,500 clocks with two blocks a multiprocessor,
+// of which the 51 products of a warp take half; 32 columns a block were slower (155 us instead of 121), and so were sums and
+// store by the loading warp (NP 64: 103 us instead of 91).
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// chunks in shared memory: the one worked on and two on their way, with states of 64 rows three; two blocks a multiprocessor
+__host__ __device__ constexpr int limb_stages(int np) { return np == 128 ? 3 : 4; }
+constexpr int kVs = 20;            // floats a row of x and of the shares of the output: lanes read different banks
+// a chunk in shared memory: [q][k] parts, the decays (decay: a row each), A's parts, the 48 numbers (state-space scan), x [16][kVs]
+__host__ __device__ constexpr int limb_stage(int kind, int np) { return limb_rows(np) + (kind == kSsm ? 0 : np) + kLimbMat + (kind == kSsm ? 48 : 0) + kQ * kVs; }
+constexpr int kLimbThreads = 6 * 32;
+
+template <int NP, int KIND>
+__global__ void __launch_bounds__(kLimbThreads, 2) walk_mma_kernel(const WalkArgs a) {
+    constexpr int CT = 16, KS = NP / 64, kRing = limb_stages(NP), kRows = limb_rows(NP), kStage = limb_stage(KIND, NP), kShare = kQ * kVs, kPart = limb_part(KIND, NP), kPlane = kQ * NP * 2;
+    constexpr int of_a[6] = {2, 0, 1, 1, 0, 0}, of_b[6] = {0, 2, 1, 0, 1, 0};      // parts of the products, the smallest first
+    extern __shared__ __align__(16) float sm[];
+    float* shares = sm + kRing * kStage;                       // [2][5 warps][16 tokens][kVs]
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(shares + 2 * 5 * kShare);      // [kRing] a chunk is there
+    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
+    const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
+    if (n_new < a.ch.least || n_new >= a.ch.most) return;
+    const int base = chunk_base(first, seq, a.ch.packed) - a.ch.from, start = a.start_pos[seq];
+    const int lo = max(0, -base), hi = min((n_new + kQ - 1) / kQ, a.ch.count - base);
+    if (lo >= hi) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t2 = (lane & 3) * 2;              // the lane's column (and g + 8), its pair of rows or tokens
+    // rows of eight tokens that an ldmatrix reads: its matrices are (tokens 0-7, piece c), (0-7, c + 1), (8-15, c), (8-15, c + 1) for
+    // the read-out, and (0-7, c), (8-15, c), (0-7, c + 1), (8-15, c + 1) for the update
+    const int tq = (lane & 7) + (lane >> 4) * 8, pq = lane >> 3 & 1, tk = (lane & 7) + (lane >> 3 & 1) * 8, pk = lane >> 4;
+    // x of a chunk: pairs of tokens t2 + {0, 1} (and 8 further) of the columns g (and g + 8)
+    auto pairs_of = [&](const float* x, float (&xv)[4][2]) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) xv[e][y] = x[(t2 + y + (e >> 1) * 8) * kVs + g + (e & 1) * 8];
+    };
+    if (tid == 0) {
+        for (int i = 0; i < kRing; ++i) tc5::mbar_init(full + i, 32 + 1);
+        tc5::mbar_init_fence();
+    }
+    __syncthreads();
+    auto there = [&](int chunk) {
+        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT);
+        return sm + (chunk - lo) % kRing * kStage;
+    };
+    auto share = [&](int chunk, const float (&o)[2][4]) {      // a warp's share of the output: columns g, g + 8; tokens t2, + 1 (and 8 further)
+        float* to = shares + ((chunk & 1) * 5 + min(warp, 4)) * kShare + g;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) to[(8 * n + t2 + (e & 1)) * kVs + (e >> 1) * 8] = o[n][e];
+    };
+
+    if (warp == 5) {
+        // a chunk's output: the warps' shares added up, eight columns of a token a lane
+        const int j = lane >> 1, c8 = (lane & 1) * 8;
+        float* y = a.y + (size_t)(first + j) * a.y_stride + (size_t)h * a.dv + col0 + c8;
+        const bool vec = (((size_t)y | (size_t)a.y_stride * 4) & 15) == 0 && col0 + c8 + 8 <= a.dv;
+        auto store = [&](int chunk) {
+            const float* from = shares + (chunk & 1) * 5 * kShare + j * kVs + c8;
+            float v[8];
+#pragma unroll
+            for (int w = 0; w < 5; ++w) {
+                const float4 low = *reinterpret_cast<const float4*>(from + w * kShare), high = *reinterpret_cast<const float4*>(from + w * kShare + 4);
+                const float u[8] = {low.x, low.y, low.z, low.w, high.x, high.y, high.z, high.w};
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = w ? v[e] + u[e] : u[e];
+            }
+            if (chunk * kQ + j < n_new) {
+                float* to = y + (size_t)chunk * kQ * a.y_stride;
+                if (vec) {
+                    reinterpret_cast<float4*>(to)[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    reinterpret_cast<float4*>(to)[1] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        if (col0 + c8 + e < a.dv) to[e] = v[e];
+                }
+            }
+        };
+        // what the tokens of a chunk read of one another.  A zero of the matrix does not silence a value that is not finite: it is
+        // taken out and joins the tokens behind it by itself.
+        for (int chunk = lo; chunk < hi; ++chunk) {
+            __syncthreads();
+            if (chunk > lo) store(chunk - 1);
+            const float* st = there(chunk);
+            const float *x = st + kStage - kShare, *mat = st + kRows + (KIND == kSsm ? 0 : NP);
+            float xv[4][2], o[2][4] = {};
+            pairs_of(x, xv);
+            unsigned most = 0, x3[3][4], b[3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    most = max(most, __float_as_uint(xv[e][y]) & 0x7fffffffu);
+                    if (!isfinite(xv[e][y])) xv[e][y] = 0.f;
+                }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tc5::split3(xv[e][0], xv[e][1], x3[0][e], x3[1][e], x3[2][e]);
+#pragma unroll
+            for (int l = 0; l < 3; ++l)
+                ldsm_x4(b[l], (unsigned)__cvta_generic_to_shared(mat) + l * kQ * kQ * 2 + tq * 32 + ((pq ^ (tq >> 2 & 1)) << 4));
+#pragma unroll
+            for (int p = 0; p < 6; ++p)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) mma_bf16(o[n], x3[of_a[p]], b[of_b[p]][2 * n], b[of_b[p]][2 * n + 1]);
+            if (__any_sync(0xffffffffu, most >= 0x7f800000u)) {
+#pragma unroll 1
+                for (int i = 0; i < kQ; ++i) {
+                    const float v0 = x[i * kVs + g], v1 = x[i * kVs + g + 8];
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int j = 8 * n + t2 + (e & 1);
+                            const float v = e >> 1 ? v1 : v0;
+                            float w = 0.f;
+#pragma unroll
+                            for (int l = 0; l < 3; ++l)
+                                w += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(reinterpret_cast<const unsigned char*>(mat) + l * kQ * kQ * 2 + limb_mat_at(j, i)));
+                            if (i <= j && !isfinite(v)) o[n][e] = fmaf(w, v, o[n][e]);
+                        }
+                }
+            }
+            share(chunk, o);
+        }
+        __syncthreads();
+        store(hi - 1);
+        return;
+    }
+    if (warp == 4) {                           // the loads
+        auto bring = [&](int chunk) {
+            if (chunk >= hi) return;
+            unsigned long long* bar = full + (chunk - lo) % kRing;
+            float* st = sm + (chunk - lo) % kRing * kStage;
+            const int at = first + chunk * kQ, nt = min(kQ, n_new - chunk * kQ);
+            constexpr unsigned kOwn = (KIND == kSsm ? kLimbMat + 48 : kPart) * 4, kShared = KIND == kSsm ? kRows * 4 : 0;
+            if (lane == 0) {
+                tc5::mbar_expect_tx(bar, kOwn + kShared);
+                auto copy = [&](float* to, const float* from, unsigned bytes) {
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(tc5::smem_u32(to)), "l"(from),
+                                 "r"(bytes), "r"(tc5::smem_u32(bar))
+                                 : "memory");
+                };
+                copy(st + kShared / 4, a.scratch + ((size_t)(base + chunk) * a.heads + h) * kPart, kOwn);
+                if (KIND == kSsm) copy(st, a.limbs + ((size_t)(base + chunk) * (a.heads / a.per_group) + h / a.per_group) * kRows, kShared);
+            }
+            const float* v = a.v.p + (size_t)at * a.v.stride + a.v.col0 + (size_t)h * a.dv + col0;
+#pragma unroll
+            for (int i = 0; i < kQ * CT / 32; ++i) {
+                const int t = (lane + 32 * i) / CT, c = (lane + 32 * i) % CT;
+                const bool on = t < nt && col0 + c < a.dv;
+                cp4(st + kStage - kShare + t * kVs + c, on ? v + t * a.v.stride + c : a.scratch, on ? 4 : 0);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(tc5::smem_u32(bar)) : "memory");
+        };
+        for (int i = 0; i < kRing - 1; ++i) bring(lo + i);
+        for (int chunk = lo; chunk < hi; ++chunk) {
+            __syncthreads();                   // the others are done with the chunk before, where the next one goes
+            bring(chunk + kRing - 1);
+        }
+        __syncthreads();
+        return;
+    }
+
+    const int row0 = warp * (NP / 4);
+    float* both = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off + (size_t)h * NP * a.dv;
+    float* fresh = both + (size_t)((start + n_new) & 1) * a.copy_stride;
+    const float* old = lo > 0 ? fresh : both + (size_t)(start & 1) * a.copy_stride;      // (behind an earlier pass: what that wrote)
+    float S[2 * KS][4];                        // tile n: columns g, g + 8; rows row0 + 8 n + t2, + 1
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + (e >> 1) * 8;
+            S[n][e] = (start > 0 || lo > 0) && col < a.dv ? old[((size_t)(row0 / 8 + n) * a.dv + col) * 8 + t2 + (e & 1)] : 0.f;
+        }
+    // What a chunk adds to the state knows nothing of the state: its operands and products come at the end of the chunk before, while
+    // that one's read-out is on its way through the tensor cores.
+    unsigned q[KS][3][4], k[KS][3][4], x3[3][4];
+    float d[KS][2][4];
+    auto ahead = [&](int chunk) {
+        const float* st = there(chunk);
+        const unsigned rows = (unsigned)__cvta_generic_to_shared(st);
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) ldsm_x4_trans(k[u][l], rows + (3 + l) * kPlane + tk * NP * 2 + (((row0 / 8 + 2 * u + pk) ^ (tk & 7)) << 4));
+        float xv[4][2];
+        pairs_of(st + kStage - kShare, xv);
+        if (KIND == kSsm) {
+            const float* nums = st + kRows + kLimbMat;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) xv[e][y] *= nums[kQ + t2 + y + (e >> 1) * 8];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tc5::split3(xv[e][0], xv[e][1], x3[0][e], x3[1][e], x3[2][e]);
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) ldsm_x4(q[u][l], rows + l * kPlane + tq * NP * 2 + (((row0 / 8 + 2 * u + pq) ^ (tq & 7)) << 4));
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) d[u][n][0] = d[u][n][1] = d[u][n][2] = d[u][n][3] = 0.f;
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) mma_bf16(d[u][n], x3[of_a[p]], k[u][of_b[p]][2 * n], k[u][of_b[p]][2 * n + 1]);
+    };
+    ahead(lo);
+    for (int chunk = lo; chunk < hi; ++chunk) {
+        __syncthreads();
+        const float* decays = sm + (chunk - lo) % kRing * kStage + kRows;
+        const float* nums = decays + kLimbMat;                 // (state-space scan)
+        unsigned s3[KS][3][4];
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tc5::split3(S[2 * u + (e >> 1)][(e & 1) * 2], S[2 * u + (e >> 1)][(e & 1) * 2 + 1], s3[u][0][e], s3[u][1][e], s3[u][2][e]);
+        float o[KS][2][4] = {};
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) mma_bf16(o[u][n], s3[u][of_a[p]], q[u][of_b[p]][2 * n], q[u][of_b[p]][2 * n + 1]);
+        // the state behind the chunk
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const float2 p2 = KIND == kSsm ? make_float2(nums[32], nums[32]) : *reinterpret_cast<const float2*>(decays + row0 + (2 * u + n) * 8 + t2);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[2 * u + n][e] = fmaf(S[2 * u + n][e], e & 1 ? p2.y : p2.x, d[u][n][e]);
+            }
+        float f[2][2];
+        if (KIND == kSsm) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) f[n][e] = nums[8 * n + t2 + e];
+        }
+        if (chunk + 1 < hi) ahead(chunk + 1);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (KS > 1) o[0][n][e] += o[KS - 1][n][e];
+                if (KIND == kSsm) o[0][n][e] *= f[n][e & 1];
+            }
+        share(chunk, o[0]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + (e >> 1) * 8;
+            if (col < a.dv) fresh[((size_t)(row0 / 8 + n) * a.dv + col) * 8 + t2 + (e & 1)] = S[n][e];
+        }
+}
+
 // Rows of a state as the scans keep them: eight times a power of two.
 static int padded_rows(int rows) {
     int n = 8;
@@ -754,6 +1130,14 @@ static int launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
     return blm_check_launch("scan_chunks (walk)");
 }
 
+template <int NP, int KIND>
+static int launch_walk_mma(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+    constexpr size_t smem = ((size_t)limb_stages(NP) * limb_stage(KIND, NP) + 2 * 5 * kQ * kVs) * sizeof(float) + 64;
+    if (int rc = allow_smem(walk_mma_kernel<NP, KIND>, smem)) return rc;
+    walk_mma_kernel<NP, KIND><<<dim3((a.dv + 15) / 16, a.heads, n_seqs), kLimbThreads, smem, stream>>>(a);
+    return blm_check_launch("scan_chunks (walk)");
+}
+
 // Rows and columns of a thread, columns of a block.  Four columns a thread: a row piece that comes from shared memory serves four
 // multiply-adds a row; 16 columns a block: a prompt of few heads still has a block for most multiprocessors.  2,048 tokens, states
 // of 128 rows (decay of 32 heads x 128 columns / state-space scan of 64 x 64 / delta rule of 16 x 128, 2,001 tokens), us:
@@ -761,31 +1145,40 @@ static int launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
 // 4 columns, 8 rows, 16 a block (64 threads) 237 / 260 / 211, 32 a block 184 / 200 / 216.
 template <int KIND>
 static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
+    if constexpr (KIND != kDelta) {
+        if (np == 64) return launch_walk_mma<64, KIND>(a, n_seqs, stream);
+        if (np == 128) return launch_walk_mma<128, KIND>(a, n_seqs, stream);
+    } else {
+        if (np == 64) return launch_walk<64, 2, 16, 16, KIND>(a, n_seqs, stream);
+        if (np == 128) return launch_walk<128, 4, 32, 16, KIND>(a, n_seqs, stream);
+    }
     switch (np) {
         case 32: return launch_walk<32, 2, 8, 32, KIND>(a, n_seqs, stream);
-        case 64: return launch_walk<64, 2, 16, 16, KIND>(a, n_seqs, stream);
-        case 128: return launch_walk<128, 4, 32, 16, KIND>(a, n_seqs, stream);
         case 256: return launch_walk<256, 4, 32, 16, KIND>(a, n_seqs, stream);
     }
     return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
 }
 
-// Chunks of a pass.
-static int chunks_at_once(int kind, int heads, int np, int n_tokens, int n_seqs, int least) {
-    const long long most = kScratch / ((long long)heads * part_floats(kind, np)), all = chunk_bound(n_tokens, n_seqs, least);
+// Floats of scratch of a chunk (`groups`: row sets of a state-space scan), and chunks of a pass.
+static long long chunk_floats(int kind, int heads, int groups, int np) {
+    if (!on_tensor_cores(kind, np)) return (long long)heads * part_floats(kind, np);
+    return (long long)heads * limb_part(kind, np) + (kind == kSsm ? (long long)groups * limb_rows(np) : 0);
+}
+static int chunks_at_once(int kind, int heads, int groups, int np, int n_tokens, int n_seqs, int least) {
+    const long long most = kScratch / chunk_floats(kind, heads, groups, np), all = chunk_bound(n_tokens, n_seqs, least);
     return (int)(all < most ? all : (most > 1 ? most : 1));
 }
 
 // Floats of scratch a step needs; 0: these kernels do not take the size (states of up to 16 or of more than 256 rows, more
 // sequences than a grid's third dimension holds).  And the number of kernels it launches.
-BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
+BLM_API long long blm_scan_chunks_scratch(int kind, int heads, int groups, int rows, int n_tokens, int n_seqs, int least) {
     const int np = padded_rows(rows);
-    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta || heads < 1 || n_seqs > 65535) return 0;
-    return (long long)chunks_at_once(kind, heads, np, n_tokens, n_seqs, least) * heads * part_floats(kind, np);
+    if (np < 32 || np > 256 || kind < kSsm || kind > kDelta || heads < 1 || groups < 1 || n_seqs > 65535) return 0;
+    return (long long)chunks_at_once(kind, heads, groups, np, n_tokens, n_seqs, least) * chunk_floats(kind, heads, groups, np);
 }
-BLM_API int blm_scan_chunks_launches(int kind, int heads, int rows, int n_tokens, int n_seqs, int least) {
-    if (blm_scan_chunks_scratch(kind, heads, rows, n_tokens, n_seqs, least) == 0) return 0;
-    const int at_once = chunks_at_once(kind, heads, padded_rows(rows), n_tokens, n_seqs, least);
+BLM_API int blm_scan_chunks_launches(int kind, int heads, int groups, int rows, int n_tokens, int n_seqs, int least) {
+    if (blm_scan_chunks_scratch(kind, heads, groups, rows, n_tokens, n_seqs, least) == 0) return 0;
+    const int at_once = chunks_at_once(kind, heads, groups, padded_rows(rows), n_tokens, n_seqs, least);
     return 2 * (int)((chunk_bound(n_tokens, n_seqs, least) + at_once - 1) / at_once);
 }
 
@@ -798,15 +1191,17 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
                                 long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                                 long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
                                 const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, int most, float* state,
-                                long long slot_stride, long long copy_stride, long long state_off, float* scratch, cudaStream_t stream) {
+                                long long slot_stride, long long copy_stride, long long state_off, float* scratch, int* status, cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
     Chunks ch = {cu_seqlens, n_seqs, least, most, chunks_packed(n_tokens, n_seqs, least), 0, 0};
     const int np = padded_rows(N), per = heads / groups;
-    SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
-                     scratch};
+    SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N, np,
+                     scratch, nullptr};
+    BLM_REQUIRE(status != nullptr, "scan_chunks: no status word");
     WalkArgs a = {};
+    a.status = status;
     a.v = {xbc, xbc_stride, x_col0};
     a.scratch = scratch;
     a.rows = xbc;
@@ -826,7 +1221,8 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
     a.slot_stride = slot_stride;
     a.copy_stride = copy_stride;
     a.state_off = state_off;
-    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(kSsm, heads, np, n_tokens, n_seqs, least);
+    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(kSsm, heads, groups, np, n_tokens, n_seqs, least);
+    if (on_tensor_cores(kSsm, np)) a.limbs = p.limbs = scratch + (size_t)at_once * heads * limb_part(kSsm, np);
     for (ch.from = 0; ch.from < all; ch.from += at_once) {
         ch.count = all - ch.from < at_once ? all - ch.from : at_once;
         p.ch = a.ch = ch;
@@ -860,7 +1256,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
                                  const float* A_log, float* o, long long o_stride, int heads, int qk_heads, int dk, int dv,
                                  int lower_bound, int read_first, const int* cu_seqlens, const int* slot_of_seq, const int* start_pos,
                                  int n_tokens, int n_seqs, int least, float* state, long long slot_stride, long long copy_stride,
-                                 long long state_off, float* scratch, cudaStream_t stream) {
+                                 long long state_off, float* scratch, int* status, cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(qk_heads > 0 && heads % qk_heads == 0 && dk > 0 && dv > 0, "scan_chunks: bad head counts");
     if (int rc = check_step(n_tokens, n_seqs, heads, least)) return rc;
@@ -872,7 +1268,9 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     PrepArgs p = {{q, q_stride, q_col0}, {k, k_stride, k_col0}, {a_raw, a_stride, a_col0}, {b_raw, b_stride, b_col0}, bias, extra, A_log,
                   ch, heads, qk_heads, dk, scratch};
     const int mode = delta ? kModeDelta : (lower_bound ? kModeLower : (read_first ? kModeExpFirst : kModeExp));
+    BLM_REQUIRE(status != nullptr, "scan_chunks: no status word");
     WalkArgs a = {};
+    a.status = status;
     a.v = {v, v_stride, v_col0};
     a.scratch = scratch;
     a.y = o;
@@ -885,7 +1283,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
     a.slot_stride = slot_stride;
     a.copy_stride = copy_stride;
     a.state_off = state_off;
-    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(delta ? kDelta : kDecay, heads, np, n_tokens, n_seqs, least);
+    const int all = (int)chunk_bound(n_tokens, n_seqs, least), at_once = chunks_at_once(delta ? kDelta : kDecay, heads, 1, np, n_tokens, n_seqs, least);
     for (ch.from = 0; ch.from < all; ch.from += at_once) {
         ch.count = all - ch.from < at_once ? all - ch.from : at_once;
         p.ch = a.ch = ch;

@@ -3,7 +3,7 @@
 // The chunks of sixteen tokens (scan_chunks.cu) are a chain of 128 links for a prompt of 2,048 tokens, each of which passes over
 // the state with fp32 multiply-adds: 230 us for 64 heads of 128 x 64, whose multiply-adds alone take 58.  Here a chunk has 64
 // tokens, its products run on the tensor cores with every float as three bfloat16 numbers (tcgen05.cuh: 24 bits, six products, sums
-// in float32), and a sequence is cut into groups of eight chunks that run side by side: 124 us.  With P(i..j) the product of the
+// in float32), and a sequence is cut into four groups of chunks that run side by side: 124 us.  With P(i..j) the product of the
 // decays of the tokens i..j and S the state in front of a chunk:
 //     out_j  = P(0..j) S^T C_j + sum_(i <= j) A_ji x_i,     A_ji = (C_j . B_i) P(i+1..j) dt_i  (+ D on the diagonal)
 //     S'     = P(0..63) S + Z,     Z = sum_j (P(j+1..63) dt_j B_j) x_j^T
@@ -26,7 +26,7 @@ BLM_API const char* blm_scan_long_last_error() { return g_blm_error; }
 using namespace tc5;
 
 constexpr int kT = 64;            // tokens of a chunk
-constexpr int kGroup = 8;         // chunks of a group
+constexpr int kGroups = 4;        // groups of a sequence: its chunks in even parts
 constexpr int kTile = kT * 128;   // bytes of 64 rows of 64 bfloat16 numbers
 
 constexpr int NR = 128, H = NR / 64;      // rows of the state as it lies, and rows of 128 bytes that its parts take
@@ -34,7 +34,7 @@ constexpr int NR = 128, H = NR / 64;      // rows of the state as it lies, and r
 __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // Sequences of `least` or more new tokens are run.  Chunk c of sequence s has the index cu[s] / 64 + s + c: distinct, and below
-// n_tokens / 64 + n_seqs.  Sums of group g of a sequence with several groups have the index (its first chunk's index) / 8, distinct too.
+// n_tokens / 64 + n_seqs.  Sums of group g of a sequence have the index 3 (cu[s] / least) + g, distinct too.
 struct Chunks {
     const int* cu;
     int n_seqs, least;
@@ -78,8 +78,8 @@ struct Sizes {
     long long rows, mats, nums, sums, decays;          // bytes
     long long all() const { return rows + mats + nums + sums + decays; }
 };
-static Sizes sizes_of(int units, int heads, int dv, long long chunks) {
-    const long long groups = chunks / kGroup + 1;
+static Sizes sizes_of(int units, int heads, int dv, long long chunks, long long sequences) {
+    const long long groups = sequences * (kGroups - 1);
     return {chunks * units * 6 * H * kTile, chunks * heads * 3 * kTile, chunks * heads * kNums * 4, groups * heads * dv * NR * 4, groups * heads * 4};
 }
 static Scratch scratch_at(float* base, const Sizes& s) {
@@ -271,7 +271,7 @@ struct RunArgs {
     const int *slot_of_seq, *start_pos;
     int units, per_unit;           // units of `rows` a chunk, heads of a unit
     int head0, heads;              // this pass: heads from head0 on
-    int dv, groups;                // groups of the longest sequence
+    int dv;
     float* y;
     long long y_stride;
     float* state;
@@ -330,12 +330,12 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 13);
     int* odd = reinterpret_cast<int*>(tmem_slot + 2);                       // [2][4]: a warp of columns has values that are not finite in the chunk
 
-    const int h = blockIdx.x * 2, seq = blockIdx.y / a.groups, group = blockIdx.y % a.groups;
+    const int h = blockIdx.x * 2, seq = blockIdx.y / kGroups, group = blockIdx.y % kGroups;
     const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
     if (n_new < a.ch.least) return;
-    const int chunks = (n_new + kT - 1) / kT, lo = group * kGroup;
-    if (lo >= chunks || (SUMS && lo + kGroup >= chunks)) return;
-    const int n = min(kGroup, chunks - lo), base = chunk_base(first, seq) + lo;
+    const int chunks = (n_new + kT - 1) / kT, size = (chunks + kGroups - 1) / kGroups, lo = group * size;
+    if (lo >= chunks || (SUMS && lo + size >= chunks)) return;
+    const int n = min(size, chunks - lo), base = chunk_base(first, seq) + lo;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(a_full, 1);
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                         for (int e = 0; e < 8; ++e) S[r8 * 8 + e] = at(old, r8)[e];
                 }
                 for (int g = 0; g < group; ++g) {          // the groups in front
-                    const size_t i = (size_t)((base - lo + g * kGroup) / kGroup) * a.heads + hl;
+                    const size_t i = (size_t)(first / a.ch.least * (kGroups - 1) + g) * a.heads + hl;
                     const float* sum = a.s.sums + (i * a.dv + min(col, a.dv - 1)) * NR + half * kHalf;
                     const float d = a.s.decays[i];
 #pragma unroll
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                 }
             }
             if (ok && SUMS) {
-                const size_t i = (size_t)(base / kGroup) * a.heads + hl;
+                const size_t i = (size_t)(first / a.ch.least * (kGroups - 1) + group) * a.heads + hl;
                 if (live) {
                     float* sum = a.s.sums + (i * a.dv + col) * NR + half * kHalf;
 #pragma unroll
@@ -697,56 +697,51 @@ static int allow_smem(K kernel, int smem) {
 // Heads at a time, in whole groups of those that share B and C, so that a pass's scratch stays within kMost bytes (256 MB: some 8,000
 // tokens of 64 heads); heads know nothing of one another, so the passes change no bit.
 constexpr long long kMost = 256ll << 20;
-static int heads_at_once(int heads, int unit, int dv, long long chunks) {
+static int heads_at_once(int heads, int unit, int dv, long long chunks, long long sequences) {
     int at_once = heads;
-    while (at_once > unit && sizes_of(at_once / unit, at_once, dv, chunks).all() > kMost) at_once = (at_once / unit + 1) / 2 * unit;
+    while (at_once > unit && sizes_of(at_once / unit, at_once, dv, chunks, sequences).all() > kMost) at_once = (at_once / unit + 1) / 2 * unit;
     return at_once;
 }
 
 // Bytes of scratch; 0: these kernels do not take the size (states of 65 to 128 rows x 33 to 64 columns, an even number of heads that share
 // B and C: `unit`).  And how many kernels are launched.
-BLM_API long long blm_scan_long_scratch(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int longest) {
-    const long long groups = ((longest + kT - 1) / kT + kGroup - 1) / kGroup;
-    if (rows <= NR / 2 || rows > NR || dv <= 32 || dv > 64 || unit < 2 || unit % 2 || heads % unit || n_seqs < 1 || n_seqs * groups > 65535) return 0;
-    const long long chunks = chunk_bound(n_tokens, n_seqs);
-    const int n = heads_at_once(heads, unit, dv, chunks);
-    return n / unit > 65535 ? 0 : sizes_of(n / unit, n, dv, chunks).all();
+BLM_API long long blm_scan_long_scratch(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int least) {
+    if (rows <= NR / 2 || rows > NR || dv <= 32 || dv > 64 || unit < 2 || unit % 2 || heads % unit || n_seqs < 1 || n_seqs * kGroups > 65535 || least < 1) return 0;
+    const long long chunks = chunk_bound(n_tokens, n_seqs), sequences = n_tokens / least + 1;
+    const int n = heads_at_once(heads, unit, dv, chunks, sequences);
+    return n / unit > 65535 ? 0 : sizes_of(n / unit, n, dv, chunks, sequences).all();
 }
-BLM_API int blm_scan_long_launches(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int longest) {
-    const int n = heads_at_once(heads, unit, dv, chunk_bound(n_tokens, n_seqs));
-    return ((heads - 1) / n + 1) * (longest > kT * kGroup ? 3 : 2);
+BLM_API int blm_scan_long_launches(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int least) {
+    return ((heads - 1) / heads_at_once(heads, unit, dv, chunk_bound(n_tokens, n_seqs), n_tokens / least + 1) + 1) * 3;
 }
 
 BLM_API int blm_scan_chunks_long_ssm(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
                                      long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                                      long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
-                                     const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int longest, int least, float* state,
+                                     const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, float* state,
                                      long long slot_stride, long long copy_stride, long long state_off, float* scratch, int* status,
                                      cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0, "scan_long: bad head counts");
     const int per = heads / groups;
-    BLM_REQUIRE(blm_scan_long_scratch(heads, per, N, dv, n_tokens, n_seqs, longest) > 0 && status && least > 0, "scan_long: %d rows, %d columns", N, dv);
-    const long long chunks = chunk_bound(n_tokens, n_seqs);
-    const int at_once = heads_at_once(heads, per, dv, chunks);
+    BLM_REQUIRE(blm_scan_long_scratch(heads, per, N, dv, n_tokens, n_seqs, least) > 0 && status, "scan_long: %d rows, %d columns", N, dv);
+    const long long chunks = chunk_bound(n_tokens, n_seqs), sequences = n_tokens / least + 1;
+    const int at_once = heads_at_once(heads, per, dv, chunks, sequences);
     const Chunks ch = {cu_seqlens, n_seqs, least};
     for (int head0 = 0; head0 < heads; head0 += at_once) {
         const int now = heads - head0 < at_once ? heads - head0 : at_once;
-        const Scratch s = scratch_at(scratch, sizes_of(now / per, now, dv, chunks));
+        const Scratch s = scratch_at(scratch, sizes_of(now / per, now, dv, chunks, sequences));
         const SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
                                head0 / per, now / per, s};
         int rc = allow_smem(long_prep_kernel, kPrepSmem);
         if (rc) return rc;
         long_prep_kernel<<<dim3((unsigned)chunks, now / per), kPrepThreads, kPrepSmem, stream>>>(p);
         if ((rc = blm_check_launch("scan_long (chunks)"))) return rc;
-        const RunArgs a = {{xbc, xbc_stride, x_col0}, s, ch, slot_of_seq, start_pos, now / per, per, head0, now, dv,
-                           ((longest + kT - 1) / kT + kGroup - 1) / kGroup, y, y_stride, state, slot_stride, copy_stride, state_off, status};
-        const dim3 grid(now / 2, n_seqs * a.groups);
-        if (a.groups > 1) {
-            if ((rc = allow_smem(long_run_kernel<true>, kRunSmem))) return rc;
-            long_run_kernel<true><<<grid, kRunThreads, kRunSmem, stream>>>(a);
-            if ((rc = blm_check_launch("scan_long (sums)"))) return rc;
-        }
+        const RunArgs a = {{xbc, xbc_stride, x_col0}, s, ch, slot_of_seq, start_pos, now / per, per, head0, now, dv, y, y_stride, state, slot_stride, copy_stride, state_off, status};
+        const dim3 grid(now / 2, n_seqs * kGroups);
+        if ((rc = allow_smem(long_run_kernel<true>, kRunSmem))) return rc;
+        long_run_kernel<true><<<grid, kRunThreads, kRunSmem, stream>>>(a);
+        if ((rc = blm_check_launch("scan_long (sums)"))) return rc;
         if ((rc = allow_smem(long_run_kernel<false>, kRunSmem))) return rc;
         long_run_kernel<false><<<grid, kRunThreads, kRunSmem, stream>>>(a);
         if ((rc = blm_check_launch("scan_long (run)"))) return rc;

@@ -143,21 +143,21 @@ _protos = {
                                  c_float, c_void_p, c_int, c_longlong, c_int, c_void_p],
     },
     "scan_chunks": {
-        "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int, c_int],
-        "blm_scan_chunks_launches": [c_int, c_int, c_int, c_int, c_int, c_int],
+        "blm_scan_chunks_scratch": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
+        "blm_scan_chunks_launches": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
         "blm_scan_chunks_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+                                c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
         "blm_scan_chunks_rows": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p,
                                  c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong,
                                  c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                 c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
+                                 c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
     },
     "scan_long": {
         "blm_scan_long_scratch": [c_int] * 7,
         "blm_scan_long_launches": [c_int] * 7,
         "blm_scan_chunks_long_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                                     c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                      c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
     },
     "retention": {
@@ -1427,15 +1427,15 @@ def scan_runs(lengths) -> tuple:
     return most >= SCAN_CHUNK_TOKENS, least < SCAN_CHUNK_TOKENS, most >= SCAN_LONG_TOKENS, least >= SCAN_LONG_TOKENS_FEW_HEADS
 
 
-def _scan_route(kind, heads, rows, step, device):
+def _scan_route(kind, heads, rows, step, device, groups=1):
     """How a step's recurrence runs: (scratch of the chunk kernels, or None without them; how many of them are launched; the length
     from which they run a sequence; the length below which the walk runs one, 0 without the walk).  Every sequence is run by
-    its own length, which the kernels read; step.scan_runs says which of the two have work (the engine's steps know)."""
+    its own length, which the kernels read (`groups`: of heads that share B and C); step.scan_runs says which of the two have work (the engine's steps know)."""
     longest = getattr(step, "max_q_len", 0)
     in_chunks, walked = (getattr(step, "scan_runs", None) or ())[:2] or (longest >= SCAN_CHUNK_RUN, step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs)
     if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
         least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
-        lib, sizes = _lib("scan_chunks"), (kind, heads, rows, step.n_tokens, step.n_seqs, least)
+        lib, sizes = _lib("scan_chunks"), (kind, heads, groups, rows, step.n_tokens, step.n_seqs, least)
         floats = int(lib.blm_scan_chunks_scratch(*sizes))
         if floats:
             return (torch.empty(floats, dtype=torch.float32, device=device), int(lib.blm_scan_chunks_launches(*sizes)), least,
@@ -1445,9 +1445,9 @@ def _scan_route(kind, heads, rows, step, device):
 
 # From this many new tokens on, a sequence's state-space scan runs in chunks of 64 tokens on the tensor cores (scan_long.cu) where that
 # kernel takes the size: where the blocks of the chunks of sixteen tokens (16 columns of a head each) fill the multiprocessors
-# more than once, and where they do not.  One prompt of 1,024 / 2,048 / 2,700 tokens, states of 128 x 64, us by chunks of sixteen and here: 64
-# heads 126 / 230 / 300 and 106 / 124 / 208, 24 heads 79 / 136 / 173 and 103 / 108 / 114; 512 tokens of 64 heads 75 and 73, 600 85 and 97.
-SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1024, 2048
+# more than once, and where they do not.  One prompt, states of 128 x 64, us by chunks of sixteen and here: 64 heads, 1,024 / 2,048 tokens
+# 86 / 151 and 106 / 122; 24 heads, 1,024 / 2,048 tokens 69 / 115 and 103 / 106.
+SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1536, 2048
 
 
 def _long_route(heads, groups, n_state, value_dim, step, device):
@@ -1457,7 +1457,7 @@ def _long_route(heads, groups, n_state, value_dim, step, device):
     if longest < SCAN_LONG_TOKENS or (runs is not None and len(runs) > 2 and not runs[2]):
         return None
     least = SCAN_LONG_TOKENS if heads * -(-value_dim // 16) > sm_count(device) else SCAN_LONG_TOKENS_FEW_HEADS
-    sizes = (heads, heads // groups, n_state, value_dim, step.n_tokens, step.n_seqs, longest)
+    sizes = (heads, heads // groups, n_state, value_dim, step.n_tokens, step.n_seqs, least)
     floats = -(-_ask("scan_long", "blm_scan_long_scratch", *sizes) // 4) if longest >= least else 0
     if floats == 0:
         return None
@@ -1484,16 +1484,17 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     if long is not None:
         _call("scan_long", "blm_scan_chunks_long_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, min(step.max_q_len, step.n_tokens), long[2], *_state_args(state, state_offset),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, long[2], *_state_args(state, state_offset),
               _ptr(long[0]), _ptr(status_word(y.device)), _stream(), kernels=long[1])
         if long[3]:
             return
     most = long[2] if long is not None else _NO_LIMIT
-    scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device)
+    scratch, launches, least, below = (None, 0, 0, _NO_LIMIT) if wide_sums else _scan_route(_SCAN_SSM, heads, n_state, step, y.device, groups)
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, most, *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, most, *_state_args(state, state_offset), _ptr(scratch),
+              _ptr(status_word(y.device)), _stream(),
               kernels=launches)
     if below == 0:
         return
@@ -1521,7 +1522,7 @@ def delta_scan(q, q_col0, k, k_col0, v, v_col0, b, b_col0, a, a_col0, dt_bias, a
     if scratch is not None:
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, *ba, *aa, _ptr(dt_bias), _ptr(None), _ptr(a_log), _ptr(out),
               out.stride(0), heads, qk_heads, key_dim, value_dim, 0, 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, least, *_state_args(state, state_offset), _ptr(scratch), _ptr(status_word(out.device)), _stream(),
               kernels=launches)
     if below == 0:
         return
@@ -1573,7 +1574,7 @@ def decay_scan(q, q_col0, k, k_col0, v, v_col0, a, a_col0, bias, extra, out, hea
         _call("scan_chunks", "blm_scan_chunks_rows", *qa, *ka, *va, 0, 0, 0, *aa, _ptr(bias), _ptr(extra), _ptr(None),
               _ptr(out), out.stride(0), heads, heads, key_dim, value_dim, 1 if kind == DECAY_LOWER_BOUND else 0,
               1 if read_first else 0, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), step.n_tokens, step.n_seqs, least,
-              *_state_args(state, state_offset), _ptr(scratch), _stream(),
+              *_state_args(state, state_offset), _ptr(scratch), _ptr(status_word(out.device)), _stream(),
               kernels=launches)
     if below == 0:
         return

@@ -80,7 +80,8 @@ def test_a_sequence_has_the_bits_it_has_alone():
     assert torch.equal(own, together)
 
 
-def test_scratch_is_bounded_and_heads_in_passes_change_no_bit():
+def test_scratch_is_bounded_and_heads_in_passes_change_no_bit(monkeypatch):
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", 1536)                            # (sums are kept for every so many tokens of a step)
     gen = torch.Generator(device="cuda")
     gen.manual_seed(4)
     heads, groups, rows, dv, n = 64, 4, 128, 64, 12000
