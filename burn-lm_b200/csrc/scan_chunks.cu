@@ -2,9 +2,9 @@
 //
 // Walked token by token (recurrent.cu) a prompt is a chain: every token waits for the sums over a state's rows of the one
 // before it, and a 2,048-token prompt took 1.1 to 1.8 ms for work that the multiprocessors' fp32 units can do in 0.07.  Here
-// a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 182, state-space scan
-// of 64 heads of 128 x 64 1,116 -> 218, and 124 in chunks of 64 (scan_long.cu), delta rule of 16 heads of 128 x 128 over 1,501 + 500
-// tokens 1,224 -> 214).  With P(i..j) the product of the decays of the tokens i..j (per row, or
+// a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 188, state-space scan
+// of 64 heads of 128 x 64 1,116 -> 151, and 124 in chunks of 64 (scan_long.cu), delta rule of 16 heads of 128 x 128 over 1,501 + 500
+// tokens 1,224 -> 170).  With P(i..j) the product of the decays of the tokens i..j (per row, or
 // one number per head) and S the state in front of the chunk:
 //     out_j  = (P(0..j) q_j)^T S + sum_(i <= j) A_ji x_i,     A_ji = sum_rows q_j P(i+1..j) k_i
 //     S'     = P(0..15) S + sum_j (P(j+1..15) k_j) x_j^T
@@ -59,14 +59,17 @@ __host__ __device__ constexpr int rows_floats(int kind, int np) { return kind ==
 __host__ __device__ constexpr int small_floats(int kind) { return kMat * (kind == kDelta ? 2 : 1) + (kind == kSsm ? 48 : 0); }
 __host__ __device__ constexpr int part_floats(int kind, int np) { return rows_floats(kind, np) + small_floats(kind); }
 
-// Where the walk runs on the tensor cores (states of 64 and 128 rows that decay), floats as three bfloat16 numbers: a (chunk, head) has
-// [q][k] [3][16][NP] (the state-space scan once a group of heads, behind all chunks' and heads'), [the chunk's decay], A [3][16][16],
+// Where the walk runs on the tensor cores (states of 128 rows, and of 64 that decay: the delta rule's chain of two barriers a chunk is
+// longer there than what the fp32 units take, 2,048 tokens of 16 heads of 64 x 64 173 us instead of 167), floats as three bfloat16 numbers: a (chunk, head) has
+// [decayed k for the correction (delta)][q][k] [3][16][NP] (the state-space scan once a group of heads, behind all chunks' and heads'), [the chunk's decay], A [3][16][16] (delta: A T, then T),
 // and for the state-space scan the 48 numbers.  Rows of tokens lie in 16-byte pieces, piece c of token t at c ^ (t % 8); rows of A,
 // two pieces, at c ^ (j / 4 % 2).
-__host__ __device__ constexpr bool on_tensor_cores(int kind, int np) { return kind != kDelta && (np == 64 || np == 128); }
+__host__ __device__ constexpr bool on_tensor_cores(int kind, int np) { return np == 128 || (np == 64 && kind != kDelta); }
 __host__ __device__ constexpr int limb_rows(int np) { return 2 * 3 * kQ * np / 2; }      // floats
 constexpr int kLimbMat = 3 * kQ * kQ / 2;
-__host__ __device__ constexpr int limb_part(int kind, int np) { return kind == kSsm ? kLimbMat + 48 : limb_rows(np) + np + kLimbMat; }
+__host__ __device__ constexpr int limb_part(int kind, int np) {
+    return kind == kSsm ? kLimbMat + 48 : (kind == kDelta ? limb_rows(np) * 3 / 2 + np + 2 * kLimbMat : limb_rows(np) + np + kLimbMat);
+}
 __device__ __forceinline__ int limb_at(int t, int r, int np) { return (t * np + (((r >> 3) ^ (t & 7)) << 3) + (r & 7)) * 2; }      // bytes
 __device__ __forceinline__ int limb_mat_at(int j, int i) { return j * 32 + (((i >> 3) ^ (j >> 2 & 1)) << 4) + (i & 7) * 2; }
 // the 16 x 16 matrix A as parts: a thread two neighbouring i
@@ -222,18 +225,20 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         const float s = sum_sixteen(v);
         if (!(lane & 1)) sums[2][warp][lane >> 1] = s;
     }
-    constexpr bool kLimbs = !DELTA && on_tensor_cores(kDecay, NP);
-    float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h) * (kLimbs ? limb_part(kDecay, NP) : part_floats(DELTA ? kDelta : kDecay, NP));
+    constexpr bool kLimbs = on_tensor_cores(DELTA ? kDelta : kDecay, NP);
+    float* out = a.scratch + ((size_t)blockIdx.x * a.heads + h) * (kLimbs ? limb_part(DELTA ? kDelta : kDecay, NP) : part_floats(DELTA ? kDelta : kDecay, NP));
     if (kLimbs && r < NP) {
         // an even lane writes its row and the next one's first eight tokens, an odd one the last eight of the row before and its own
         const bool up = lane & 1;
         unsigned char* rows = reinterpret_cast<unsigned char*>(out);
-        float qd[kQ], kd[kQ], p = 1.f;
+        constexpr int kSets = DELTA ? 3 : 2, kDecays = limb_rows(NP) / 2 * kSets;
+        float kc[kQ], qd[kQ], kd[kQ], p = 1.f;
 #pragma unroll
         for (int t = 0; t < kQ; ++t) {
             if (kFirst) qd[t] = qq[t] * p;
             p *= w[t];
             if (!kFirst) qd[t] = qq[t] * p;
+            kc[t] = kk[t] * p;
         }
         p = 1.f;
 #pragma unroll
@@ -241,12 +246,13 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
             kd[t] = kk[t] * p;
             p *= w[t];
         }
-        out[limb_rows(NP) + r] = p;
+        out[kDecays + r] = p;
 #pragma unroll
-        for (int which = 0; which < 2; ++which)
+        for (int which = 0; which < kSets; ++which)
 #pragma unroll
             for (int t = 0; t < kQ / 2; ++t) {
-                const float low = which ? kd[t] : qd[t], high = which ? kd[t + 8] : qd[t + 8];
+                const float(&from)[kQ] = which == kSets - 1 ? kd : (which == kSets - 2 ? qd : kc);
+                const float low = from[t], high = from[t + 8];
                 const float other = __shfl_xor_sync(0xffffffffu, up ? low : high, 1);
                 unsigned l[3];
                 tc5::split3(up ? other : low, up ? high : other, l[0], l[1], l[2]);
@@ -338,7 +344,7 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         As[r][r] = s;
     }
     __syncthreads();
-    if (kLimbs) {
+    if (kLimbs && !DELTA) {
         store_limb_mat(out + limb_rows(NP) + NP, As, r);
         return;
     }
@@ -361,16 +367,34 @@ __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepA
         for (int j = 0; j < kQ; ++j) Ts[j][r] = x[j];
     }
     __syncthreads();
-    for (int e = r; e < kMat; e += T) {
-        const int j = e / kMs, i = e % kMs;
-        float s = 0.f;
-        if (i < kQ) {
+    if constexpr (kLimbs) {
+        // (nothing of a later token: its place is zero, whatever the solution left there)
+        for (int e = r; e < kQ * kQ; e += T) {
+            const int j = e / kQ, i = e % kQ;
+            float s = 0.f;
 #pragma unroll
             for (int y = 0; y < kQ; ++y)
-                if (y <= j) s += As[j][y] * Ts[y][i];           // (nothing of a later token, not even times zero)
+                if (y <= j) s += As[j][y] * Ts[y][i];
+            Cs[j][i] = i > j ? 0.f : s;
         }
-        m[e] = s;
-        m[kMat + e] = i < kQ ? Ts[j][i] : 0.f;
+        __syncthreads();
+        for (int e = r; e < kQ * kQ; e += T)
+            if (e % kQ > e / kQ) Ts[e / kQ][e % kQ] = 0.f;
+        __syncthreads();
+        store_limb_mat(out + limb_rows(NP) * 3 / 2 + NP, Cs, r);
+        store_limb_mat(out + limb_rows(NP) * 3 / 2 + NP + kLimbMat, Ts, r);
+    } else {
+        for (int e = r; e < kMat; e += T) {
+            const int j = e / kMs, i = e % kMs;
+            float s = 0.f;
+            if (i < kQ) {
+#pragma unroll
+                for (int y = 0; y < kQ; ++y)
+                    if (y <= j) s += As[j][y] * Ts[y][i];           // (nothing of a later token, not even times zero)
+            }
+            m[e] = s;
+            m[kMat + e] = i < kQ ? Ts[j][i] : 0.f;
+        }
     }
 }
 
@@ -1106,6 +1130,229 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_mma_kernel(const WalkArg
         }
 }
 
+// ---------------------------------------------------------------------------------------------
+// the delta rule on the tensor cores: the same layout, with a second barrier, behind which every warp forms the corrected values
+// x = T (v - k S) for itself from the warps' shares of k S (as many products as the tokens' among themselves), and a warp of its own
+// the output q S + A T (v - k S).  1,501 + 500 tokens of 16 heads of 128 x 128: 176 -> 119 us (the launch before it 46 -> 51), 2,048 tokens
+// 228 -> 202 with it, four times 500 232 -> 169; the parts of a chunk, 40 KB, leave room for two chunks and two blocks a multiprocessor.
+// ---------------------------------------------------------------------------------------------
+constexpr int kDeltaRing = 2, kDeltaStage = limb_part(kDelta, 128) + kQ * kVs;      // chunks in shared memory, floats of one
+
+__global__ void __launch_bounds__(kLimbThreads, 2) walk_delta_kernel(const WalkArgs a) {
+    constexpr int NP = 128, CT = 16, KS = NP / 64, kRing = kDeltaRing, kStage = kDeltaStage, kShare = 2 * kQ * kVs, kPart = limb_part(kDelta, NP), kPlane = kQ * NP * 2;
+    constexpr int kDecays = limb_rows(NP) * 3 / 2, kMats = kDecays + NP;
+    constexpr int of_a[6] = {2, 0, 1, 1, 0, 0}, of_b[6] = {0, 2, 1, 0, 1, 0};      // parts of the products, the smallest first
+    extern __shared__ __align__(16) float sm[];
+    float* shares = sm + kRing * kStage;                       // [4 warps][k S, q S][16 tokens][kVs]
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(shares + 4 * kShare);      // [kRing] a chunk is there
+    const int h = blockIdx.y, seq = blockIdx.z, col0 = blockIdx.x * CT;
+    const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
+    if (n_new < a.ch.least || n_new >= a.ch.most) return;
+    const int base = chunk_base(first, seq, a.ch.packed) - a.ch.from, start = a.start_pos[seq];
+    const int lo = max(0, -base), hi = min((n_new + kQ - 1) / kQ, a.ch.count - base);
+    if (lo >= hi) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t2 = (lane & 3) * 2;              // the lane's column (and g + 8), its pair of rows or tokens
+    const int tq = (lane & 7) + (lane >> 4) * 8, pq = lane >> 3 & 1, tk = (lane & 7) + (lane >> 3 & 1) * 8, pk = lane >> 4;      // as above
+    if (tid == 0) {
+        for (int i = 0; i < kRing; ++i) tc5::mbar_init(full + i, 32 + 1);
+        tc5::mbar_init_fence();
+    }
+    __syncthreads();
+    auto there = [&](int chunk) {
+        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT);
+        return sm + (chunk - lo) % kRing * kStage;
+    };
+
+    if (warp == 4) {                           // the loads
+        auto bring = [&](int chunk) {
+            if (chunk >= hi) return;
+            unsigned long long* bar = full + (chunk - lo) % kRing;
+            float* st = sm + (chunk - lo) % kRing * kStage;
+            const int at = first + chunk * kQ, nt = min(kQ, n_new - chunk * kQ);
+            if (lane == 0) {
+                tc5::mbar_expect_tx(bar, kPart * 4);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(tc5::smem_u32(st)),
+                             "l"(a.scratch + ((size_t)(base + chunk) * a.heads + h) * kPart), "r"(kPart * 4), "r"(tc5::smem_u32(bar))
+                             : "memory");
+            }
+            const float* v = a.v.p + (size_t)at * a.v.stride + a.v.col0 + (size_t)h * a.dv + col0;
+#pragma unroll
+            for (int i = 0; i < kQ * CT / 32; ++i) {
+                const int t = (lane + 32 * i) / CT, c = (lane + 32 * i) % CT;
+                const bool on = t < nt && col0 + c < a.dv;
+                cp4(st + kPart + t * kVs + c, on ? v + t * a.v.stride + c : a.scratch, on ? 4 : 0);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(tc5::smem_u32(bar)) : "memory");
+        };
+        for (int i = 0; i < kRing - 1; ++i) bring(lo + i);
+        for (int chunk = lo; chunk < hi; ++chunk) {
+            __syncthreads();                   // the others are done with the chunk before, where the next one goes
+            bring(chunk + kRing - 1);
+            __syncthreads();
+        }
+        return;
+    }
+
+    // v - k S of a token and column, once the warps' shares are there
+    auto left = [&](const float* st, int t, int c) {
+        float s = shares[t * kVs + c];
+#pragma unroll
+        for (int w = 1; w < 4; ++w) s += shares[w * kShare + t * kVs + c];
+        return st[kPart + t * kVs + c] - s;
+    };
+    // the matrix (`which` 0: A T, 1: T) times v - k S: columns g, g + 8; tokens t2, + 1 (and 8 further).  A zero of the matrix does not
+    // silence a value that is not finite: it is taken out and joins the tokens behind it by itself.
+    auto corrected = [&](const float* st, int which, float (&o)[2][4]) {
+        const float* mat = st + kMats + which * kLimbMat;
+        float wv[4][2];
+        unsigned most = 0, w3[3][4], b[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const float v = left(st, t2 + y + (e >> 1) * 8, g + (e & 1) * 8);
+                most = max(most, __float_as_uint(v) & 0x7fffffffu);
+                wv[e][y] = isfinite(v) ? v : 0.f;
+            }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tc5::split3(wv[e][0], wv[e][1], w3[0][e], w3[1][e], w3[2][e]);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) ldsm_x4(b[l], (unsigned)__cvta_generic_to_shared(mat) + l * kQ * kQ * 2 + tq * 32 + ((pq ^ (tq >> 2 & 1)) << 4));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma_bf16(o[n], w3[of_a[p]], b[of_b[p]][2 * n], b[of_b[p]][2 * n + 1]);
+        if (__any_sync(0xffffffffu, most >= 0x7f800000u)) {
+#pragma unroll 1
+            for (int i = 0; i < kQ; ++i) {
+                const float v0 = left(st, i, g), v1 = left(st, i, g + 8);
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int j = 8 * n + t2 + (e & 1);
+                        const float v = e >> 1 ? v1 : v0;
+                        float w = 0.f;
+#pragma unroll
+                        for (int l = 0; l < 3; ++l)
+                            w += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(reinterpret_cast<const unsigned char*>(mat) + l * kQ * kQ * 2 + limb_mat_at(j, i)));
+                        if (i <= j && !isfinite(v)) o[n][e] = fmaf(w, v, o[n][e]);
+                    }
+            }
+        }
+    };
+
+    if (warp == 5) {                           // the output
+        for (int chunk = lo; chunk < hi; ++chunk) {
+            __syncthreads();
+            const float* st = there(chunk);
+            __syncthreads();
+            float o[2][4];
+            corrected(st, 0, o);
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = 8 * n + t2 + (e & 1), c = g + (e >> 1) * 8;
+                    float s = o[n][e];
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) s += shares[w * kShare + kQ * kVs + j * kVs + c];
+                    if (chunk * kQ + j < n_new && col0 + c < a.dv) a.y[(size_t)(first + chunk * kQ + j) * a.y_stride + (size_t)h * a.dv + col0 + c] = s;
+                }
+        }
+        return;
+    }
+
+    const int row0 = warp * (NP / 4);
+    float* both = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off + (size_t)h * NP * a.dv;
+    float* fresh = both + (size_t)((start + n_new) & 1) * a.copy_stride;
+    const float* old = lo > 0 ? fresh : both + (size_t)(start & 1) * a.copy_stride;      // (behind an earlier pass: what that wrote)
+    float S[2 * KS][4];                        // tile n: columns g, g + 8; rows row0 + 8 n + t2, + 1
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + (e >> 1) * 8;
+            S[n][e] = (start > 0 || lo > 0) && col < a.dv ? old[((size_t)(row0 / 8 + n) * a.dv + col) * 8 + t2 + (e & 1)] : 0.f;
+        }
+    for (int chunk = lo; chunk < hi; ++chunk) {
+        __syncthreads();
+        const float* st = there(chunk);
+        const unsigned rows = (unsigned)__cvta_generic_to_shared(st);
+        // the rows of the state in front of the chunk against those of k and of q
+        {
+            unsigned s3[KS][3][4], b[2][KS][3][4];
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+#pragma unroll
+                for (int l = 0; l < 3; ++l)
+#pragma unroll
+                    for (int which = 0; which < 2; ++which)
+                        ldsm_x4(b[which][u][l], rows + (which * 3 + l) * kPlane + tq * NP * 2 + (((row0 / 8 + 2 * u + pq) ^ (tq & 7)) << 4));
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) tc5::split3(S[2 * u + (e >> 1)][(e & 1) * 2], S[2 * u + (e >> 1)][(e & 1) * 2 + 1], s3[u][0][e], s3[u][1][e], s3[u][2][e]);
+            float o[2][KS][2][4] = {};
+#pragma unroll
+            for (int p = 0; p < 6; ++p)
+#pragma unroll
+                for (int which = 0; which < 2; ++which)
+#pragma unroll
+                    for (int u = 0; u < KS; ++u)
+#pragma unroll
+                        for (int n = 0; n < 2; ++n) mma_bf16(o[which][u][n], s3[u][of_a[p]], b[which][u][of_b[p]][2 * n], b[which][u][of_b[p]][2 * n + 1]);
+#pragma unroll
+            for (int which = 0; which < 2; ++which)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float s = KS > 1 ? o[which][0][n][e] + o[which][KS - 1][n][e] : o[which][0][n][e];
+                        shares[warp * kShare + which * kQ * kVs + (8 * n + t2 + (e & 1)) * kVs + g + (e >> 1) * 8] = s;
+                    }
+        }
+        unsigned k[KS][3][4];
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int l = 0; l < 3; ++l) ldsm_x4_trans(k[u][l], rows + (6 + l) * kPlane + tk * NP * 2 + (((row0 / 8 + 2 * u + pk) ^ (tk & 7)) << 4));
+        float2 p2[KS][2];
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) p2[u][n] = *reinterpret_cast<const float2*>(st + kDecays + row0 + (2 * u + n) * 8 + t2);
+        __syncthreads();
+        float x[2][4], d[KS][2][4] = {};
+        corrected(st, 1, x);
+        unsigned x3[3][4];                     // (tile n's pairs of tokens of the columns g and g + 8)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tc5::split3(x[e >> 1][(e & 1) * 2], x[e >> 1][(e & 1) * 2 + 1], x3[0][e], x3[1][e], x3[2][e]);
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int u = 0; u < KS; ++u)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) mma_bf16(d[u][n], x3[of_a[p]], k[u][of_b[p]][2 * n], k[u][of_b[p]][2 * n + 1]);
+#pragma unroll
+        for (int u = 0; u < KS; ++u)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[2 * u + n][e] = fmaf(S[2 * u + n][e], e & 1 ? p2[u][n].y : p2[u][n].x, d[u][n][e]);
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int col = col0 + g + (e >> 1) * 8;
+            if (col < a.dv) fresh[((size_t)(row0 / 8 + n) * a.dv + col) * 8 + t2 + (e & 1)] = S[n][e];
+        }
+}
+
 // Rows of a state as the scans keep them: eight times a power of two.
 static int padded_rows(int rows) {
     int n = 8;
@@ -1138,11 +1385,16 @@ static int launch_walk_mma(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
     return blm_check_launch("scan_chunks (walk)");
 }
 
-// Rows and columns of a thread, columns of a block.  Four columns a thread: a row piece that comes from shared memory serves four
-// multiply-adds a row; 16 columns a block: a prompt of few heads still has a block for most multiprocessors.  2,048 tokens, states
-// of 128 rows (decay of 32 heads x 128 columns / state-space scan of 64 x 64 / delta rule of 16 x 128, 2,001 tokens), us:
-// 4 columns, 4 rows, 16 a block 177 / 202 / 174; 32 a block 198 / 208 / 249; 2 columns, 8 rows, 16 a block 206 / 216 / 188;
-// 4 columns, 8 rows, 16 a block (64 threads) 237 / 260 / 211, 32 a block 184 / 200 / 216.
+static int launch_walk_delta(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+    constexpr size_t smem = ((size_t)kDeltaRing * kDeltaStage + 4 * 2 * kQ * kVs) * sizeof(float) + 64;
+    if (int rc = allow_smem(walk_delta_kernel, smem)) return rc;
+    walk_delta_kernel<<<dim3((a.dv + 15) / 16, a.heads, n_seqs), kLimbThreads, smem, stream>>>(a);
+    return blm_check_launch("scan_chunks (walk)");
+}
+
+// States of 128 rows, and of 64 that decay, are walked on the tensor cores.  The others with rows and columns of a thread, columns of a
+// block: four columns a thread, a row piece that comes from shared memory serves four multiply-adds a row; 16 columns a block, a
+// prompt of few heads still has a block for most multiprocessors.
 template <int KIND>
 static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
     if constexpr (KIND != kDelta) {
@@ -1150,7 +1402,7 @@ static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
         if (np == 128) return launch_walk_mma<128, KIND>(a, n_seqs, stream);
     } else {
         if (np == 64) return launch_walk<64, 2, 16, 16, KIND>(a, n_seqs, stream);
-        if (np == 128) return launch_walk<128, 4, 32, 16, KIND>(a, n_seqs, stream);
+        if (np == 128) return launch_walk_delta(a, n_seqs, stream);
     }
     switch (np) {
         case 32: return launch_walk<32, 2, 8, 32, KIND>(a, n_seqs, stream);
