@@ -14,8 +14,12 @@
 //   the values, transposed:  O^T += V^T M^T: rows are value lanes, k runs over keys, columns are eight head rows, of which four
 //     belong to the key/value head.  Two queries fill both halves: the second query's rows cross over by one shuffle.
 // Weights, their mix and the outputs never leave registers; shared memory holds keys, values, the queries' and talk's fragments.
-// 1,536 tokens of 32 heads of 64 on 8: 695 -> 167 us; 64 single tokens over 1,088 keys: 220 -> 38 us (3.7 TB/s).
-#include "common.cuh"
+// 1,536 tokens of 32 heads of 64 on 8, the kernel alone: 695 us with shared memory between the three, 167 with blocks of four warps
+// that met at a barrier a tile, 130 with tiles by TMA and no barrier (quad_rows_kernel); 64 single tokens over 1,088 keys: 220, 38
+// and 33 us (4.3 TB/s).
+#include <type_traits>
+
+#include "tcgen05.cuh"
 
 BLM_API const char* blm_attention_quads_last_error() { return g_blm_error; }
 
@@ -117,61 +121,61 @@ __device__ __forceinline__ void stage_talk(uint4* to, const QuadArgs& a, int tid
 }
 
 // The queries' fragments of one pair of queries: [key/value head][32 lanes of a key][lane] of 16 bytes (two steps of sixteen; the
-// second one zero beyond the last); column n is head n / 2, query n % 2 (rows row0, row0 + 1; a query beyond `rows` is zero).
-__device__ __forceinline__ void stage_queries(uint4* to, const QuadArgs& a, size_t row0, int rows, int lane) {
-    const int per = a.H / a.G, steps = a.dk / 16, pairs = (steps + 1) / 2, n = lane >> 2, h = n >> 1, x = n & 1;
+// second one zero beyond the last); column n is head n / 2, query n % 2 (rows row0, row0 + 1; a query beyond `rows` is zero).  Warps
+// take every `by`-th piece from `from` on, and eight of a warp's pieces are on their way together: one after another they held a
+// block some 5 us before its first product.
+template <int KS, bool FULL>
+__device__ __forceinline__ void stage_queries(uint4* to, const QuadArgs& a, size_t row0, int rows, int lane, int from, int by) {
+    const int per = a.H / a.G, steps = FULL ? KS : a.dk / 16, pairs = (steps + 1) / 2, n = lane >> 2, h = n >> 1, x = n & 1;
+    const int G = FULL ? kQuads : a.G;
     const bool live = h < per && x < rows;
     const __nv_bfloat16* q = a.q + (row0 + (live ? x : 0)) * a.H * a.dk + (lane & 3) * 2;
-    for (int g = 0; g < a.G; ++g)
-        for (int s = 0; s < pairs; ++s) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (live) {
-                const __nv_bfloat16* p = q + (g * per + h) * a.dk + s * 32;
-                v.x = *reinterpret_cast<const unsigned*>(p);
-                v.y = *reinterpret_cast<const unsigned*>(p + 8);
-                if (2 * s + 1 < steps) {
-                    v.z = *reinterpret_cast<const unsigned*>(p + 16);
-                    v.w = *reinterpret_cast<const unsigned*>(p + 24);
-                }
+#pragma unroll 8
+    for (int i = from; i < G * pairs; i += by) {
+        const int g = i / pairs, s = i % pairs;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (live) {
+            const unsigned* p = reinterpret_cast<const unsigned*>(q + (g * per + h) * a.dk + s * 32);
+            v.x = __ldg(p);
+            v.y = __ldg(p + 4);
+            if (2 * s + 1 < steps) {
+                v.z = __ldg(p + 8);
+                v.w = __ldg(p + 12);
             }
-            to[(g * pairs + s) * 32 + lane] = v;
         }
+        to[i * 32 + lane] = v;
+    }
 }
 
 // Rows of keys and values in shared memory are 128 bytes (256 beyond 64 lanes); the 16-byte piece c of row r lies in place
 // c ^ (r % 8), so that the eight rows an ldmatrix reads at one piece lie in eight different groups of banks.
 //
-// Scores of a tile of sixteen keys (keys at `k`, rows of `row` bytes, a key/value head every `head` bytes) for the staged queries.
+// Scores of a tile of sixteen keys (keys at `k`, rows of `row` bytes, a key/value head every `head` bytes) for the staged queries:
+// key/value heads u0 to u0 + 3, whose products are independent, so that one's latency hides behind the others'.
 template <int KS, bool FULL>
-__device__ __forceinline__ void score_tile(float (&c)[kQuads][4], unsigned k, int row, int head, const uint4* qf, int G, int steps, int lane) {
+__device__ __forceinline__ void score_tile(float (&c)[4][4], int u0, unsigned k, int row, int head, const uint4* qf, int G, int steps, int lane) {
     const unsigned at = k + ((lane & 7) + (lane >> 3 & 1) * 8) * row, turn = ((lane >> 4) ^ (lane & 7)) * 16;
     const int pairs = FULL ? KS / 2 : (steps + 1) / 2;
 #pragma unroll
-    for (int u = 0; u < kQuads; ++u) c[u][0] = c[u][1] = c[u][2] = c[u][3] = 0.f;
+    for (int u = 0; u < 4; ++u) c[u][0] = c[u][1] = c[u][2] = c[u][3] = 0.f;
 #pragma unroll
     for (int s = 0; s < KS / 2; ++s) {
         if (FULL || s < pairs) {
-            // (four heads at a time: their products are independent, so that one's latency hides behind the others')
+            unsigned f[4][4];
+            uint4 b[4];
 #pragma unroll
-            for (int u0 = 0; u0 < kQuads; u0 += 4) {
-                if (FULL || u0 < G) {
-                    unsigned f[4][4];
-                    uint4 b[4];
+            for (int u = 0; u < 4; ++u) {
+                const int v = FULL || u0 + u < G ? u0 + u : 0;
+                ldsm_x4(f[u], at + v * head + (turn ^ (s * 64)));
+                b[u] = qf[(v * pairs + s) * 32 + lane];
+            }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int v = FULL || u0 + u < G ? u0 + u : 0;
-                        ldsm_x4(f[u], at + v * head + (turn ^ (s * 64)));
-                        b[u] = qf[(v * pairs + s) * 32 + lane];
-                    }
+            for (int u = 0; u < 4; ++u) mma_bf16(c[u], f[u], b[u].x, b[u].y);
+            if (FULL || 2 * s + 1 < steps) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) mma_bf16(c[u0 + u], f[u], b[u].x, b[u].y);
-                    if (FULL || 2 * s + 1 < steps) {
+                for (int u = 0; u < 4; ++u) ldsm_x4(f[u], at + (FULL || u0 + u < G ? u0 + u : 0) * head + (turn ^ (s * 64 + 32)));
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) ldsm_x4(f[u], at + (FULL || u0 + u < G ? u0 + u : 0) * head + (turn ^ (s * 64 + 32)));
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) mma_bf16(c[u0 + u], f[u], b[u].z, b[u].w);
-                    }
-                }
+                for (int u = 0; u < 4; ++u) mma_bf16(c[u], f[u], b[u].z, b[u].w);
             }
         }
     }
@@ -192,55 +196,41 @@ __device__ __forceinline__ float rcp_fast(float v) {
 // cap tanh(x) = cap - 2 cap / (1 + exp(2 x)), so that with a cap the exponent is one multiply-add of a reciprocal.
 struct WeighConsts {
     float in, out;                 // exp2(s in); exponent: start + out / (1 + that), or start + s out without a cap
-    bool cap;
 };
 __device__ __forceinline__ WeighConsts weigh_consts(float scale, float cap) {
     constexpr float kLog2e = 1.4426950408889634f;
     WeighConsts w;
-    w.cap = cap > 0.f;
-    w.in = w.cap ? 2.0f * scale / cap * kLog2e : 0.f;
-    w.out = w.cap ? 2.0f * cap * kLog2e : -scale * kLog2e;
+    w.in = cap > 0.f ? 2.0f * scale / cap * kLog2e : 0.f;
+    w.out = cap > 0.f ? 2.0f * cap * kLog2e : -scale * kLog2e;
     return w;
 }
 __device__ __forceinline__ float weigh_start(float cap, float bias) { return -(cap > 0.f ? cap + bias : bias) * 1.4426950408889634f; }
 
 // Scores to weights, in place; key of c[.][2 r + x]: j + 8 r (j: the lane's first), query x at position p0 + x.
-template <int X>
-__device__ __forceinline__ void weigh(float (&c)[kQuads][4], const float (&start)[kQuads], int j, int p0, bool open, const WeighConsts& k) {
-    if (k.cap) {
+template <int X, bool CAP, bool OPEN>
+__device__ __forceinline__ void weigh(float (&c)[4][4], const float* start, int j, int p0, const WeighConsts& k) {
 #pragma unroll
-        for (int u = 0; u < kQuads; ++u)
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
+        for (int r = 0; r < 2; ++r)
 #pragma unroll
-                for (int x = 0; x < X; ++x) {
-                    const float t = rcp_fast(1.0f + exp2_fast(c[u][2 * r + x] * k.in));
-                    c[u][2 * r + x] = rcp_fast(1.0f + exp2_fast(fmaf(k.out, t, start[u])));
-                }
-    } else {
-#pragma unroll
-        for (int u = 0; u < kQuads; ++u)
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int x = 0; x < X; ++x) c[u][2 * r + x] = rcp_fast(1.0f + exp2_fast(fmaf(k.out, c[u][2 * r + x], start[u])));
-    }
-    if (!open) {
-#pragma unroll
-        for (int u = 0; u < kQuads; ++u)
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int x = 0; x < X; ++x)
-                    if (j + 8 * r > p0 + x) c[u][2 * r + x] = 0.f;
-    }
+            for (int x = 0; x < X; ++x) {
+                float& v = c[u][2 * r + x];
+                const float t = CAP ? rcp_fast(1.0f + exp2_fast(v * k.in)) : v;
+                v = rcp_fast(1.0f + exp2_fast(fmaf(k.out, t, start[u])));
+                if (!OPEN && j + 8 * r > p0 + x) v = 0.f;
+            }
 }
 
-// The mix of X queries' weights, packed: p[query][row tile][row half][key half] is head row (lane / 4) + 8 half at keys
-// 2 (lane % 4), + 1.  A k tile's talk serves every query and key half, and their products do not wait for one another.  Of the
-// nine products of limbs the three below 2^-24 of a product are left out; the smallest are added first.
-template <int X, bool FULL>
-__device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[kQuads][4], const uint4* talk, int G, int lane) {
+// The mixed weights of X queries for a tile of sixteen keys, packed: p[query][row tile][row half][key half] is head row
+// (lane / 4) + 8 half at keys 2 (lane % 4), + 1.  Four key/value heads at a time go from scores to their share of the mix, without a
+// branch in between: one half's products can run under the other half's exponentials.  A k tile's talk serves every query and
+// key half, and their products do not wait for one another.  Of the nine products of limbs the three below 2^-24 of a product
+// are left out; the smallest are added first.
+template <int KS, int X, bool FULL, bool CAP, bool OPEN, typename F>
+__device__ __forceinline__ void mixed_tile_of(unsigned (&p)[X][2][2][2], unsigned k, int row, int head, const uint4* qf, const uint4* talk,
+                                              const float (&start)[kQuads], int j, int p0, const WeighConsts& consts, int G, int steps,
+                                              int lane, F done) {
     float c[X][2][2][4];
 #pragma unroll
     for (int x = 0; x < X; ++x)
@@ -251,13 +241,17 @@ __device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         if (FULL || 4 * t < G) {
+            float w[4][4];
+            score_tile<KS, FULL>(w, 4 * t, k, row, head, qf, G, steps, lane);
+            if (t == 1 || (!FULL && G <= 4)) done();
+            weigh<X, CAP, OPEN>(w, start + 4 * t, j, p0, consts);
             Limbs b[X][2][2];
 #pragma unroll
             for (int x = 0; x < X; ++x)
 #pragma unroll
                 for (int r = 0; r < 2; ++r)
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) b[x][r][half] = split_bf16(w[4 * t + 2 * half][2 * r + x], w[4 * t + 2 * half + 1][2 * r + x]);
+                    for (int half = 0; half < 2; ++half) b[x][r][half] = split_bf16(w[2 * half][2 * r + x], w[2 * half + 1][2 * r + x]);
 #pragma unroll
             for (int m = 0; m < 2; ++m) {
                 if (FULL || 4 * m < G) {
@@ -286,212 +280,327 @@ __device__ __forceinline__ void mix(unsigned (&p)[X][2][2][2], const float (&w)[
 #pragma unroll
                 for (int r = 0; r < 2; ++r) p[x][m][half][r] = pack_bf16(c[x][m][r][2 * half], c[x][m][r][2 * half + 1]);
 }
-
-// ---------------------------------------------------------------------------------------------
-// portions: a block owns eight queries of a sequence and a range of its keys; a team of T warps owns two queries.
-// T = 1 (keys and values of up to 64 lanes): four warps, tiles of 16 keys in two buffers, two blocks a multiprocessor: the warps
-// of one block go through scores, exponentials, mix and values in step, so that one block's tensor cores idle while its special
-// function units work; a second one fills them (one block of eight warps: 206 us for 1,536 tokens of 32 heads on 8, two of
-// four 164).
-// T = 2: eight warps; two warps take 16 keys each up to the mix, hand the mixed weights to each other through shared memory, and
-// take 64 value lanes each.  Tiles of 32 keys, keys and values in one buffer each, the next tile's keys on their way from the
-// end of the scores, its values from the end of the value product.
-// ---------------------------------------------------------------------------------------------
-__host__ __device__ constexpr int portion_warps(int T) { return T == 1 ? 4 : 8; }
-
-struct PortionLayout {
-    int keys, krow, vrow, stages;             // keys of a tile; bytes of a row of keys and of values
-    size_t talk, q, swap, k, v, total;
-};
-__host__ __device__ inline PortionLayout portion_layout(int G, int dk, int T) {
-    PortionLayout l;
-    l.keys = 16 * T;
-    l.krow = l.vrow = 128 * T;
-    l.stages = T == 1 ? 2 : 1;
-    l.talk = 0;
-    l.q = kTalkBytes;
-    l.swap = l.q + (size_t)(portion_warps(T) / T) * G * ((dk + 16) / 32) * 32 * 16;
-    l.k = l.swap + (T == 1 ? 0 : (size_t)portion_warps(T) * 16 * 32 * 4);
-    l.v = l.k + (size_t)l.stages * G * l.keys * l.krow;
-    l.total = l.v + (size_t)l.stages * G * l.keys * l.vrow;
-    return l;
+// (`open`: every query sees all sixteen keys; `done` is called when the keys have been read)
+template <int KS, int X, bool FULL, bool CAP, typename F>
+__device__ __forceinline__ void mixed_tile(unsigned (&p)[X][2][2][2], unsigned k, int row, int head, const uint4* qf, const uint4* talk,
+                                           const float (&start)[kQuads], int j, int p0, bool open, const WeighConsts& consts, int G, int steps,
+                                           int lane, F done) {
+    if (open) mixed_tile_of<KS, X, FULL, CAP, true>(p, k, row, head, qf, talk, start, j, p0, consts, G, steps, lane, done);
+    else mixed_tile_of<KS, X, FULL, CAP, false>(p, k, row, head, qf, talk, start, j, p0, consts, G, steps, lane, done);
 }
 
-template <int KS, int T, bool FULL>
-__global__ void __launch_bounds__(portion_warps(T) * 32, T == 1 ? 2 : 1) quad_portions_kernel(const QuadArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int G = FULL ? kQuads : a.G;
-    const PortionLayout L = portion_layout(G, a.dk, T);
-    constexpr int kWarps = portion_warps(T), kBQ = 2 * kWarps / T, kKeys = 16 * T;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, team = warp / T, part = warp % T;
-    const int seq = blockIdx.x / a.q_tiles, tile = a.q_tiles - 1 - blockIdx.x % a.q_tiles;     // the rows with the most keys first
-    const int first = a.cu_seqlens[seq], n_new = a.cu_seqlens[seq + 1] - first, i0 = tile * kBQ;
-    if (i0 >= n_new) return;
-    const int start = a.start_pos[seq], kv_hi = start + min(i0 + kBQ, n_new);
-    const int tiles = (kv_hi + kKeys - 1) / kKeys, per = tiles_of_range(tiles, a.ranges, 256 / kKeys);
-    const int lo = blockIdx.y * per, hi = min(tiles, lo + per);
-    if (lo >= hi) return;
-    const int* table = a.block_table + (size_t)a.slot_of_seq[seq] * a.table_stride;
-    const uint4* talk = reinterpret_cast<const uint4*>(smem + L.talk);
-    const int steps = FULL ? KS : a.dk / 16, kp = 2 * steps, vp = FULL ? 8 * T : a.dv / 8;
-    uint4* qf = reinterpret_cast<uint4*>(smem + L.q) + (size_t)team * G * ((steps + 1) / 2) * 32;
-    const unsigned ks = smem_at(smem + L.k), vs = smem_at(smem + L.v);
-    const int khead = kKeys * L.krow, vhead = kKeys * L.vrow;
-    const size_t page_elems = (size_t)G * a.page * (a.dk + a.dv);
-    const int iq = i0 + 2 * team, p0 = start + iq;             // the team's queries: rows iq, iq + 1, positions p0, p0 + 1
+// The mixed weights of two queries as operands of the value products: b[parity] is the even and the odd key/value heads' of every
+// pair, both queries in one operand.
+__device__ __forceinline__ void cross(unsigned (&b)[2][2][2][2], const unsigned (&p)[2][2][2][2], int lane) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const unsigned other = __shfl_xor_sync(0xffffffffu, p[1][m][half][r], 16);
+                b[0][m][half][r] = lane < 16 ? p[0][m][half][r] : other;
+                b[1][m][half][r] = lane < 16 ? other : p[0][m][half][r];
+            }
+}
 
-    auto load_keys = [&](int t, int stage, int pg) {
-        if (t < hi) {
-            const int j0 = t * kKeys, live = kv_hi - j0;
-            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)(j0 % a.page) * a.dk;
-            const unsigned to = ks + stage * G * khead;
-            for (int e = tid; e < G * kKeys * kp; e += kWarps * 32) {
-                const int c = e % kp, j = e / kp % kKeys, g = e / (kp * kKeys);
-                cp16(to + g * khead + j * L.krow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dk + c * 8, j < live);
+// Sixteen keys of values (64 lanes from the address on, rows of `row` bytes, a key/value head every `head` bytes) times the packed
+// weights of both queries.
+template <bool FULL>
+__device__ __forceinline__ void value_tile(float (&o)[kQuads][4][4], unsigned v, int row, int head, const unsigned (&b)[2][2][2][2], int G,
+                                           int lane) {
+    const unsigned at = v + ((lane & 7) + (lane >> 4) * 8) * row, turn = ((lane >> 3 & 1) ^ (lane & 7)) * 16;
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u) {
+        if (FULL || u < G) {
+            const unsigned b0 = b[u & 1][u >> 2][u >> 1 & 1][0], b1 = b[u & 1][u >> 2][u >> 1 & 1][1];
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+                unsigned f[4];
+                ldsm_x4_trans(f, at + u * head + (turn ^ (d * 32)));
+                mma_bf16(o[u][d], f, b0, b1);
             }
         }
-    };
-    auto load_values = [&](int t, int stage, int pg) {
-        if (t < hi) {
-            const int j0 = t * kKeys, live = kv_hi - j0;
-            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)G * a.page * a.dk + (size_t)(j0 % a.page) * a.dv;
-            const unsigned to = vs + stage * G * vhead;
-            for (int e = tid; e < G * kKeys * vp; e += kWarps * 32) {
-                const int c = e % vp, j = e / vp % kKeys, g = e / (vp * kKeys);
-                cp16(to + g * vhead + j * L.vrow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dv + c * 8, j < live);
-            }
-        }
-    };
-    auto page_of = [&](int t) { return t < hi ? table[t * kKeys / a.page] : 0; };
-
-    int ahead = 0;                                             // the page of the next tile to be asked for
-    if (T == 1) {
-        const int pg = page_of(lo);
-        load_keys(lo, 0, pg);
-        load_values(lo, 0, pg);
-        cp_commit();
-        ahead = page_of(lo + 1);
-    } else {
-        const int pg = page_of(lo);
-        load_keys(lo, 0, pg);
-        cp_commit();
-        load_values(lo, 0, pg);
-        cp_commit();
-        ahead = page_of(lo + 1);
     }
-    stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, kWarps * 32);
-    if (part == 0) stage_queries(qf, a, (size_t)first + min(iq, n_new - 1), max(0, min(2, n_new - iq)), lane);
-    const WeighConsts consts = weigh_consts(a.scale, a.softcap);
-    float begin[kQuads];
-    {
-        const int per_kv = a.H / a.G;
-#pragma unroll
-        for (int u = 0; u < kQuads; ++u)
-            begin[u] = weigh_start(a.softcap, a.head_bias && u < G && (lane & 3) < per_kv ? a.head_bias[u * per_kv + (lane & 3)] : 0.f);
-    }
-    float o[kQuads][4][4];
-#pragma unroll
-    for (int u = 0; u < kQuads; ++u)
-#pragma unroll
-        for (int d = 0; d < 4; ++d) o[u][d][0] = o[u][d][1] = o[u][d][2] = o[u][d][3] = 0.f;
+}
 
-    // one tile of sixteen keys of values (64 lanes from the address on) times the packed weights of both queries
-    auto values = [&](unsigned v, const unsigned (&b)[2][2][2][2]) {
-        const unsigned at = v + ((lane & 7) + (lane >> 4) * 8) * L.vrow, turn = ((lane >> 3 & 1) ^ (lane & 7)) * 16;
-#pragma unroll
-        for (int u = 0; u < kQuads; ++u) {
-            if (FULL || u < G) {
-                const unsigned b0 = b[u & 1][u >> 2][u >> 1 & 1][0], b1 = b[u & 1][u >> 2][u >> 1 & 1][1];
-#pragma unroll
-                for (int d = 0; d < 4; ++d) {
-                    unsigned f[4];
-                    ldsm_x4_trans(f, at + u * vhead + (turn ^ (d * 32)));
-                    mma_bf16(o[u][d], f, b0, b1);
-                }
-            }
-        }
-    };
-
-    for (int t = lo; t < hi; ++t) {
-        const int stage = T == 1 ? (t - lo) & 1 : 0;
-        cp_wait<T == 1 ? 0 : 1>();
-        __syncthreads();                                       // T 1: this tile is there, the one before done with; T 2: its keys
-        if (T == 1) {
-            load_keys(t + 1, stage ^ 1, ahead);
-            load_values(t + 1, stage ^ 1, ahead);
-            cp_commit();
-            ahead = page_of(t + 2);
-        }
-        const int j0 = t * kKeys + part * 16;
-        const bool some = j0 <= p0 + 1;                        // the warp's queries see some of its keys
-        float c[kQuads][4];
-        if (some) score_tile<KS, FULL>(c, ks + stage * G * khead + part * 16 * L.krow, L.krow, khead, qf, G, steps, lane);
-        if (T > 1) {
-            __syncthreads();                                   // the keys are done with
-            load_keys(t + 1, 0, ahead);
-            cp_commit();
-        }
-        // b[parity]: the weights of the even and the odd key/value heads of every pair, both queries in one operand
-        unsigned b[2][2][2][2];
-        if (some) {
-            weigh<2>(c, begin, j0 + (lane >> 2), p0, j0 + 15 <= p0, consts);
-            unsigned p[2][2][2][2];
-            mix<2, FULL>(p, c, talk, G, lane);
-#pragma unroll
-            for (int m = 0; m < 2; ++m)
-#pragma unroll
-                for (int half = 0; half < 2; ++half)
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const unsigned other = __shfl_xor_sync(0xffffffffu, p[1][m][half][r], 16);
-                        b[0][m][half][r] = lane < 16 ? p[0][m][half][r] : other;
-                        b[1][m][half][r] = lane < 16 ? other : p[0][m][half][r];
-                    }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = 0u;
-        }
-        if (T == 1) {
-            if (some) values(vs + stage * G * vhead, b);
-        } else {
-            unsigned* mine = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)warp * 16 * 32 + lane;
-            const unsigned* theirs = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)(warp ^ 1) * 16 * 32 + lane;
-#pragma unroll
-            for (int e = 0; e < 16; ++e) mine[e * 32] = b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1];
-            cp_wait<1>();                                      // the values; the next keys may be on their way
-            __syncthreads();
-            const unsigned v = vs + part * 128;                // (a piece's place keeps its upper bit: 64 lanes are 8 pieces)
-            const bool own = FULL || part * 64 < a.dv;         // the warp has value lanes
-            if (own) values(v + part * 16 * L.vrow, b);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = theirs[e * 32];
-            if (own) values(v + (part ^ 1) * 16 * L.vrow, b);
-            __syncthreads();                                   // the values and the weights are done with
-            load_values(t + 1, 0, ahead);
-            cp_commit();
-            ahead = page_of(t + 2);
-        }
-    }
-    // column n of key/value head u: head n % 4; an even u's columns 0 .. 3 are query 0's, an odd one's query 1's
+// Two queries' outputs (rows row0, row0 + 1, of which `rows` exist), value lanes lane0 and on, to the result or to the range's share.
+// Column n of key/value head u: head n % 4; an even u's columns 0 .. 3 are query 0's, an odd one's query 1's.
+__device__ __forceinline__ void store_rows(const QuadArgs& a, const float (&o)[kQuads][4][4], size_t row0, int rows, int lane0, int range, int G,
+                                           int lane) {
     const int per_kv = a.H / a.G, HD = a.H * a.dv;
 #pragma unroll
     for (int u = 0; u < kQuads; ++u)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int n = 2 * (lane & 3) + e, h = n & 3, x = (n >> 2) ^ (u & 1);
-            if (u >= G || h >= per_kv || iq + x >= n_new) continue;
-            const size_t at = (size_t)(first + iq + x) * HD + (u * per_kv + h) * a.dv;
+            if (u >= G || h >= per_kv || x >= rows) continue;
+            const size_t at = (row0 + x) * HD + (u * per_kv + h) * a.dv;
 #pragma unroll
             for (int d = 0; d < 4; ++d)
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const int lanev = part * 64 + d * 16 + (lane >> 2) + 8 * r;
+                    const int lanev = lane0 + d * 16 + (lane >> 2) + 8 * r;
                     if (lanev < a.dv) {
-                        if (a.ranges > 1) a.partial[(size_t)blockIdx.y * a.n_tokens * HD + at + lanev] = o[u][d][2 * r + e];
+                        if (a.ranges > 1) a.partial[(size_t)range * a.n_tokens * HD + at + lanev] = o[u][d][2 * r + e];
                         else a.out[at + lanev] = __float2bfloat16_rn(o[u][d][2 * r + e]);
                     }
                 }
         }
+}
+
+__device__ __forceinline__ void head_starts(float (&begin)[kQuads], const QuadArgs& a, int G, int lane) {
+    const int per_kv = a.H / a.G;
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+        begin[u] = weigh_start(a.softcap, a.head_bias && u < G && (lane & 3) < per_kv ? a.head_bias[u * per_kv + (lane & 3)] : 0.f);
+}
+
+// A portion block's sequence, queries and range of keys: the longest blocks first (the last rows of the longest sequences see the
+// most keys, a row's ranges are of one length).
+struct PortionWork {
+    int seq, first, n_new, i0, start, kv_hi, lo, hi, range;
+};
+__device__ __forceinline__ PortionWork portion_work(const QuadArgs& a, int bq, int keys) {
+    PortionWork w;
+    w.range = blockIdx.x % a.ranges;
+    const int at = blockIdx.x / a.ranges;
+    w.seq = at % a.n_seqs;
+    w.i0 = (a.q_tiles - 1 - at / a.n_seqs) * bq;
+    w.first = a.cu_seqlens[w.seq];
+    w.n_new = a.cu_seqlens[w.seq + 1] - w.first;
+    w.start = a.start_pos[w.seq];
+    w.kv_hi = w.start + min(w.i0 + bq, w.n_new);
+    const int tiles = (w.kv_hi + keys - 1) / keys, per = tiles_of_range(tiles, a.ranges, 256 / keys);
+    w.lo = w.range * per;
+    w.hi = w.i0 < w.n_new ? min(tiles, w.lo + per) : 0;
+    return w;
+}
+
+// ---------------------------------------------------------------------------------------------
+// portions, keys and values of up to 64 lanes: a block of eight warps owns sixteen queries of a sequence and a range of its keys; a
+// warp owns two queries.  Tiles of 16 keys come by TMA (whose 128-byte swizzle is the order of the pieces above) into a ring of four,
+// and a warp goes through them at its own pace: no barrier between the warps, so that one's scores and products run under
+// another's exponentials.  The last warp to leave a tile asks for the one four further on into its place.
+// What bounds it (1,536 tokens of 32 heads of 64 on 8, 130 us): no unit alone; a tile's 160 products, its 128 special functions, the
+// 1,700 instructions around them and the 1,700 cycles of shared-memory reads (every two queries read all keys and values again)
+// take 30 to 40 % of the time each, and two warps a scheduler, all that the outputs' registers leave room for, hide only part of
+// one under another.  Left out one at a time, copies, scores, weights, mix and values each took 24 to 37 us off the form before.
+// Measured on the way: copies by TMA and no barrier 167 -> 145 us; the queries' pieces fetched together 145 -> 135; scores, weights and
+// mix by halves of the key/value heads 135 -> 130.  A late start for half of the warps: 137.  Limbs cut off instead of rounded: 129.
+// ---------------------------------------------------------------------------------------------
+constexpr int kRowWarps = 8, kRowStages = 4, kRowBytes = 128;
+
+struct RowLayout {
+    size_t talk, q, tiles, stage, sync, total;
+};
+__host__ __device__ inline RowLayout row_layout(int G, int dk) {
+    RowLayout l;
+    l.talk = 0;
+    l.q = kTalkBytes;
+    l.tiles = (l.q + (size_t)kRowWarps * G * ((dk + 16) / 32) * 32 * 16 + 1023) / 1024 * 1024;
+    l.stage = (size_t)2 * G * 16 * kRowBytes;
+    l.sync = l.tiles + kRowStages * l.stage;
+    l.total = l.sync + kRowStages * 16;
+    return l;
+}
+
+template <bool FULL, bool CAP>
+__global__ void __launch_bounds__(kRowWarps * 32, 1)
+    quad_rows_kernel(const QuadArgs a, const __grid_constant__ CUtensorMap keys, const __grid_constant__ CUtensorMap values, int* status) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int G = FULL ? kQuads : a.G;
+    const RowLayout L = row_layout(G, a.dk);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const PortionWork w = portion_work(a, 2 * kRowWarps, 16);
+    if (w.lo >= w.hi) return;
+    const int* table = a.block_table + (size_t)a.slot_of_seq[w.seq] * a.table_stride;
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(smem + L.sync);
+    unsigned* left = reinterpret_cast<unsigned*>(smem + L.sync + kRowStages * 8);        // warps that have left a place's tiles, in all
+    const int half = G * 16 * kRowBytes;
+    auto load = [&](int t, int place, int pg) {
+        unsigned char* to = smem + L.tiles + place * L.stage;
+        tc5::mbar_expect_tx(full + place, 2 * half);
+        tc5::tma_load_4d(to, &keys, 0, t * 16 % a.page, 0, pg, full + place);
+        tc5::tma_load_4d(to + half, &values, 0, t * 16 % a.page, 0, pg, full + place);
+    };
+    auto page_of = [&](int t) { return t < w.hi ? table[t * 16 / a.page] : 0; };
+    if (tid == 0) {
+        for (int p = 0; p < kRowStages; ++p) {
+            tc5::mbar_init(full + p, 1);
+            left[p] = 0;
+        }
+        tc5::mbar_init_fence();
+        for (int p = 0; p < kRowStages && w.lo + p < w.hi; ++p) load(w.lo + p, p, page_of(w.lo + p));
+    }
+    const uint4* talk = reinterpret_cast<const uint4*>(smem + L.talk);
+    const int steps = FULL ? 4 : a.dk / 16, iq = w.i0 + 2 * warp, p0 = w.start + iq;     // the warp's queries: rows iq, iq + 1 at p0, p0 + 1
+    uint4* qf = reinterpret_cast<uint4*>(smem + L.q) + (size_t)warp * G * ((steps + 1) / 2) * 32;
+    stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, kRowWarps * 32);
+    stage_queries<4, FULL>(qf, a, (size_t)w.first + min(iq, w.n_new - 1), max(0, min(2, w.n_new - iq)), lane, 0, 1);
+    const WeighConsts consts = weigh_consts(a.scale, a.softcap);
+    float begin[kQuads];
+    head_starts(begin, a, G, lane);
+    float o[kQuads][4][4];
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) o[u][d][0] = o[u][d][1] = o[u][d][2] = o[u][d][3] = 0.f;
+    __syncthreads();
+
+    const unsigned ring = smem_at(smem + L.tiles);
+    const int khead = 16 * kRowBytes;
+    for (int t = w.lo; t < w.hi; ++t) {
+        const int place = (t - w.lo) % kRowStages, ahead = page_of(t + kRowStages), j0 = t * 16;
+        if (!tc5::mbar_wait(full + place, (t - w.lo) / kRowStages & 1)) {
+            if (status) *status = tc5::TC5_TIMEOUT;
+            return;
+        }
+        if (j0 + 16 > w.kv_hi) {                               // the sequence's last tile (no other follows): values of rows that
+            __syncthreads();                                   // no key has may be anything and count as zero
+            unsigned char* v = smem + L.tiles + place * L.stage + half;
+            const int from = (w.kv_hi - j0) * (kRowBytes / 16), pieces = 16 * (kRowBytes / 16);
+            for (int e = tid; e < G * pieces; e += kRowWarps * 32)
+                if (e % pieces >= from) reinterpret_cast<uint4*>(v)[e] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+        }
+        if (j0 <= p0 + 1) {                                    // the warp's queries see some of the keys
+            const unsigned at = ring + place * (unsigned)L.stage;
+            unsigned p[2][2][2][2], b[2][2][2][2];
+            mixed_tile<4, 2, FULL, CAP>(p, at, kRowBytes, khead, qf, talk, begin, j0 + (lane >> 2), p0, j0 + 15 <= p0, consts, G, steps, lane,
+                                        [] {});
+            cross(b, p, lane);
+            value_tile<FULL>(o, at + half, kRowBytes, khead, b, G, lane);
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0 && t + kRowStages < w.hi && atomicAdd(left + place, 1u) % kRowWarps == kRowWarps - 1) {
+            __threadfence_block();
+            tc5::fence_async_smem();
+            load(t + kRowStages, place, ahead);
+        }
+    }
+    store_rows(a, o, (size_t)w.first + iq, w.n_new - iq, 0, w.range, G, lane);
+}
+
+// ---------------------------------------------------------------------------------------------
+// portions, more than 64 lanes: a block of eight warps owns eight queries; a team of two warps owns two queries.  The two take 16 keys
+// each up to the mix, hand the mixed weights to each other through shared memory, and take 64 value lanes each.  Tiles of 32 keys,
+// keys and values in one buffer each, the next tile's keys on their way from the end of the scores, its values from the end of
+// the value product.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTeamWarps = 8, kTeamKeys = 32, kTeamRow = 256;
+
+struct PortionLayout {
+    size_t talk, q, swap, k, v, total;
+};
+__host__ __device__ inline PortionLayout portion_layout(int G, int dk) {
+    PortionLayout l;
+    l.talk = 0;
+    l.q = kTalkBytes;
+    l.swap = l.q + (size_t)(kTeamWarps / 2) * G * ((dk + 16) / 32) * 32 * 16;
+    l.k = l.swap + (size_t)kTeamWarps * 16 * 32 * 4;
+    l.v = l.k + (size_t)G * kTeamKeys * kTeamRow;
+    l.total = l.v + (size_t)G * kTeamKeys * kTeamRow;
+    return l;
+}
+
+template <int KS, bool FULL, bool CAP>
+__global__ void __launch_bounds__(kTeamWarps * 32, 1) quad_portions_kernel(const QuadArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int G = FULL ? kQuads : a.G;
+    const PortionLayout L = portion_layout(G, a.dk);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, team = warp / 2, part = warp % 2;
+    const PortionWork w = portion_work(a, kTeamWarps, kTeamKeys);
+    if (w.lo >= w.hi) return;
+    const int kv_hi = w.kv_hi, hi = w.hi;
+    const int* table = a.block_table + (size_t)a.slot_of_seq[w.seq] * a.table_stride;
+    const uint4* talk = reinterpret_cast<const uint4*>(smem + L.talk);
+    const int steps = FULL ? KS : a.dk / 16, kp = 2 * steps, vp = FULL ? 16 : a.dv / 8;
+    uint4* qf = reinterpret_cast<uint4*>(smem + L.q) + (size_t)team * G * ((steps + 1) / 2) * 32;
+    const unsigned ks = smem_at(smem + L.k), vs = smem_at(smem + L.v);
+    const int khead = kTeamKeys * kTeamRow;
+    const size_t page_elems = (size_t)G * a.page * (a.dk + a.dv);
+    const int iq = w.i0 + 2 * team, p0 = w.start + iq;         // the team's queries: rows iq, iq + 1, positions p0, p0 + 1
+
+    auto load_keys = [&](int t, int pg) {
+        if (t < hi) {
+            const int j0 = t * kTeamKeys, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)(j0 % a.page) * a.dk;
+            for (int e = tid; e < G * kTeamKeys * kp; e += kTeamWarps * 32) {
+                const int c = e % kp, j = e / kp % kTeamKeys, g = e / (kp * kTeamKeys);
+                cp16(ks + g * khead + j * kTeamRow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dk + c * 8, j < live);
+            }
+        }
+        cp_commit();
+    };
+    auto load_values = [&](int t, int pg) {
+        if (t < hi) {
+            const int j0 = t * kTeamKeys, live = kv_hi - j0;
+            const __nv_bfloat16* from = a.pool + (size_t)pg * page_elems + (size_t)G * a.page * a.dk + (size_t)(j0 % a.page) * a.dv;
+            for (int e = tid; e < G * kTeamKeys * vp; e += kTeamWarps * 32) {
+                const int c = e % vp, j = e / vp % kTeamKeys, g = e / (vp * kTeamKeys);
+                cp16(vs + g * khead + j * kTeamRow + (c ^ (j & 7)) * 16, from + ((size_t)g * a.page + j) * a.dv + c * 8, j < live);
+            }
+        }
+        cp_commit();
+    };
+    auto page_of = [&](int t) { return t < hi ? table[t * kTeamKeys / a.page] : 0; };
+
+    {
+        const int pg = page_of(w.lo);
+        load_keys(w.lo, pg);
+        load_values(w.lo, pg);
+    }
+    int ahead = page_of(w.lo + 1);                             // the page of the next tile to be asked for
+    stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, kTeamWarps * 32);
+    stage_queries<KS, FULL>(qf, a, (size_t)w.first + min(iq, w.n_new - 1), max(0, min(2, w.n_new - iq)), lane, part, 2);
+    const WeighConsts consts = weigh_consts(a.scale, a.softcap);
+    float begin[kQuads];
+    head_starts(begin, a, G, lane);
+    float o[kQuads][4][4];
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u)
+#pragma unroll
+        for (int d = 0; d < 4; ++d) o[u][d][0] = o[u][d][1] = o[u][d][2] = o[u][d][3] = 0.f;
+
+    for (int t = w.lo; t < hi; ++t) {
+        cp_wait<1>();
+        __syncthreads();                                       // this tile's keys are there
+        const int j0 = t * kTeamKeys + part * 16;
+        const bool some = j0 <= p0 + 1;                        // the warp's queries see some of its keys
+        unsigned b[2][2][2][2];
+        auto refill = [&] {                                    // (warps come here from two places: a barrier of its own)
+            asm volatile("bar.sync 1, %0;\n" ::"n"(kTeamWarps * 32) : "memory");
+            load_keys(t + 1, ahead);
+        };
+        if (some) {
+            unsigned p[2][2][2][2];
+            mixed_tile<KS, 2, FULL, CAP>(p, ks + part * 16 * kTeamRow, kTeamRow, khead, qf, talk, begin, j0 + (lane >> 2), p0, j0 + 15 <= p0, consts, G,
+                                         steps, lane, refill);
+            cross(b, p, lane);
+        } else {
+            refill();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = 0u;
+        }
+        unsigned* mine = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)warp * 16 * 32 + lane;
+        const unsigned* theirs = reinterpret_cast<unsigned*>(smem + L.swap) + (size_t)(warp ^ 1) * 16 * 32 + lane;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) mine[e * 32] = b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1];
+        cp_wait<1>();                                          // the values; the next keys may be on their way
+        __syncthreads();
+        const unsigned v = vs + part * 128;                    // (a piece's place keeps its upper bit: 64 lanes are 8 pieces)
+        const bool own = FULL || part * 64 < a.dv;             // the warp has value lanes
+        if (own) value_tile<FULL>(o, v + part * 16 * kTeamRow, kTeamRow, khead, b, G, lane);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) b[e >> 3][e >> 2 & 1][e >> 1 & 1][e & 1] = theirs[e * 32];
+        if (own) value_tile<FULL>(o, v + (part ^ 1) * 16 * kTeamRow, kTeamRow, khead, b, G, lane);
+        __syncthreads();                                       // the values and the weights are done with
+        load_values(t + 1, ahead);
+        ahead = page_of(t + 2);
+    }
+    store_rows(a, o, (size_t)w.first + iq, w.n_new - iq, part * 64, w.range, G, lane);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -518,9 +627,9 @@ __host__ __device__ inline SingleLayout single_layout(int G, int dk, int dv) {
     return l;
 }
 
-template <int KS, int DT, bool FULL>
+template <int KS, int DT, bool FULL, bool CAP>
 __global__ void __launch_bounds__(192, 1) quad_singles_kernel(const QuadArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int G = FULL ? kQuads : a.G;
     const SingleLayout L = single_layout(G, a.dk, a.dv);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = L.warps * 32;
@@ -569,7 +678,7 @@ __global__ void __launch_bounds__(192, 1) quad_singles_kernel(const QuadArgs a) 
     }
     int ahead = page_of(lo + warp + L.warps);
     stage_talk(reinterpret_cast<uint4*>(smem + L.talk), a, tid, threads);
-    if (warp == 0) stage_queries(qf, a, (size_t)first, 1, lane);
+    stage_queries<KS, FULL>(qf, a, (size_t)first, 1, lane, warp, L.warps);
     const int per_kv = a.H / a.G;
     const WeighConsts consts = weigh_consts(a.scale, a.softcap);
     float begin[kQuads];
@@ -587,13 +696,11 @@ __global__ void __launch_bounds__(192, 1) quad_singles_kernel(const QuadArgs a) 
         ahead = page_of(t + 2 * L.warps);
         cp_wait<1>();
         __syncwarp();
-        float c[kQuads][4];
-        score_tile<KS, FULL>(c, ks, L.krow, khead, qf, G, steps, lane);
-        __syncwarp();
-        load_keys(t + L.warps, pg);
-        weigh<1>(c, begin, t * 16 + (lane >> 2), pos, t * 16 + 15 <= pos, consts);
         unsigned p[1][2][2][2];
-        mix<1, FULL>(p, c, talk, G, lane);
+        mixed_tile<KS, 1, FULL, CAP>(p, ks, L.krow, khead, qf, talk, begin, t * 16 + (lane >> 2), pos, t * 16 + 15 <= pos, consts, G, steps, lane, [&] {
+            __syncwarp();
+            load_keys(t + L.warps, pg);
+        });
         cp_wait<1>();
         __syncwarp();
         const unsigned at = vs + ((lane & 7) + (lane >> 4) * 8) * L.vrow, turn = ((lane >> 3 & 1) ^ (lane & 7)) * 16;
@@ -682,6 +789,9 @@ BLM_API int blm_attention_quads_takes(int H, int G, int dk, int dv, int page) {
     return dk % 16 == 0 && dk >= 16 && dk <= 128 && dv % 8 == 0 && dv >= 8 && dv <= 128 && page % 32 == 0;
 }
 
+// Query rows of a portion block.
+BLM_API int blm_attention_quads_rows(int dk, int dv) { return dv > 64 || dk > 64 ? kTeamWarps : 2 * kRowWarps; }
+
 template <typename K>
 static int allow_smem(K kernel, size_t smem) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -691,7 +801,8 @@ static int allow_smem(K kernel, size_t smem) {
 BLM_API int blm_attention_quads(const void* q, const void* pool, const int* block_table, int table_stride, const int* cu_seqlens,
                                 const int* slot_of_seq, const int* start_pos, const int* token_seq, const float* talk,
                                 const float* head_bias, void* out, float* partial, int n_tokens, int n_seqs, int max_q_len, int H, int G,
-                                int dk, int dv, int page, int ranges, float scale, float softcap, cudaStream_t stream) {
+                                int dk, int dv, int page, long long n_pages, int ranges, float scale, float softcap, int* status,
+                                cudaStream_t stream) {
     if (n_tokens == 0 || n_seqs == 0) return BLM_OK;
     BLM_REQUIRE(blm_attention_quads_takes(H, G, dk, dv, page) && max_q_len > 0, "attention_quads: %d heads on %d, %d + %d lanes", H, G, dk, dv);
     BLM_REQUIRE(ranges >= 1 && ranges <= 65535 && (ranges == 1 || partial != nullptr), "attention_quads: several key ranges need a workspace");
@@ -703,25 +814,51 @@ BLM_API int blm_attention_quads(const void* q, const void* pool, const int* bloc
     int bq = 1, keys = 16;
     if (max_q_len == 1) {
         const SingleLayout l = single_layout(G, dk, dv);
-        auto k = !full ? quad_singles_kernel<8, 8, false>
-                 : dk == 64 ? (dv == 64 ? quad_singles_kernel<4, 4, true> : quad_singles_kernel<4, 8, true>)
-                            : (dv == 64 ? quad_singles_kernel<8, 4, true> : quad_singles_kernel<8, 8, true>);
+        auto pick = [&](auto cap) {
+            constexpr bool CAP = decltype(cap)::value;
+            return !full ? quad_singles_kernel<8, 8, false, CAP>
+                   : dk == 64 ? (dv == 64 ? quad_singles_kernel<4, 4, true, CAP> : quad_singles_kernel<4, 8, true, CAP>)
+                              : (dv == 64 ? quad_singles_kernel<8, 4, true, CAP> : quad_singles_kernel<8, 8, true, CAP>);
+        };
+        auto k = softcap > 0.f ? pick(std::true_type()) : pick(std::false_type());
         BLM_REQUIRE(l.warps >= 1, "attention_quads: shared memory");
         if (int rc = allow_smem(k, l.total)) return rc;
         k<<<dim3(n_seqs, ranges), l.warps * 32, l.total, stream>>>(a);
     } else {
-        const int T = dv > 64 || dk > 64 ? 2 : 1;
-        bq = 2 * portion_warps(T) / T;
-        keys = 16 * T;
+        const bool wide = dv > 64 || dk > 64;
+        bq = blm_attention_quads_rows(dk, dv);
+        keys = wide ? kTeamKeys : 16;
         a.q_tiles = (max_q_len + bq - 1) / bq;
-        BLM_REQUIRE((long long)n_seqs * a.q_tiles <= 0x7fffffffLL, "attention_quads: grid too large");
-        const PortionLayout l = portion_layout(G, dk, T);
-        auto k = T == 1 ? (full ? quad_portions_kernel<4, 1, true> : quad_portions_kernel<4, 1, false>)
-                 : !full || dv == 64 ? quad_portions_kernel<8, 2, false>
-                                     : (dk == 64 ? quad_portions_kernel<4, 2, true> : quad_portions_kernel<8, 2, true>);
-        BLM_REQUIRE(l.total <= 227 * 1024, "attention_quads: shared memory");
-        if (int rc = allow_smem(k, l.total)) return rc;
-        k<<<dim3(n_seqs * a.q_tiles, ranges), portion_warps(T) * 32, l.total, stream>>>(a);
+        const long long blocks = (long long)n_seqs * a.q_tiles * ranges;
+        BLM_REQUIRE(blocks <= 0x7fffffffLL, "attention_quads: grid too large");
+        if (wide) {
+            const PortionLayout l = portion_layout(G, dk);
+            auto pick = [&](auto cap) {
+                constexpr bool CAP = decltype(cap)::value;
+                return !full || dv == 64 ? quad_portions_kernel<8, false, CAP>
+                                         : (dk == 64 ? quad_portions_kernel<4, true, CAP> : quad_portions_kernel<8, true, CAP>);
+            };
+            auto k = softcap > 0.f ? pick(std::true_type()) : pick(std::false_type());
+            BLM_REQUIRE(l.total <= 227 * 1024, "attention_quads: shared memory");
+            if (int rc = allow_smem(k, l.total)) return rc;
+            k<<<(unsigned)blocks, kTeamWarps * 32, l.total, stream>>>(a);
+        } else {
+            const RowLayout l = row_layout(G, dk);
+            auto k = softcap > 0.f ? (full ? quad_rows_kernel<true, true> : quad_rows_kernel<false, true>)
+                                   : (full ? quad_rows_kernel<true, false> : quad_rows_kernel<false, false>);
+            // the pages as [page][key/value head][row][lane]; a box is sixteen rows of every head, lanes that are not there read as zero
+            const long long page_bytes = (long long)G * page * (dk + dv) * 2;
+            CUtensorMap km, vm;
+            BLM_REQUIRE(n_pages > 0 &&
+                            tc5::make_map_4d(&km, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.pool, {dk, page, G, n_pages},
+                                             {dk * 2LL, page * dk * 2LL, page_bytes}, {64, 16, G, 1}, CU_TENSOR_MAP_SWIZZLE_128B) &&
+                            tc5::make_map_4d(&vm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.pool + (size_t)G * page * dk, {dv, page, G, n_pages},
+                                             {dv * 2LL, page * dv * 2LL, page_bytes}, {64, 16, G, 1}, CU_TENSOR_MAP_SWIZZLE_128B),
+                        "attention_quads: no tensor map for %lld pages of %d heads of %d + %d lanes", n_pages, G, dk, dv);
+            BLM_REQUIRE(l.total <= 227 * 1024, "attention_quads: shared memory");
+            if (int rc = allow_smem(k, l.total)) return rc;
+            k<<<(unsigned)blocks, kRowWarps * 32, l.total, stream>>>(a, km, vm, status);
+        }
     }
     if (int rc = blm_check_launch("attention_quads")) return rc;
     if (ranges == 1) return BLM_OK;

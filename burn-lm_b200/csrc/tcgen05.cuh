@@ -52,6 +52,12 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, unsigned long long* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar))
+        : "memory");
+}
 // one lane of a converged warp
 __device__ __forceinline__ bool elect() {
     unsigned is;
@@ -150,15 +156,30 @@ static inline EncodeTiledFn encode_tiled() {
     }();
     return fn;
 }
-// A three-dimensional view (strides of the second and third dimension in bytes, multiples of 16); what lies outside reads as zero.
-static inline bool make_map_3d(CUtensorMap* out, CUtensorMapDataType type, const void* base, const long long (&dims)[3],
-                               const long long (&strides)[2], const int (&box)[3], CUtensorMapSwizzle swizzle) {
+// A view of R dimensions (strides of all but the first in bytes, multiples of 16); what lies outside reads as zero.
+template <int R>
+static inline bool make_map(CUtensorMap* out, CUtensorMapDataType type, const void* base, const long long (&dims)[R],
+                            const long long (&strides)[R - 1], const int (&box)[R], CUtensorMapSwizzle swizzle) {
     const EncodeTiledFn encode = encode_tiled();
     if (!encode) return false;
-    const cuuint64_t d[3] = {(cuuint64_t)dims[0], (cuuint64_t)dims[1], (cuuint64_t)dims[2]}, s[2] = {(cuuint64_t)strides[0], (cuuint64_t)strides[1]};
-    const cuuint32_t b[3] = {(cuuint32_t)box[0], (cuuint32_t)box[1], (cuuint32_t)box[2]}, e[3] = {1, 1, 1};
-    return encode(out, type, 3, const_cast<void*>(base), d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    cuuint64_t d[R], s[R - 1];
+    cuuint32_t b[R], e[R];
+    for (int i = 0; i < R; ++i) {
+        d[i] = (cuuint64_t)dims[i];
+        b[i] = (cuuint32_t)box[i];
+        e[i] = 1;
+        if (i) s[i - 1] = (cuuint64_t)strides[i - 1];
+    }
+    return encode(out, type, R, const_cast<void*>(base), d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+static inline bool make_map_3d(CUtensorMap* out, CUtensorMapDataType type, const void* base, const long long (&dims)[3],
+                               const long long (&strides)[2], const int (&box)[3], CUtensorMapSwizzle swizzle) {
+    return make_map<3>(out, type, base, dims, strides, box, swizzle);
+}
+static inline bool make_map_4d(CUtensorMap* out, CUtensorMapDataType type, const void* base, const long long (&dims)[4],
+                               const long long (&strides)[3], const int (&box)[4], CUtensorMapSwizzle swizzle) {
+    return make_map<4>(out, type, base, dims, strides, box, swizzle);
 }
 
 }  // namespace tc5

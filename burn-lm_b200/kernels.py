@@ -179,8 +179,10 @@ _protos = {
     },
     "attention_quads": {
         "blm_attention_quads_takes": [c_int, c_int, c_int, c_int, c_int],
+        "blm_attention_quads_rows": [c_int, c_int],
         "blm_attention_quads": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
+                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_int, c_float, c_float,
+                                c_void_p, c_void_p],
     },
     "attention_latent": {
         "blm_latent_prepare": [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_float, c_void_p, c_int, c_void_p, c_void_p,
@@ -1760,12 +1762,14 @@ def sigmoid_attention_ranges(step, n_heads, n_kv, key_dim, value_dim, dtype, dev
     sms = sm_count(device)
     if sigmoid_attention_in_registers(dtype, n_heads, n_kv, key_dim, value_dim):
         # single tokens: one round of blocks, which fill a multiprocessor each (64 sequences of 1,088 keys, the whole mixer: 1 / 2 /
-        # 3 / 4 ranges 78 / 60 / 78 / 72 us).  Portions: blocks are of unequal length, so enough of them that the last round
-        # weighs little (1,536 tokens: 1 / 2 / 4 / 5 / 6 ranges 346 / 247 / 241 / 234 / 247 us)
+        # 3 / 4 ranges 78 / 60 / 78 / 72 us).  Portions: blocks are of unequal length and start longest first, so twice as many as
+        # multiprocessors where they own sixteen rows (1,536 tokens, attention and merge of the ranges: 2 / 4 / 5 ranges
+        # 157 / 138 / 147 us); wider heads' blocks own eight rows, and six times as many
         if step.max_q_len == 1:
             return max(1, min(sms // step.n_seqs, step.max_kv_len // PAGE, 64))
-        tiles = step.n_seqs * -(-step.max_q_len // 8)
-        return max(1, min(-(-6 * sms // tiles), step.max_kv_len // 256, 8))
+        rows = _ask("attention_quads", "blm_attention_quads_rows", key_dim, value_dim)
+        tiles = step.n_seqs * -(-step.max_q_len // rows)
+        return max(1, min(-(-(2 if rows == 16 else 6) * sms // tiles), step.max_kv_len // 256, 8))
     tiles = step.n_seqs * ((step.max_q_len + 15) // 16)
     want = (4 if step.max_q_len == 1 else 2) * sms                  # single rows: small blocks, four an SM
     shortest = PAGE if step.max_q_len == 1 else 256                 # a single row's range may be one page
@@ -1777,8 +1781,8 @@ def sigmoid_attention(q, pool, block_table, step, out, n_heads, n_kv, key_dim, v
     """Causal attention whose weights are sigmoid(cap(scale q.k) + head_bias) without a normalisation over the keys, mixed
     across heads by talk [heads, heads] (row h: what head h takes of every head's weights) before they meet the values.
     q [N, heads * key_dim] and out [N, heads * value_dim] in the cache's dtype (out must hold zeros in rows of no
-    sequence); `ranges` > 1 cuts every query's keys over that many blocks whose partial outputs (`partial`, float32
-    with room for ranges * N * heads * value_dim) are added in order.  bfloat16 runs the tensor-core
+    sequence where `ranges` is 1); `ranges` > 1 cuts every query's keys over that many blocks whose partial outputs (`partial`,
+    float32 with room for ranges * N * heads * value_dim) are added in order, rows of no sequence to zero.  bfloat16 runs the tensor-core
     kernels where they take the shape (key lanes in multiples of 16, value lanes of 8; up to eight key/value heads of up to
     four query heads each: attention_quads.cu, others attention_sigmoid.cu); `scalar_only` keeps it off them."""
     _need_cuda(q, pool, block_table, out, talk, head_bias, partial)
@@ -1796,8 +1800,9 @@ def sigmoid_attention(q, pool, block_table, step, out, n_heads, n_kv, key_dim, v
             t is None or t.data_ptr() % 16 == 0 for t in (q, pool, out, partial)):
         _call("attention_quads", "blm_attention_quads", _ptr(q), _ptr(pool), _ptr(block_table), block_table.shape[1], _ptr(step.cu_seqlens),
               _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias), _ptr(out),
-              _ptr(partial if ranges > 1 else None), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE, int(ranges),
-              scale, softcap, _stream(), kernels=2 if ranges > 1 else 1)
+              _ptr(partial if ranges > 1 else None), n, step.n_seqs, step.max_q_len, n_heads, n_kv, key_dim, value_dim, PAGE,
+              pool.numel() // (n_kv * PAGE * (key_dim + value_dim)), int(ranges), scale, softcap, _ptr(status_word(pool.device)), _stream(),
+              kernels=2 if ranges > 1 else 1)
         return
     _call("attention_sigmoid", "blm_sigmoid_attention", _ptr(q), _ptr(pool), _code(pool.dtype), _ptr(block_table), block_table.shape[1],
           _ptr(step.cu_seqlens), _ptr(step.slot_of_seq), _ptr(step.start_pos), _ptr(step.token_seq), _ptr(talk), _ptr(head_bias),

@@ -96,9 +96,10 @@ class SigmoidAttention(Part):
         q = torch.empty((n, s.n_heads * s.head_dim), dtype=rt.dtype, device=proj.device)
         K.bias_rope_append(proj, self.bias, self.freq, s.rotary_dim, q, cache.pool, cache.block_table, step, s.n_heads,
                            s.n_kv_heads, s.head_dim, s.value_dim)
-        out = torch.zeros((n, s.n_heads * s.value_dim), dtype=rt.dtype, device=proj.device)   # rows of no sequence stay zero
         ranges = K.sigmoid_attention_ranges(step, s.n_heads, s.n_kv_heads, s.head_dim, s.value_dim, rt.dtype, rt.device)
         partial = None
+        # rows of no sequence are zeros: written by the merge of several ranges, by nothing where there is one
+        out = (torch.empty if ranges > 1 else torch.zeros)((n, s.n_heads * s.value_dim), dtype=rt.dtype, device=proj.device)
         if ranges > 1:
             partial = step.workspace.scratch("sigmoid_attention", ranges * n * s.n_heads * s.value_dim)
         K.sigmoid_attention(q, cache.pool, cache.block_table, step, out, s.n_heads, s.n_kv_heads, s.head_dim, s.value_dim, s.scale,
