@@ -97,3 +97,37 @@ def test_the_mix_keeps_every_bit_of_the_weights(H, G, dk, dv, lens):
                         H, G, dk, dv, 1.0, talk=talk)
     want = (talk.double().sum(1) * 0.5)[:, None].expand(H, dv).reshape(-1)     # every position sees the first one's value; the others' are zero
     assert ((out.double() - want).abs() <= 2.0 ** -7 * want.abs()).all()      # (bfloat16 rounds what is left, twice)
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(32, 8, 64, 64), (12, 3, 16, 24), (16, 4, 64, 8)])
+@pytest.mark.parametrize("lens,starts,ranges", [([15, 16, 17], [0, 0, 0], 1), ([2, 31, 33], [47, 48, 49], 1), ([5], [60], 1),       # four and five tiles
+                                                ([18, 1], [1006, 2030], 8), ([400, 0, 9], [113, 7, 1], 2)])
+def test_portions_at_the_edges_of_rings_and_blocks(H, G, dk, dv, lens, starts, ranges):
+    """Blocks of sixteen rows, a ring of four tiles of sixteen keys (passed several times), a last tile that is full, ragged or all the
+    sequence has, fewer lanes than a box of the copies."""
+    test_weights_mix_and_values(H, G, dk, dv, lens, starts, ranges)
+
+
+@pytest.mark.parametrize("most", [1, 20])
+def test_several_ranges_write_every_row(most):
+    """Where a query's keys are cut into ranges, rows of no sequence come out as zeros whatever lay there."""
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(most)
+    n, pages = most + 2, 12
+    step = SimpleNamespace(n_tokens=n, n_seqs=1, max_q_len=most, max_kv_len=pages * K.PAGE, cu_seqlens=i32([0, most]),
+                           token_seq=i32([0] * most + [-1] * 2), slot_of_seq=i32([0]), start_pos=i32([pages * K.PAGE - most]))
+    pool = torch.randn((pages, 8 * K.PAGE * 128), generator=gen, device="cuda").bfloat16()
+    q = torch.randn((n, 32 * 64), generator=gen, device="cuda").bfloat16()
+    table, outs = i32([list(range(pages))]), []
+    for ranges, fill in ((1, 0.0), (3, float("nan"))):
+        out = torch.full((n, 32 * 64), fill, dtype=torch.bfloat16, device="cuda")
+        partial = torch.full((ranges * n * 32 * 64,), float("nan"), device="cuda")
+        K.sigmoid_attention(q, pool, table, step, out, 32, 8, 64, 64, 0.125, ranges=ranges, partial=partial)
+        outs.append(out.float())
+    assert not outs[1][most:].any()
+    # sums of some 800 products of about one in another order (800 * 2^-20 is generous), each rounded once to the eight bits of a
+    # bfloat16 number: by up to 2^-8 of it, so that two differ by up to 2^-7 of the larger
+    room = 2.0 ** -7 * torch.maximum(outs[0].abs(), outs[1].abs()) + 800 * 2.0 ** -20
+    diff = (outs[0] - outs[1]).abs()
+    assert (diff <= room).all(), (diff - room).max()
