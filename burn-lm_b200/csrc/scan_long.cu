@@ -11,8 +11,10 @@
 //
 // Three launches.  (1) What does not depend on the state is formed for all chunks at once and left as the tensor cores read it: C,
 // B and the 64 x 64 matrices A, split into bfloat16 parts, in the 128-byte swizzle (29 us).  (2) Every group but a sequence's last is
-// run from an empty state: what it adds to the state (28).  (3) Every group folds the groups in front of it into its first state
-// and runs (59): a block owns a group and two neighbouring heads that share B and C, whose 2 x 64 columns are the lanes of
+// run from an empty state: what it adds to the state (28); the first one also copies the state that the sequence brings.  (3)
+// Every group folds the groups in front of it into that copy and runs (59); the last one writes the sequence's state.  The state
+// itself is not read in this launch, whose groups run in no order: for an even number of tokens it is what the last group writes (a
+// sequence of one group reads and writes its own).  A block owns a group and two neighbouring heads that share B and C, whose 2 x 64 columns are the lanes of
 // tensor memory.  S lives in registers (a lane a column, half of the rows a warp); its parts, the operand of the read-out, are
 // written to tensor memory, and so are x's.
 // A chunk takes 10,000 clocks, of which the 120 tcgen05.mma, issued one every 40, take 4,800; the rest are the hand-overs between them
@@ -34,7 +36,7 @@ constexpr int NR = 128, H = NR / 64;      // rows of the state as it lies, and r
 __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 // Sequences of `least` or more new tokens are run.  Chunk c of sequence s has the index cu[s] / 64 + s + c: distinct, and below
-// n_tokens / 64 + n_seqs.  Sums of group g of a sequence have the index 3 (cu[s] / least) + g, distinct too.
+// n_tokens / 64 + n_seqs.  Sums of group g of a sequence have the index 3 (cu[s] / least) + g, distinct too, its first state cu[s] / least.
 struct Chunks {
     const int* cu;
     int n_seqs, least;
@@ -69,22 +71,24 @@ struct RowsIn {                    // a column range of a float32 [N, *] tensor
 //   mats   [chunk][head][3][64 j][64 i]                                                bfloat16
 //   nums   [chunk][head][kNums]: 64 factors of the read-out, 64 of what a token writes, the chunk's decay
 //   sums   [group][head][column][NR], decays [group][head]
+//   firsts [sequence][head][column][NR]: the state in front of the sequence's first group
 constexpr int kNums = 132;
 struct Scratch {
     unsigned char *rows, *mats;
-    float *nums, *sums, *decays;
+    float *nums, *sums, *firsts, *decays;
 };
 struct Sizes {
-    long long rows, mats, nums, sums, decays;          // bytes
-    long long all() const { return rows + mats + nums + sums + decays; }
+    long long rows, mats, nums, sums, firsts, decays;  // bytes
+    long long all() const { return rows + mats + nums + sums + firsts + decays; }
 };
 static Sizes sizes_of(int units, int heads, int dv, long long chunks, long long sequences) {
     const long long groups = sequences * (kGroups - 1);
-    return {chunks * units * 6 * H * kTile, chunks * heads * 3 * kTile, chunks * heads * kNums * 4, groups * heads * dv * NR * 4, groups * heads * 4};
+    return {chunks * units * 6 * H * kTile, chunks * heads * 3 * kTile, chunks * heads * kNums * 4, groups * heads * dv * NR * 4,
+            sequences * heads * dv * NR * 4, groups * heads * 4};
 }
 static Scratch scratch_at(float* base, const Sizes& s) {
-    unsigned char* p = reinterpret_cast<unsigned char*>(base);
-    return {p, p + s.rows, (float*)(p + s.rows + s.mats), (float*)(p + s.rows + s.mats + s.nums), (float*)(p + s.rows + s.mats + s.nums + s.sums)};
+    unsigned char *mats = reinterpret_cast<unsigned char*>(base) + s.rows, *nums = mats + s.mats, *sums = nums + s.nums, *firsts = sums + s.sums;
+    return {mats - s.rows, mats, (float*)nums, (float*)sums, (float*)firsts, (float*)(firsts + s.firsts)};
 }
 
 // where row (8 a multiple of 4) `c` of token t lies in a tile of rows of 128 bytes
@@ -502,13 +506,28 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
             float S[kHalf];
 #pragma unroll
             for (int r = 0; r < kHalf; ++r) S[r] = 0.f;
+            const bool lone = size >= chunks;          // (the sequence is one group)
+            float* kept = a.s.firsts + (((size_t)(first / a.ch.least) * a.heads + hl) * a.dv + min(col, a.dv - 1)) * NR + half * kHalf;
+            if ((SUMS ? group == 0 : lone) && start > 0 && live) {
+                float* old = both + (size_t)(start & 1) * a.copy_stride;
+#pragma unroll
+                for (int r8 = 0; r8 < NR / 16; ++r8)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        if constexpr (SUMS) kept[r8 * 8 + e] = at(old, r8)[e];
+                        else S[r8 * 8 + e] = at(old, r8)[e];
+                    }
+            }
             if (!SUMS) {
-                if (start > 0 && live) {
-                    float* old = both + (size_t)(start & 1) * a.copy_stride;
+                if (!lone && start > 0 && live) {
 #pragma unroll
-                    for (int r8 = 0; r8 < NR / 16; ++r8)
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) S[r8 * 8 + e] = at(old, r8)[e];
+                    for (int r = 0; r < kHalf; r += 4) {
+                        const float4 s4 = *reinterpret_cast<const float4*>(kept + r);
+                        S[r] = s4.x;
+                        S[r + 1] = s4.y;
+                        S[r + 2] = s4.z;
+                        S[r + 3] = s4.w;
+                    }
                 }
                 for (int g = 0; g < group; ++g) {          // the groups in front
                     const size_t i = (size_t)(first / a.ch.least * (kGroups - 1) + g) * a.heads + hl;

@@ -61,6 +61,28 @@ def test_long_sequences_against_the_walk_in_float64(heads, groups, rows, dv, len
     assert K.check_status("cuda") is None
 
 
+def test_groups_in_any_order_read_the_state_the_sequence_brings(monkeypatch):
+    """An even number of tokens: the state is written where it was read.  With more blocks than the chip holds at a time the last
+    sequences' groups start one after another."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(6)
+    heads, groups, rows, dv, lens, starts = 64, 2, 128, 64, [512, 194, 512, 512, 514], [2, 4, 3, 6, 8]
+    step, n = step_of(lens, starts), sum(lens)
+    state = state_of(step, heads, rows, dv, 0, gen)
+    x, b0, dt, dt_bias, a_log, skip = args = inputs(heads, groups, rows, dv, n, gen)
+    step.scan_runs = (False, True)                                            # walked token by token; then as long sequences
+    walked, run = state.clone(), state.clone()
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", K._NO_LIMIT)
+    want = scan(*args, heads, groups, rows, dv, step, walked, 0)
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", 64)
+    step.scan_runs = K.scan_runs(lens)
+    route = K._long_route(heads, groups, rows, dv, step, "cuda")
+    assert route is not None and route[3] and K.sm_count("cuda") < heads // 2 * 4 * len(lens)
+    got = scan(*args, heads, groups, rows, dv, step, run, 0)
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()                # both within 1e-5 of 64 bits
+    assert (run - walked).abs().max() <= 2e-5 * walked.abs().max()
+
+
 def test_a_sequence_has_the_bits_it_has_alone():
     gen = torch.Generator(device="cuda")
     gen.manual_seed(3)
