@@ -1089,8 +1089,11 @@ def status_word(device) -> torch.Tensor:
     if w is None:
         dev = torch.device(device)
         if dev.index is None:
-            return status_word(torch.device(dev.type, torch.cuda.current_device()))
-        w = _status[dev] = torch.zeros(1, dtype=torch.int32, device=dev)
+            dev = torch.device(dev.type, torch.cuda.current_device())
+        # one word a device, however the device is spelled and whichever thread asks first: captured graphs hold its address
+        w = _status.get(dev)
+        if w is None:
+            w = _status.setdefault(dev, torch.zeros(1, dtype=torch.int32, device=dev))
     return w
 
 
