@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1)
     for (int t = w.lo; t < w.hi; ++t) {
         const int place = (t - w.lo) % kRowStages, ahead = page_of(t + kRowStages), j0 = t * 16;
         if (!tc5::mbar_wait(full + place, (t - w.lo) / kRowStages & 1)) {
-            if (status) *status = tc5::TC5_TIMEOUT;
+            if (status) *status = tc5::TC5_TIMEOUT_QUADS;
             return;
         }
         if (j0 + 16 > w.kv_hi) {                               // the sequence's last tile (no other follows): values of rows that

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
     auto wait = [&](unsigned long long* bar, unsigned phase) {
         if (ok && !mbar_wait(bar, phase)) {
             ok = false;
-            if (lane == 0) atomicCAS(a.status, TC5_OK, TC5_TIMEOUT);
+            if (lane == 0) atomicCAS(a.status, TC5_OK, TC5_TIMEOUT_PRODUCT);
         }
         return ok;
     };

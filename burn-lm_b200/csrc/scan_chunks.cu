@@ -905,7 +905,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_mma_kernel(const WalkArg
     }
     __syncthreads();
     auto there = [&](int chunk) {
-        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT);
+        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT_SCAN_CHUNKS);
         return sm + (chunk - lo) % kRing * kStage;
     };
     auto share = [&](int chunk, const float (&o)[2][4]) {      // a warp's share of the output: columns g, g + 8; tokens t2, + 1 (and 8 further)
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_delta_kernel(const WalkA
     }
     __syncthreads();
     auto there = [&](int chunk) {
-        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT);
+        if (!tc5::mbar_wait(full + (chunk - lo) % kRing, (chunk - lo) / kRing & 1) && lane == 0) atomicCAS(a.status, tc5::TC5_OK, tc5::TC5_TIMEOUT_SCAN_CHUNKS);
         return sm + (chunk - lo) % kRing * kStage;
     };
 

@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
     auto wait = [&](unsigned long long* bar, unsigned phase) {
         if (ok && !mbar_wait(bar, phase & 1)) {
             ok = false;
-            if (lane == 0) atomicCAS(a.status, TC5_OK, TC5_TIMEOUT);
+            if (lane == 0) atomicCAS(a.status, TC5_OK, TC5_TIMEOUT_SCAN_LONG);
         }
         return ok;
     };

@@ -12,7 +12,8 @@
 namespace tc5 {
 
 constexpr unsigned kSpinLimit = 1u << 18;
-enum { TC5_OK = 0, TC5_TIMEOUT = 15 };
+// what a kernel whose wait ran out leaves in the status word: a code for every file that includes this one
+enum { TC5_OK = 0, TC5_TIMEOUT_PRODUCT = 15, TC5_TIMEOUT_SCAN_CHUNKS = 16, TC5_TIMEOUT_SCAN_LONG = 17, TC5_TIMEOUT_QUADS = 18 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {

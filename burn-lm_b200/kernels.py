@@ -1097,23 +1097,28 @@ def status_word(device) -> torch.Tensor:
     return w
 
 
+_WAITS = {
+    1: "gemv: a consumer waited in vain for a weight stage", 2: "gemv: the producer waited in vain for a free stage",
+    11: "gemm_tc: the tensor-core thread waited in vain for a stage", 12: "gemm_tc: the producer waited in vain for a free stage",
+    13: "gemm_tc: the epilogue waited in vain for the accumulator", 14: "gemm_tc: a tile was not read in time",
+    15: "float32 product: a wait ran out", 16: "recurrence in chunks of sixteen tokens: a wait ran out",
+    17: "state-space scan in chunks of 64 tokens: a wait ran out", 18: "sigmoid attention of prompts: a wait ran out",
+    21: "decode attention: a consumer waited in vain for a page", 22: "decode attention: the producer waited in vain for a free stage",
+    31: "prompt attention: the query tile did not arrive", 32: "prompt attention: a key tile did not arrive",
+    33: "prompt attention: a value tile did not arrive", 34: "prompt attention: the scores did not arrive",
+    35: "prompt attention: the probabilities were not written", 36: "prompt attention: the product with the values did not arrive",
+    37: "prompt attention: the producer waited in vain for a free stage",
+    41: "gemm_sk: the tensor-core thread waited in vain for a stage", 42: "gemm_sk: the producer waited in vain for a free stage",
+    43: "gemm_sk: the epilogue waited in vain for the accumulator"}
+
+
 def check_status(device) -> None:
     """Raise if a kernel gave up a bounded wait since the last check (reads one word from the device)."""
     w = status_word(device)
     code = int(w.item())
     if code:
         w.zero_()
-        what = {21: "decode attention: a consumer waited in vain for a page", 22: "decode attention: the producer waited in vain for a free stage",
-                1: "gemv: a consumer waited in vain for a weight stage", 2: "gemv: the producer waited in vain for a free stage",
-                31: "prompt attention: the query tile did not arrive", 32: "prompt attention: a key tile did not arrive",
-                33: "prompt attention: a value tile did not arrive", 34: "prompt attention: the scores did not arrive",
-                35: "prompt attention: the probabilities were not written", 36: "prompt attention: the product with the values did not arrive",
-                37: "prompt attention: the producer waited in vain for a free stage",
-                15: "float32 product: a wait on an mbarrier ran out", 11: "gemm_tc: the tensor-core thread waited in vain for a stage", 12: "gemm_tc: the producer waited in vain for a free stage",
-                13: "gemm_tc: the epilogue waited in vain for the accumulator",
-                41: "gemm_sk: the tensor-core thread waited in vain for a stage", 42: "gemm_sk: the producer waited in vain for a free stage",
-                43: "gemm_sk: the epilogue waited in vain for the accumulator"}
-        raise KernelError(f"{what.get(code, 'status ' + str(code))}; the step's results are not valid")
+        raise KernelError(f"{_WAITS.get(code, 'status ' + str(code))}; the step's results are not valid")
 
 
 SQUARES_ROWS = 16     # row length of the sums of squares that go with a handed-over norm
