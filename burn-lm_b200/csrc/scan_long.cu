@@ -3,24 +3,27 @@
 // The chunks of sixteen tokens (scan_chunks.cu) are a chain of 128 links for a prompt of 2,048 tokens, each of which passes over
 // the state with fp32 multiply-adds: 230 us for 64 heads of 128 x 64, whose multiply-adds alone take 58.  Here a chunk has 64
 // tokens, its products run on the tensor cores with every float as three bfloat16 numbers (tcgen05.cuh: 24 bits, six products, sums
-// in float32), and a sequence is cut into four groups of chunks that run side by side: 124 us.  With P(i..j) the product of the
+// in float32), and a sequence (beyond 4,096 tokens each such segment of it, one after another) is cut into four groups of chunks that
+// run side by side: 124 us.  With P(i..j) the product of the
 // decays of the tokens i..j and S the state in front of a chunk:
 //     out_j  = P(0..j) S^T C_j + sum_(i <= j) A_ji x_i,     A_ji = (C_j . B_i) P(i+1..j) dt_i  (+ D on the diagonal)
 //     S'     = P(0..63) S + Z,     Z = sum_j (P(j+1..63) dt_j B_j) x_j^T
 // Every factor is a product of decays, never a quotient of two: nothing overflows however strong a decay is.
 //
 // Three launches.  (1) What does not depend on the state is formed for all chunks at once and left as the tensor cores read it: C,
-// B and the 64 x 64 matrices A, split into bfloat16 parts, in the 128-byte swizzle (29 us).  (2) Every group but a sequence's last is
-// run from an empty state: what it adds to the state (28); the first one also copies the state that the sequence brings.  (3)
+// B and the 64 x 64 matrices A, split into bfloat16 parts, in the 128-byte swizzle (29 us).  (2) Every group but a segment's last is
+// run from an empty state: what it adds to the state (28); the first one also copies the state that the segment starts from.  (3)
 // Every group folds the groups in front of it into that copy and runs (59); the last one writes the sequence's state.  The state
 // itself is not read in this launch, whose groups run in no order: for an even number of tokens it is what the last group writes (a
-// sequence of one group reads and writes its own).  A block owns a group and two neighbouring heads that share B and C, whose 2 x 64 columns are the lanes of
+// segment of one group reads and writes its own).  A block owns a group and two neighbouring heads that share B and C, whose 2 x 64 columns are the lanes of
 // tensor memory.  S lives in registers (a lane a column, half of the rows a warp); its parts, the operand of the read-out, are
 // written to tensor memory, and so are x's.
 // A chunk takes 10,000 clocks, of which the 120 tcgen05.mma, issued one every 40, take 4,800; the rest are the hand-overs between them
 // (x's parts, the reading of A x, of Z and of the output).  That is no faster a chain than sixteen tokens at a time, so only
 // long sequences of enough heads gain (kernels.py has the border and both sides' times), and decays per row, whose 64 x 64
 // matrices and decayed rows are each head's own (119 us to form them for 32 heads of 128 x 128), do not at all.
+#include <algorithm>
+
 #include "tcgen05.cuh"
 
 BLM_API const char* blm_scan_long_last_error() { return g_blm_error; }
@@ -28,30 +31,60 @@ BLM_API const char* blm_scan_long_last_error() { return g_blm_error; }
 using namespace tc5;
 
 constexpr int kT = 64;            // tokens of a chunk
-constexpr int kGroups = 4;        // groups of a sequence: its chunks in even parts
+constexpr int kSegment = 64;      // chunks of a segment: a sequence is run segment by segment
+constexpr int kGroups = 4;        // groups of a segment: its chunks in even parts
 constexpr int kTile = kT * 128;   // bytes of 64 rows of 64 bfloat16 numbers
 
 constexpr int NR = 128, H = NR / 64;      // rows of the state as it lies, and rows of 128 bytes that its parts take
 
 __device__ __forceinline__ float softplus_r(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
-// Sequences of `least` or more new tokens are run.  Chunk c of sequence s has the index cu[s] / 64 + s + c: distinct, and below
-// n_tokens / 64 + n_seqs.  Sums of group g of a sequence have the index 3 (cu[s] / least) + g, distinct too, its first state cu[s] / least.
+// Sequences of `least` or more new tokens are run, in segments of kSegment chunks one after another: what a pass needs of scratch
+// does not grow with a sequence, and where a segment begins depends on its own sequence alone, so a sequence has the bits it has alone.
+// Chunk c of sequence s has the index cu[s] / 64 + s + c: distinct, and below n_tokens / 64 + n_seqs (a step of one sequence: c).  A pass runs
+// the segments whose first chunk has an index from `from` up to from + count; their chunks have indexes below from + count + a
+// segment's chunks - 1.  Each has a slot of its own for its groups' sums: sequences begin `gap` indexes apart at least, so every `gap`
+// indexes hold the beginning of one at most; where sequences have several segments a pass counts no more than kSegment indexes,
+// which hold one at most that is not its sequence's first (slot 0; `later`: there may be both).
 struct Chunks {
     const int* cu;
     int n_seqs, least;
+    int from, count, gap, later;
 };
 static long long chunk_bound(int n_tokens, int n_seqs) { return (long long)n_tokens / kT + n_seqs; }
-__device__ __forceinline__ int chunk_base(int cu, int seq) { return cu / kT + seq; }
+__device__ __forceinline__ int chunk_base(const Chunks& ch, int seq) { return ch.n_seqs > 1 ? ch.cu[seq] / kT + seq : 0; }
 
+// The sequence and chunk of the pass's chunk `idx`; false: there is none.  All threads of the block call it.
 __device__ __forceinline__ bool find_chunk(int idx, const Chunks& ch, int* found, int& seq, int& chunk) {
+    idx += ch.from;
     if (threadIdx.x == 0) found[0] = -1;
     __syncthreads();
     for (int s = threadIdx.x; s < ch.n_seqs; s += blockDim.x) {
-        const int lo = ch.cu[s], n = ch.cu[s + 1] - lo, base = chunk_base(lo, s);
-        if (n >= ch.least && idx >= base && idx < base + (n + kT - 1) / kT) {
+        const int n = ch.cu[s + 1] - ch.cu[s], c = idx - chunk_base(ch, s);
+        if (n < ch.least || c < 0 || c >= (n + kT - 1) / kT) continue;
+        const int begin = idx - c % kSegment;
+        if (begin >= ch.from && begin < ch.from + ch.count) {
             found[0] = s;
-            found[1] = idx - base;
+            found[1] = c;
+        }
+    }
+    __syncthreads();
+    seq = found[0];
+    chunk = found[1];
+    return seq >= 0;
+}
+
+// The sequence and the first chunk of the pass's segment in a slot; false: there is none.  All threads of the block call it.
+__device__ __forceinline__ bool find_segment(int slot, const Chunks& ch, int* found, int& seq, int& chunk) {
+    if (threadIdx.x == 0) found[0] = -1;
+    __syncthreads();
+    for (int s = threadIdx.x; s < ch.n_seqs; s += blockDim.x) {
+        const int n = ch.cu[s + 1] - ch.cu[s], ahead = max(0, ch.from - chunk_base(ch, s));
+        if (n < ch.least) continue;
+        const int c = (ahead + kSegment - 1) / kSegment * kSegment, at = chunk_base(ch, s) + c - ch.from;
+        if (c < (n + kT - 1) / kT && at < ch.count && slot == (c > 0 ? 0 : ch.later + at / ch.gap)) {
+            found[0] = s;
+            found[1] = c;
         }
     }
     __syncthreads();
@@ -70,8 +103,8 @@ struct RowsIn {                    // a column range of a float32 [N, *] tensor
 //   rows   [chunk][unit][C, B][3 parts][NR / 64][64 tokens][64 rows of the state]      bfloat16
 //   mats   [chunk][head][3][64 j][64 i]                                                bfloat16
 //   nums   [chunk][head][kNums]: 64 factors of the read-out, 64 of what a token writes, the chunk's decay
-//   sums   [group][head][column][NR], decays [group][head]
-//   firsts [sequence][head][column][NR]: the state in front of the sequence's first group
+//   sums   [slot][kGroups - 1][head][column][NR], decays [slot][kGroups - 1][head]
+//   firsts [slot][head][column][NR]: the state in front of the segment
 constexpr int kNums = 132;
 struct Scratch {
     unsigned char *rows, *mats;
@@ -81,10 +114,10 @@ struct Sizes {
     long long rows, mats, nums, sums, firsts, decays;  // bytes
     long long all() const { return rows + mats + nums + sums + firsts + decays; }
 };
-static Sizes sizes_of(int units, int heads, int dv, long long chunks, long long sequences) {
-    const long long groups = sequences * (kGroups - 1);
+static Sizes sizes_of(int units, int heads, int dv, long long chunks, long long slots) {
+    const long long groups = slots * (kGroups - 1);
     return {chunks * units * 6 * H * kTile, chunks * heads * 3 * kTile, chunks * heads * kNums * 4, groups * heads * dv * NR * 4,
-            sequences * heads * dv * NR * 4, groups * heads * 4};
+            slots * heads * dv * NR * 4, groups * heads * 4};
 }
 static Scratch scratch_at(float* base, const Sizes& s) {
     unsigned char *mats = reinterpret_cast<unsigned char*>(base) + s.rows, *nums = mats + s.mats, *sums = nums + s.nums, *firsts = sums + s.sums;
@@ -333,13 +366,16 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                        *d_read = bars + 11, *raw_full = bars + 12;
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 13);
     int* odd = reinterpret_cast<int*>(tmem_slot + 2);                       // [2][4]: a warp of columns has values that are not finite in the chunk
+    int* found = odd + 8;                      // (not beside them: shared memory then begins where addresses are known at compile time)
 
-    const int h = blockIdx.x * 2, seq = blockIdx.y / kGroups, group = blockIdx.y % kGroups;
-    const int first = a.ch.cu[seq], n_new = a.ch.cu[seq + 1] - first;
-    if (n_new < a.ch.least) return;
-    const int chunks = (n_new + kT - 1) / kT, size = (chunks + kGroups - 1) / kGroups, lo = group * size;
-    if (lo >= chunks || (SUMS && lo + size >= chunks)) return;
-    const int n = min(size, chunks - lo), base = chunk_base(first, seq) + lo;
+    const int h = blockIdx.x * 2, slot = blockIdx.y / kGroups, group = blockIdx.y % kGroups;
+    int seq, begin;                            // the segment's sequence, and its first chunk
+    if (!find_segment(slot, a.ch, found, seq, begin)) return;
+    const int n_new = a.ch.cu[seq + 1] - a.ch.cu[seq];
+    const int length = min(kSegment, (n_new + kT - 1) / kT - begin), size = (length + kGroups - 1) / kGroups, lo = group * size;      // of the segment
+    if (lo >= length || (SUMS && lo + size >= length)) return;
+    const int n = min(size, length - lo), base = chunk_base(a.ch, seq) - a.ch.from + begin + lo;
+    const int first = a.ch.cu[seq] + (begin + lo) * kT, rest = n_new - (begin + lo) * kT;      // the group's first token, and how many the sequence has from there on
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         mbar_init(a_full, 1);
@@ -396,7 +432,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
         const int in4 = (lane & 15) * 4, at4 = (lane >> 4) * a.dv + in4;
         auto bring_x = [&](int c) {
             float* to = xs + c % kXSlots * kT * 128;
-            const int t0 = first + (lo + c) * kT, nt = min(kT, n_new - (lo + c) * kT);
+            const int t0 = first + c * kT, nt = min(kT, rest - c * kT);
             if (vec) {
                 const float* src = v + (size_t)t0 * a.v.stride + at4;
 #pragma unroll 4
@@ -499,38 +535,30 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
         const unsigned lanes = (unsigned)(quarter * 32) << 16;
         {
             const bool live = col < a.dv;
+            // the half's first eight rows of the column as the state lies, [head][row / 8][column][row % 8]; where the sequence leaves it
             const int start = a.start_pos[seq];
-            // as it lies: [head][row / 8][column][row % 8]
-            float* both = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off + (size_t)(a.head0 + hl) * NR * a.dv;
-            auto at = [&](float* s, int r8) { return s + ((size_t)(half * (NR / 16) + r8) * a.dv + col) * 8; };
+            float* fresh = a.state + (size_t)a.slot_of_seq[seq] * a.slot_stride + a.state_off +
+                           (((size_t)(a.head0 + hl) * (NR / 8) + half * (NR / 16)) * a.dv + col) * 8 + (size_t)((start + n_new) & 1) * a.copy_stride;
+            const bool lone = size >= length, some = live && (start > 0 || begin > 0);      // (the segment is one group; there is a state)
+            // what the segment starts from: the sequence's state, behind another segment what that wrote, and its copy
+            const float* old = fresh + (begin > 0 ? 0 : (start & 1) - ((start + n_new) & 1)) * a.copy_stride;
+            float* kept = a.s.firsts + (((size_t)slot * a.heads + hl) * a.dv + min(col, a.dv - 1)) * NR + half * kHalf;
+            if (SUMS && group == 0 && some) {
+#pragma unroll
+                for (int r = 0; r < kHalf; ++r) kept[r] = old[r / 8 * 8 * a.dv + r % 8];
+            }
             float S[kHalf];
 #pragma unroll
             for (int r = 0; r < kHalf; ++r) S[r] = 0.f;
-            const bool lone = size >= chunks;          // (the sequence is one group)
-            float* kept = a.s.firsts + (((size_t)(first / a.ch.least) * a.heads + hl) * a.dv + min(col, a.dv - 1)) * NR + half * kHalf;
-            if ((SUMS ? group == 0 : lone) && start > 0 && live) {
-                float* old = both + (size_t)(start & 1) * a.copy_stride;
-#pragma unroll
-                for (int r8 = 0; r8 < NR / 16; ++r8)
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        if constexpr (SUMS) kept[r8 * 8 + e] = at(old, r8)[e];
-                        else S[r8 * 8 + e] = at(old, r8)[e];
-                    }
-            }
             if (!SUMS) {
-                if (!lone && start > 0 && live) {
+                if (some) {
+                    const float* from = lone ? old : kept;
+                    const int by = lone ? 8 * a.dv : 8;
 #pragma unroll
-                    for (int r = 0; r < kHalf; r += 4) {
-                        const float4 s4 = *reinterpret_cast<const float4*>(kept + r);
-                        S[r] = s4.x;
-                        S[r + 1] = s4.y;
-                        S[r + 2] = s4.z;
-                        S[r + 3] = s4.w;
-                    }
+                    for (int r = 0; r < kHalf; ++r) S[r] = from[r / 8 * by + r % 8];
                 }
                 for (int g = 0; g < group; ++g) {          // the groups in front
-                    const size_t i = (size_t)(first / a.ch.least * (kGroups - 1) + g) * a.heads + hl;
+                    const size_t i = (size_t)(slot * (kGroups - 1) + g) * a.heads + hl;
                     const float* sum = a.s.sums + (i * a.dv + min(col, a.dv - 1)) * NR + half * kHalf;
                     const float d = a.s.decays[i];
 #pragma unroll
@@ -604,19 +632,16 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                 }
             }
             if (ok && SUMS) {
-                const size_t i = (size_t)(first / a.ch.least * (kGroups - 1) + group) * a.heads + hl;
+                const size_t i = (size_t)(slot * (kGroups - 1) + group) * a.heads + hl;
                 if (live) {
                     float* sum = a.s.sums + (i * a.dv + col) * NR + half * kHalf;
 #pragma unroll
                     for (int r = 0; r < kHalf; r += 4) *reinterpret_cast<float4*>(sum + r) = make_float4(S[r], S[r + 1], S[r + 2], S[r + 3]);
                 }
                 if ((quarter & 1) == 0 && half == 0 && lane == 0) a.s.decays[i] = all;
-            } else if (ok && lo + n == chunks && live) {
-                float* fresh = both + (size_t)((start + n_new) & 1) * a.copy_stride;
+            } else if (ok && lo + n == length && live) {
 #pragma unroll
-                for (int r8 = 0; r8 < NR / 16; ++r8)
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) at(fresh, r8)[e] = S[r8 * 8 + e];
+                for (int r = 0; r < kHalf; ++r) fresh[r / 8 * 8 * a.dv + r % 8] = S[r];
             }
         }
     } else {
@@ -646,7 +671,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                     if (c + 1 < n) begin(c + 1);
                     continue;
                 }
-                const int t0 = first + (lo + c) * kT, nt = min(kT, n_new - (lo + c) * kT);
+                const int t0 = first + c * kT, nt = min(kT, rest - c * kT);
                 const float* nums = nums_of(c);
                 const float* x = xs + c % kXSlots * kT * 128 + v0;
                 const bool odd_here = some;
@@ -713,57 +738,89 @@ static int allow_smem(K kernel, int smem) {
     return e == cudaSuccess ? BLM_OK : blm_fail(BLM_CUDA_ERROR, "scan_long: %s", cudaGetErrorString(e));
 }
 
-// Heads at a time, in whole groups of those that share B and C, so that a pass's scratch stays within kMost bytes (256 MB: some 8,000
-// tokens of 64 heads); heads know nothing of one another, so the passes change no bit.
+// How a step is run: passes over the chunks' indexes (Chunks) and over the heads, in whole groups of those that share B and C, so that a
+// pass's scratch stays within kMost bytes.  Heads know nothing of one another and segments are their sequences' own: passes change no bit.
+// With 64 heads of 128 x 64 and one group a segment of 4,096 tokens is 118 MB.  Passes over heads alone, each over the whole prompt, held fewer blocks
+// than the chip and were slower than chunks of sixteen: 64 heads in 8 groups, 16,384 tokens 2,124 us, by segments 895, by chunks of sixteen
+// 1,144; 32,768 tokens 7,773, 1,811 and 2,268.
 constexpr long long kMost = 256ll << 20;
-static int heads_at_once(int heads, int unit, int dv, long long chunks, long long sequences) {
-    int at_once = heads;
-    while (at_once > unit && sizes_of(at_once / unit, at_once, dv, chunks, sequences).all() > kMost) at_once = (at_once / unit + 1) / 2 * unit;
-    return at_once;
+struct Passes {
+    int heads, count, gap, later, slots;
+    long long all, chunks;         // indexes of the step, chunks of a pass
+    Sizes sizes;
+    int number(int of_heads) const { return (int)((all + count - 1) / count) * ((of_heads + heads - 1) / heads); }
+};
+static bool passes_of(Passes& p, int heads, int unit, int dv, int n_tokens, int n_seqs, int longest, int least) {
+    p.all = n_seqs > 1 ? chunk_bound(n_tokens, n_seqs) : (n_tokens + kT - 1) / kT;
+    const int longest_chunks = (std::min(longest, n_tokens) + kT - 1) / kT, segment = std::min(kSegment, longest_chunks);
+    const bool several = longest_chunks > kSegment;    // sequences of several segments
+    p.gap = n_seqs > 1 ? std::min(kSegment, std::max(1, least / kT)) : kSegment;
+    p.later = several && n_seqs > 1;
+    const long long limit = several ? std::min<long long>(p.all, kSegment) : p.all;
+    auto with = [&](long long count) {
+        p.count = (int)count;
+        p.slots = (int)((count + p.gap - 1) / p.gap) + p.later;
+        p.chunks = n_seqs > 1 ? std::min(p.all, count + segment - 1) : count;
+        p.sizes = sizes_of(p.heads / unit, p.heads, dv, p.chunks, p.slots);
+        return p.sizes.all() <= kMost && p.heads / unit <= 65535 && p.slots * kGroups <= 65535;
+    };
+    for (p.heads = heads;; p.heads = (p.heads / unit + 1) / 2 * unit) {
+        if (with(limit)) return true;
+        // as many indexes as fit, in even parts, unless they are few beside the chunks that reach beyond them
+        const double chunk = (double)sizes_of(p.heads / unit, p.heads, dv, 1, 0).all(), slot = (double)sizes_of(p.heads / unit, p.heads, dv, 0, 1).all();
+        const long long most = (long long)((kMost - chunk * (segment - 1) - slot * (1 + p.later)) / (chunk + slot / p.gap));
+        if (n_seqs > 1 && most >= (segment + 1) / 2) {
+            const long long parts = (limit + most - 1) / most;
+            if (with((limit + parts - 1) / parts)) return true;
+        }
+        if (p.heads <= unit) return false;
+    }
 }
 
-// Bytes of scratch; 0: these kernels do not take the size (states of 65 to 128 rows x 33 to 64 columns, an even number of heads that share
-// B and C: `unit`).  And how many kernels are launched.
-BLM_API long long blm_scan_long_scratch(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int least) {
-    if (rows <= NR / 2 || rows > NR || dv <= 32 || dv > 64 || unit < 2 || unit % 2 || heads % unit || n_seqs < 1 || n_seqs * kGroups > 65535 || least < 1) return 0;
-    const long long chunks = chunk_bound(n_tokens, n_seqs), sequences = n_tokens / least + 1;
-    const int n = heads_at_once(heads, unit, dv, chunks, sequences);
-    return n / unit > 65535 ? 0 : sizes_of(n / unit, n, dv, chunks, sequences).all();
+// Bytes of scratch; 0: these kernels do not take the step (states of 65 to 128 rows x 33 to 64 columns, an even number of heads that share
+// B and C: `unit`; `longest`: no sequence brings more tokens).  And how many kernels are launched.
+BLM_API long long blm_scan_long_scratch(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int longest, int least) {
+    if (rows <= NR / 2 || rows > NR || dv <= 32 || dv > 64 || unit < 2 || unit % 2 || heads % unit || n_seqs < 1 || n_tokens < 1 || longest < 1 || least < 1)
+        return 0;
+    Passes p;
+    return passes_of(p, heads, unit, dv, n_tokens, n_seqs, longest, least) ? p.sizes.all() : 0;
 }
-BLM_API int blm_scan_long_launches(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int least) {
-    return ((heads - 1) / heads_at_once(heads, unit, dv, chunk_bound(n_tokens, n_seqs), n_tokens / least + 1) + 1) * 3;
+BLM_API int blm_scan_long_launches(int heads, int unit, int rows, int dv, int n_tokens, int n_seqs, int longest, int least) {
+    Passes p;
+    return passes_of(p, heads, unit, dv, n_tokens, n_seqs, longest, least) ? 3 * p.number(heads) : 0;
 }
 
 BLM_API int blm_scan_chunks_long_ssm(const float* xbc, long long xbc_stride, int x_col0, int b_col0, int c_col0, const float* dt_raw,
                                      long long dt_stride, int dt_col0, const float* dt_bias, const float* A_log, const float* D, float* y,
                                      long long y_stride, int heads, int groups, int N, int dv, const int* cu_seqlens,
-                                     const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int least, float* state,
+                                     const int* slot_of_seq, const int* start_pos, int n_tokens, int n_seqs, int longest, int least, float* state,
                                      long long slot_stride, long long copy_stride, long long state_off, float* scratch, int* status,
                                      cudaStream_t stream) {
     if (n_seqs == 0 || n_tokens == 0) return BLM_OK;
     BLM_REQUIRE(groups > 0 && heads % groups == 0, "scan_long: bad head counts");
     const int per = heads / groups;
-    BLM_REQUIRE(blm_scan_long_scratch(heads, per, N, dv, n_tokens, n_seqs, least) > 0 && status, "scan_long: %d rows, %d columns", N, dv);
-    const long long chunks = chunk_bound(n_tokens, n_seqs), sequences = n_tokens / least + 1;
-    const int at_once = heads_at_once(heads, per, dv, chunks, sequences);
-    const Chunks ch = {cu_seqlens, n_seqs, least};
-    for (int head0 = 0; head0 < heads; head0 += at_once) {
-        const int now = heads - head0 < at_once ? heads - head0 : at_once;
-        const Scratch s = scratch_at(scratch, sizes_of(now / per, now, dv, chunks, sequences));
-        const SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
-                               head0 / per, now / per, s};
-        int rc = allow_smem(long_prep_kernel, kPrepSmem);
-        if (rc) return rc;
-        long_prep_kernel<<<dim3((unsigned)chunks, now / per), kPrepThreads, kPrepSmem, stream>>>(p);
-        if ((rc = blm_check_launch("scan_long (chunks)"))) return rc;
-        const RunArgs a = {{xbc, xbc_stride, x_col0}, s, ch, slot_of_seq, start_pos, now / per, per, head0, now, dv, y, y_stride, state, slot_stride, copy_stride, state_off, status};
-        const dim3 grid(now / 2, n_seqs * kGroups);
-        if ((rc = allow_smem(long_run_kernel<true>, kRunSmem))) return rc;
-        long_run_kernel<true><<<grid, kRunThreads, kRunSmem, stream>>>(a);
-        if ((rc = blm_check_launch("scan_long (sums)"))) return rc;
-        if ((rc = allow_smem(long_run_kernel<false>, kRunSmem))) return rc;
-        long_run_kernel<false><<<grid, kRunThreads, kRunSmem, stream>>>(a);
-        if ((rc = blm_check_launch("scan_long (run)"))) return rc;
-    }
+    BLM_REQUIRE(blm_scan_long_scratch(heads, per, N, dv, n_tokens, n_seqs, longest, least) > 0 && status, "scan_long: %d rows, %d columns", N, dv);
+    Passes pass;
+    passes_of(pass, heads, per, dv, n_tokens, n_seqs, longest, least);
+    if (int rc = allow_smem(long_prep_kernel, kPrepSmem)) return rc;
+    if (int rc = allow_smem(long_run_kernel<true>, kRunSmem)) return rc;
+    if (int rc = allow_smem(long_run_kernel<false>, kRunSmem)) return rc;
+    for (int head0 = 0; head0 < heads; head0 += pass.heads)
+        for (long long from = 0; from < pass.all; from += pass.count) {
+            const Chunks ch = {cu_seqlens, n_seqs, least, (int)from, pass.count, pass.gap, pass.later};
+            const int now = std::min(heads - head0, pass.heads);
+            const Scratch s = scratch_at(scratch, sizes_of(now / per, now, dv, pass.chunks, pass.slots));
+            const SsmPrepArgs p = {{xbc, xbc_stride, x_col0}, {dt_raw, dt_stride, dt_col0}, b_col0, c_col0, dt_bias, A_log, D, ch, heads, groups, N,
+                                   head0 / per, now / per, s};
+            int rc;
+            long_prep_kernel<<<dim3((unsigned)std::min(pass.chunks, pass.all - from), now / per), kPrepThreads, kPrepSmem, stream>>>(p);
+            if ((rc = blm_check_launch("scan_long (chunks)"))) return rc;
+            const RunArgs a = {{xbc, xbc_stride, x_col0}, s, ch, slot_of_seq, start_pos, now / per, per, head0, now, dv, y, y_stride, state, slot_stride, copy_stride, state_off, status};
+            const dim3 grid(now / 2, pass.slots * kGroups);
+            long_run_kernel<true><<<grid, kRunThreads, kRunSmem, stream>>>(a);
+            if ((rc = blm_check_launch("scan_long (sums)"))) return rc;
+            long_run_kernel<false><<<grid, kRunThreads, kRunSmem, stream>>>(a);
+            if ((rc = blm_check_launch("scan_long (run)"))) return rc;
+        }
     return BLM_OK;
 }

@@ -154,10 +154,10 @@ _protos = {
                                  c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
     },
     "scan_long": {
-        "blm_scan_long_scratch": [c_int] * 7,
-        "blm_scan_long_launches": [c_int] * 7,
+        "blm_scan_long_scratch": [c_int] * 8,
+        "blm_scan_long_launches": [c_int] * 8,
         "blm_scan_chunks_long_ssm": [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                     c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                      c_void_p, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
     },
     "retention": {
@@ -1462,12 +1462,12 @@ SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1536, 2048
 
 def _long_route(heads, groups, n_state, value_dim, step, device):
     """How a step's long sequences run: (scratch of scan_long.cu, how many of its kernels are launched, the length from which they run
-    a sequence, whether every sequence is as long), or None where they run none."""
+    a sequence, whether every sequence is as long), or None where they run none: also where the scratch would be more than 256 MB."""
     longest, runs = min(getattr(step, "max_q_len", 0), step.n_tokens), getattr(step, "scan_runs", None)
     if longest < SCAN_LONG_TOKENS or (runs is not None and len(runs) > 2 and not runs[2]):
         return None
     least = SCAN_LONG_TOKENS if heads * -(-value_dim // 16) > sm_count(device) else SCAN_LONG_TOKENS_FEW_HEADS
-    sizes = (heads, heads // groups, n_state, value_dim, step.n_tokens, step.n_seqs, least)
+    sizes = (heads, heads // groups, n_state, value_dim, step.n_tokens, step.n_seqs, longest, least)
     floats = -(-_ask("scan_long", "blm_scan_long_scratch", *sizes) // 4) if longest >= least else 0
     if floats == 0:
         return None
@@ -1494,7 +1494,7 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
     if long is not None:
         _call("scan_long", "blm_scan_chunks_long_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, long[2], *_state_args(state, state_offset),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, min(step.max_q_len, step.n_tokens), long[2], *_state_args(state, state_offset),
               _ptr(long[0]), _ptr(status_word(y.device)), _stream(), kernels=long[1])
         if long[3]:
             return

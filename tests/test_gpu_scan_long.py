@@ -122,6 +122,44 @@ def test_scratch_is_bounded_and_heads_in_passes_change_no_bit(monkeypatch):
     assert torch.equal(state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(own.shape), own)
 
 
+LARGEST = 256 << 20                                                           # bytes of scratch
+
+
+@pytest.mark.parametrize("heads,groups", [(64, 1), (64, 4), (64, 8), (64, 32), (128, 8), (24, 1), (8, 4)])
+@pytest.mark.parametrize("n_seqs,longest", [(1, 2048), (1, 16384), (1, 131072), (4, 2048), (3, 20000), (200, 2000), (20, 65536)])
+def test_scratch_does_not_grow_with_the_tokens(heads, groups, n_seqs, longest):
+    least, n = 1536, n_seqs * longest
+    used = K._ask("scan_long", "blm_scan_long_scratch", heads, heads // groups, 128, 64, n, n_seqs, longest, least)
+    launches = K._ask("scan_long", "blm_scan_long_launches", heads, heads // groups, 128, 64, n, n_seqs, longest, least)
+    assert 0 < used <= LARGEST and launches % 3 == 0 and 0 < launches <= 3 * (2 if heads == 128 or groups == 32 else 1) * (-(-n // 2048) + n_seqs + 1)
+
+
+@pytest.mark.parametrize("lens,starts", [([4096], [2]), ([4097], [1]), ([8256], [4]), ([9000, 70, 2, 4160, 4096, 100], [2, 0, 3, 6, 1, 8])])
+def test_segments_against_the_walk(lens, starts, monkeypatch):
+    """Sequences of several segments, whose edges fall between those of others, in passes of their own."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(sum(lens))
+    heads, groups, rows, dv = 4, 1, 128, 64
+    step, n = step_of(lens, starts), sum(lens)
+    state = state_of(step, heads, rows, dv, 0, gen)
+    x, b0, dt, dt_bias, a_log, skip = args = inputs(heads, groups, rows, dv, n, gen)
+    step.scan_runs = K.scan_runs(lens)
+    assert K._long_route(heads, groups, rows, dv, step, "cuda")[1] >= (3 if n <= 4096 else 6)
+    run, own, walked = state.clone(), state.clone(), state.clone()
+    got, at = scan(*args, heads, groups, rows, dv, step, run, 0), 0
+    for s, m in enumerate(lens):                                              # the bits it has alone
+        alone = step_of([m], [starts[s]])
+        alone.slot_of_seq, alone.scan_runs = step.slot_of_seq[s:s + 1], K.scan_runs([m])
+        assert torch.equal(got[at:at + m], scan(x[at:at + m], b0, dt[at:at + m], dt_bias, a_log, skip, heads, groups, rows, dv, alone, own, 0)), s
+        at += m
+    assert torch.equal(run, own)
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", K._NO_LIMIT)
+    step.scan_runs = (False, True)
+    want = scan(*args, heads, groups, rows, dv, step, walked, 0)
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()                # both within 1e-5 of 64 bits
+    assert (run - walked).abs().max() <= 2e-5 * walked.abs().max()
+
+
 @pytest.mark.parametrize("where", ["value", "key", "dt"])
 def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(where):
     gen = torch.Generator(device="cuda")
