@@ -166,7 +166,7 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
 // finite is formed again with fmaf from the floats themselves.  Operands below 2^-109 lose their last bits (x3 would be below
 // the smallest bfloat16 number).
 // With 16,384 x 2,048 / 2,048 x 8,192 weights, us (FFMA above): 1 row 40 / 30, 16 rows 40 / 30, 64 rows 44 / 32, 160 rows 62 / 44, 317 rows
-// 110 / 69, 2,000 rows 603 / 390 (3,000 / 1,513); the error against 64 bits 1.5e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
+// 110 / 69, 2,000 rows 603 / 390 (3,000 / 1,513); the error against 64 bits 1.2e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
 // of which the tensor core works 1,920: x's parts have room for two steps only.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTcLeast = 64;

@@ -2,7 +2,7 @@
 // instructions and descriptors, and the split of a float into three bfloat16 numbers.
 //
 // A float has 24 bits of mantissa, a bfloat16 number 8 and the same exponents, so x = x1 + x2 + x3 exactly (x1 = x's first bits,
-// x2 = the next, x3 = what is left).  x w is then nine products that the tensor cores form exactly; the six with i + j <= 4 are
+// x2 = what is left rounded, x3 = the rest).  x w is then nine products that the tensor cores form exactly; the six with i + j <= 4 are
 // summed (in float32, the smallest first), the other three are below 2^-21 of the product and 2^-24 on average.
 #pragma once
 #include <cuda.h>
@@ -133,15 +133,17 @@ __device__ __forceinline__ void tmem_free(unsigned base, int cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(base), "r"(cols));
 }
 
-// Two floats as three pairs of bfloat16 numbers (the first float in the lower half): x1 and x2 are cut off, not rounded, which
-// leaves x3 exact all the same.
+// Two floats as three pairs of bfloat16 numbers (the first float in the lower half).  x1 is cut off, so that no finite float becomes an
+// infinity; x2 is rounded, so that the products left out are of either sign (both cut off they all had the product's own: errors of
+// recurrences and products 1.1 to 1.7 times as large); x3 is exact.  As many instructions as with both cut off.
 __device__ __forceinline__ void split3(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
     p1 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
     a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
     b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-    p2 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-    a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
-    b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+    p2 = *reinterpret_cast<const unsigned*>(&m);
+    a -= __uint_as_float(p2 << 16);
+    b -= __uint_as_float(p2 & 0xffff0000u);
     p3 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
