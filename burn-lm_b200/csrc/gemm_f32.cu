@@ -2,7 +2,7 @@
 // This is the matrix product of the 32-bit path.  The sum over K runs in one fixed order that depends on neither N nor M, so a
 // token's result is the same whatever else is in the batch: K is cut into shares, each is summed in order, and the shares' sums are
 // added in order.  Two kernels: on the tensor cores (further down) where K and W's rows come in 16-byte pieces, and FFMA for
-// everything else.
+// small weights and everything else.
 //
 // FFMA: what bounds it is fp32 multiply-adds from some 50 rows on (74 TFLOP/s on this chip at best), the weights' way in below.  Both
 // operands lie along K and stay so in shared memory (rows padded by a 16-byte piece, so that eight rows start in eight different
@@ -83,11 +83,12 @@ __global__ void __launch_bounds__(TN * TM) gemm_f32_kernel(const GemmArgs a) {
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    float acc[AN][AM];
+    // rows in 16-byte pieces: a slice is summed by itself and then added (one chain of 256 places: 2.9e-7 off, so 1.2e-7)
+    float acc[AN][AM], sum[AN][AM];
 #pragma unroll
     for (int i = 0; i < AN; ++i)
 #pragma unroll
-        for (int j = 0; j < AM; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < AM; ++j) acc[i][j] = sum[i][j] = 0.f;
     for (int s = 0; s < kSlices - 1; ++s) load(s);
     for (int slice = 0; slice < slices; ++slice) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kSlices - 2) : "memory");
@@ -110,6 +111,15 @@ __global__ void __launch_bounds__(TN * TM) gemm_f32_kernel(const GemmArgs a) {
 #pragma unroll
                     for (int j = 0; j < AM; ++j)
                         acc[i][j] = fmaf((&xv[i].x)[e], (&wv[j].x)[e], acc[i][j]);
+            if (VEC && k == kBK - 4) {
+#pragma unroll
+                for (int i = 0; i < AN; ++i)
+#pragma unroll
+                    for (int j = 0; j < AM; ++j) {
+                        sum[i][j] += acc[i][j];
+                        acc[i][j] = 0.f;
+                    }
+            }
         }
     }
     float* y = a.shares > 1 ? a.y + ((size_t)share * a.batch + b) * a.N * a.M : a.y + (size_t)b * a.by;
@@ -119,7 +129,7 @@ __global__ void __launch_bounds__(TN * TM) gemm_f32_kernel(const GemmArgs a) {
 #pragma unroll
         for (int j = 0; j < AM; ++j) {
             const int n = n0 + tn + TN * i, m = m0 + tm + TM * j;
-            if (n < a.N && m < a.M) y[(size_t)n * ldy + m] = acc[i][j];
+            if (n < a.N && m < a.M) y[(size_t)n * ldy + m] = VEC ? sum[i][j] : acc[i][j];
         }
 }
 
@@ -150,8 +160,8 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
 }
 
 // ---------------------------------------------------------------------------------------------
-// The product on the tensor cores, for K a multiple of 4 from kTcLeast on and rows of W at multiples of 16 bytes: a choice by K and
-// W's layout alone, so that a row's bits depend on neither N nor M.
+// The product on the tensor cores, for K a multiple of 4 from kTcLeast on and rows of W at multiples of 16 bytes, unless the weight is
+// small: a choice by the weight alone, so that a row's bits do not depend on what else is in the batch.
 //
 // Both operands as three bfloat16 numbers a float (tcgen05.cuh): 24 bits and six products, 282 TFLOP/s of the chip's 1,692 against
 // 74 of FFMA.  x is split once by a launch of its own (it is read by every tile of W's rows); W, which is read once or a few times,
@@ -170,6 +180,11 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
 // of which the tensor core works 1,920: x's parts have room for two steps only.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTcLeast = 64;
+// Floats of W and K up to which FFMA is the faster one: a launch less, no tensor memory to take, tiles of 16 x 32.  us, FFMA and so, 17 / 317 / 2,000 rows:
+// 64 x 64 2.4 / 2.4 / 3.0 and 6.3 / 6.4 / 6.8; 512 x 64 2.3 / 3.1 / 5.9 and 6.5 / 6.7 / 7.8; 128 x 256 4.9 / 4.9 / 8.1 and 7.9 / 8.0 / 8.4; 64 x 512
+// 8.2 / 8.2 / 9.4 and 9.8 / 9.8 / 11.  Twice as many: 1,024 x 64 2.2 / 3.8 / 11 and 6.5 / 7.0 / 9.0; 256 x 256 4.7 / 5.3 / 11 and 7.9 / 8.0 / 9.0.
+// (Large batches of such products are the exception: 64 of 128 x 256, 2,000 rows 207 and 136.)  From 1,024 places on FFMA gains nothing.
+constexpr int kTcWeight = 1 << 15, kTcSmall = 512;
 constexpr int kTcShare = 1024;    // places of K of a share at most
 constexpr int kTcK = 32;          // of a slice; two slices are a step
 constexpr int kTcRows = 128;      // rows of W of a tile
@@ -466,24 +481,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
     }
 }
 
-// x's rows as three bfloat16 numbers a float: planes [batch][3][N][pitch]
+// x's rows as three bfloat16 numbers a float: planes [batch][3][N][pitch].  A thread four places of K of a row: a block holds many
+// short rows or a part of a long one (a block a row: 64 products of 2,000 rows of 64 places 168 us, of which the products take 30).
 template <bool VEC>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, int N, int K, int pitch,
                                                          long long ldx, long long bx) {
     pdl_launch_dependents();
-    const int n = blockIdx.x, b = blockIdx.z;
+    const unsigned pieces = K / 4;
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = e / pieces;
+    if (n >= N) return;
+    const int c = (int)(e - n * pieces) * 4, b = blockIdx.y;
     const float* row = x + (size_t)b * bx + (size_t)n * ldx;
-    __nv_bfloat16* to = out + ((size_t)b * 3 * N + n) * pitch;
+    __nv_bfloat16* to = out + ((size_t)b * 3 * N + n) * pitch + c;
     const size_t plane = (size_t)N * pitch;
-    for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4; c < K; c += gridDim.y * blockDim.x * 4) {
-        const float4 v = VEC ? *reinterpret_cast<const float4*>(row + c) : make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
-        uint2 p1, p2, p3;
-        tc5::split3(v.x, v.y, p1.x, p2.x, p3.x);
-        tc5::split3(v.z, v.w, p1.y, p2.y, p3.y);
-        *reinterpret_cast<uint2*>(to + c) = p1;
-        *reinterpret_cast<uint2*>(to + plane + c) = p2;
-        *reinterpret_cast<uint2*>(to + 2 * plane + c) = p3;
-    }
+    const float4 v = VEC ? *reinterpret_cast<const float4*>(row + c) : make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
+    uint2 p1, p2, p3;
+    tc5::split3(v.x, v.y, p1.x, p2.x, p3.x);
+    tc5::split3(v.z, v.w, p1.y, p2.y, p3.y);
+    *reinterpret_cast<uint2*>(to) = p1;
+    *reinterpret_cast<uint2*>(to + plane) = p2;
+    *reinterpret_cast<uint2*>(to + 2 * plane) = p3;
 }
 
 template <int TN, int TM, int AN, int AM>
@@ -525,9 +542,10 @@ static Plan tc_plan(int batch, int N, int M, int K, int sms) {
     return best;
 }
 
-// The tensor cores take it: by K and how W lies, never by N or M.
-static bool tc_takes(const float* w, int K, long long ldw, long long bw) {
-    return K >= kTcLeast && K % 4 == 0 && ((size_t)w & 15) == 0 && ldw > 0 && ldw % 4 == 0 && ldw < (1ll << 37) && bw >= 0 && bw % 4 == 0 &&
+// The tensor cores take it: by W's size and how it lies, never by N.
+static bool tc_size(int M, int K) { return K >= kTcLeast && K % 4 == 0 && (K > kTcSmall || (long long)M * K > kTcWeight); }
+static bool tc_takes(const float* w, int M, int K, long long ldw, long long bw) {
+    return tc_size(M, K) && ((size_t)w & 15) == 0 && ldw > 0 && ldw % 4 == 0 && ldw < (1ll << 37) && bw >= 0 && bw % 4 == 0 &&
            bw < (1ll << 37) && tc5::encode_tiled() != nullptr;
 }
 
@@ -557,7 +575,7 @@ static int launch_tc(const GemmArgs& g, const Plan& plan, float* scratch, int* s
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem + 1024);
     if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "gemm_f32: %s", cudaGetErrorString(e));
     const bool vec = ((size_t)g.x & 15) == 0 && g.ldx % 4 == 0 && g.bx % 4 == 0;
-    const dim3 grid(g.N, std::min(8, (g.K + 1023) / 1024), g.batch);
+    const dim3 grid((unsigned)(((long long)g.N * (g.K / 4) + 255) / 256), g.batch);
     if (vec) split_rows_kernel<true><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
     else split_rows_kernel<false><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
     if (int rc = blm_check_launch("gemm_f32 (parts)")) return rc;
@@ -619,10 +637,10 @@ static long long scratch_of(bool tc, int batch, int N, int M, int K) {
 BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
     if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
     const long long ffma = scratch_of(false, batch, N, M, K);
-    return K >= kTcLeast && K % 4 == 0 ? std::max(ffma, scratch_of(true, batch, N, M, K)) : ffma;
+    return tc_size(M, K) ? std::max(ffma, scratch_of(true, batch, N, M, K)) : ffma;
 }
 // whether the tensor cores form it, and how many kernels it launches.
-BLM_API int blm_gemm_f32_tensor(const float* w, int K, long long ldw, long long bw) { return tc_takes(w, K, ldw, bw); }
+BLM_API int blm_gemm_f32_tensor(const float* w, int M, int K, long long ldw, long long bw) { return tc_takes(w, M, K, ldw, bw); }
 BLM_API int blm_gemm_f32_launches(int tensor, int batch, int N, int M, int K) {
     if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
     const Pass p = pass_of(tensor, batch, N, M, K);
@@ -634,7 +652,7 @@ BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int b
                                  long long ldy, long long bx, long long bw, long long by, float* scratch, int* status, cudaStream_t stream) {
     if (N == 0 || M == 0 || batch == 0) return BLM_OK;
     BLM_REQUIRE(N > 0 && M > 0 && K > 0 && batch > 0, "gemm_f32: bad sizes %d x %d %d %d", batch, N, M, K);
-    const bool tc = tc_takes(w, K, ldw, batch > 1 ? bw : 0);
+    const bool tc = tc_takes(w, M, K, ldw, batch > 1 ? bw : 0);
     const int shares = shares_of(tc, K);
     BLM_REQUIRE(batch <= 65535 && shares <= 65535 && N <= 64 * 65535, "gemm_f32: too many rows or products (%d x %d)", batch, N);
     BLM_REQUIRE((shares == 1 && !tc) || (scratch != nullptr && status != nullptr), "gemm_f32: a sum over %d places needs scratch and a status word", K);
@@ -652,9 +670,11 @@ BLM_API int blm_gemm_f32_batched(const float* x, const float* w, float* y, int b
                 const GemmArgs a = {x + (size_t)b0 * bx + (size_t)n0 * ldx, w + (size_t)b0 * bw + (size_t)m0 * ldw, planes ? sums : to,
                                     rows, cols, K, shares, products, ldx, ldw, ldy, bx, bw, by};
                 // few rows: what takes the time is the weights' way in, which wants many small blocks (16 rows of 16,384 x 2,048 weights
-                // 49 us, with tiles of 32 rows 73); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
+                // 49 us, with tiles of 32 rows 73); so do small weights, a block's slices following one another (317 rows of 256 x 256
+                // 5.5 us, with tiles of 64 rows 10.5); then the smallest tile that holds the rows (48 rows: 101 us, in tiles of 64 rows 121)
+                const bool few = rows <= 16 || (vec && (long long)((rows + 15) / 16) * ((cols + 31) / 32) * products * shares <= 4 * blm_sm_count());
                 const int rc = tc           ? launch_tc(a, {tc_plan(products, rows, cols, K, blm_sm_count()).nt, planes}, scratch, status, stream)
-                               : rows <= 16 ? launch<4, 16, 4, 2>(a, vec, stream)
+                               : few        ? launch<4, 16, 4, 2>(a, vec, stream)
                                : rows <= 32 ? launch<8, 16, 4, 4>(a, vec, stream)
                                : rows <= 48 ? launch<8, 16, 6, 4>(a, vec, stream)
                                             : launch<8, 16, 8, 4>(a, vec, stream);

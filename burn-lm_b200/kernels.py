@@ -222,7 +222,7 @@ _protos = {
         "blm_gemm_f32_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                  c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
         "blm_gemm_f32_scratch": [c_int, c_int, c_int, c_int],
-        "blm_gemm_f32_tensor": [c_void_p, c_int, c_longlong, c_longlong],
+        "blm_gemm_f32_tensor": [c_void_p, c_int, c_int, c_longlong, c_longlong],
         "blm_gemm_f32_launches": [c_int, c_int, c_int, c_int, c_int],
     },
     "gemv": {
@@ -903,9 +903,9 @@ def _gemm_f32_scratch(batch, n, m, k, device, w=None):
     lib = _lib("gemm")
     floats = int(lib.blm_gemm_f32_scratch(batch, n, m, k))
     if w is None:
-        tensor = lib.blm_gemm_f32_tensor(None, k, 4, 0)
+        tensor = lib.blm_gemm_f32_tensor(None, m, k, 4, 0)
     else:
-        tensor = lib.blm_gemm_f32_tensor(_ptr(w), k, w.stride(-2), w.stride(0) if w.dim() == 3 and batch > 1 else 0)
+        tensor = lib.blm_gemm_f32_tensor(_ptr(w), m, k, w.stride(-2), w.stride(0) if w.dim() == 3 and batch > 1 else 0)
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, int(lib.blm_gemm_f32_launches(tensor, batch, n, m, k))
 
 

@@ -48,3 +48,19 @@ def test_what_is_not_finite():
     y, want = K.gemm_f32(x, w), (x[:, None] * w[None]).sum(-1)
     assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
     assert torch.equal(y[y.isinf()], want[want.isinf()])
+
+
+@pytest.mark.parametrize("m,k,tensor", [(512, 64, 0), (513, 64, 1), (64, 512, 0), (65, 512, 1), (1, 516, 1), (64, 64, 0), (200, 160, 0), (200, 66, 0)])
+def test_small_weights_take_one_launch(m, k, tensor):
+    """A weight's size says which kernel forms its products, and a row has the bits it has alone, on either side of the border."""
+    x, w = _operands(1700, m, k, m + k)
+    assert K._ask("gemm", "blm_gemm_f32_tensor", w.data_ptr(), m, k, k, 0) == tensor
+    scratch, launches = K._gemm_f32_scratch(1, 1700, m, k, "cuda", w)
+    assert launches == 1 + tensor and (scratch is None) == (not tensor)
+    y, want = K.gemm_f32(x, w), x.double() @ w.double().T
+    # FFMA: roundings of partial sums that grow with the square root of their length, 32 places at a time where rows come in 16-byte pieces;
+    # the tensor cores: four additions a step of 64 places
+    chain = k if k % 4 else 32
+    assert (y.double() - want).norm() / want.norm() <= (1.5e-7 if tensor else (chain / 2 + k / chain / 2) ** 0.5 * 2.0 ** -24 / 3 ** 0.5)
+    for n in (1, 16, 17, 40, 130, 700):                      # tiles of every size
+        assert torch.equal(K.gemm_f32(x[:n].contiguous(), w), y[:n]), n
