@@ -633,14 +633,16 @@ static long long scratch_of(bool tc, int batch, int N, int M, int K) {
     return (planes_of(tc, p, K) ? (long long)shares_of(tc, K) * p.products * p.rows * p.cols : 0) + (tc ? tc_parts(p.products, p.rows, K) : 0);
 }
 
-// Floats of scratch a product needs, however W lies (planes of sums, x's parts);
-BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
-    if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
-    const long long ffma = scratch_of(false, batch, N, M, K);
-    return tc_size(M, K) ? std::max(ffma, scratch_of(true, batch, N, M, K)) : ffma;
-}
-// whether the tensor cores form it, and how many kernels it launches.
+// Whether the tensor cores form a product (`w`, its strides: what the product itself is given),
 BLM_API int blm_gemm_f32_tensor(const float* w, int M, int K, long long ldw, long long bw) { return tc_takes(w, M, K, ldw, bw); }
+// floats of scratch that it then needs (planes of sums, x's parts), or however W lies, and how many kernels it launches.
+BLM_API long long blm_gemm_f32_scratch_as(int tensor, int batch, int N, int M, int K) {
+    return batch <= 0 || N <= 0 || M <= 0 || K <= 0 ? 0 : scratch_of(tensor, batch, N, M, K);
+}
+BLM_API long long blm_gemm_f32_scratch(int batch, int N, int M, int K) {
+    const long long ffma = blm_gemm_f32_scratch_as(0, batch, N, M, K);
+    return tc_size(M, K) ? std::max(ffma, blm_gemm_f32_scratch_as(1, batch, N, M, K)) : ffma;
+}
 BLM_API int blm_gemm_f32_launches(int tensor, int batch, int N, int M, int K) {
     if (batch <= 0 || N <= 0 || M <= 0 || K <= 0) return 0;
     const Pass p = pass_of(tensor, batch, N, M, K);

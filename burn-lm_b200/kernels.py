@@ -222,6 +222,7 @@ _protos = {
         "blm_gemm_f32_batched": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                                  c_longlong, c_longlong, c_longlong, c_void_p, c_void_p, c_void_p],
         "blm_gemm_f32_scratch": [c_int, c_int, c_int, c_int],
+        "blm_gemm_f32_scratch_as": [c_int, c_int, c_int, c_int, c_int],
         "blm_gemm_f32_tensor": [c_void_p, c_int, c_int, c_longlong, c_longlong],
         "blm_gemm_f32_launches": [c_int, c_int, c_int, c_int, c_int],
     },
@@ -261,7 +262,7 @@ _protos = {
 _bound: dict[str, ctypes.CDLL] = {}
 
 
-_LONG_RESULTS = ("blm_scan_chunks_scratch", "blm_scan_long_scratch", "blm_gemm_f32_scratch")     # entry points that return a number of floats instead of a status
+_LONG_RESULTS = ("blm_scan_chunks_scratch", "blm_scan_long_scratch", "blm_gemm_f32_scratch", "blm_gemm_f32_scratch_as")     # entry points that return a number of floats instead of a status
 
 
 def _lib(module: str) -> ctypes.CDLL:
@@ -890,23 +891,20 @@ def gemm_f32(x, w, out=None):
         out = torch.empty((n, m), dtype=torch.float32, device=x.device)
     elif tuple(out.shape) != (n, m) or out.dtype != torch.float32:
         raise KernelError("gemm_f32: out must be float32 [N, M]")
-    scratch, launches = _gemm_f32_scratch(1, n, m, k, x.device, w)
+    scratch, launches = _gemm_f32_scratch(1, n, m, k, x.device, w, k)
     _call("gemm", "blm_gemm_f32", _ptr(x), _ptr(w), _ptr(out), n, m, k, k, k, m, _ptr(scratch), _ptr(status_word(x.device)), _stream(),
           kernels=launches)
     return out
 
 
-def _gemm_f32_scratch(batch, n, m, k, device, w=None):
+def _gemm_f32_scratch(batch, n, m, k, device, w=None, ldw=4, bw=0):
     """(scratch of a float32 product, None where it needs none: a plane of sums for every share of K that it cuts its sums into, and x
     in three bfloat16 numbers a float where the tensor cores form it; the kernels it launches: products that would need more than
-    256 MB run in several passes).  `w` [M, K] or [B, M, K]: the weights; without them, rows at multiples of 16 bytes."""
-    lib = _lib("gemm")
-    floats = int(lib.blm_gemm_f32_scratch(batch, n, m, k))
-    if w is None:
-        tensor = lib.blm_gemm_f32_tensor(None, m, k, 4, 0)
-    else:
-        tensor = lib.blm_gemm_f32_tensor(_ptr(w), m, k, w.stride(-2), w.stride(0) if w.dim() == 3 and batch > 1 else 0)
-    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, int(lib.blm_gemm_f32_launches(tensor, batch, n, m, k))
+    256 MB run in several passes).  `w`, `ldw`, `bw`: the weights and their strides as the product is given them, which say how it is
+    formed; without them, rows at multiples of 16 bytes."""
+    tensor = _ask("gemm", "blm_gemm_f32_tensor", _ptr(w), m, k, ldw, bw if batch > 1 else 0)
+    floats = _ask("gemm", "blm_gemm_f32_scratch_as", tensor, batch, n, m, k)
+    return torch.empty(floats, dtype=torch.float32, device=device) if floats else None, _ask("gemm", "blm_gemm_f32_launches", tensor, batch, n, m, k)
 
 
 def batched_product(x, w, out=None, out_dtype=None):
@@ -927,7 +925,7 @@ def batched_product(x, w, out=None, out_dtype=None):
             out = torch.empty((b, n, m), dtype=torch.float32, device=x.device)
         if out.dtype != torch.float32 or tuple(out.shape) != (b, n, m) or any(t.stride(2) != 1 for t in (x, w, out)):
             raise KernelError("batched_product: float32 out [B, N, M]; unit stride along the last axis")
-        scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device, w)
+        scratch, launches = _gemm_f32_scratch(b, n, m, k, x.device, w, w.stride(1), w.stride(0))
         _call("gemm", "blm_gemm_f32_batched", _ptr(x), _ptr(w), _ptr(out), b, n, m, k, x.stride(1), w.stride(1),
               out.stride(1), x.stride(0), w.stride(0), out.stride(0), _ptr(scratch),
               _ptr(status_word(x.device)), _stream(), kernels=launches)
@@ -1445,10 +1443,10 @@ def _scan_route(kind, heads, rows, step, device, groups=1):
     in_chunks, walked = (getattr(step, "scan_runs", None) or ())[:2] or (longest >= SCAN_CHUNK_RUN, step.n_tokens < SCAN_CHUNK_MEAN * step.n_seqs)
     if in_chunks and min(longest, step.n_tokens) >= SCAN_CHUNK_TOKENS:
         least = SCAN_CHUNK_TOKENS if walked else 1                  # without the walk the chunk kernels run whatever there is
-        lib, sizes = _lib("scan_chunks"), (kind, heads, groups, rows, step.n_tokens, step.n_seqs, least)
-        floats = int(lib.blm_scan_chunks_scratch(*sizes))
+        sizes = (kind, heads, groups, rows, step.n_tokens, step.n_seqs, least)
+        floats = _ask("scan_chunks", "blm_scan_chunks_scratch", *sizes)
         if floats:
-            return (torch.empty(floats, dtype=torch.float32, device=device), int(lib.blm_scan_chunks_launches(*sizes)), least,
+            return (torch.empty(floats, dtype=torch.float32, device=device), _ask("scan_chunks", "blm_scan_chunks_launches", *sizes), least,
                     SCAN_CHUNK_TOKENS if walked else 0)
     return None, 0, 0, _NO_LIMIT
 

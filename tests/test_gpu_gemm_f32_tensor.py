@@ -55,7 +55,7 @@ def test_small_weights_take_one_launch(m, k, tensor):
     """A weight's size says which kernel forms its products, and a row has the bits it has alone, on either side of the border."""
     x, w = _operands(1700, m, k, m + k)
     assert K._ask("gemm", "blm_gemm_f32_tensor", w.data_ptr(), m, k, k, 0) == tensor
-    scratch, launches = K._gemm_f32_scratch(1, 1700, m, k, "cuda", w)
+    scratch, launches = K._gemm_f32_scratch(1, 1700, m, k, "cuda", w, k)
     assert launches == 1 + tensor and (scratch is None) == (not tensor)
     y, want = K.gemm_f32(x, w), x.double() @ w.double().T
     # FFMA: roundings of partial sums that grow with the square root of their length, 32 places at a time where rows come in 16-byte pieces;
@@ -64,3 +64,14 @@ def test_small_weights_take_one_launch(m, k, tensor):
     assert (y.double() - want).norm() / want.norm() <= (1.5e-7 if tensor else (chain / 2 + k / chain / 2) ** 0.5 * 2.0 ** -24 / 3 ** 0.5)
     for n in (1, 16, 17, 40, 130, 700):                      # tiles of every size
         assert torch.equal(K.gemm_f32(x[:n].contiguous(), w), y[:n]), n
+
+
+def test_scratch_is_that_of_the_kernel_that_runs():
+    parts = 600 * 2048 * 3 // 2                              # x in three bfloat16 numbers a float
+    w = torch.empty((16384, 2052), device="cuda")
+    assert K._gemm_f32_scratch(1, 600, 16384, 2048, "cuda", w, 2052)[0].numel() == parts
+    assert K._gemm_f32_scratch(1, 600, 16384, 2048, "cuda", w.view(-1)[1:], 2052)[0].numel() == 2 * 600 * 16384      # FFMA's planes
+    # one row of a wider matrix says it is contiguous, whatever its stride
+    x, wide = _operands(5, 1, 2048, 8)[0], torch.randn((3, 2049), device="cuda")
+    w = wide[1:2, 3:2051 - 2].as_strided((1, 2048), (2049, 1), 2052)
+    assert w.is_contiguous() and (K.gemm_f32(x, w).double() - x.double() @ w.double().T).abs().max() <= 1e-3
