@@ -1490,9 +1490,11 @@ def ssm_scan(xbc, x_col0, b_col0, c_col0, dt, dt_col0, dt_bias, a_log, d_skip, y
         raise KernelError("ssm_scan: y float32 [N, heads * value_dim]")
     long = None if wide_sums else _long_route(heads, groups, n_state, value_dim, step, y.device)
     if long is not None:
+        # alone in a step that does not know its lengths, a sequence is run whatever its length is (n_tokens may count rows of no sequence)
+        least = 1 if long[3] and step.n_seqs == 1 else long[2]
         _call("scan_long", "blm_scan_chunks_long_ssm", xp, xs, xc, int(b_col0), int(c_col0), dp, ds, dc, _ptr(dt_bias), _ptr(a_log),
               _ptr(d_skip), _ptr(y), y.stride(0), heads, groups, n_state, value_dim, _ptr(step.cu_seqlens), _ptr(step.slot_of_seq),
-              _ptr(step.start_pos), step.n_tokens, step.n_seqs, min(step.max_q_len, step.n_tokens), long[2], *_state_args(state, state_offset),
+              _ptr(step.start_pos), step.n_tokens, step.n_seqs, min(step.max_q_len, step.n_tokens), least, *_state_args(state, state_offset),
               _ptr(long[0]), _ptr(status_word(y.device)), _stream(), kernels=long[1])
         if long[3]:
             return

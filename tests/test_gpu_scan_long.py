@@ -122,6 +122,24 @@ def test_scratch_is_bounded_and_heads_in_passes_change_no_bit(monkeypatch):
     assert torch.equal(state.view(state.shape[0], 2, heads, -1)[:, :, :few].reshape(own.shape), own)
 
 
+@pytest.mark.parametrize("m", [1, 63, 64, 130, 700])
+def test_a_lone_sequence_among_rows_of_none(m):
+    """A step that knows no lengths but the bounds of a captured size: its one sequence is run however short it is."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m)
+    heads, groups, rows, dv, n = 4, 2, 128, 64, 4500
+    step, real = step_of([m], [3]), step_of([m], [3])
+    step.n_tokens = step.max_q_len = n
+    state = state_of(step, heads, rows, dv, 0, gen)
+    x, b0, dt, dt_bias, a_log, skip = args = inputs(heads, groups, rows, dv, n, gen)
+    assert K._long_route(heads, groups, rows, dv, step, "cuda")[3]
+    own, walked, real.scan_runs = state.clone(), state.clone(), (False, True)
+    out = scan(*args, heads, groups, rows, dv, step, own, 0)
+    want = scan(x[:m], b0, dt[:m], dt_bias, a_log, skip, heads, groups, rows, dv, real, walked, 0)
+    assert not out[m:].any()
+    assert (out[:m] - want).abs().max() <= 2e-5 * want.abs().max() and (own - walked).abs().max() <= 2e-5 * walked.abs().max()
+
+
 LARGEST = 256 << 20                                                           # bytes of scratch
 
 
