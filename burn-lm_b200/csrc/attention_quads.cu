@@ -454,6 +454,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1)
         const int place = (t - w.lo) % kRowStages, ahead = page_of(t + kRowStages), j0 = t * 16;
         if (!tc5::mbar_wait(full + place, (t - w.lo) / kRowStages & 1)) {
             if (status) *status = tc5::TC5_TIMEOUT_QUADS;
+            for (int u = t; u < min(w.hi, t + kRowStages); ++u)        // (no copy is on its way when the block ends)
+                tc5::mbar_wait(full + (u - w.lo) % kRowStages, (u - w.lo) / kRowStages & 1);
             return;
         }
         if (j0 + 16 > w.kv_hi) {                               // the sequence's last tile (no other follows): values of rows that

@@ -334,12 +334,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
                 r.next(stages);
             }
         }
+        // no copy is on its way when the block ends, not even where a wait ran out
+        for (int s = 0; s < (free ? r.at : stages); ++s) mbar_wait(full + s, s < r.at ? r.phase : r.phase ^ 1);
     } else if (warp < 3) {
         // ---------------- the tensor core: a warp the even steps, one the odd ones (one warp for all: 64 rows of x 128 us instead of 114) ----------------
         const int b = warp - 1;
         const unsigned idesc = instruction(a.nt), d = tmem_base + (unsigned)(b * a.nt);
         const unsigned long long x_desc = operand(x_ring, 2, 1024);
-        RingAt r;
+        RingAt r, last;                        // (last: where the last products went, if any)
+        last.at = -1;
         unsigned turn = 0;
         for (long long t = first_unit; t < units && ok; t = next_unit(t)) {
             const int steps = unit_at(t).steps;
@@ -363,8 +366,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
                     commit(done + r.at);
                 }
                 __syncwarp();
+                last = r;
             }
         }
+        if (last.at >= 0) mbar_wait(done + last.at, last.phase);       // nor are products
     } else if (warp < 3 + kConverters) {
         // ---------------- W's floats into parts: a lane a row; four warps both slices of a step, or eight one each ----------------
         const int row = (warp & 3) * 32 + lane, only = (warp - 3) >> 2;

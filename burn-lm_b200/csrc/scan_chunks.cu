@@ -1025,6 +1025,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_mma_kernel(const WalkArg
             bring(chunk + kRing - 1);
         }
         __syncthreads();
+        for (int chunk = max(lo, hi - kRing); chunk < hi; ++chunk) there(chunk);       // (no copy is on its way when the block ends, not even where a wait ran out)
         return;
     }
 
@@ -1191,6 +1192,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_delta_kernel(const WalkA
             bring(chunk + kRing - 1);
             __syncthreads();
         }
+        for (int chunk = max(lo, hi - kRing); chunk < hi; ++chunk) there(chunk);       // (no copy is on its way when the block ends, not even where a wait ran out)
         return;
     }
 

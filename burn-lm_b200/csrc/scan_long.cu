@@ -461,25 +461,35 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(raw_full + c % kXSlots)) : "memory");
         };
         bring_x(0);
+        int as = 0, ks = 0, qs = 0;            // copies asked for
         for (int c = 0; c < n && ok; ++c) {
             const unsigned char* rows = a.s.rows + ((size_t)(base + c) * a.units + h / a.per_unit) * 6 * H * kTile;
             if (!SUMS) {
                 if (c > 0 && !wait(intra_done, c - 1)) break;
                 copy(a_img, a.s.mats + ((size_t)(base + c) * a.heads + h) * 3 * kTile, 6 * kTile, a_full);
+                ++as;
             }
             if (c > 0 && !wait(upd_done, c - 1)) break;
             copy(k_img, rows + rows_bytes, rows_bytes, k_full);
+            ++ks;
             if (c > 0 && !wait(d_read, c - 1)) break;      // (the state may ask for the values of chunk c - 1)
             if (c + 1 < n) bring_x(c + 1);
             if (!SUMS) {
                 if (c > 0 && !wait(out_done, c - 1)) break;
                 copy(q_img, rows, rows_bytes, q_full);
+                ++qs;
             }
         }
+        // no copy is on its way when the block ends, not even where a wait ran out
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (as > 0) mbar_wait(a_full, (as - 1) & 1);
+        if (ks > 0) mbar_wait(k_full, (ks - 1) & 1);
+        if (qs > 0) mbar_wait(q_full, (qs - 1) & 1);
     } else if (warp == 1) {
         // ---------------- the products, the smallest first ----------------
         constexpr unsigned of_a = 0x001102, of_b = 0x010120;      // a nibble a product
         const unsigned long long qd = operand(q_img, 2, 1024), kd = operand(k_img, 2, 1024, kTile), ad = operand(a_img, 2, 1024);
+        int intra = 0, updates = 0, outs = 0;  // products issued and committed
         for (int c = 0; c < n && ok; ++c) {
             if (!SUMS) {
                 if (c > 0) wait(out_read, c - 1);
@@ -509,6 +519,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                     commit(intra_done);
                 }
                 __syncwarp();
+                ++intra;
             }
             if (!SUMS) wait(intra_read, c);
             wait(xs_full, c);
@@ -524,6 +535,7 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                 commit(upd_done);
             }
             __syncwarp();
+            ++updates;
             if (!SUMS) {
                 wait(q_full, c);
                 if (!wait(s_full, c)) break;
@@ -538,8 +550,17 @@ __global__ void __launch_bounds__(kRunThreads, 1) long_run_kernel(const RunArgs 
                     commit(out_done);
                 }
                 __syncwarp();
+                ++outs;
             }
         }
+        if (!ok) {                             // (those of the lower head may have no commit of their own)
+            if (elect()) commit(intra_done);
+            __syncwarp();
+            ++intra;
+        }
+        if (intra > 0) mbar_wait(intra_done, (intra - 1) & 1);         // nor are products
+        if (updates > 0) mbar_wait(upd_done, (updates - 1) & 1);
+        if (outs > 0) mbar_wait(out_done, (outs - 1) & 1);
     } else if (warp < 2 + kSWarps) {
         // ---------------- the state: a lane a column, half of the rows a warp ----------------
         const int quarter = warp & 3, half = warp >= 6, v0 = quarter * 32 + lane, col = v0 & 63;
