@@ -1430,9 +1430,10 @@ _NO_LIMIT = (1 << 31) - 1
 
 def scan_runs(lengths) -> tuple:
     """What a step's new tokens by sequence bring the matrix-state scans: (some sequence is run in chunks, some is
-    walked, some may be run as a long one, all are)."""
+    walked, some may be run as a long one, all are where heads are few, all are where they are not)."""
     least, most = min(lengths, default=0), max(lengths, default=0)
-    return most >= SCAN_CHUNK_TOKENS, least < SCAN_CHUNK_TOKENS, most >= SCAN_LONG_TOKENS, least >= SCAN_LONG_TOKENS_FEW_HEADS
+    return (most >= SCAN_CHUNK_TOKENS, least < SCAN_CHUNK_TOKENS, most >= SCAN_LONG_TOKENS, least >= SCAN_LONG_TOKENS_FEW_HEADS,
+            least >= SCAN_LONG_TOKENS)
 
 
 def _scan_route(kind, heads, rows, step, device, groups=1):
@@ -1453,9 +1454,10 @@ def _scan_route(kind, heads, rows, step, device, groups=1):
 
 # From this many new tokens on, a sequence's state-space scan runs in chunks of 64 tokens on the tensor cores (scan_long.cu) where that
 # kernel takes the size: where the blocks of the chunks of sixteen tokens (16 columns of a head each) fill the multiprocessors
-# more than once, and where they do not.  One prompt, states of 128 x 64, us by chunks of sixteen and here: 64 heads, 1,024 / 2,048 tokens
-# 86 / 151 and 106 / 122; 24 heads, 1,024 / 2,048 tokens 69 / 115 and 103 / 106.
-SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1536, 2048
+# more than once, and where they do not.  One prompt, states of 128 x 64, us by chunks of sixteen and here, 1,024 / 1,536 / 2,048 / 4,096 tokens:
+# 64 heads in 8 groups 84 / 120 / 158 / 292 and 85 / 109 / 125 / 208; 48 in one 80 / 110 / 144 / 276 and 88 / 102 / 115 / 186; 36 in one 63 / 83 / 104 / 215
+# and 88 / 102 / 116 / 181; 24 in one 59 / 77 / 98 / 187 and 85 / 99 / 113 / 171; 8 in one 57 / 77 / 96 / 172 and 80 / 94 / 107 / 165.
+SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1536, 4096
 
 
 def _long_route(heads, groups, n_state, value_dim, step, device):
@@ -1469,7 +1471,10 @@ def _long_route(heads, groups, n_state, value_dim, step, device):
     floats = -(-_ask("scan_long", "blm_scan_long_scratch", *sizes) // 4) if longest >= least else 0
     if floats == 0:
         return None
-    alone = runs[3] if runs is not None and len(runs) > 3 else runs is None and step.n_seqs == 1 and longest == step.n_tokens
+    if runs is not None:
+        alone = any(runs[3:4 if least > SCAN_LONG_TOKENS else 5])             # (the border of few heads is the higher one)
+    else:
+        alone = step.n_seqs == 1 and longest == step.n_tokens
     return torch.empty(floats, dtype=torch.float32, device=device), _ask("scan_long", "blm_scan_long_launches", *sizes), least, alone
 
 

@@ -7,6 +7,7 @@ from burn_lm_b200 import kernels as K
 from test_gpu_scan_chunks import read_state, state_of, step_of, walk
 
 pytestmark = pytest.mark.gpu
+BORDERS = K.SCAN_LONG_TOKENS, K.SCAN_LONG_TOKENS_FEW_HEADS
 
 
 @pytest.fixture(autouse=True)
@@ -138,6 +139,18 @@ def test_a_lone_sequence_among_rows_of_none(m):
     want = scan(x[:m], b0, dt[:m], dt_bias, a_log, skip, heads, groups, rows, dv, real, walked, 0)
     assert not out[m:].any()
     assert (out[:m] - want).abs().max() <= 2e-5 * want.abs().max() and (own - walked).abs().max() <= 2e-5 * walked.abs().max()
+
+
+@pytest.mark.parametrize("heads,lens,long,alone", [(36, [4095], False, None), (36, [4096], True, True), (38, [1535], False, None), (38, [1536], True, True),
+                                                   (36, [4096, 2000], True, False), (38, [1536, 2000], True, True), (38, [1536, 1], True, False)])
+def test_where_the_long_scans_begin(heads, lens, long, alone, monkeypatch):
+    """Thirty-six heads of 64 columns are one block a multiprocessor in chunks of sixteen, thirty-eight more."""
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS", BORDERS[0])
+    monkeypatch.setattr(K, "SCAN_LONG_TOKENS_FEW_HEADS", BORDERS[1])
+    step = step_of(lens, [0] * len(lens))
+    step.scan_runs = K.scan_runs(lens)
+    route = K._long_route(heads, 1, 128, 64, step, "cuda")
+    assert (route is not None) == long and (not long or route[3] == alone)
 
 
 LARGEST = 256 << 20                                                           # bytes of scratch
