@@ -12,7 +12,8 @@
 // C_ji = k_j . P(i+1..j) k_i below the diagonal, so that the sixteen corrections, each of which waits for the one before it,
 // are one small triangular product.  Every factor is a product of at most 16 decays, never a quotient of two: nothing
 // overflows however strong a decay is, and all of it is float32 sums of products of whole floats, as in the walk: multiply-adds, or
-// six tensor-core products of bfloat16 parts.
+// six tensor-core products of bfloat16 parts.  An infinity has parts that are not numbers: where the products are of parts, what an infinite
+// state, key or value reaches is not a number, where the walk's multiply-adds may leave an infinity; it reaches no more than there.
 //
 // Two launches.  What does not depend on the state (decayed rows, A, T) is formed for all chunks at once; then a block owns
 // (sequence, head, 16 or 32 value columns), holds its part of S in registers, and walks the sequence's chunks, while one more

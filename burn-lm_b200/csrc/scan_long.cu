@@ -310,7 +310,8 @@ __global__ void __launch_bounds__(kPrepThreads, 2) long_prep_kernel(const SsmPre
 // Warp 0 brings the chunk's operands (three barriers: each is asked for as soon as its product of the chunk before is done), one
 // thread of warp 1 issues the products, warps 2 to 9 keep the state, warps 10 to 13 split x and write the output.
 // A value that is not finite must not reach earlier tokens through a matrix's zeros, so it is taken out of x and joins the later
-// tokens' outputs and the state by itself.
+// tokens' outputs and the state by itself.  An infinite state, B or C has parts that are not numbers, and so is what it reaches, where the
+// walk's multiply-adds may leave an infinity; it reaches no more than there.
 // ---------------------------------------------------------------------------------------------
 struct RunArgs {
     RowsIn v;

@@ -177,6 +177,29 @@ def scan_of(kind, heads, rows, dv, n, gen):
                                                      K.DECAY_EXP_EXP if exp else K.DECAY_LOWER_BOUND, exp, step, state, 0)
 
 
+@pytest.mark.parametrize("heads,rows,dv", [(2, 20, 5), (3, 64, 64), (2, 128, 100)])
+@pytest.mark.parametrize("kind", ["ssm", "wkv", "delta"])
+def test_an_infinite_state_stays_in_its_column(kind, heads, rows, dv):
+    """Where products are formed of parts it comes out as not a number rather than as an infinity; no other column sees it, and without
+    the delta rule no other row of the state."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows)
+    step, h, r, c = step_of([40, 35], [0, 3]), 1, 3, 2
+    state, slot = state_of(step, heads, rows, dv, 0, gen), int(step.slot_of_seq[1])
+    run = scan_of(kind, heads, rows, dv, 75, gen)
+    outs, states = [], []
+    for value in (1.0, float("inf")):
+        own, out = state.clone(), torch.zeros((75, heads, dv), device="cuda")
+        own[slot, 1].view(heads, -1, dv, 8)[h, r // 8, c, r % 8] = value
+        run(slice(0, 75), out.view(75, -1), step, own)
+        outs.append(out)
+        states.append(read_state(own, slot, (3 + 35) & 1, 0, heads, dv))
+    assert not torch.isfinite(outs[1][40:, h, c]).any() and not torch.isfinite(states[1][h, r, c])
+    outs[1][40:, h, c] = outs[0][40:, h, c]
+    states[1][h, r if kind != "delta" else slice(None), c] = states[0][h, r if kind != "delta" else slice(None), c]
+    assert torch.equal(*outs) and torch.equal(*states)
+
+
 @pytest.mark.parametrize("lens", [[1, 1, 1, 40, 1, 13, 0, 35, 0], [15, 16, 17, 31], [1] * 15 + [4], [0, 64, 1]])
 @pytest.mark.parametrize("heads,rows,dv", [(3, 64, 64), (2, 128, 100)])
 @pytest.mark.parametrize("kind", ["ssm", "wkv", "lower", "delta"])

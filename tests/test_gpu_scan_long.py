@@ -191,6 +191,23 @@ def test_segments_against_the_walk(lens, starts, monkeypatch):
     assert (run - walked).abs().max() <= 2e-5 * walked.abs().max()
 
 
+def test_an_infinite_state_stays_in_its_column():
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(9)
+    heads, rows, dv, h, r, c = 4, 128, 64, 1, 70, 33
+    step = step_of([70, 640], [0, 3])
+    state, slot = state_of(step, heads, rows, dv, 0, gen), int(step.slot_of_seq[1])
+    args, outs, states = inputs(heads, 1, rows, dv, 710, gen), [], []
+    for value in (1.0, float("inf")):
+        own = state.clone()
+        own[slot, 1].view(heads, -1, dv, 8)[h, r // 8, c, r % 8] = value
+        outs.append(scan(*args, heads, 1, rows, dv, step, own, 0).view(710, heads, dv))
+        states.append(read_state(own, slot, (3 + 640) & 1, 0, heads, dv))
+    assert not torch.isfinite(outs[1][70:, h, c]).any() and not torch.isfinite(states[1][h, r, c])
+    outs[1][70:, h, c], states[1][h, r, c] = outs[0][70:, h, c], states[0][h, r, c]
+    assert torch.equal(*outs) and torch.equal(*states)
+
+
 @pytest.mark.parametrize("where", ["value", "key", "dt"])
 def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(where):
     gen = torch.Generator(device="cuda")
