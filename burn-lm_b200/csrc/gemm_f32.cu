@@ -1,5 +1,5 @@
 // y[N, M] = x[N, K] . W[M, K]^T in 32 bits: all 24 bits of both operands, float32 sums.
-// This is the matrix product of the 32-bit path.  The sum over K runs in one fixed order that depends on neither N nor M, so a
+// This is the matrix product of the 32-bit path.  The sum over K runs in one fixed order that depends on the weight alone, so a
 // token's result is the same whatever else is in the batch: K is cut into shares, each is summed in order, and the shares' sums are
 // added in order.  Two kernels: on the tensor cores (further down) where K and W's rows come in 16-byte pieces, and FFMA for
 // small weights and everything else.
@@ -9,8 +9,9 @@
 // groups of banks): a slice comes by cp.async two slices ahead, nothing is transposed, and twelve 16-byte loads feed 128
 // multiply-adds of a thread with 8 x 4 outputs.  The shares of 1,024 give a product of few columns as many blocks as one of many
 // (317 x 2,048 x 8,192: 160 tiles, 1,280 blocks); a second kernel adds their sums.  Two places of K an instruction (fma.rn.f32x2) ran at the
-// same rate, 8 x 8 outputs a thread too (four blocks a multiprocessor hide the loads, two do not).  With 16,384 x 2,048 / 2,048 x 8,192 weights,
-// us: 1 row 50 / 36, 16 rows 58 / 36, 64 rows 128 / 77, 317 rows 507 / 263.
+// same rate, 8 x 8 outputs a thread too (four blocks a multiprocessor hide the loads, two do not).  Rows in 16-byte pieces run here if the
+// weight is small (kTcWeight has the times) or K is below kTcLeast; others by pieces of four bytes: with 16,384 x 2,050 / 2,048 x 8,190
+// weights, us, 1 row 59 / 37, 16 rows 60 / 39, 64 rows 143 / 74, 317 rows 628 / 317 (in 16-byte pieces 50 / 36, 58 / 36, 128 / 77, 507 / 263).
 #include <algorithm>
 
 #include "tcgen05.cuh"
@@ -176,7 +177,7 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
 // finite is formed again with fmaf from the floats themselves.  Operands below 2^-109 lose their last bits (x3 would be below
 // the smallest bfloat16 number).
 // With 16,384 x 2,048 / 2,048 x 8,192 weights, us (FFMA above): 1 row 40 / 30, 16 rows 40 / 30, 64 rows 44 / 32, 160 rows 62 / 44, 317 rows
-// 110 / 69, 2,000 rows 603 / 390 (3,000 / 1,513); the error against 64 bits 1.2e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
+// 110 / 69, 2,000 rows 603 / 390 (FFMA in 16-byte pieces 3,000 / 1,513); launched back to back 28 / 17, 29 / 18, 33 / 20, 56 / 32, 104 / 59; the error against 64 bits 1.2e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
 // of which the tensor core works 1,920: x's parts have room for two steps only.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTcLeast = 64;
@@ -596,8 +597,8 @@ static int shares_of(bool tc, int K) { return tc ? (K + kTcShare - 1) / kTcShare
 // pass is cut so that its planes of sums stay within kPlanes floats (256 MB; on the tensor cores 192 MB, beside 24 MB for x's parts, which stay in L2), in
 // even parts of whole tiles along the longer side (every pass reads the shorter side's operand again): a large product would
 // otherwise hold K / 1,024 times its result (2,048 rows of logits over 128,256 columns and K 4,096: 4.2 GB).  Every pass ends in a
-// round of blocks that is not full: FFMA, 600 x 32,768 x 4,096 in two passes 3,731 -> 3,776 us, 2,048 x 4,096 x 14,336
-// 5,198 -> 5,229 (in six and eight: 3,842, 5,492).
+// round of blocks that is not full: FFMA with rows in 16-byte pieces, 600 x 32,768 x 4,096 in two passes 3,731 -> 3,776 us, 2,048 x 4,096 x
+// 14,336 5,198 -> 5,229 (in six and eight: 3,842, 5,492); by pieces of four bytes, as they run here, 4,825 and 6,676.
 constexpr long long kPlanes = 64 << 20, kTcPlanes = 48 << 20, kTcParts = 6 << 20;
 struct Pass {
     int products, rows, cols;

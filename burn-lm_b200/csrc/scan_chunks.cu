@@ -3,8 +3,8 @@
 // Walked token by token (recurrent.cu) a prompt is a chain: every token waits for the sums over a state's rows of the one
 // before it, and a 2,048-token prompt took 1.1 to 1.8 ms for work that the multiprocessors' fp32 units can do in 0.07.  Here
 // a chunk of 16 tokens costs one pass over the state (both launches, us: decay of 32 heads of 128 x 128 1,827 -> 188, state-space scan
-// of 64 heads of 128 x 64 1,116 -> 151, and 124 in chunks of 64 (scan_long.cu), delta rule of 16 heads of 128 x 128 over 1,501 + 500
-// tokens 1,224 -> 170).  With P(i..j) the product of the decays of the tokens i..j (per row, or
+// of 64 heads of 128 x 64 1,116 -> 158, and 125 in chunks of 64 (scan_long.cu), delta rule of 16 heads of 128 x 128 over 1,501 + 500
+// tokens 1,224 -> 173).  With P(i..j) the product of the decays of the tokens i..j (per row, or
 // one number per head) and S the state in front of the chunk:
 //     out_j  = (P(0..j) q_j)^T S + sum_(i <= j) A_ji x_i,     A_ji = sum_rows q_j P(i+1..j) k_i
 //     S'     = P(0..15) S + sum_j (P(j+1..15) k_j) x_j^T

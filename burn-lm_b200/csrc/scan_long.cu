@@ -1,10 +1,9 @@
 // Long prompts of the state-space scan, sixty-four tokens at a time on tcgen05.
 //
-// The chunks of sixteen tokens (scan_chunks.cu) are a chain of 128 links for a prompt of 2,048 tokens, each of which passes over
-// the state with fp32 multiply-adds: 230 us for 64 heads of 128 x 64, whose multiply-adds alone take 58.  Here a chunk has 64
-// tokens, its products run on the tensor cores with every float as three bfloat16 numbers (tcgen05.cuh: 24 bits, six products, sums
+// The chunks of sixteen tokens (scan_chunks.cu) are a chain of 128 links for a prompt of 2,048 tokens: 150 to 158 us for 64 heads of 128
+// x 64 (eight to one groups that share B and C), whose multiply-adds alone take 58 on the fp32 units.  Here a chunk has 64 tokens, its products run on the tensor cores with every float as three bfloat16 numbers (tcgen05.cuh: 24 bits, six products, sums
 // in float32), and a sequence (beyond 4,096 tokens each such segment of it, one after another) is cut into four groups of chunks that
-// run side by side: 124 us.  With P(i..j) the product of the
+// run side by side: 119 to 125 us.  With P(i..j) the product of the
 // decays of the tokens i..j and S the state in front of a chunk:
 //     out_j  = P(0..j) S^T C_j + sum_(i <= j) A_ji x_i,     A_ji = (C_j . B_i) P(i+1..j) dt_i  (+ D on the diagonal)
 //     S'     = P(0..63) S + Z,     Z = sum_j (P(j+1..63) dt_j B_j) x_j^T

@@ -1415,9 +1415,9 @@ def causal_conv(x, x_col0, channels, taps, bias, out, out_col0, step, state, sta
 
 # From this many new tokens on, a sequence's recurrence runs in chunks of sixteen tokens (scan_chunks.cu), below it token by token
 # (recurrent.cu), each by its own length, whatever shares the step.  Chunks against the walk, us on the device, sequences of
-# 16 / 24 / 32 / 64 tokens: state-space scan of 64 heads of 128 x 64, one 15 / 9, 17 / 12, 16 / 15, 20 / 27, sixteen 67 / 55, 88 / 77,
-# 88 / 98, 133 / 188; delta rule of 16 heads of 128 x 128, one 13 / 14, 15 / 19, 15 / 24, 18 / 45, sixteen 60 / 46, 78 / 64, 78 / 83,
-# 128 / 159; WKV of 32 heads of 128 x 128, one 12 / 13, 13 / 18, 13 / 23, 17 / 43, sixteen 61 / 72, 83 / 106, 85 / 139, 133 / 290.  The line
+# 16 / 24 / 32 / 64 tokens: state-space scan of 64 heads of 128 x 64, one 14 / 9, 14 / 12, 15 / 15, 17 / 27, sixteen 45 / 54, 60 / 75,
+# 62 / 97, 96 / 187; delta rule of 16 heads of 128 x 128, one 13 / 14, 14 / 19, 14 / 24, 16 / 45, sixteen 35 / 45, 46 / 64, 46 / 83,
+# 83 / 158; WKV of 32 heads of 128 x 128, one 11 / 13, 11 / 18, 11 / 22, 14 / 42, sixteen 46 / 71, 67 / 104, 69 / 137, 109 / 284.  The line
 # lies at the lower end because a walk beside chunks comes on top of them, up to a microsecond a token of its longest sequence.  A
 # single token costs a chunk all the same (255 of them beside 64 tokens 899 / 260 for the state-space scan).
 SCAN_CHUNK_TOKENS = 16
@@ -1457,6 +1457,8 @@ def _scan_route(kind, heads, rows, step, device, groups=1):
 # more than once, and where they do not.  One prompt, states of 128 x 64, us by chunks of sixteen and here, 1,024 / 1,536 / 2,048 / 4,096 tokens:
 # 64 heads in 8 groups 84 / 120 / 158 / 292 and 85 / 109 / 125 / 208; 48 in one 80 / 110 / 144 / 276 and 88 / 102 / 115 / 186; 36 in one 63 / 83 / 104 / 215
 # and 88 / 102 / 116 / 181; 24 in one 59 / 77 / 98 / 187 and 85 / 99 / 113 / 171; 8 in one 57 / 77 / 96 / 172 and 80 / 94 / 107 / 165.
+# Several prompts of 64 heads in 8 groups: three of 1,536 tokens 326 and 250, two / four of 2,048 293 / 553 and 226 / 450; three of 2,048 with 24
+# heads 157 and 126, which the border for one prompt gives away: a sequence's bits do not depend on what shares its step.
 SCAN_LONG_TOKENS, SCAN_LONG_TOKENS_FEW_HEADS = 1536, 4096
 
 
