@@ -149,6 +149,7 @@ enum { kModeDelta = 0, kModeExp = 1, kModeExpFirst = 2, kModeLower = 3 };
 
 template <int NP, int MODE>
 __global__ void __launch_bounds__(prep_threads(NP)) prep_rows_kernel(const PrepArgs a) {
+    pdl_launch_dependents();
     constexpr bool DELTA = MODE == kModeDelta, kFirst = MODE == kModeExpFirst;
     constexpr int T = prep_threads(NP), W = T / 32, NS = NP + 4;
     extern __shared__ __align__(16) float levels[];          // [4][16][NS], then (delta) the odd blocks' k [4][8][NS]
@@ -416,6 +417,7 @@ struct SsmPrepArgs {
 };
 
 __global__ void __launch_bounds__(256) prep_ssm_kernel(const SsmPrepArgs a) {
+    pdl_launch_dependents();
     __shared__ int found[2];
     __shared__ float Bs[kQ][65], Cs[kQ][65];   // 64 rows of the state at a time
     __shared__ float As[kQ][kMs];
@@ -1020,6 +1022,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_mma_kernel(const WalkArg
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(tc5::smem_u32(bar)) : "memory");
         };
+        pdl_wait();                            // (the parts; the state, x and the barriers were there before)
         for (int i = 0; i < kRing - 1; ++i) bring(lo + i);
         for (int chunk = lo; chunk < hi; ++chunk) {
             __syncthreads();                   // the others are done with the chunk before, where the next one goes
@@ -1187,6 +1190,7 @@ __global__ void __launch_bounds__(kLimbThreads, 2) walk_delta_kernel(const WalkA
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(tc5::smem_u32(bar)) : "memory");
         };
+        pdl_wait();                            // (the parts; the state, x and the barriers were there before)
         for (int i = 0; i < kRing - 1; ++i) bring(lo + i);
         for (int chunk = lo; chunk < hi; ++chunk) {
             __syncthreads();                   // the others are done with the chunk before, where the next one goes
@@ -1380,32 +1384,45 @@ static int launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
     return blm_check_launch("scan_chunks (walk)");
 }
 
-template <int NP, int KIND>
-static int launch_walk_mma(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
-    constexpr size_t smem = ((size_t)limb_stages(NP) * limb_stage(KIND, NP) + 2 * 5 * kQ * kVs) * sizeof(float) + 64;
-    if (int rc = allow_smem(walk_mma_kernel<NP, KIND>, smem)) return rc;
-    walk_mma_kernel<NP, KIND><<<dim3((a.dv + 15) / 16, a.heads, n_seqs), kLimbThreads, smem, stream>>>(a);
+// The walk's blocks may find their places while the chunks' own products are formed: a microsecond less (WKV of 32 heads of 128 x 128, 16 / 64
+// tokens 10.4 / 14.4 -> 9.3 / 13.1 us).  Blocks that come early share the first multiprocessors that have room, `per` each, where others stay
+// idle: a walk of fewer blocks takes up to half as long again (8 heads of 64 x 64, 1,200 tokens 52 -> 82 us), so it begins early where
+// every multiprocessor has `per` blocks or one less, and in steps of three chunks at most (32 heads of 64 x 64, 32 / 64 tokens 10.2 / 12.3 and 9.4 / 12.7).
+static int launch_limbs(void (*kernel)(const WalkArgs), const WalkArgs& a, int n_seqs, int n_tokens, int per, size_t smem, cudaStream_t stream) {
+    const dim3 grid((a.dv + 15) / 16, a.heads, n_seqs);
+    if ((long long)grid.x * grid.y * grid.z > (per - 1) * blm_sm_count() || n_tokens <= 3 * kQ) {
+        cudaError_t e = blm_launch_dependent(kernel, grid, dim3(kLimbThreads), smem, stream, a);
+        if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "scan_chunks: %s", cudaGetErrorString(e));
+    } else {
+        kernel<<<grid, kLimbThreads, smem, stream>>>(a);
+    }
     return blm_check_launch("scan_chunks (walk)");
 }
 
-static int launch_walk_delta(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+template <int NP, int KIND>
+static int launch_walk_mma(const WalkArgs& a, int n_seqs, int n_tokens, cudaStream_t stream) {
+    constexpr size_t smem = ((size_t)limb_stages(NP) * limb_stage(KIND, NP) + 2 * 5 * kQ * kVs) * sizeof(float) + 64;
+    if (int rc = allow_smem(walk_mma_kernel<NP, KIND>, smem)) return rc;
+    return launch_limbs(walk_mma_kernel<NP, KIND>, a, n_seqs, n_tokens, NP == 64 ? 3 : 2, smem, stream);
+}
+
+static int launch_walk_delta(const WalkArgs& a, int n_seqs, int n_tokens, cudaStream_t stream) {
     constexpr size_t smem = ((size_t)kDeltaRing * kDeltaStage + 4 * 2 * kQ * kVs) * sizeof(float) + 64;
     if (int rc = allow_smem(walk_delta_kernel, smem)) return rc;
-    walk_delta_kernel<<<dim3((a.dv + 15) / 16, a.heads, n_seqs), kLimbThreads, smem, stream>>>(a);
-    return blm_check_launch("scan_chunks (walk)");
+    return launch_limbs(walk_delta_kernel, a, n_seqs, n_tokens, 2, smem, stream);
 }
 
 // States of 128 rows, and of 64 that decay, are walked on the tensor cores.  The others with rows and columns of a thread, columns of a
 // block: four columns a thread, a row piece that comes from shared memory serves four multiply-adds a row; 16 columns a block, a
 // prompt of few heads still has a block for most multiprocessors.
 template <int KIND>
-static int walk(const WalkArgs& a, int np, int n_seqs, cudaStream_t stream) {
+static int walk(const WalkArgs& a, int np, int n_seqs, int n_tokens, cudaStream_t stream) {
     if constexpr (KIND != kDelta) {
-        if (np == 64) return launch_walk_mma<64, KIND>(a, n_seqs, stream);
-        if (np == 128) return launch_walk_mma<128, KIND>(a, n_seqs, stream);
+        if (np == 64) return launch_walk_mma<64, KIND>(a, n_seqs, n_tokens, stream);
+        if (np == 128) return launch_walk_mma<128, KIND>(a, n_seqs, n_tokens, stream);
     } else {
         if (np == 64) return launch_walk<64, 2, 16, 16, KIND>(a, n_seqs, stream);
-        if (np == 128) return launch_walk_delta(a, n_seqs, stream);
+        if (np == 128) return launch_walk_delta(a, n_seqs, n_tokens, stream);
     }
     switch (np) {
         case 32: return launch_walk<32, 2, 8, 32, KIND>(a, n_seqs, stream);
@@ -1483,7 +1500,7 @@ BLM_API int blm_scan_chunks_ssm(const float* xbc, long long xbc_stride, int x_co
         p.ch = a.ch = ch;
         prep_ssm_kernel<<<dim3(ch.count, groups * ((per + kSsmHeads - 1) / kSsmHeads)), 256, 0, stream>>>(p);
         if (int rc = blm_check_launch("scan_chunks (state-space scan)")) return rc;
-        if (int rc = walk<kSsm>(a, np, n_seqs, stream)) return rc;
+        if (int rc = walk<kSsm>(a, np, n_seqs, n_tokens, stream)) return rc;
     }
     return BLM_OK;
 }
@@ -1551,7 +1568,7 @@ BLM_API int blm_scan_chunks_rows(const float* q, long long q_stride, int q_col0,
             case 256: rc = prep<256>(p, mode, grid, stream); break;
             default: return blm_fail(BLM_BAD_ARGUMENT, "scan_chunks: states of %d rows", np);
         }
-        if (rc == BLM_OK) rc = delta ? walk<kDelta>(a, np, n_seqs, stream) : walk<kDecay>(a, np, n_seqs, stream);
+        if (rc == BLM_OK) rc = delta ? walk<kDelta>(a, np, n_seqs, n_tokens, stream) : walk<kDecay>(a, np, n_seqs, n_tokens, stream);
         if (rc != BLM_OK) return rc;
     }
     return BLM_OK;
