@@ -1387,10 +1387,11 @@ static int launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
 // The walk's blocks may find their places while the chunks' own products are formed: a microsecond less (WKV of 32 heads of 128 x 128, 16 / 64
 // tokens 10.4 / 14.4 -> 9.3 / 13.1 us).  Blocks that come early share the first multiprocessors that have room, `per` each, where others stay
 // idle: a walk of fewer blocks takes up to half as long again (8 heads of 64 x 64, 1,200 tokens 52 -> 82 us), so it begins early where
-// every multiprocessor has `per` blocks or one less, and in steps of three chunks at most (32 heads of 64 x 64, 32 / 64 tokens 10.2 / 12.3 and 9.4 / 12.7).
+// a single sequence gives every multiprocessor `per` blocks or one less (the delta rule of 16 heads, 1,501 + 500 tokens, whose longer
+// sequence has 128 blocks: the layer 279 -> 321 us), and in steps of three chunks at most (32 heads of 64 x 64, 32 / 64 tokens 10.2 / 12.3 and 9.4 / 12.7).
 static int launch_limbs(void (*kernel)(const WalkArgs), const WalkArgs& a, int n_seqs, int n_tokens, int per, size_t smem, cudaStream_t stream) {
     const dim3 grid((a.dv + 15) / 16, a.heads, n_seqs);
-    if ((long long)grid.x * grid.y * grid.z > (per - 1) * blm_sm_count() || n_tokens <= 3 * kQ) {
+    if ((long long)grid.x * grid.y > (per - 1) * blm_sm_count() || n_tokens <= 3 * kQ) {
         cudaError_t e = blm_launch_dependent(kernel, grid, dim3(kLimbThreads), smem, stream, a);
         if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "scan_chunks: %s", cudaGetErrorString(e));
     } else {
