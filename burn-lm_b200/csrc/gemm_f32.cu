@@ -173,8 +173,10 @@ __global__ void add_shares_kernel(const float* __restrict__ part, float* __restr
 // tensor core's additions cut bits off, so no more than a step is left to it (four additions of the large products); the sums over
 // the steps are float32 additions in order, and so are those over shares of 1,024 places of K.  The shares of a tile are a
 // block's, which adds them up in y, or where there are few tiles a block each and planes of sums: the same additions.
+// x's parts are rounded, which leaves the products left out of either sign, W's cut off: their conversion is on the way of every step (rounded, too,
+// 444 rows of 10,752 x 816 weights 43.3 us for 42.3).
 // Infinities: an infinite x1 makes x2 not a number, and a zero x2 times an infinity is not one either, so an output that is not
-// finite is formed again with fmaf from the floats themselves.  Operands below 2^-109 lose their last bits (x3 would be below
+// finite is formed again with fmaf from the floats themselves (so is one of an x whose x1 rounds to infinity).  Operands below 2^-109 lose their last bits (x3 would be below
 // the smallest bfloat16 number).
 // With 16,384 x 2,048 / 2,048 x 8,192 weights, us (FFMA above): 1 row 40 / 30, 16 rows 40 / 30, 64 rows 44 / 32, 160 rows 62 / 44, 317 rows
 // 110 / 69, 2,000 rows 603 / 390 (FFMA in 16-byte pieces 3,000 / 1,513); launched back to back 28 / 17, 29 / 18, 33 / 20, 56 / 32, 104 / 59; the error against 64 bits 1.2e-7 (5.7e-7).  A step of 160 rows of x takes some 2,900 clocks
@@ -393,8 +395,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
                     unsigned p[3][kTcPart];
 #pragma unroll
                     for (int c = 0; c < kTcK / 4; ++c) {
-                        split3(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
-                        split3(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
+                        split3_as<false, false>(v[c].x, v[c].y, p[0][2 * c], p[1][2 * c], p[2][2 * c]);
+                        split3_as<false, false>(v[c].z, v[c].w, p[0][2 * c + 1], p[1][2 * c + 1], p[2][2 * c + 1]);
                     }
 #pragma unroll
                     for (int i = 0; i < 3; ++i) tmem_st16(to + ((o.at * 2 + half) * 3 + i) * kTcPart, p[i]);
@@ -487,26 +489,35 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_f32_tc_kernel(const TcArgs
     }
 }
 
-// x's rows as three bfloat16 numbers a float: planes [batch][3][N][pitch].  A thread four places of K of a row: a block holds many
-// short rows or a part of a long one (a block a row: 64 products of 2,000 rows of 64 places 168 us, of which the products take 30).
+// x's rows as three bfloat16 numbers a float: planes [batch][3][N][pitch].  A thread four places of K of a row; `rows` short rows a block, or
+// (0) a block a row or a part of one (64 products of 2,000 rows of 64 places 168 us so, of which the products take 30; but the division
+// shows in long rows, 104 us of a product for 103).
 template <bool VEC>
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ out, int N, int K, int pitch,
-                                                         long long ldx, long long bx) {
+                                                         long long ldx, long long bx, int rows) {
     pdl_launch_dependents();
-    const unsigned pieces = K / 4;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = e / pieces;
+    int n = blockIdx.x, first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+    if (rows > 0) {
+        const int own = threadIdx.x / (K / 4);
+        if (own >= rows) return;
+        n = n * rows + own;
+        first = threadIdx.x - own * (K / 4);
+        step = K;
+    }
     if (n >= N) return;
-    const int c = (int)(e - n * pieces) * 4, b = blockIdx.y;
+    const int b = blockIdx.z;
     const float* row = x + (size_t)b * bx + (size_t)n * ldx;
-    __nv_bfloat16* to = out + ((size_t)b * 3 * N + n) * pitch + c;
+    __nv_bfloat16* to = out + ((size_t)b * 3 * N + n) * pitch;
     const size_t plane = (size_t)N * pitch;
-    const float4 v = VEC ? *reinterpret_cast<const float4*>(row + c) : make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
-    uint2 p1, p2, p3;
-    tc5::split3(v.x, v.y, p1.x, p2.x, p3.x);
-    tc5::split3(v.z, v.w, p1.y, p2.y, p3.y);
-    *reinterpret_cast<uint2*>(to) = p1;
-    *reinterpret_cast<uint2*>(to + plane) = p2;
-    *reinterpret_cast<uint2*>(to + 2 * plane) = p3;
+    for (int c = first * 4; c < K; c += step * 4) {
+        const float4 v = VEC ? *reinterpret_cast<const float4*>(row + c) : make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
+        uint2 p1, p2, p3;
+        tc5::split3_as<true, true>(v.x, v.y, p1.x, p2.x, p3.x);
+        tc5::split3_as<true, true>(v.z, v.w, p1.y, p2.y, p3.y);
+        *reinterpret_cast<uint2*>(to + c) = p1;
+        *reinterpret_cast<uint2*>(to + plane + c) = p2;
+        *reinterpret_cast<uint2*>(to + 2 * plane + c) = p3;
+    }
 }
 
 template <int TN, int TM, int AN, int AM>
@@ -581,9 +592,10 @@ static int launch_tc(const GemmArgs& g, const Plan& plan, float* scratch, int* s
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem + 1024);
     if (e != cudaSuccess) return blm_fail(BLM_CUDA_ERROR, "gemm_f32: %s", cudaGetErrorString(e));
     const bool vec = ((size_t)g.x & 15) == 0 && g.ldx % 4 == 0 && g.bx % 4 == 0;
-    const dim3 grid((unsigned)(((long long)g.N * (g.K / 4) + 255) / 256), g.batch);
-    if (vec) split_rows_kernel<true><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
-    else split_rows_kernel<false><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx);
+    const int rows = g.K <= 512 ? 256 / (g.K / 4) : 0;
+    const dim3 grid(rows ? (g.N + rows - 1) / rows : g.N, rows ? 1 : std::min(8, (g.K + 1023) / 1024), g.batch);
+    if (vec) split_rows_kernel<true><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx, rows);
+    else split_rows_kernel<false><<<grid, 256, 0, stream>>>(g.x, parts, g.N, g.K, pitch, g.ldx, g.bx, rows);
     if (int rc = blm_check_launch("gemm_f32 (parts)")) return rc;
     const long long tiles = (long long)a.n_tiles * a.m_tiles * (a.planes ? g.shares : 1) * g.batch;
     e = blm_launch_dependent(kernel, dim3((unsigned)std::min<long long>(tiles, blm_sm_count())), dim3(kTcThreads), smem, stream, a, xmap, wmap);

@@ -2,7 +2,7 @@
 // instructions and descriptors, and the split of a float into three bfloat16 numbers.
 //
 // A float has 24 bits of mantissa, a bfloat16 number 8 and the same exponents, so x = x1 + x2 + x3 exactly (x1 = x's first bits,
-// x2 = what is left rounded, x3 = the rest).  x w is then nine products that the tensor cores form exactly; the six with i + j <= 4 are
+// x2 = the next, x3 = what is left; split3_as).  x w is then nine products that the tensor cores form exactly; the six with i + j <= 4 are
 // summed (in float32, the smallest first), the other three are below 2^-21 of the product and 2^-24 on average.
 #pragma once
 #include <cuda.h>
@@ -133,19 +133,24 @@ __device__ __forceinline__ void tmem_free(unsigned base, int cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(base), "r"(cols));
 }
 
-// Two floats as three pairs of bfloat16 numbers (the first float in the lower half).  x1 is cut off, so that no finite float becomes an
-// infinity; x2 is rounded, so that the products left out are of either sign (both cut off they all had the product's own: errors of
-// recurrences and products 1.1 to 1.7 times as large); x3 is exact.  As many instructions as with both cut off.
-__device__ __forceinline__ void split3(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
-    p1 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-    a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
-    b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-    const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
-    p2 = *reinterpret_cast<const unsigned*>(&m);
-    a -= __uint_as_float(p2 << 16);
-    b -= __uint_as_float(p2 & 0xffff0000u);
+// Two floats as three pairs of bfloat16 numbers (the first float in the lower half); x3 is exact whichever of the first two are rounded.
+// Where all are cut off in both operands, the products left out have the product's own sign and add up: errors of recurrences and products
+// 1.1 to 1.7 times as large.  Rounding either operand's leaves them of either sign.  With x1 cut off no finite float becomes an infinity, so
+// that is what recurrences take, x2 rounded.  As many instructions each; a conversion takes longer than a byte permutation.
+template <bool ROUND1, bool ROUND2>
+__device__ __forceinline__ void split3_as(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) {
+    auto part = [&](bool round) {
+        const __nv_bfloat162 m = __floats2bfloat162_rn(a, b);
+        const unsigned p = round ? *reinterpret_cast<const unsigned*>(&m) : __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+        a -= __uint_as_float(round ? p << 16 : __float_as_uint(a) & 0xffff0000u);
+        b -= __uint_as_float(round ? p & 0xffff0000u : __float_as_uint(b) & 0xffff0000u);
+        return p;
+    };
+    p1 = part(ROUND1);
+    p2 = part(ROUND2);
     p3 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
+__device__ __forceinline__ void split3(float a, float b, unsigned& p1, unsigned& p2, unsigned& p3) { split3_as<false, true>(a, b, p1, p2, p3); }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
